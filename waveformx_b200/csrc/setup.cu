@@ -316,6 +316,11 @@ __global__ void __launch_bounds__(kWholeBlock, MIN_BLOCKS) k_setup_whole(const d
 // table and the head of binary b, part 1 + m its higher mode m. Each
 // computes the (2,2) set-up its part reads (setup_xhm.cuh). The status
 // (zeroed beforehand) gathers the parts' bits.
+// The part is the block's (blockIdx.y), and each mode's table is compiled for
+// its mode: a warp runs the code of one mode (with the parts in adjacent
+// threads every warp ran all five in turn: 170 us for 1 to 1024 binaries
+// against 102 to 112; the tangents below 1256 us at 1024 against 720). What
+// is left is one thread's chain, waiting on instruction fetch.
 constexpr int kXhmSetupBlock = 64;
 constexpr int kXhmParts = 5;
 
@@ -323,10 +328,9 @@ __global__ void __launch_bounds__(kXhmSetupBlock)
     k_setup_xhm(const double* __restrict__ params, int64_t B, const double* __restrict__ f_min, int64_t f_min_stride,
                 double amp_scale, double rmf, double* __restrict__ table64, float* __restrict__ table32,
                 int32_t* __restrict__ status) {
-  const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= B * kXhmParts) return;
-  const int64_t b = c / kXhmParts;
-  const int part = static_cast<int>(c % kXhmParts);
+  const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (b >= B) return;
+  const int part = static_cast<int>(blockIdx.y);
   double p[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) p[k] = params[b * 8 + k];
@@ -358,7 +362,13 @@ __global__ void __launch_bounds__(kXhmSetupBlock)
   }
   const int m = part - 1;
   double out[xhm::kModeSize];
-  const bool ok = xhm::mode_table(in, tab, m, out);
+  bool ok;
+  switch (m) {
+    case 0: ok = xhm::mode_table(in, tab, 0, out); break;
+    case 1: ok = xhm::mode_table(in, tab, 1, out); break;
+    case 2: ok = xhm::mode_table(in, tab, 2, out); break;
+    default: ok = xhm::mode_table(in, tab, 3, out);
+  }
   if (status != nullptr && !ok) atomicOr(&status[b], static_cast<int32_t>(kStatusSolve));
   if (row64 != nullptr) {
     double* mrow = row64 + H_MODES + m * kXhmModeStride64;
@@ -399,11 +409,10 @@ __global__ void __launch_bounds__(kXhmJvpBlock)
     k_setup_xhm_jvp(const double* __restrict__ params, int64_t B, const double* __restrict__ f_min,
                     int64_t f_min_stride, double amp_scale, double rmf, double* __restrict__ dtable) {
   const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= B * kXhmParts * kDirections) return;
+  if (c >= B * kDirections) return;
   const int j = static_cast<int>(c % kDirections);
-  const int64_t bp = c / kDirections;
-  const int64_t b = bp / kXhmParts;
-  const int part = static_cast<int>(bp % kXhmParts);
+  const int64_t b = c / kDirections;
+  const int part = static_cast<int>(blockIdx.y);
   Dual p[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) p[k] = Dual(params[b * 8 + k], 0.0);
@@ -610,8 +619,7 @@ int wfx_xhm_setup(const double* params, int64_t B, const double* f_min, int64_t 
     const cudaError_t rc = cudaMemsetAsync(status, 0, sizeof(int32_t) * B, s);
     if (rc != cudaSuccess) return static_cast<int>(rc);
   }
-  const int64_t threads = B * kXhmParts;
-  const unsigned grid = static_cast<unsigned>((threads + kXhmSetupBlock - 1) / kXhmSetupBlock);
+  const dim3 grid(static_cast<unsigned>((B + kXhmSetupBlock - 1) / kXhmSetupBlock), kXhmParts);
   k_setup_xhm<<<grid, kXhmSetupBlock, 0, s>>>(params, B, f_min, f_min_stride, amp_scale, reference_mf, table64,
                                               table32, status);
   return launched();
@@ -627,8 +635,7 @@ int wfx_xhm_setup_jvp(const double* params, int64_t B, const double* f_min, int6
                                  stream);
     if (rc != 0) return rc;
   }
-  const int64_t threads = B * kXhmParts * kDirections;
-  const unsigned grid = static_cast<unsigned>((threads + kXhmJvpBlock - 1) / kXhmJvpBlock);
+  const dim3 grid(static_cast<unsigned>((B * kDirections + kXhmJvpBlock - 1) / kXhmJvpBlock), kXhmParts);
   k_setup_xhm_jvp<<<grid, kXhmJvpBlock, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       params, B, f_min, f_min_stride, amp_scale, reference_mf, dtable);
   return launched();

@@ -316,7 +316,7 @@ struct Mode {
 };
 
 template <class R>
-inline WFX_HDI Mode<R> mode_struct(const xas::Internals<R>& w, int mode_int, R psi4tostrain) {
+WFX_HD Mode<R> mode_struct(const xas::Internals<R>& w, int mode_int, R psi4tostrain) {
   Mode<R> hm;
   hm.mode_int = mode_int;
   hm.tag = mode_int == 0 ? 21 : (mode_int == 1 ? 33 : (mode_int == 2 ? 32 : 44));
@@ -354,7 +354,7 @@ inline WFX_HDI Mode<R> mode_struct(const xas::Internals<R>& w, int mode_int, R p
 
 // The arguments of the fits (hm_fit_code.h).
 template <class R>
-inline WFX_HDI hmfit::Args<R> fit_args(const xas::Internals<R>& w) {
+WFX_HD hmfit::Args<R> fit_args(const xas::Internals<R>& w) {
   hmfit::Args<R> a;
   a.sq = w_sqrt(w.eta);
   a.delta = w.delta;
@@ -374,7 +374,7 @@ inline WFX_HDI hmfit::Args<R> fit_args(const xas::Internals<R>& w) {
 // (reference.py:441-443).
 
 template <class R, class T>
-inline WFX_HDI T ins_dphase22(const xas::Internals<R>& w, const Powers<T>& q) {
+WFX_HD T ins_dphase22(const xas::Internals<R>& w, const Powers<T>& q) {
   const R d2 = 3.0 / 5.0 * w.phi2, d3 = 2.0 / 5.0 * w.phi3, d4 = 1.0 / 5.0 * w.phi4, d5 = -3.0 / 5.0 * w.phi5l;
   const R d6 = -(1.0 / 5.0) * w.phi6 - 3.0 / 5.0 * w.phi6l, d6l = -1.0 / 5.0 * w.phi6l, d7 = -2.0 / 5.0 * w.phi7;
   const R d8 = -(3.0 / 5.0) * w.phi8 - 3.0 / 5.0 * w.phi8l, d8l = -3.0 / 5.0 * w.phi8l;
@@ -386,7 +386,7 @@ inline WFX_HDI T ins_dphase22(const xas::Internals<R>& w, const Powers<T>& q) {
 }
 
 template <class R, class T>
-inline WFX_HDI T ins_phase22(const xas::Internals<R>& w, const Powers<T>& q) {
+WFX_HD T ins_phase22(const xas::Internals<R>& w, const Powers<T>& q) {
   const R phi_norm = -(3.0 * fit::LALPI_M_FIVE_THIRDS) / 128.0;
   T x = 1.0 + w.phi2 * q.two_thirds + w.phi3 * q.itself + w.phi4 * q.four_thirds + w.phi5l * q.five_thirds * q.log_ +
         w.phi6 * q.two + w.phi6l * q.two * q.log_ + w.phi7 * q.seven_thirds + w.phi8 * q.eight_thirds +
@@ -397,7 +397,7 @@ inline WFX_HDI T ins_phase22(const xas::Internals<R>& w, const Powers<T>& q) {
 }
 
 template <class R, class T>
-inline WFX_HDI T dphase22(const xas::Internals<R>& w, const T& f, bool connected = true) {
+WFX_HD T dphase22(const xas::Internals<R>& w, const T& f, bool connected = true) {
   const Powers<T> q(f);
   if (value(f) < w.f_phase_in) return ins_dphase22(w, q);
   if (value(f) >= w.f_phase_im) {
@@ -412,7 +412,7 @@ inline WFX_HDI T dphase22(const xas::Internals<R>& w, const T& f, bool connected
 
 // The (2,2) ringdown amplitude ansatz (_generated/ringdown.py:55-61).
 template <class R, class T>
-inline WFX_HDI T amp22_ringdown(const xas::Internals<R>& w, const T& mf) {
+WFX_HD T amp22_ringdown(const xas::Internals<R>& w, const T& mf) {
   const R gamma_d13 = w.f_damp * w.gamma1 * w.gamma3;
   const R gamma_r = w.gamma2 / (w.gamma3 * w.f_damp);
   const R gamma_d2 = (w.f_damp * w.gamma3) * (w.f_damp * w.gamma3);
@@ -424,7 +424,7 @@ inline WFX_HDI T amp22_ringdown(const xas::Internals<R>& w, const T& mf) {
 // (core.py:193-205): the table's rest plus, in the inspiral and with
 // `leading`, T0 f^-5/3.
 template <class R, class T>
-inline WFX_HDI T rest22(const R* tab22, const T& mf, R m_sec, bool leading, bool& past) {
+WFX_HD T rest22(const R* tab22, const T& mf, R m_sec, bool leading, bool& past) {
   const T f = mf / m_sec;
   T lf;
   T rest = xas::rest_at<T, R>(tab22, f, past, lf);
@@ -447,7 +447,7 @@ struct Amp {
 
 // IMRPhenomXHM_GetPNAmplitudeCoefficients (hm/inspiral.py:45-216).
 template <class R>
-inline WFX_HDI void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& amp) {
+WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& amp) {
   const R chi_a = hm.chi_a, chi_s = hm.chi_s, eta = w.eta, delta = w.delta;
   const R pi = fit::PI;
   const R sqrt_5_7 = w_sqrt(5.0 / 7.0);
@@ -585,7 +585,7 @@ inline WFX_HDI void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, 
 
 // The PN amplitude times pnGlobalFactor ampNorm f^-7/6 (reference.py:152-162).
 template <class R, class T>
-inline WFX_HDI T pn_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
+WFX_HD T pn_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
   const T terms[6] = {p.one_third, p.two_thirds, p.itself, p.four_thirds, p.five_thirds, p.two};
   T re(amp.pn_re[0]), im(amp.pn_im[0]);
   for (int k = 0; k < 6; ++k) {
@@ -597,7 +597,7 @@ inline WFX_HDI T pn_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
 
 // PN plus pseudo-PN terms (reference.py:165-172).
 template <class R, class T>
-inline WFX_HDI T inspiral_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
+WFX_HD T inspiral_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
   T pseudo = p.seven_thirds / amp.fcut_7_3 * amp.ins[0] + p.eight_thirds / amp.fcut_8_3 * amp.ins[1];
   pseudo = p.three / amp.fcut_3 * amp.ins[2] + pseudo;
   return pn_amp_ansatz(p, amp) + pseudo * p.m_seven_sixths * amp.pn_dominant;
@@ -606,7 +606,7 @@ inline WFX_HDI T inspiral_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
 // The Lorentzian of the ringdown amplitude and its derivative
 // (reference.py:195-214).
 template <class R, class T>
-inline WFX_HDI T lorentzian(const T& mf, const Mode<R>& hm, const R* rd) {
+WFX_HD T lorentzian(const T& mf, const Mode<R>& hm, const R* rd) {
   const R fda = hm.f_damp;
   const T dfr = mf - hm.f_ring;
   const R dfd = fda * rd[2];
@@ -614,7 +614,7 @@ inline WFX_HDI T lorentzian(const T& mf, const Mode<R>& hm, const R* rd) {
 }
 
 template <class R>
-inline WFX_HDI R rd_amp_dansatz(R mf, const Mode<R>& hm, const R* rd) {
+WFX_HD R rd_amp_dansatz(R mf, const Mode<R>& hm, const R* rd) {
   const R fda = hm.f_damp;
   const R dfr = mf - hm.f_ring;
   const R numerator = rd[0] * (fda * fda * rd[1] * rd[2] * rd[2] + (dfr * dfr * rd[1] + 2.0 * fda * dfr * rd[2]));
@@ -626,7 +626,7 @@ inline WFX_HDI R rd_amp_dansatz(R mf, const Mode<R>& hm, const R* rd) {
 // The ringdown amplitude ansatz: the Lorentzian, the cubic of the (3,2)
 // below fRDAux, the fall-off above fAmpRDfalloff (reference.py:217-229).
 template <class R, class T>
-inline WFX_HDI T rd_amp_ansatz(const T& mf, const Mode<R>& hm, const Amp<R>& amp) {
+WFX_HD T rd_amp_ansatz(const T& mf, const Mode<R>& hm, const Amp<R>& amp) {
   T out = value(mf) >= hm.f_amp_rd_falloff ? amp.rd[3] * w_exp(-amp.rd[4] * (mf - hm.f_amp_rd_falloff))
                                             : lorentzian(mf, hm, amp.rd);
   if (hm.mixing && value(mf) < amp.f_rd_aux) {
@@ -650,7 +650,7 @@ struct RdPhase {
 };
 
 template <class R, class T>
-inline WFX_HDI T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
+WFX_HD T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
   const R frd = hm.f_ring, fda = hm.f_damp;
   const T den = fda * fda + (ff - frd) * (ff - frd);
   if (!hm.mixing) return frd * frd * ph.alpha2 * p.m_two + ph.alpha0 + (ph.alpha_l * fda) / den;
@@ -659,7 +659,7 @@ inline WFX_HDI T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, c
 }
 
 template <class R, class T>
-inline WFX_HDI T rd_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
+WFX_HD T rd_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
   const R frd = hm.f_ring, fda = hm.f_damp;
   const T arctan = w_atan((ff - frd) / fda);
   if (!hm.mixing) {
@@ -687,7 +687,7 @@ struct Rotation {
 // ansatz rescaled by its leading order with the phase of the (2,2) without
 // its anchor.
 template <class R, class T>
-inline WFX_HDI void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
+WFX_HD void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
   const xas::Internals<R>& w = *r.w;
   const Powers<T> p(mf);
   const T a22 = amp22_ringdown(w, mf) * w.amp_norm * p.m_seven_sixths;
@@ -708,13 +708,13 @@ inline WFX_HDI void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
 }
 
 template <int N, class R>
-inline WFX_HDI bool solve_n(R (&a)[N][N], R (&b)[N]) {
+WFX_HD bool solve_n(R (&a)[N][N], R (&b)[N]) {
   return solve<R, N>(a, b);
 }
 
 // IMRPhenomXHM_GetAmplitudeCoefficients (reference.py:337-348).
 template <class R>
-inline WFX_HDI bool amplitude_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
+WFX_HD bool amplitude_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
                                     Rotation<R>& rot, Amp<R>& amp) {
   using F1 = typename Deriv<R>::F1;
   bool ok = true;
@@ -937,7 +937,7 @@ struct Phase {
 };
 
 template <class R, class T>
-inline WFX_HDI T ins_phase_int(const T& mf, const Powers<T>& p, const Phase<R>& ph, bool leading = true) {
+WFX_HD T ins_phase_int(const T& mf, const Powers<T>& p, const Phase<R>& ph, bool leading = true) {
   const T freqs[13] = {p.m_five_thirds, p.m_four_thirds, p.m_one, p.m_two_thirds, p.m_one_third, T(1.0),
                        p.one_third, p.two_thirds, mf, p.four_thirds, p.five_thirds, p.two, p.seven_thirds};
   const T log_mf = p.log_;
@@ -947,7 +947,7 @@ inline WFX_HDI T ins_phase_int(const T& mf, const Powers<T>& p, const Phase<R>& 
 }
 
 template <class R, class T>
-inline WFX_HDI T ins_dphase(const T& mf, const Powers<T>& p, const Phase<R>& ph) {
+WFX_HD T ins_dphase(const T& mf, const Powers<T>& p, const Phase<R>& ph) {
   const R coeffs[13] = {-5.0 / 3.0, -4.0 / 3.0, -1.0, -2.0 / 3.0, -1.0 / 3.0, 0.0, 1.0 / 3.0, 2.0 / 3.0, 1.0,
                              4.0 / 3.0, 5.0 / 3.0, 2.0, 7.0 / 3.0};
   const T freqs[13] = {p.m_eight_thirds, p.m_seven_thirds, p.m_two, p.m_five_thirds, p.m_four_thirds, p.m_one,
@@ -962,7 +962,7 @@ inline WFX_HDI T ins_dphase(const T& mf, const Powers<T>& p, const Phase<R>& ph)
 }
 
 template <class R, class T>
-inline WFX_HDI T int_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
+WFX_HD T int_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
   const R fda = hm.f_damp, frd = hm.f_ring;
   const T lor = (ph.c_l * fda) / (fda * fda + (ff - frd) * (ff - frd));
   T d = ph.c1 * p.m_one + ph.c0;
@@ -973,7 +973,7 @@ inline WFX_HDI T int_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, 
 }
 
 template <class R, class T>
-inline WFX_HDI T int_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
+WFX_HD T int_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
   const R fda = hm.f_damp, frd = hm.f_ring;
   T x = ph.c0 * ff + ph.c1 * p.log_;
   x = -ph.c2 * p.m_one + x;
@@ -983,7 +983,7 @@ inline WFX_HDI T int_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, c
 }
 
 template <class R>
-inline WFX_HDI R phase_fit(const hmfit::Args<R>& fa, int tag, int i) {
+WFX_HD R phase_fit(const hmfit::Args<R>& fa, int tag, int i) {
 #define WFX_PF(t)                                                                                        \
   case t:                                                                                                \
     switch (i) {                                                                                         \
@@ -1007,7 +1007,7 @@ inline WFX_HDI R phase_fit(const hmfit::Args<R>& fa, int tag, int i) {
 // IMRPhenomXHM_Insp_Phase_LambdaPN (_generated/hm_inspiral.py:26-42) or the
 // extreme-mass-ratio fit.
 template <class R>
-inline WFX_HDI R lambda_pn(const hmfit::Args<R>& fa, R eta, int tag) {
+WFX_HD R lambda_pn(const hmfit::Args<R>& fa, R eta, int tag) {
   if (eta > 0.01) {
     const R pi = fit::PI;
     R out = 0.0;
@@ -1028,7 +1028,7 @@ inline WFX_HDI R lambda_pn(const hmfit::Args<R>& fa, R eta, int tag) {
 
 // IMRPhenomXHM_PN21AmpSign (hm/phase.py:214-227).
 template <class R>
-inline WFX_HDI bool pn21_amp_sign(R ff, const xas::Internals<R>& w) {
+WFX_HD bool pn21_amp_sign(R ff, const xas::Internals<R>& w) {
   const R eta = w.eta, chi1 = w.chi1, chi2 = w.chi2;
   const R delta = w_sqrt(-4.0 * eta + 1.0);
   const R sqrt5 = w_sqrt(5.0);
@@ -1042,7 +1042,7 @@ inline WFX_HDI bool pn21_amp_sign(R ff, const xas::Internals<R>& w) {
 }
 
 template <class R>
-inline WFX_HDI bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
+WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
                                 Rotation<R>& rot, Phase<R>& ph) {
   using J2 = typename Deriv<R>::J2;
   bool ok = true;
@@ -1211,7 +1211,7 @@ inline WFX_HDI bool phase_coefficients(const xas::Internals<R>& w, const hmfit::
 // The spheroidal (3,2) ringdown aligned with the (2,2) ringdown, without the
 // anchor of the (2,2) in phi0_s (core.py:208-234).
 template <class R>
-inline WFX_HDI bool spheroidal(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const R* tab22,
+WFX_HD bool spheroidal(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const R* tab22,
                         const Mode<R>& hm, Spheroidal<R>& sp) {
   const R fringlm = hm.f_ring, fdamplm = hm.f_damp;
   const R freqs[4] = {w.f_ring, -1.5 * fdamplm + fringlm, -0.5 * fdamplm + fringlm, 0.5 * fdamplm + fringlm};
@@ -1254,7 +1254,7 @@ struct SPowers {
 };
 
 template <class R>
-inline WFX_HDI SPowers<R> s_powers(R s) {
+WFX_HD SPowers<R> s_powers(R s) {
   const Powers<R> p(s);
   SPowers<R> o;
   o.p[B_M3] = p.m_three;
@@ -1277,7 +1277,7 @@ inline WFX_HDI SPowers<R> s_powers(R s) {
 
 // b: the basis index of x^a (no log); log_index: that of x^a log x (or -1).
 template <class R>
-inline WFX_HDI void add_term(R* row, const SPowers<R>& sp, R c, int b, int log_index) {
+WFX_HD void add_term(R* row, const SPowers<R>& sp, R c, int b, int log_index) {
   const R scaled = c * sp.p[b];
   if (log_index < 0) {
     row[b] = row[b] + scaled;
@@ -1291,7 +1291,7 @@ inline WFX_HDI void add_term(R* row, const SPowers<R>& sp, R c, int b, int log_i
 // odd modes of equal masses and spins. Returns false if a collocation
 // system is singular.
 template <class R>
-inline WFX_HDI bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int, R* out) {
+WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int, R* out) {
   for (int k = 0; k < kModeSize; ++k) out[k] = 0.0;
   const hmfit::Args<R> fa = fit_args(w);
   const R psi4_args[4] = {w.eta, w.s_tot_r, w.dchi, sqrt_nonneg(-4.0 * w.eta + 1.0)};
@@ -1414,7 +1414,7 @@ inline WFX_HDI bool mode_table(const xas::Internals<R>& w, const R* tab22, int m
 
 // Wigner's d^l_{m' m}(beta) (the convention of LAL's XLALWignerdMatrix).
 template <class R>
-inline WFX_HDI R wigner_d(int ell, int mp, int m, R beta) {
+WFX_HD R wigner_d(int ell, int mp, int m, R beta) {
   auto fact = [](int n) {
     R r = 1.0;
     for (int i = 2; i <= n; ++i) r *= i;
@@ -1435,7 +1435,7 @@ inline WFX_HDI R wigner_d(int ell, int mp, int m, R beta) {
 
 // -2Y_lm(theta, pi/2) as (re, im).
 template <class R>
-inline WFX_HDI void swsh(R theta, int ell, int m, R& re, R& im) {
+WFX_HD void swsh(R theta, int ell, int m, R& re, R& im) {
   const R norm = w_sqrt((2 * ell + 1) / (4.0 * fit::PI));
   const R d = norm * wigner_d(ell, m, 2, theta);
   const R x = static_cast<double>(m) * (fit::PI / 2.0);
@@ -1446,7 +1446,7 @@ inline WFX_HDI void swsh(R theta, int ell, int m, R& re, R& im) {
 // factors[4 k .. 4 k + 4) = Re F+, Im F+, Re Fx, Im Fx of mode k of
 // (2,2), (2,1), (3,3), (3,2), (4,4).
 template <class R>
-inline WFX_HDI void mode_factors(R inclination, R* factors) {
+WFX_HD void mode_factors(R inclination, R* factors) {
   const int ells[5] = {2, 2, 3, 3, 4}, emms[5] = {2, 1, 3, 2, 4};
   for (int k = 0; k < 5; ++k) {
     const int ell = ells[k], emm = emms[k];
