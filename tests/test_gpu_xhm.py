@@ -502,3 +502,32 @@ def test_keyword_polarizations(cuda, approximant, fixture):
     if approximant in ("IMRPhenomXAS", "IMRPhenomXHM"):
         with pytest.raises(wb.InvalidParameterError):  # (IMRPhenomX's mass-ratio limit)
             wb.polarizations(approximant, f, mass_1=2000.0, mass_2=1.0)
+
+
+@pytest.mark.parametrize("n, batch", [(1, 3), (31, 3), (32, 3), (33, 3), (128, 3), (129, 3), (300, 1600)])
+def test_gradient_sums_over_frequencies(cuda, n, batch):
+    """ops.xhm_vjp at the edges of its spans (128 frequencies, 32 a warp) and
+    with several spans a block (1600 x 300): the gradient of a grid is the
+    sum of the gradients of its frequencies, each taken as a row of its own
+    of a ragged grid. Bar: 1e-9 of the sum of the terms' magnitudes (the sums
+    round to 1e-14 of it, and a row's slots cancel by at most 1e5 in the
+    product with the set-up's tangents)."""
+    import torch
+
+    from waveformx_b200 import ops
+
+    base = golden("xhm_random")["params"][:3]
+    grid = torch.as_tensor(np.geomspace(20.0, 600.0, n) if n > 1 else np.array([90.0]), device=cuda)
+    rng = np.random.default_rng(n)
+    params = torch.as_tensor(np.tile(base, (batch // 3 + 1, 1))[:batch], device=cuda)
+    t_c = torch.as_tensor(np.tile([0.01, -0.02, 0.0], batch // 3 + 1)[:batch], device=cuda)
+    cot = [torch.as_tensor(rng.normal(size=(3, n)) + 1j * rng.normal(size=(3, n)), device=cuda) for _ in range(2)]
+    whole = ops.xhm_vjp(params, grid[:1], grid, None, t_c,
+                        *(c.repeat(batch // 3 + 1, 1)[:batch].contiguous() for c in cot))
+    rows = torch.arange(3, device=cuda).repeat_interleave(n)
+    parts = ops.xhm_vjp(params[:3][rows].contiguous(), grid[:1], grid.repeat(3),
+                        torch.arange(3 * n + 1, device=cuda), t_c[:3][rows].contiguous(),
+                        *(c.reshape(-1) for c in cot)).reshape(3, n, 9)
+    bar = 1e-9 * parts.abs().sum(1)
+    error = (whole - parts.sum(1).repeat(batch // 3 + 1, 1)[:batch]).abs()
+    assert bool((error <= bar.repeat(batch // 3 + 1, 1)[:batch]).all()), (error / bar.repeat(batch // 3 + 1, 1)[:batch]).max()
