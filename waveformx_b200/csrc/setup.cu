@@ -9,7 +9,9 @@
 //    IMRPhenomXAS and IMRPhenomD, where it shortens the chain a block waits
 //    on and spills less (measured, XAS: 72 us at 1024 binaries either way;
 //    84 against 103 us at 4096, 268 against 314 at 16384, 1.01 against
-//    1.28 ms at 65536; the same dtable bit for bit).
+//    1.28 ms at 65536; the same dtable bit for bit). With the tangents'
+//    systems solved by the values' elimination (setup_common.cuh, solve): 66
+//    us at 1024, 79 at 4096, 250 at 16384.
 //
 // This file is compiled without FMA contraction (-fmad=false): the value
 // part of the dual-number set-up then rounds exactly as the plain one, so a
@@ -312,134 +314,246 @@ __global__ void __launch_bounds__(kWholeBlock, MIN_BLOCKS) k_setup_whole(const d
 }
 
 
-// IMRPhenomXHM: thread (b, part) of 5 per binary; part 0 writes the (2,2)
-// table and the head of binary b, part 1 + m its higher mode m. Each
-// computes the (2,2) set-up its part reads (setup_xhm.cuh). The status
-// (zeroed beforehand) gathers the parts' bits.
-// The part is the block's (blockIdx.y), and each mode's table is compiled for
-// its mode: a warp runs the code of one mode (with the parts in adjacent
-// threads every warp ran all five in turn: 170 us for 1 to 1024 binaries
-// against 102 to 112; the tangents below 1256 us at 1024 against 720). What
-// is left is one thread's chain, waiting on instruction fetch.
+// IMRPhenomXHM: nine parts per binary, each on its own blocks (blockIdx.y):
+// part 0 writes the (2,2) table and the head, part 1 + m the amplitude of the
+// higher mode m, part 5 + m its phase and the rest of its table. A part
+// computes what it reads of the (2,2) set-up (setup_xhm.cuh): a higher mode's
+// amplitude only the waveform variables, its phase the (2,2)'s phase, the
+// (3,2) both. The status (zeroed beforehand) gathers the parts' bits.
+//
+// What binds it is one thread's chain, waiting on instruction fetch. The parts
+// in adjacent threads (every warp running them all in turn) took 170 us for 1
+// to 1024 binaries, a mode a block 102 to 112; 58 to 64 us (98 at 4096) with
+// the amplitudes apart from the phases, the amplitudes' collocation points as
+// divided differences and the powers of constants as numbers. The tangents:
+// 154 us at 250 binaries, 223 at 1024, 726 at 4096, from 394, 720 and 2053
+// (four dual-number directions rather than eight besides). (The duals do not
+// write the values too: a form that did, saving the values' launch, did not
+// come to an end on the device, though its host build did.)
 constexpr int kXhmSetupBlock = 64;
-constexpr int kXhmParts = 5;
+constexpr int kXhmParts = 9;
 
-__global__ void __launch_bounds__(kXhmSetupBlock)
-    k_setup_xhm(const double* __restrict__ params, int64_t B, const double* __restrict__ f_min, int64_t f_min_stride,
-                double amp_scale, double rmf, double* __restrict__ table64, float* __restrict__ table32,
-                int32_t* __restrict__ status) {
-  const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const int part = static_cast<int>(blockIdx.y);
-  double p[8];
+// The slots of the amplitudes that scale with 1 / distance.
+__device__ __forceinline__ constexpr bool xhm_scale_slot(int k) {
+  return (k >= xhm::M_PN_RE && k < xhm::M_INTER_C) || k == xhm::M_RD || k == xhm::M_FALLOFF ||
+         (k >= xhm::M_AUX && k < xhm::M_F_AUX);
+}
+
+// Part PART (xhm::kModeAmp, kModePhase) of the higher mode M of binary b: the
+// values on double, the tangents along parameter d on Dual. The duals of d = 0
+// also write the tangents along the parameters that no dual number carries:
+// the distance (1 / distance in the amplitudes), phi_ref and f_ref. These two
+// shift the (2,2)'s phase by delta, and with it each region's constant by
+// (m/2) delta, but the (3,2)'s: its spheroidal phase by delta and its ringdown,
+// which rotates the (2,2), not at all (its D and its ringdown's constant
+// cancel).
+template <int M, int PART, class R>
+__device__ __forceinline__ void xhm_mode_part(const R* p, int d, int64_t b, double f_min, double amp_scale, double rmf,
+                                              double* table64, float* table32, double* dtable, int32_t* status) {
+  constexpr bool kAmp = PART == xhm::kModeAmp, kDual = sizeof(R) != sizeof(double);
+  constexpr int kXasRole = M == 2 ? kRoleAll : (kAmp ? kRoleNone : kRolePhase);
+  R tab[kTableStride];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) p[k] = params[b * 8 + k];
-  // (zeroed: the slots the FP64 (2,2) table leaves unused are written too)
-  double tab[kTableStride];
+  for (int k = 0; k < kTableStride; ++k) tab[k] = R(0.0);
+  xas::Internals<R> in;
+  const xas::Vars<R> v = xas::variables<R>(p);
+  const DirectFits<R, xas::Vars<R>> fits{v};
+  xas::setup<R, DirectFits<R, xas::Vars<R>>, kXasRole>(p, f_min, amp_scale, rmf, tab, fits, &in);
+  R out[xhm::kModeSize];
+  const bool ok = xhm::mode_table<M, PART>(in, tab, out);
+  if constexpr (kDual) {
+    double* drow = dtable + (b * kXhmStride64 + H_MODES + M * kXhmModeStride64) * kDirections + d;
 #pragma unroll
-  for (int k = 0; k < kTableStride; ++k) tab[k] = 0.0;
-  xas::Internals<double> in;
-  const xas::Vars<double> v = xas::variables<double>(p);
-  const int32_t st = xas::setup(p, f_min[b * f_min_stride], amp_scale, rmf, tab,
-                                DirectFits<double, xas::Vars<double>>{v}, &in);
-  double* row64 = table64 != nullptr ? table64 + b * kXhmStride64 : nullptr;
-  float* row32 = table32 != nullptr ? table32 + b * kXhmStride32 : nullptr;
-  if (part == 0) {
-    write_tables<kModelXas>(kRoleAll, tab, 0, row64, row32);
-    double head[H_MODES - H_FACTORS];
-    xhm::mode_factors(p[5], head);
-    for (int k = 0; k < xhm::kHeadFactors; ++k) head[k] = st != 0 ? NAN : head[k];
-    head[H_AMP0 - H_FACTORS] = in.amp0;
-    head[H_S - H_FACTORS] = in.m_sec;
-    head[H_COS_A - H_FACTORS] = cos(tab[X_ANCHOR]);
-    head[H_SIN_A - H_FACTORS] = sin(tab[X_ANCHOR]);
-    for (int k = 0; k < H_MODES - H_FACTORS; ++k) {
-      if (row64 != nullptr) row64[H_FACTORS + k] = head[k];
-      if (row32 != nullptr) row32[H_FACTORS + k] = static_cast<float>(head[k]);
+    for (int k = 0; k < xhm::kModeSize; ++k) {
+      if (xhm::mode_amp_slot(k) == kAmp) drow[k * kDirections] = out[k].d;
     }
-    if (status != nullptr && st != 0) atomicOr(&status[b], st);
+    if (d != 0) return;
+    const double inv = 1.0 / value(p[4]);
+    double phi = 0.0, fref = 0.0;
+    if constexpr (!kAmp) {
+      if (!xhm::mode_vanishes<M>(in)) {
+        double tv[kTableStride], pv[8];
+#pragma unroll
+        for (int k = 0; k < kTableStride; ++k) tv[k] = value(tab[k]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) pv[k] = value(p[k]);
+        const Tail<kModelXas> t = tail_derivatives<kModelXas>(tv, pv, rmf);
+        phi = t.constant_phi;
+        fref = t.constant_fref;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < xhm::kModeSize; ++k) {
+      if (xhm::mode_amp_slot(k) != kAmp) continue;
+      double* at = drow + k * kDirections + kDualDirections;
+      const bool constant = k == xhm::M_PHASE + xhm::B_1 || k == xhm::M_PHASE + xhm::kBasis + xhm::B_1 ||
+                            (M != 2 && k == xhm::M_PHASE + 2 * xhm::kBasis + xhm::B_1) ||
+                            (M == 2 && k == xhm::M_SPH + 1);
+      const double m_over_2 = xhm::ModeConst<M>::emm * 0.5;
+      at[0] = xhm_scale_slot(k) ? -value(out[k]) * inv : 0.0;
+      at[1] = 0.0;
+      at[2] = constant ? m_over_2 * phi : 0.0;
+      at[3] = constant ? m_over_2 * fref : 0.0;
+    }
     return;
   }
-  const int m = part - 1;
-  double out[xhm::kModeSize];
-  bool ok;
-  switch (m) {
-    case 0: ok = xhm::mode_table(in, tab, 0, out); break;
-    case 1: ok = xhm::mode_table(in, tab, 1, out); break;
-    case 2: ok = xhm::mode_table(in, tab, 2, out); break;
-    default: ok = xhm::mode_table(in, tab, 3, out);
-  }
   if (status != nullptr && !ok) atomicOr(&status[b], static_cast<int32_t>(kStatusSolve));
-  if (row64 != nullptr) {
-    double* mrow = row64 + H_MODES + m * kXhmModeStride64;
-    for (int k = 0; k < xhm::kModeSize; ++k) mrow[k] = out[k];
-  }
-  if (row32 != nullptr) {
-    // FP32: the leading term (m/2)^(8/3) T0 and each region's coefficient of
-    // f as double-floats, each region's constant less (m/2) A modulo 2 pi
-    // (models/xhm/core.py:544-546)
-    float* mrow = row32 + H_MODES + m * kXhmModeStride32;
-    for (int k = 0; k < xhm::kModeSize; ++k) mrow[k] = static_cast<float>(out[k]);
-    const double m_over_2 = (m == 0 ? 1 : (m == 1 ? 3 : (m == 2 ? 2 : 4))) * 0.5;
-    const double t0 = pow(m_over_2, 8.0 / 3.0) * tab[X_T0];
-    mrow[HM32_T0_HI] = static_cast<float>(t0);
-    mrow[HM32_T0_LO] = static_cast<float>(t0 - static_cast<double>(mrow[HM32_T0_HI]));
-    const double two_pi = 6.283185307179586;
-    for (int r = 0; r < 3; ++r) {
-      const int cs = xhm::M_PHASE + r * xhm::kBasis + xhm::B_1, ls = xhm::M_PHASE + r * xhm::kBasis + xhm::B_F;
-      double cr = out[cs] - m_over_2 * tab[X_ANCHOR];
-      cr = cr - two_pi * rint(cr / two_pi);
-      mrow[cs] = static_cast<float>(cr);
-      mrow[HM32_LIN_LO + r] = static_cast<float>(out[ls] - static_cast<double>(mrow[ls]));
+  if (table64 != nullptr) {
+    double* row = table64 + b * kXhmStride64 + H_MODES + M * kXhmModeStride64;
+#pragma unroll
+    for (int k = 0; k < xhm::kModeSize; ++k) {
+      if (xhm::mode_amp_slot(k) == kAmp) row[k] = value(out[k]);
     }
-    for (int k = HM32_LIN_LO + 3; k < kXhmModeStride32; ++k) mrow[k] = 0.0f;
+  }
+  if (table32 != nullptr) {
+    float* row = table32 + b * kXhmStride32 + H_MODES + M * kXhmModeStride32;
+#pragma unroll
+    for (int k = 0; k < xhm::kModeSize; ++k) {
+      if (xhm::mode_amp_slot(k) == kAmp) row[k] = static_cast<float>(value(out[k]));
+    }
+    if constexpr (!kAmp) {
+      // the leading term (m/2)^(8/3) T0 and each region's coefficient of f as
+      // double-floats, each region's constant less (m/2) A modulo 2 pi
+      // (models/xhm/core.py:544-546)
+      constexpr double m_over_2 = xhm::ModeConst<M>::emm * 0.5;
+      const double t0 = xhm::ModeConst<M>::half(0) * value(tab[X_T0]);
+      const float hi = static_cast<float>(t0);
+      row[HM32_T0_HI] = hi;
+      row[HM32_T0_LO] = static_cast<float>(t0 - static_cast<double>(hi));
+      const double two_pi = 6.283185307179586;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const int cs = xhm::M_PHASE + r * xhm::kBasis + xhm::B_1, ls = xhm::M_PHASE + r * xhm::kBasis + xhm::B_F;
+        double cr = value(out[cs]) - m_over_2 * value(tab[X_ANCHOR]);
+        cr = cr - two_pi * rint(cr / two_pi);
+        row[cs] = static_cast<float>(cr);
+        const double l = value(out[ls]);
+        row[HM32_LIN_LO + r] = static_cast<float>(l - static_cast<double>(static_cast<float>(l)));
+      }
+#pragma unroll
+      for (int k = HM32_LIN_LO + 3; k < kXhmModeStride32; ++k) row[k] = 0.0f;
+    }
   }
 }
 
-
-// IMRPhenomXHM's d table / d params: thread (b, part, j) runs its part's
-// set-up (as k_setup_xhm) on dual numbers seeded along parameter j and
-// writes the tangents of the FP64 row's slots its part owns to
-// dtable[(b * kXhmStride64 + k) * 8 + j]. f_ref = 0 stands for the first
-// frequency (or reference_mf / M): its column is zero there. Where the (2,2)
-// set-up failed the head's factors and their tangents are NaN.
-constexpr int kXhmJvpBlock = 64;
-
-__global__ void __launch_bounds__(kXhmJvpBlock)
-    k_setup_xhm_jvp(const double* __restrict__ params, int64_t B, const double* __restrict__ f_min,
-                    int64_t f_min_stride, double amp_scale, double rmf, double* __restrict__ dtable) {
-  const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= B * kDirections) return;
-  const int j = static_cast<int>(c % kDirections);
-  const int64_t b = c / kDirections;
-  const int part = static_cast<int>(blockIdx.y);
-  Dual p[8];
+// Part 0 of binary b: the (2,2) table and the head, as xhm_mode_part. Where
+// the (2,2) set-up failed the head's factors and their tangents are NaN.
+template <class R>
+__device__ __forceinline__ void xhm_head_part(const R* p, int d, int64_t b, double f_min, double amp_scale, double rmf,
+                                              double* table64, float* table32, double* dtable, int32_t* status) {
+  constexpr bool kDual = sizeof(R) != sizeof(double);
+  constexpr int kHead = H_MODES - H_FACTORS;
+  R tab[kTableStride];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) p[k] = Dual(params[b * 8 + k], 0.0);
-  p[j].d = j == 7 && p[7].v == 0.0 ? 0.0 : 1.0;
-  Dual tab[kTableStride];
-  xas::Internals<Dual> in;
-  const xas::Vars<Dual> v = xas::variables<Dual>(p);
-  const int32_t st = xas::setup(p, f_min[b * f_min_stride], amp_scale, rmf, tab,
-                                DirectFits<Dual, xas::Vars<Dual>>{v}, &in);
-  double* drow = dtable + b * kXhmStride64 * kDirections + j;
-  if (part == 0) {
+  for (int k = 0; k < kTableStride; ++k) tab[k] = R(0.0);
+  xas::Internals<R> in;
+  const xas::Vars<R> v = xas::variables<R>(p);
+  const DirectFits<R, xas::Vars<R>> fits{v};
+  const int32_t st = xas::setup<R>(p, f_min, amp_scale, rmf, tab, fits, &in);
+  double* row64 = table64 != nullptr ? table64 + b * kXhmStride64 : nullptr;
+  float* row32 = table32 != nullptr ? table32 + b * kXhmStride32 : nullptr;
+  if constexpr (kDual) {
+    double* drow = dtable + b * kXhmStride64 * kDirections + d;
+#pragma unroll
     for (int k = 0; k < kTableStride; ++k) drow[k * kDirections] = tab[k].d;
-    Dual head[H_MODES - H_FACTORS];
-    xhm::mode_factors(p[5], head);
-    for (int k = 0; k < xhm::kHeadFactors; ++k) head[k].d = st != 0 ? NAN : head[k].d;
-    head[H_AMP0 - H_FACTORS] = in.amp0;
-    head[H_S - H_FACTORS] = in.m_sec;
-    head[H_COS_A - H_FACTORS] = w_cos(tab[X_ANCHOR]);
-    head[H_SIN_A - H_FACTORS] = w_sin(tab[X_ANCHOR]);
-    for (int k = 0; k < H_MODES - H_FACTORS; ++k) drow[(H_FACTORS + k) * kDirections] = head[k].d;
-    return;
+#pragma unroll
+    for (int k = 0; k < kHead; ++k) {
+      double t = k < xhm::kHeadFactors && st != 0 ? NAN : 0.0;
+      if (k == H_AMP0 - H_FACTORS) t = in.amp0.d;
+      if (k == H_S - H_FACTORS) t = in.m_sec.d;
+      if (k == H_COS_A - H_FACTORS) t = w_cos(tab[X_ANCHOR]).d;
+      if (k == H_SIN_A - H_FACTORS) t = w_sin(tab[X_ANCHOR]).d;
+      drow[(H_FACTORS + k) * kDirections] = t;
+    }
   }
-  const int m = part - 1;
-  Dual out[xhm::kModeSize];
-  xhm::mode_table(in, tab, m, out);
-  double* mrow = drow + (H_MODES + m * kXhmModeStride64) * kDirections;
-  for (int k = 0; k < xhm::kModeSize; ++k) mrow[k * kDirections] = out[k].d;
+  if (kDual && d != 0) return;
+  double tv[kTableStride], pv[8], head[kHead];
+#pragma unroll
+  for (int k = 0; k < kTableStride; ++k) tv[k] = value(tab[k]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) pv[k] = value(p[k]);
+  // (the factors depend on the inclination alone, their values here and, on
+  // Dual, their tangents along it)
+  R factors[xhm::kHeadFactors];
+  R inclination = pv[5];
+  if constexpr (kDual) inclination.d = 1.0;
+  xhm::mode_factors(inclination, factors);
+#pragma unroll
+  for (int k = 0; k < xhm::kHeadFactors; ++k) head[k] = st != 0 ? NAN : value(factors[k]);
+  head[H_AMP0 - H_FACTORS] = value(in.amp0);
+  head[H_S - H_FACTORS] = value(in.m_sec);
+  head[H_COS_A - H_FACTORS] = cos(tv[X_ANCHOR]);
+  head[H_SIN_A - H_FACTORS] = sin(tv[X_ANCHOR]);
+  if constexpr (kDual) {
+    // the distance, the inclination, phi_ref and f_ref, as write_chain
+    const Tail<kModelXas> t = tail_derivatives<kModelXas>(tv, pv, rmf);
+    double* tail = dtable + b * kXhmStride64 * kDirections + kDualDirections;
+#pragma unroll
+    for (int k = 0; k < kTableStride; ++k) {
+      double* at = tail + k * kDirections;
+      at[0] = normalisation_slot<kModelXas>(k) && !isnan(tv[k]) ? -tv[k] / pv[4] : 0.0;
+      at[1] = k == X_KP ? t.kp : (k == X_KC ? t.kc : 0.0);
+      at[2] = constant_slot<kModelXas>(k) ? t.constant_phi : 0.0;
+      at[3] = constant_slot<kModelXas>(k) ? t.constant_fref : (k == X_ANCHOR ? t.anchor_fref : 0.0);
+    }
+    const double refused = st != 0 ? NAN : 0.0;
+#pragma unroll
+    for (int k = 0; k < kHead; ++k) {
+      double* at = tail + (H_FACTORS + k) * kDirections;
+      const bool factor = k < xhm::kHeadFactors;
+      at[0] = factor ? refused : (k == H_AMP0 - H_FACTORS ? -head[k] / pv[4] : 0.0);
+      at[1] = factor ? refused + factors[factor ? k : 0].d : 0.0;
+      at[2] = factor ? refused : 0.0;
+      at[3] = factor ? refused
+                     : (k == H_COS_A - H_FACTORS ? -head[H_SIN_A - H_FACTORS] * t.anchor_fref
+                                                 : (k == H_SIN_A - H_FACTORS ? head[H_COS_A - H_FACTORS] * t.anchor_fref
+                                                                             : 0.0));
+    }
+  }
+  if constexpr (kDual) return;
+  if (status != nullptr && st != 0) atomicOr(&status[b], st);
+  write_tables<kModelXas>(kRoleAll, tv, 0, row64, row32);
+#pragma unroll
+  for (int k = 0; k < kHead; ++k) {
+    if (row64 != nullptr) row64[H_FACTORS + k] = head[k];
+    if (row32 != nullptr) row32[H_FACTORS + k] = static_cast<float>(head[k]);
+  }
+}
+
+// The set-up of B binaries on R = double (the values), or on Dual: chains
+// (binary, direction d < kDualDirections) that write d table64 / d params
+// (dtable[(b * kXhmStride64 + k) * 8 + j]). f_ref = 0 stands for the first
+// frequency (or reference_mf / M): its column is zero there.
+template <class R>
+__global__ void __launch_bounds__(kXhmSetupBlock)
+    k_setup_xhm(const double* __restrict__ params, int64_t B, const double* __restrict__ f_min, int64_t f_min_stride,
+                double amp_scale, double rmf, double* __restrict__ table64, float* __restrict__ table32,
+                double* __restrict__ dtable, int32_t* __restrict__ status) {
+  constexpr int kChains = sizeof(R) == sizeof(double) ? 1 : kDualDirections;
+  const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (c >= B * kChains) return;
+  const int64_t b = c / kChains;
+  const int d = static_cast<int>(c % kChains);
+  R p[8];
+  chain_params(params, c, kChains, p);
+  const double fm = f_min[b * f_min_stride];
+  switch (blockIdx.y) {
+#define WFX_XHM_PART(k, m, part)                                                                                  \
+  case k:                                                                                                        \
+    xhm_mode_part<m, part, R>(p, d, b, fm, amp_scale, rmf, table64, table32, dtable, status);                  \
+    break;
+    WFX_XHM_PART(1, 0, xhm::kModeAmp)
+    WFX_XHM_PART(2, 1, xhm::kModeAmp)
+    WFX_XHM_PART(3, 2, xhm::kModeAmp)
+    WFX_XHM_PART(4, 3, xhm::kModeAmp)
+    WFX_XHM_PART(5, 0, xhm::kModePhase)
+    WFX_XHM_PART(6, 1, xhm::kModePhase)
+    WFX_XHM_PART(7, 2, xhm::kModePhase)
+    WFX_XHM_PART(8, 3, xhm::kModePhase)
+#undef WFX_XHM_PART
+    default:
+      xhm_head_part<R>(p, d, b, fm, amp_scale, rmf, table64, table32, dtable, status);
+  }
 }
 
 
@@ -620,8 +734,8 @@ int wfx_xhm_setup(const double* params, int64_t B, const double* f_min, int64_t 
     if (rc != cudaSuccess) return static_cast<int>(rc);
   }
   const dim3 grid(static_cast<unsigned>((B + kXhmSetupBlock - 1) / kXhmSetupBlock), kXhmParts);
-  k_setup_xhm<<<grid, kXhmSetupBlock, 0, s>>>(params, B, f_min, f_min_stride, amp_scale, reference_mf, table64,
-                                              table32, status);
+  k_setup_xhm<double><<<grid, kXhmSetupBlock, 0, s>>>(params, B, f_min, f_min_stride, amp_scale, reference_mf, table64,
+                                                      table32, nullptr, status);
   return launched();
 }
 
@@ -635,9 +749,10 @@ int wfx_xhm_setup_jvp(const double* params, int64_t B, const double* f_min, int6
                                  stream);
     if (rc != 0) return rc;
   }
-  const dim3 grid(static_cast<unsigned>((B * kDirections + kXhmJvpBlock - 1) / kXhmJvpBlock), kXhmParts);
-  k_setup_xhm_jvp<<<grid, kXhmJvpBlock, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      params, B, f_min, f_min_stride, amp_scale, reference_mf, dtable);
+  const int64_t chains = B * kDualDirections;
+  const dim3 grid(static_cast<unsigned>((chains + kXhmSetupBlock - 1) / kXhmSetupBlock), kXhmParts);
+  k_setup_xhm<Dual><<<grid, kXhmSetupBlock, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      params, B, f_min, f_min_stride, amp_scale, reference_mf, nullptr, nullptr, dtable, nullptr);
   return launched();
 }
 

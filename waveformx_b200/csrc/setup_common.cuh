@@ -30,10 +30,10 @@ WFX_HD R fit5(int id, const R& a, const R& b, const R& c, const R& d, const R& e
 }
 
 // The parts of a set-up: its amplitude coefficients, its phase
-// coefficients (with the alignment, f_cut and the projection), or both. The
-// two parts share only the fits and the QNM frequencies, so that different
-// blocks can compute them.
-enum Role : int { kRoleAmp = 1, kRolePhase = 2, kRoleAll = 3 };
+// coefficients (with the alignment, f_cut and the projection), both, or
+// neither (IMRPhenomXHM's Internals alone). The two parts share only the fits
+// and the QNM frequencies, so that different blocks can compute them.
+enum Role : int { kRoleNone = 0, kRoleAmp = 1, kRolePhase = 2, kRoleAll = 3 };
 
 // Where a set-up takes its fit values from: evaluated in place from the
 // binary's variables (DirectFits; fit_value of the model's namespace), or
@@ -137,6 +137,88 @@ WFX_HDI bool solve(R (&a)[N][N], R (&b)[N]) {
     for (int c = r + 1; c < N; ++c) s = s - a[r][c] * b[c];
     b[r] = s / a[r][r];
   }
+  return ok;
+}
+
+// The same on dual numbers: the elimination runs once, on the values, and the
+// tangent of the solution solves the same system, A dx = db - dA x, by the
+// elimination's steps again (a third of the work of an elimination in dual
+// arithmetic, and no tangent of the matrix in registers beside it). The
+// values are those of the plain solve.
+template <int N>
+WFX_HD bool solve(Dual (&a)[N][N], Dual (&b)[N]) {
+  double m[N][N], x[N], r[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    x[i] = b[i].v;
+#pragma unroll
+    for (int j = 0; j < N; ++j) m[i][j] = a[i][j].v;
+  }
+  bool ok = true;
+  unsigned swaps = 0;  // bit k: the k-th compare-and-swap exchanged its rows
+  int k = 0;
+#pragma unroll
+  for (int col = 0; col < N; ++col) {
+#pragma unroll
+    for (int i = col + 1; i < N; ++i, ++k) {
+      const bool larger = fabs(m[i][col]) > fabs(m[col][col]);
+      swaps |= static_cast<unsigned>(larger) << k;
+#pragma unroll
+      for (int j = col; j < N; ++j) {
+        const double top = m[col][j], other = m[i][j];
+        m[col][j] = larger ? other : top;
+        m[i][j] = larger ? top : other;
+      }
+      const double top = x[col], other = x[i];
+      x[col] = larger ? other : top;
+      x[i] = larger ? top : other;
+    }
+    ok = ok && fabs(m[col][col]) > 0.0;
+#pragma unroll
+    for (int i = col + 1; i < N; ++i) {
+      const double l = m[i][col] / m[col][col];
+#pragma unroll
+      for (int j = col + 1; j < N; ++j) m[i][j] = m[i][j] - l * m[col][j];
+      x[i] = x[i] - l * x[col];
+      m[i][col] = l;
+    }
+  }
+#pragma unroll
+  for (int i = N - 1; i >= 0; --i) {
+    double s = x[i];
+#pragma unroll
+    for (int j = i + 1; j < N; ++j) s = s - m[i][j] * x[j];
+    x[i] = s / m[i][i];
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    double s = b[i].d;
+#pragma unroll
+    for (int j = 0; j < N; ++j) s = s - a[i][j].d * x[j];
+    r[i] = s;
+  }
+  k = 0;
+#pragma unroll
+  for (int col = 0; col < N; ++col) {
+#pragma unroll
+    for (int i = col + 1; i < N; ++i, ++k) {
+      const bool larger = (swaps >> k) & 1u;
+      const double top = r[col], other = r[i];
+      r[col] = larger ? other : top;
+      r[i] = larger ? top : other;
+    }
+#pragma unroll
+    for (int i = col + 1; i < N; ++i) r[i] = r[i] - m[i][col] * r[col];
+  }
+#pragma unroll
+  for (int i = N - 1; i >= 0; --i) {
+    double s = r[i];
+#pragma unroll
+    for (int j = i + 1; j < N; ++j) s = s - m[i][j] * r[j];
+    r[i] = s / m[i][i];
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) b[i] = Dual(x[i], r[i]);
   return ok;
 }
 

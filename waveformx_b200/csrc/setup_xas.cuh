@@ -152,9 +152,9 @@ WFX_HDI R fit_value(int id, const Vars<R>& v) {
 // ROLE (Role) selects the part of the table computed: the other part's
 // slots are left as they are. A failed amplitude solve makes the amplitude
 // slots NaN; any other refusal makes kp, kc NaN.
-// `out`, when given, receives the Internals (a full set-up, ROLE kRoleAll).
+// `out`, when given, receives the Internals that ROLE computes.
 template <class R, class Fits, int ROLE = kRoleAll>
-WFX_HDI int32_t setup(const R* p, double f_min, double amp_scale, double reference_mf, R* tab, const Fits& fits,
+WFX_HD int32_t setup(const R* p, double f_min, double amp_scale, double reference_mf, R* tab, const Fits& fits,
                       Internals<R>* out = nullptr) {
   using fit::MTSUN_SI;
   using fit::PI;

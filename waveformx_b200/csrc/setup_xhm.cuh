@@ -305,31 +305,102 @@ enum HmBasis : int {
   B_LOG, B_1_3_LOG, B_F_LOG, B_4_3_LOG, kBasis
 };
 
-// The variables of one higher mode (hm/variables.py:100-169 for release
-// 122022 with the QNM fits in 1 - a_final, reference.py:84-104).
-template <class R>
-struct Mode {
-  int tag, ell, emm, mode_int;
-  bool mixing;
-  R f_ring, f_damp, f_meco_lm, chi_s, chi_a, delta_t, f_amp_rd_falloff;
-  R mix[4][2];
+// The constants of mode M (LAL's modeInt): l, m, the powers of 2 / m and m / 2
+// (hm/inspiral.py:30-41, reference.py:419-436) and the PN amplitude's prefactor
+// (hm/inspiral.py:45-52), as numbers: at run time each is a power or logarithm
+// a thread (two on dual numbers).
+template <int M>
+struct ModeConst;
+template <>
+struct ModeConst<0> {
+  static constexpr int tag = 21, ell = 2, emm = 1;
+  static constexpr double kPrefactor = 0.4714045207910317;        // sqrt(2) / 3
+  static constexpr double kM76 = 0.44544935907016964;             // (2/m)^(-7/6)
+  static constexpr double kLogHalf = -0.6931471805599453;         // log(m/2)
+  WFX_HD static constexpr double two_over_m(int k) {              // (2/m)^(k/3)
+    constexpr double c[7] = {1.0, 1.2599210498948732, 1.5874010519681996, 2.0, 2.5198420997897464,
+                             3.174802103936399, 4.0};
+    return c[k];
+  }
+  WFX_HD static constexpr double half(int i) {                    // (m/2)^((8 - i)/3)
+    constexpr double c[13] = {0.15749013123685915, 0.19842513149602495, 0.25, 0.3149802624737183, 0.3968502629920499,
+                              0.5, 0.6299605249474366, 0.7937005259840998, 1.0, 1.2599210498948732,
+                              1.5874010519681996, 2.0, 2.5198420997897464};
+    return c[i];
+  }
+};
+template <>
+struct ModeConst<1> {
+  static constexpr int tag = 33, ell = 3, emm = 3;
+  static constexpr double kPrefactor = 0.6338656910463875;        // (3/4) sqrt(5/7)
+  static constexpr double kM76 = 1.6048697909004945;
+  static constexpr double kLogHalf = 0.4054651081081644;
+  WFX_HD static constexpr double two_over_m(int k) {
+    constexpr double c[7] = {1.0, 0.8735804647362989, 0.7631428283688879, 0.6666666666666666, 0.5823869764908659,
+                             0.5087618855792586, 0.4444444444444444};
+    return c[k];
+  }
+  WFX_HD static constexpr double half(int i) {
+    constexpr double c[13] = {2.948334068485009, 2.575607045744997, 2.25, 1.9655560456566725, 1.7170713638299977,
+                              1.5, 1.3103706971044482, 1.1447142425533319, 1.0, 0.8735804647362989,
+                              0.7631428283688879, 0.6666666666666666, 0.5823869764908659};
+    return c[i];
+  }
+};
+template <>
+struct ModeConst<2> {
+  static constexpr int tag = 32, ell = 3, emm = 2;
+  static constexpr double kPrefactor = 0.2817180849095055;        // sqrt(5/7) / 3
+  static constexpr double kM76 = 1.0, kLogHalf = 0.0;
+  WFX_HD static constexpr double two_over_m(int) { return 1.0; }
+  WFX_HD static constexpr double half(int) { return 1.0; }
+};
+template <>
+struct ModeConst<3> {
+  static constexpr int tag = 44, ell = 4, emm = 4;
+  static constexpr double kPrefactor = 0.5312127152597305;        // (4/9) sqrt(2) sqrt(5/7)
+  static constexpr double kM76 = 2.244924096618746;
+  static constexpr double kLogHalf = 0.6931471805599453;
+  WFX_HD static constexpr double two_over_m(int k) {
+    constexpr double c[7] = {1.0, 0.7937005259840998, 0.6299605249474366, 0.5, 0.3968502629920499, 0.3149802624737183,
+                             0.25};
+    return c[k];
+  }
+  WFX_HD static constexpr double half(int i) {
+    constexpr double c[13] = {6.349604207872798, 5.039684199579493, 4.0, 3.174802103936399, 2.5198420997897464, 2.0,
+                              1.5874010519681996, 1.2599210498948732, 1.0, 0.7937005259840998, 0.6299605249474366,
+                              0.5, 0.3968502629920499};
+    return c[i];
+  }
 };
 
-template <class R>
-WFX_HD Mode<R> mode_struct(const xas::Internals<R>& w, int mode_int, R psi4tostrain) {
-  Mode<R> hm;
-  hm.mode_int = mode_int;
-  hm.tag = mode_int == 0 ? 21 : (mode_int == 1 ? 33 : (mode_int == 2 ? 32 : 44));
-  hm.ell = hm.tag / 10;
-  hm.emm = hm.tag % 10;
-  hm.mixing = hm.tag == 32;
+// The variables of one higher mode (hm/variables.py:100-169 for release
+// 122022 with the QNM fits in 1 - a_final, reference.py:84-104).
+template <class R, int M>
+struct Mode : ModeConst<M> {
+  using C = ModeConst<M>;
+  static constexpr bool mixing = C::tag == 32;
+  R f_ring, f_damp, f_meco_lm, chi_s, chi_a, delta_t, f_amp_rd_falloff;
+  R mix[2][2];  // the (3,2)'s overlaps with the (2,2) and with itself
+};
+
+template <int M, class R>
+WFX_HD Mode<R, M> mode_struct(const xas::Internals<R>& w, R psi4tostrain) {
+  Mode<R, M> hm;
   const R af = w.a_final;
-  R fr = 0.0, fd = 0.0;
-  switch (hm.tag) {
-    case 21: fr = hmfit::fring21(af); fd = hmfit::fdamp21(af); break;
-    case 33: fr = hmfit::fring33(af); fd = hmfit::fdamp33(af); break;
-    case 32: fr = hmfit::fring32(af); fd = hmfit::fdamp32(af); break;
-    default: fr = hmfit::fring44(af); fd = hmfit::fdamp44(af); break;
+  R fr, fd;
+  if constexpr (M == 0) {
+    fr = hmfit::fring21(af);
+    fd = hmfit::fdamp21(af);
+  } else if constexpr (M == 1) {
+    fr = hmfit::fring33(af);
+    fd = hmfit::fdamp33(af);
+  } else if constexpr (M == 2) {
+    fr = hmfit::fring32(af);
+    fd = hmfit::fdamp32(af);
+  } else {
+    fr = hmfit::fring44(af);
+    fd = hmfit::fdamp44(af);
   }
   hm.f_ring = fr / w.m_final;
   hm.f_damp = fd / w.m_final;
@@ -338,16 +409,11 @@ WFX_HD Mode<R> mode_struct(const xas::Internals<R>& w, int mode_int, R psi4tostr
   hm.chi_a = (w.chi1 - w.chi2) * 0.5;
   hm.delta_t = -2.0 * fit::PI * (500.0 + psi4tostrain);
   hm.f_amp_rd_falloff = 2.0 * hm.f_damp + hm.f_ring;
-  for (int i = 0; i < 4; ++i) hm.mix[i][0] = hm.mix[i][1] = 0.0;
-  if (hm.mixing) {
-    hm.mix[0][0] = hmfit::re_l2m2lp2(af);
-    hm.mix[0][1] = hmfit::im_l2m2lp2(af);
-    hm.mix[1][0] = hmfit::re_l2m2lp3(af);
-    hm.mix[1][1] = hmfit::im_l2m2lp3(af);
-    hm.mix[2][0] = -hmfit::re_l3m2lp2(af);
-    hm.mix[2][1] = -hmfit::im_l3m2lp2(af);
-    hm.mix[3][0] = -hmfit::re_l3m2lp3(af);
-    hm.mix[3][1] = -hmfit::im_l3m2lp3(af);
+  if constexpr (M == 2) {
+    hm.mix[0][0] = -hmfit::re_l3m2lp2(af);
+    hm.mix[0][1] = -hmfit::im_l3m2lp2(af);
+    hm.mix[1][0] = -hmfit::re_l3m2lp3(af);
+    hm.mix[1][1] = -hmfit::im_l3m2lp3(af);
   }
   return hm;
 }
@@ -439,33 +505,30 @@ template <class R>
 struct Amp {
   R amp_norm, pn_dominant, f_rd_aux, f_amp_match_in, f_amp_match_im;
   R pn_re[7], pn_im[7], pn_global_factor;
-  R fcut_7_3, fcut_8_3, fcut_3, ins[3];
+  R c_cut;   // the cube root of the inspiral's matching frequency
+  R ins[3];  // the pseudo-PN terms of (f / f_cut)^(7/3), (8/3), (3)
   R rd[5], rd_aux[4];
   R inter[8], inter_center, inter_half;
-  int n_inter;
 };
 
+constexpr double kLn16 = 2.772588722239781, kLn15 = 0.4054651081081644;
+
 // IMRPhenomXHM_GetPNAmplitudeCoefficients (hm/inspiral.py:45-216).
-template <class R>
-WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& amp) {
+template <class R, int M>
+WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R, M>& hm, Amp<R>& amp) {
   const R chi_a = hm.chi_a, chi_s = hm.chi_s, eta = w.eta, delta = w.delta;
-  const R pi = fit::PI;
-  const R sqrt_5_7 = w_sqrt(5.0 / 7.0);
-  const R prefactors[4] = {w_sqrt(2.0) / 3.0, 0.75 * sqrt_5_7, sqrt_5_7 / 3.0, 4.0 * w_sqrt(2.0) / 9.0 * sqrt_5_7};
-  amp.pn_global_factor = w_pow(2.0 / hm.emm, -7.0 / 6.0) * prefactors[hm.mode_int];
+  const double pi = fit::PI;
+  amp.pn_global_factor = hm.kM76 * hm.kPrefactor;
   for (int k = 0; k < 7; ++k) amp.pn_re[k] = amp.pn_im[k] = 0.0;
-  // the powers of the constant 2/m of the mode (hm/inspiral.py:30-41)
-  const R base = hm.tag == 21 ? 2.0 : (hm.tag == 33 ? 2.0 / 3.0 : 0.5);
-  const Powers<R> p2(base);
-  if (hm.tag == 21) {
+  if constexpr (M == 0) {
     R re = 3427.0 * chi_a;
     re = re + 3427.0 * chi_s * delta;
     re = re - 8404.0 * chi_a * eta;
     re = re - 3860.0 * chi_s * delta * eta;
     re = re - 1344.0 * delta * pi;
     R im = -(672.0 * delta);
-    im = im - 672.0 * delta * w_log(16.0);
-    R scale = fit::LALPI_FOUR_THIRDS * p2.four_thirds;
+    im = im - 672.0 * delta * kLn16;
+    R scale = fit::LALPI_FOUR_THIRDS * hm.two_over_m(4);
     amp.pn_re[4] = re / 1344.0 * scale;
     amp.pn_im[4] = im / 1344.0 * scale;
     re = 143063173.0 * chi_a;
@@ -476,11 +539,11 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     re = re + 20176128.0 * delta * eta * pi;
     re = re + 61725888.0 * chi_s * delta * chi_a * chi_a;
     re = re - 81285120.0 * chi_s * delta * eta * chi_a * chi_a;
-    re = re + 20575296.0 * w_pow(chi_a, 3.0);
-    re = re - 81285120.0 * eta * w_pow(chi_a, 3.0);
+    re = re + 20575296.0 * (chi_a * chi_a * chi_a);
+    re = re - 81285120.0 * eta * (chi_a * chi_a * chi_a);
     re = re + 61725888.0 * chi_a * chi_s * chi_s;
     re = re - 165618432.0 * chi_a * eta * chi_s * chi_s;
-    re = re + 20575296.0 * delta * w_pow(chi_s, 3.0);
+    re = re + 20575296.0 * delta * (chi_s * chi_s * chi_s);
     re = re - 1016064.0 * delta * eta * chi_s * chi_s * chi_s;
     re = re + 128873808.0 * chi_a * eta * eta;
     re = re - 3859632.0 * chi_s * delta * eta * eta;
@@ -488,7 +551,7 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     im = im - 72043776.0 * delta * eta;
     im = im - 5402880.0 * delta * fit::LN_2;
     im = im - 17224704.0 * delta * eta * fit::LN_2;
-    scale = fit::LALPI_TWO * p2.two;
+    scale = fit::LALPI_TWO * hm.two_over_m(6);
     amp.pn_re[6] = re / 5.419008e6 * scale;
     amp.pn_im[6] = im / 5.419008e6 * scale;
     const R five = 21535920.0 * delta * eta * eta + (39626496.0 * delta * eta * chi_s * chi_s + (
@@ -496,12 +559,12 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
             -(77982912.0 * delta * chi_a) * chi_a + (24385536.0 * chi_s * delta * pi + (
                 24385536.0 * chi_a * pi + (-(23670792.0 * delta) * eta + (
                     432843264.0 * chi_a * chi_s * eta + (-155965824.0 * chi_a * chi_s - 964357.0 * delta)))))))));
-    amp.pn_re[1] = delta * fit::LALPI_ONE_THIRD * p2.one_third;
-    amp.pn_re[2] = -3.0 * (chi_s * delta + chi_a) / 2.0 * fit::LALPI_TWO_THIRDS * p2.two_thirds;
-    amp.pn_re[3] = (335.0 * delta + 1404.0 * delta * eta) / 672.0 * pi * p2.itself;
-    amp.pn_re[5] = five / 8.128512e6 * fit::LALPI_FIVE_THIRDS * p2.five_thirds;
-  } else if (hm.tag == 33) {
-    const R ln15 = w_log(1.5);
+    amp.pn_re[1] = delta * fit::LALPI_ONE_THIRD * hm.two_over_m(1);
+    amp.pn_re[2] = -3.0 * (chi_s * delta + chi_a) / 2.0 * fit::LALPI_TWO_THIRDS * hm.two_over_m(2);
+    amp.pn_re[3] = (335.0 * delta + 1404.0 * delta * eta) / 672.0 * pi * hm.two_over_m(3);
+    amp.pn_re[5] = five / 8.128512e6 * fit::LALPI_FIVE_THIRDS * hm.two_over_m(5);
+  } else if constexpr (M == 1) {
+    const double ln15 = kLn15;
     R re = 325.0 * chi_a;
     re = re + 325.0 * chi_s * delta;
     re = re - 1120.0 * chi_a * eta;
@@ -509,7 +572,7 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     re = re + 120.0 * delta * pi;
     R im = -(504.0 * delta);
     im = im + 720.0 * delta * ln15;
-    R scale = fit::LALPI_FOUR_THIRDS * p2.four_thirds;
+    R scale = fit::LALPI_FOUR_THIRDS * hm.two_over_m(4);
     amp.pn_re[4] = re / 120.0 * scale;
     amp.pn_im[4] = im / 120.0 * scale;
     re = 22007835.0 * chi_a;
@@ -524,17 +587,17 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     im = im - 98774368.0 * delta * eta;
     im = im - 37810800.0 * delta * ln15;
     im = im + 37558080.0 * delta * eta * ln15;
-    scale = fit::LALPI_TWO * p2.two;
+    scale = fit::LALPI_TWO * hm.two_over_m(6);
     amp.pn_re[6] = re / 2.17728e6 * scale;
     amp.pn_im[6] = im / 2.17728e6 * scale;
     const R five = 2966264784.0 * delta * eta * eta + (55883520.0 * delta * eta * chi_s * chi_s + (
         -(1131641280.0 * delta * chi_s) * chi_s + (4470681600.0 * delta * eta * chi_a * chi_a + (
             -(1131641280.0 * delta * chi_a) * chi_a + (-(5926068792.0 * delta) * eta + (
                 9053130240.0 * chi_a * chi_s * eta + (-2263282560.0 * chi_a * chi_s - 1077664867.0 * delta)))))));
-    amp.pn_re[1] = delta * fit::LALPI_ONE_THIRD * p2.one_third;
-    amp.pn_re[3] = (-1945.0 * delta + 2268.0 * delta * eta) / 672.0 * pi * p2.itself;
-    amp.pn_re[5] = five / 4.4706816e8 * fit::LALPI_FIVE_THIRDS * p2.five_thirds;
-  } else if (hm.tag == 32) {
+    amp.pn_re[1] = delta * fit::LALPI_ONE_THIRD * hm.two_over_m(1);
+    amp.pn_re[3] = (-1945.0 * delta + 2268.0 * delta * eta) / 672.0 * pi * hm.two_over_m(3);
+    amp.pn_re[5] = five / 4.4706816e8 * fit::LALPI_FIVE_THIRDS * hm.two_over_m(5);
+  } else if constexpr (M == 2) {
     R re = 0.0 - 3955.0 * chi_s;
     re = re - 3955.0 * chi_a * delta;
     re = re + 10810.0 * chi_s * eta;
@@ -545,7 +608,7 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     const R scale = fit::LALPI_FIVE_THIRDS;
     amp.pn_re[5] = re / 840.0 * scale;
     amp.pn_im[5] = im / 840.0 * scale;
-    const R six = 5907445488.0 * w_pow(eta, 3.0) + (5830513920.0 * chi_s * chi_s * eta * eta + (
+    const R six = 5907445488.0 * (eta * eta * eta) + (5830513920.0 * chi_s * chi_s * eta * eta + (
         13412044800.0 * chi_a * chi_a * eta * eta + (-(13202119896.0 * eta) * eta + (
             -(11870591040.0 * eta * chi_s) * chi_s + (1131641280.0 * chi_s * chi_s + (
                 -(7865605440.0 * eta * chi_a) * chi_a + (1131641280.0 * chi_a * chi_a + (
@@ -567,54 +630,58 @@ WFX_HD void pn_amplitude(const xas::Internals<R>& w, const Mode<R>& hm, Amp<R>& 
     im = im + 3579.0 * eta;
     im = im + 960.0 * fit::LN_2;
     im = im - 2880.0 * eta * fit::LN_2;
-    const R scale = fit::LALPI_FIVE_THIRDS * p2.five_thirds;
+    const R scale = fit::LALPI_FIVE_THIRDS * hm.two_over_m(5);
     amp.pn_re[5] = re / 120.0 * scale;
     amp.pn_im[5] = im / 120.0 * scale;
-    const R six = -805075876080.0 * w_pow(eta, 3.0) + (-(10897286400.0 * chi_s * chi_s * eta) * eta + (
+    const R six = -805075876080.0 * (eta * eta * eta) + (-(10897286400.0 * chi_s * chi_s * eta) * eta + (
         -(871782912000.0 * chi_a * chi_a * eta) * eta + (2271682065240.0 * eta * eta + (
             224302478400.0 * eta * chi_s * chi_s + (-(73556683200.0 * chi_s) * chi_s + (
                 511264353600.0 * eta * chi_a * chi_a + (-(73556683200.0 * chi_a) * chi_a + (
                     441340099200.0 * chi_a * chi_s * delta * eta + (-745140957231.0 * eta + (
                         -(147113366400.0 * chi_a * chi_s) * delta + 7888301437.0))))))))));
-    amp.pn_re[2] = (-3.0 * eta + 1.0) * fit::LALPI_TWO_THIRDS * p2.two_thirds;
+    amp.pn_re[2] = (-3.0 * eta + 1.0) * fit::LALPI_TWO_THIRDS * hm.two_over_m(2);
     amp.pn_re[4] = (-(446460.0 * eta) * eta + (641105.0 * eta - 158383.0)) / 36960.0 * fit::LALPI_FOUR_THIRDS *
-                   p2.four_thirds;
-    amp.pn_re[6] = six / 2.90594304e10 * fit::LALPI_TWO * p2.two;
+                   hm.two_over_m(4);
+    amp.pn_re[6] = six / 2.90594304e10 * fit::LALPI_TWO * hm.two_over_m(6);
   }
 }
 
-// The PN amplitude times pnGlobalFactor ampNorm f^-7/6 (reference.py:152-162).
+// The PN amplitude times pnGlobalFactor ampNorm f^-7/6 (reference.py:152-162)
+// at c = f^1/3, m76 = f^-7/6.
 template <class R, class T>
-WFX_HD T pn_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
-  const T terms[6] = {p.one_third, p.two_thirds, p.itself, p.four_thirds, p.five_thirds, p.two};
-  T re(amp.pn_re[0]), im(amp.pn_im[0]);
-  for (int k = 0; k < 6; ++k) {
-    re = re + terms[k] * amp.pn_re[k + 1];
-    im = im + terms[k] * amp.pn_im[k + 1];
+WFX_HD T pn_amp_ansatz(const T& c, const T& m76, const Amp<R>& amp) {
+  T re(amp.pn_re[6]), im(amp.pn_im[6]);
+#pragma unroll
+  for (int k = 5; k >= 0; --k) {
+    re = re * c + amp.pn_re[k];
+    im = im * c + amp.pn_im[k];
   }
-  return w_hypot(re, im) * (amp.pn_global_factor * p.m_seven_sixths * amp.amp_norm);
+  return w_hypot(re, im) * (amp.pn_global_factor * m76 * amp.amp_norm);
 }
 
 // PN plus pseudo-PN terms (reference.py:165-172).
 template <class R, class T>
-WFX_HD T inspiral_amp_ansatz(const Powers<T>& p, const Amp<R>& amp) {
-  T pseudo = p.seven_thirds / amp.fcut_7_3 * amp.ins[0] + p.eight_thirds / amp.fcut_8_3 * amp.ins[1];
-  pseudo = p.three / amp.fcut_3 * amp.ins[2] + pseudo;
-  return pn_amp_ansatz(p, amp) + pseudo * p.m_seven_sixths * amp.pn_dominant;
+WFX_HD T inspiral_amp_ansatz(const T& f, const Amp<R>& amp) {
+  const T c = w_cbrt(f);
+  const T m76 = 1.0 / (f * w_sqrt(c));
+  const T r = c / amp.c_cut;
+  const T r2 = r * r, r4 = r2 * r2;
+  const T pseudo = (r4 * r2 * r) * ((amp.ins[2] * r + amp.ins[1]) * r + amp.ins[0]);
+  return pn_amp_ansatz(c, m76, amp) + pseudo * m76 * amp.pn_dominant;
 }
 
 // The Lorentzian of the ringdown amplitude and its derivative
 // (reference.py:195-214).
-template <class R, class T>
-WFX_HD T lorentzian(const T& mf, const Mode<R>& hm, const R* rd) {
+template <class R, int M, class T>
+WFX_HD T lorentzian(const T& mf, const Mode<R, M>& hm, const R* rd) {
   const R fda = hm.f_damp;
   const T dfr = mf - hm.f_ring;
   const R dfd = fda * rd[2];
   return rd[0] * fda / (w_exp(rd[1] / dfd * dfr) * (dfr * dfr + dfd * dfd));
 }
 
-template <class R>
-WFX_HD R rd_amp_dansatz(R mf, const Mode<R>& hm, const R* rd) {
+template <class R, int M>
+WFX_HD R rd_amp_dansatz(R mf, const Mode<R, M>& hm, const R* rd) {
   const R fda = hm.f_damp;
   const R dfr = mf - hm.f_ring;
   const R numerator = rd[0] * (fda * fda * rd[1] * rd[2] * rd[2] + (dfr * dfr * rd[1] + 2.0 * fda * dfr * rd[2]));
@@ -625,13 +692,15 @@ WFX_HD R rd_amp_dansatz(R mf, const Mode<R>& hm, const R* rd) {
 
 // The ringdown amplitude ansatz: the Lorentzian, the cubic of the (3,2)
 // below fRDAux, the fall-off above fAmpRDfalloff (reference.py:217-229).
-template <class R, class T>
-WFX_HD T rd_amp_ansatz(const T& mf, const Mode<R>& hm, const Amp<R>& amp) {
+template <class R, int M, class T>
+WFX_HD T rd_amp_ansatz(const T& mf, const Mode<R, M>& hm, const Amp<R>& amp) {
   T out = value(mf) >= hm.f_amp_rd_falloff ? amp.rd[3] * w_exp(-amp.rd[4] * (mf - hm.f_amp_rd_falloff))
                                             : lorentzian(mf, hm, amp.rd);
-  if (hm.mixing && value(mf) < amp.f_rd_aux) {
-    const R* a = amp.rd_aux;
-    out = ((a[3] * mf + a[2]) * mf + a[1]) * mf + a[0];
+  if constexpr (M == 2) {
+    if (value(mf) < amp.f_rd_aux) {
+      const R* a = amp.rd_aux;
+      out = ((a[3] * mf + a[2]) * mf + a[1]) * mf + a[0];
+    }
   }
   return out;
 }
@@ -649,8 +718,8 @@ struct RdPhase {
   R alpha0, alpha2, alpha_l;
 };
 
-template <class R, class T>
-WFX_HD T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
+template <class R, int M, class T>
+WFX_HD T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R, M>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
   const R frd = hm.f_ring, fda = hm.f_damp;
   const T den = fda * fda + (ff - frd) * (ff - frd);
   if (!hm.mixing) return frd * frd * ph.alpha2 * p.m_two + ph.alpha0 + (ph.alpha_l * fda) / den;
@@ -658,8 +727,8 @@ WFX_HD T rd_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdP
   return sp.alpha4_s * p.m_four + d + (sp.alpha_l_s * fda) / den;
 }
 
-template <class R, class T>
-WFX_HD T rd_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
+template <class R, int M, class T>
+WFX_HD T rd_phase(const T& ff, const Powers<T>& p, const Mode<R, M>& hm, const RdPhase<R>& ph, const Spheroidal<R>& sp) {
   const R frd = hm.f_ring, fda = hm.f_damp;
   const T arctan = w_atan((ff - frd) / fda);
   if (!hm.mixing) {
@@ -674,11 +743,11 @@ WFX_HD T rd_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const RdPh
 
 // The data of the rotation of the (3,2) ringdown (core.py:250-262,
 // reference.py:354-367): the (2,2) whose ringdown it recycles.
-template <class R>
+template <class R, int M>
 struct Rotation {
   const xas::Internals<R>* w;
   const R* tab22;
-  const Mode<R>* hm;
+  const Mode<R, M>* hm;
   const Amp<R>* amp;
   Spheroidal<R> sp;
 };
@@ -686,8 +755,8 @@ struct Rotation {
 // conj(a322) h22 + conj(a323) h32_spheroidal as (re, im), the (2,2) ringdown
 // ansatz rescaled by its leading order with the phase of the (2,2) without
 // its anchor.
-template <class R, class T>
-WFX_HD void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
+template <class R, int M, class T>
+WFX_HD void rotated(const Rotation<R, M>& r, const T& mf, T& re, T& im) {
   const xas::Internals<R>& w = *r.w;
   const Powers<T> p(mf);
   const T a22 = amp22_ringdown(w, mf) * w.amp_norm * p.m_seven_sixths;
@@ -695,9 +764,9 @@ WFX_HD void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
   const T phi22 = rest22(r.tab22, mf, w.m_sec, true, past);
   const T c22 = a22 * w_cos(phi22), s22 = a22 * w_sin(phi22);
   const T amplm = rd_amp_ansatz(mf, *r.hm, *r.amp);
-  const RdPhase<R> none{0.0, 0.0, 0.0};
+  const RdPhase<R> none{R(0.0), R(0.0), R(0.0)};
   const T philm = rd_phase(mf, p, *r.hm, none, r.sp);
-  const R m2r = r.hm->mix[2][0], m2i = r.hm->mix[2][1], m3r = r.hm->mix[3][0], m3i = r.hm->mix[3][1];
+  const R m2r = r.hm->mix[0][0], m2i = r.hm->mix[0][1], m3r = r.hm->mix[1][0], m3i = r.hm->mix[1][1];
   const T a_re = c22 * m2r + s22 * m2i;
   const T a_im = s22 * m2r - c22 * m2i;
   const T b_re = amplm * m3r;
@@ -707,221 +776,206 @@ WFX_HD void rotated(const Rotation<R>& r, const T& mf, T& re, T& im) {
   im = a_im + (b_re * s + b_im * c);
 }
 
-template <int N, class R>
-WFX_HD bool solve_n(R (&a)[N][N], R (&b)[N]) {
-  return solve<R, N>(a, b);
+// The matching frequencies of the amplitude (reference.py:118-147).
+template <class R, int M>
+WFX_HD void amplitude_frequencies(const xas::Internals<R>& w, const Mode<R, M>& hm, Amp<R>& amp) {
+  amp.amp_norm = w.amp_norm;
+  amp.pn_dominant = w.amp_norm * hm.kM76;
+  amp.f_rd_aux = hm.mixing ? hm.f_ring - hm.f_damp : R(0.0);
+  const R eta = w.eta, chi1 = w.chi1;
+  const R fcut_emr = 1.25 * static_cast<double>(hm.emm) *
+                     ((0.000316707064291237 * chi1 * chi1 + (-0.0000858396080377194 * chi1 + 0.011671068725758493)) *
+                      (6.2873167352395125 * eta + 0.8447212540381764)) /
+                     (-0.9977728883419751 * chi1 + 1.2857082764038923);
+  const R funcs = 0.5 * w_tanh((eta - 0.0192234) / 0.004) + 0.5;
+  amp.f_amp_match_in = w.q < 20.0 ? hm.f_meco_lm : funcs * hm.f_meco_lm + (1.0 - funcs) * fcut_emr;
+  amp.f_amp_match_im = hm.mixing ? -0.5 * w.f_damp + w.f_ring : hm.f_ring - hm.f_damp;
 }
 
-// IMRPhenomXHM_GetAmplitudeCoefficients (reference.py:337-348).
-template <class R>
-WFX_HD bool amplitude_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
-                                    Rotation<R>& rot, Amp<R>& amp) {
-  using F1 = typename Deriv<R>::F1;
-  bool ok = true;
-  amp.amp_norm = w.amp_norm;
-  amp.pn_dominant = w.amp_norm * w_pow(2.0 / hm.emm, -7.0 / 6.0);
-  amp.f_rd_aux = hm.mixing ? hm.f_ring - hm.f_damp : 0.0;
-  // fcut of the inspiral (reference.py:118-140) and of the ringdown (:143-147)
-  {
-    const R emm = static_cast<double>(hm.emm), eta = w.eta, chi1 = w.chi1;
-    const R fcut_emr = 1.25 * emm *
-                            ((0.000316707064291237 * chi1 * chi1 + (-0.0000858396080377194 * chi1 + 0.011671068725758493)) *
-                             (6.2873167352395125 * eta + 0.8447212540381764)) /
-                            (-0.9977728883419751 * chi1 + 1.2857082764038923);
-    const R funcs = 0.5 * w_tanh((eta - 0.0192234) / 0.004) + 0.5;
-    amp.f_amp_match_in = w.q < 20.0 ? hm.f_meco_lm : funcs * hm.f_meco_lm + (1.0 - funcs) * fcut_emr;
-  }
-  amp.f_amp_match_im = hm.mixing ? -0.5 * w.f_damp + w.f_ring : hm.f_ring - hm.f_damp;
+// The inspiral: three collocation points of the pseudo-PN terms at 0.5, 0.75
+// and 1 of f_cut (reference.py:175-190). sum_j ins_j x^((7 + j)/3) = b(x) is a
+// parabola in x^1/3 after division by x^(7/3): its divided differences, the
+// nodes being constants.
+template <class R, int M>
+WFX_HD void amplitude_inspiral(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R, M>& hm,
+                               Amp<R>& amp) {
   pn_amplitude(w, hm, amp);
-  // the inspiral: three collocation points of the pseudo-PN terms
-  // (reference.py:175-190; the constant system solved here)
-  {
-    const R fcut = amp.f_amp_match_in;
-    const Powers<R> fin(fcut);
-    amp.fcut_7_3 = fin.seven_thirds;
-    amp.fcut_8_3 = fin.eight_thirds;
-    amp.fcut_3 = fin.three;
-    const R g[3] = {0.5, 0.75, 1.0};
-    R values[3];
-    switch (hm.tag) {
-      case 21: values[0] = hmfit::amp_21_iv1(fa); values[1] = hmfit::amp_21_iv2(fa); values[2] = hmfit::amp_21_iv3(fa); break;
-      case 33: values[0] = hmfit::amp_33_iv1(fa); values[1] = hmfit::amp_33_iv2(fa); values[2] = hmfit::amp_33_iv3(fa); break;
-      case 32: values[0] = hmfit::amp_32_iv1(fa); values[1] = hmfit::amp_32_iv2(fa); values[2] = hmfit::amp_32_iv3(fa); break;
-      default: values[0] = hmfit::amp_44_iv1(fa); values[1] = hmfit::amp_44_iv2(fa); values[2] = hmfit::amp_44_iv3(fa); break;
-    }
-    R a[3][3], b[3];
-    for (int i = 0; i < 3; ++i) {
-      const Powers<R> fi(g[i] * fcut);
-      const R pn = pn_amp_ansatz(fi, amp);
-      b[i] = (w_abs(values[i]) - pn) / amp.pn_dominant / fi.m_seven_sixths;
-      a[i][0] = w_pow(g[i], 7.0 / 3.0);
-      a[i][1] = w_pow(g[i], 8.0 / 3.0);
-      a[i][2] = w_pow(g[i], 3.0);
-    }
-    ok = solve_n<3>(a, b) && ok;
-    amp.ins[0] = b[0];
-    amp.ins[1] = b[1];
-    amp.ins[2] = b[2];
+  const R fcut = amp.f_amp_match_in;
+  amp.c_cut = w_cbrt(fcut);
+  const R p76 = fcut * w_sqrt(amp.c_cut);
+  const R m76 = 1.0 / p76;
+  constexpr double kT[3] = {0.7937005259840998, 0.9085602964160698, 1.0};      // x^1/3
+  constexpr double kM73[3] = {5.039684199579493, 1.9566976289745937, 1.0};     // x^-7/3
+  constexpr double kM76[3] = {2.244924096618746, 1.3988200845621976, 1.0};     // x^-7/6
+  R values[3];
+  if constexpr (M == 0) {
+    values[0] = hmfit::amp_21_iv1(fa), values[1] = hmfit::amp_21_iv2(fa), values[2] = hmfit::amp_21_iv3(fa);
+  } else if constexpr (M == 1) {
+    values[0] = hmfit::amp_33_iv1(fa), values[1] = hmfit::amp_33_iv2(fa), values[2] = hmfit::amp_33_iv3(fa);
+  } else if constexpr (M == 2) {
+    values[0] = hmfit::amp_32_iv1(fa), values[1] = hmfit::amp_32_iv2(fa), values[2] = hmfit::amp_32_iv3(fa);
+  } else {
+    values[0] = hmfit::amp_44_iv1(fa), values[1] = hmfit::amp_44_iv2(fa), values[2] = hmfit::amp_44_iv3(fa);
   }
-  // the ringdown (reference.py:232-264)
-  {
-    const R fdamp = hm.f_damp;
-    R rd[3];
-    if (hm.tag == 32) {
-      rd[0] = w_abs(hmfit::amp_32_alambda(fa));
-      rd[1] = hmfit::amp_32_lambda(fa);
-      rd[2] = hmfit::amp_32_sigma(fa);
-    } else {
-      R c1, c2, c3;
-      if (hm.tag == 21) {
-        c1 = hmfit::amp_21_rdcp1(fa); c2 = hmfit::amp_21_rdcp2(fa); c3 = hmfit::amp_21_rdcp3(fa);
-      } else if (hm.tag == 33) {
-        c1 = hmfit::amp_33_rdcp1(fa); c2 = hmfit::amp_33_rdcp2(fa); c3 = hmfit::amp_33_rdcp3(fa);
-      } else {
-        c1 = hmfit::amp_44_rdcp1(fa); c2 = hmfit::amp_44_rdcp2(fa); c3 = hmfit::amp_44_rdcp3(fa);
-      }
-      c1 = w_abs(c1);
-      c2 = w_abs(c2);
-      c3 = w_abs(c3);
-      // the vetoes
-      if (c3 >= c2 * c2 / c1) c3 = 0.5 * c2 * c2 / c1;
-      if (c3 > c2) c3 = 0.5 * c2;
-      if (c1 < c2 && c3 > c1) c3 = c1;
-      R deno = w_sqrt(c1 / c3) - c1 / c2;
-      if (deno <= 0.0) deno = 1e-16;
-      const R a_lambda = c1 * fdamp / deno;
-      const R sigma = w_sqrt(a_lambda / (c2 * fdamp));
-      rd[0] = a_lambda;
-      rd[1] = 0.5 * sigma * w_log(c1 / c3);
-      rd[2] = sigma;
-    }
-    const R falloff = hm.f_amp_rd_falloff;
-    const R v = lorentzian(falloff, hm, rd);
-    amp.rd[0] = rd[0];
-    amp.rd[1] = rd[1];
-    amp.rd[2] = rd[2];
-    amp.rd[3] = v;
-    amp.rd[4] = -1.0 * rd_amp_dansatz(falloff, hm, rd) / v;
-    for (int j = 0; j < 4; ++j) amp.rd_aux[j] = 0.0;
-    if (hm.mixing) {
-      const R faux = amp.f_rd_aux, fim = amp.f_amp_match_im;
-      R b[4] = {w_abs(hmfit::amp_32_rdaux1(fa)), w_abs(hmfit::amp_32_rdaux2(fa)), lorentzian(faux, hm, amp.rd),
-                     rd_amp_dansatz(faux, hm, amp.rd)};
-      const R freqs[3] = {fim, 0.5 * (fim + faux), faux};
-      R a[4][4];
-      for (int i = 0; i < 3; ++i) {
-        const R f = freqs[i];
-        a[i][0] = 1.0;
-        a[i][1] = f;
-        a[i][2] = f * f;
-        a[i][3] = f * f * f;
-      }
-      a[3][0] = 0.0;
-      a[3][1] = 1.0;
-      a[3][2] = 2.0 * faux;
-      a[3][3] = 3.0 * faux * faux;
-      ok = solve_n<4>(a, b) && ok;
-      for (int j = 0; j < 4; ++j) amp.rd_aux[j] = b[j];
-    }
+  R y[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const R pn = pn_amp_ansatz(kT[i] * amp.c_cut, kM76[i] * m76, amp);
+    y[i] = (w_abs(values[i]) - pn) / amp.pn_dominant * (p76 * (kM73[i] / kM76[i]));
   }
-  // the intermediate: a polynomial in u = (f - f_c) / f_h times f^-7/6
-  // through equispaced collocation points (reference.py:267-322)
-  {
-    const int version21[6] = {1, 1, 0, 1, 0, 2};
-    const int version_other[6] = {2, 1, 1, 1, 1, 2};
-    const int* version = hm.tag == 21 ? version21 : version_other;
-    const R f_in = amp.f_amp_match_in, f_rd = amp.f_amp_match_im;
-    const R deltaf = (f_rd - f_in) / 5.0;
-    const R center = 0.5 * (f_rd + f_in), half = 0.5 * (f_rd - f_in);
-    amp.inter_center = center;
-    amp.inter_half = half;
-    const int n = hm.tag == 21 ? 5 : 8;
-    amp.n_inter = n;
-    const F1 ins = inspiral_amp_ansatz(Powers<F1>(F1(f_in, 1.0)), amp);
-    R rd_value, rd_derivative;
-    if (hm.mixing) {
-      F1 re, im;
-      rotated(rot, F1(f_rd, 1.0), re, im);
-      const F1 h = w_hypot(re, im);
-      rd_value = h.v;
-      rd_derivative = h.d;
+  const R d01 = (y[1] - y[0]) * (1.0 / (kT[1] - kT[0])), d12 = (y[2] - y[1]) * (1.0 / (kT[2] - kT[1]));
+  const R d = (d12 - d01) * (1.0 / (kT[2] - kT[0]));
+  amp.ins[0] = y[0] - d01 * kT[0] + d * (kT[0] * kT[1]);
+  amp.ins[1] = d01 - d * (kT[0] + kT[1]);
+  amp.ins[2] = d;
+}
+
+// The ringdown (reference.py:232-264). Returns false where the (3,2)'s cubic
+// has no two frequencies to go through.
+template <class R, int M>
+WFX_HD bool amplitude_ringdown(const hmfit::Args<R>& fa, const Mode<R, M>& hm, Amp<R>& amp) {
+  const R fdamp = hm.f_damp;
+  R rd[3];
+  if constexpr (M == 2) {
+    rd[0] = w_abs(hmfit::amp_32_alambda(fa));
+    rd[1] = hmfit::amp_32_lambda(fa);
+    rd[2] = hmfit::amp_32_sigma(fa);
+  } else {
+    R c1, c2, c3;
+    if constexpr (M == 0) {
+      c1 = hmfit::amp_21_rdcp1(fa), c2 = hmfit::amp_21_rdcp2(fa), c3 = hmfit::amp_21_rdcp3(fa);
+    } else if constexpr (M == 1) {
+      c1 = hmfit::amp_33_rdcp1(fa), c2 = hmfit::amp_33_rdcp2(fa), c3 = hmfit::amp_33_rdcp3(fa);
     } else {
-      rd_value = rd_amp_ansatz(f_rd, hm, amp);
-      rd_derivative = rd_amp_dansatz(f_rd, hm, amp.rd);
+      c1 = hmfit::amp_44_rdcp1(fa), c2 = hmfit::amp_44_rdcp2(fa), c3 = hmfit::amp_44_rdcp3(fa);
     }
+    c1 = w_abs(c1);
+    c2 = w_abs(c2);
+    c3 = w_abs(c3);
+    // the vetoes
+    if (c3 >= c2 * c2 / c1) c3 = 0.5 * c2 * c2 / c1;
+    if (c3 > c2) c3 = 0.5 * c2;
+    if (c1 < c2 && c3 > c1) c3 = c1;
+    R deno = w_sqrt(c1 / c3) - c1 / c2;
+    if (deno <= 0.0) deno = 1e-16;
+    const R a_lambda = c1 * fdamp / deno;
+    const R sigma = w_sqrt(a_lambda / (c2 * fdamp));
+    rd[0] = a_lambda;
+    rd[1] = 0.5 * sigma * w_log(c1 / c3);
+    rd[2] = sigma;
+  }
+  const R falloff = hm.f_amp_rd_falloff;
+  const R v = lorentzian(falloff, hm, rd);
+  amp.rd[0] = rd[0];
+  amp.rd[1] = rd[1];
+  amp.rd[2] = rd[2];
+  amp.rd[3] = v;
+  amp.rd[4] = -1.0 * rd_amp_dansatz(falloff, hm, rd) / v;
+  if constexpr (M == 2) {
+    // the cubic below fRDAux: values at fim, half way and faux, the
+    // derivative at faux, in v = (f - fim) / (faux - fim) = 0, 1/2, 1, 1
+    const R faux = amp.f_rd_aux, fim = amp.f_amp_match_im;
+    const R h = faux - fim, r = 1.0 / h;
+    const R y0 = w_abs(hmfit::amp_32_rdaux1(fa)), y1 = w_abs(hmfit::amp_32_rdaux2(fa));
+    const R y2 = lorentzian(faux, hm, amp.rd), dy = h * rd_amp_dansatz(faux, hm, amp.rd);
+    const R d01 = 2.0 * (y1 - y0), d12 = 2.0 * (y2 - y1);
+    const R e0 = d12 - d01, e1 = 2.0 * (dy - d12);
+    const R q3 = (e1 - e0) * (r * r * r);
+    const R q2 = (e0 - 1.5 * (e1 - e0)) * (r * r);
+    const R q1 = (d01 - 0.5 * e0 + 0.5 * (e1 - e0)) * r;
+    amp.rd_aux[3] = q3;
+    amp.rd_aux[2] = q2 - 3.0 * fim * q3;
+    amp.rd_aux[1] = q1 + fim * (3.0 * fim * q3 - 2.0 * q2);
+    amp.rd_aux[0] = y0 + fim * (fim * (q2 - fim * q3) - q1);
+    return fabs(value(h)) > 0.0;
+  }
+  return true;
+}
+
+// The intermediate: a polynomial in u = (f - f_c) / f_h times f^-7/6 through
+// the values (and slopes) at equispaced frequencies (reference.py:267-322): u
+// = -1, -0.6, ..., 1, constants, so that the polynomial is Newton's on them
+// (a repeated node takes the slope) rather than the solution of an 8 x 8
+// system.
+template <class R, int M>
+WFX_HD bool amplitude_intermediate(const hmfit::Args<R>& fa, const Mode<R, M>& hm, const Rotation<R, M>& rot,
+                                   Amp<R>& amp) {
+  using F1 = typename Deriv<R>::F1;
+  const R f_in = amp.f_amp_match_in, f_rd = amp.f_amp_match_im;
+  const R deltaf = (f_rd - f_in) / 5.0;
+  const R half = 0.5 * (f_rd - f_in);
+  amp.inter_center = 0.5 * (f_rd + f_in);
+  amp.inter_half = half;
+  const F1 ins = inspiral_amp_ansatz(F1(f_in, 1.0), amp);
+  R rd_value, rd_derivative;
+  if constexpr (M == 2) {
+    F1 re, im;
+    rotated(rot, F1(f_rd, 1.0), re, im);
+    const F1 h = w_hypot(re, im);
+    rd_value = h.v;
+    rd_derivative = h.d;
+  } else {
+    rd_value = rd_amp_ansatz(f_rd, hm, amp);
+    rd_derivative = rd_amp_dansatz(f_rd, hm, amp.rd);
+  }
+  // the polynomial's value and slope in u at a frequency where the amplitude
+  // has the value b and the slope db
+  const auto scaled = [&](const R& f, const R& b) { return b * f * w_sqrt(w_cbrt(f)); };
+  const auto slope = [&](const R& f, const R& b, const R& db) {
+    const R s6 = w_sqrt(w_cbrt(f));
+    return half * s6 * (db * f + (7.0 / 6.0) * b);
+  };
+  const auto at = [&](int i) { return deltaf * static_cast<double>(i) + f_in; };
+  constexpr int N = M == 0 ? 5 : 8;
+  R c[N], d_in(0.0);
+  const R d_rd = slope(f_rd, rd_value, rd_derivative);
+  if constexpr (M == 0) {
+    c[0] = scaled(f_in, ins.v);
+    c[1] = scaled(at(1), w_abs(hmfit::amp_21_int1(fa)));
+    c[2] = scaled(at(3), w_abs(hmfit::amp_21_int3(fa)));
+  } else {
+    d_in = slope(f_in, ins.v, ins.d);
+    c[0] = c[1] = scaled(f_in, ins.v);
     R fits_int[4];
-    switch (hm.tag) {
-      case 21: fits_int[0] = hmfit::amp_21_int1(fa); fits_int[1] = hmfit::amp_21_int2(fa);
-               fits_int[2] = hmfit::amp_21_int3(fa); fits_int[3] = hmfit::amp_21_int4(fa); break;
-      case 33: fits_int[0] = hmfit::amp_33_int1(fa); fits_int[1] = hmfit::amp_33_int2(fa);
-               fits_int[2] = hmfit::amp_33_int3(fa); fits_int[3] = hmfit::amp_33_int4(fa); break;
-      case 32: fits_int[0] = hmfit::amp_32_int1(fa); fits_int[1] = hmfit::amp_32_int2(fa);
-               fits_int[2] = hmfit::amp_32_int3(fa); fits_int[3] = hmfit::amp_32_int4(fa); break;
-      default: fits_int[0] = hmfit::amp_44_int1(fa); fits_int[1] = hmfit::amp_44_int2(fa);
-               fits_int[2] = hmfit::amp_44_int3(fa); fits_int[3] = hmfit::amp_44_int4(fa); break;
-    }
-    R a[8][8], b[8];
-    for (int i = 0; i < 8; ++i) {
-      b[i] = 0.0;
-      for (int j = 0; j < 8; ++j) a[i][j] = i == j ? 1.0 : 0.0;  // (unused rows of the 5-point system)
-    }
-    int row = 0;
-    auto value_row = [&](R f) {
-      const R m76 = w_pow(f, -7.0 / 6.0);
-      const R u = (f - center) / half;
-      R uj = 1.0;
-      for (int j = 0; j < n; ++j) {
-        a[row][j] = m76 * uj;
-        uj = uj * u;
-      }
-    };
-    auto derivative_row = [&](R f) {
-      const R m76 = w_pow(f, -7.0 / 6.0);
-      const R u = (f - center) / half;
-      R uj = 1.0, ujm1 = 0.0;
-      for (int j = 0; j < n; ++j) {
-        a[row][j] = m76 * (-(7.0 / 6.0) / f * uj + (j ? j * ujm1 / half : 0.0));
-        ujm1 = uj;
-        uj = uj * u;
-      }
-    };
-    for (int i = 0; i < 6; ++i) {
-      const R f = deltaf * static_cast<double>(i) + f_in;
-      const int digit = version[i];
-      if (digit == 0) continue;
-      if (i == 0) {
-        value_row(f);
-        b[row++] = ins.v;
-        if (digit == 2) {
-          derivative_row(f);
-          b[row++] = ins.d;
-        }
-      } else if (i == 5) {
-        value_row(f);
-        b[row++] = rd_value;
-        if (digit == 2) {
-          derivative_row(f);
-          b[row++] = rd_derivative;
-        }
-      } else {
-        value_row(f);
-        b[row++] = w_abs(fits_int[i - 1]);
-      }
-    }
-    if (n == 5) {
-      R a5[5][5], b5[5];
-      for (int i = 0; i < 5; ++i) {
-        b5[i] = b[i];
-        for (int j = 0; j < 5; ++j) a5[i][j] = a[i][j];
-      }
-      ok = solve_n<5>(a5, b5) && ok;
-      for (int j = 0; j < 8; ++j) amp.inter[j] = j < 5 ? b5[j] : 0.0;
+    if constexpr (M == 1) {
+      fits_int[0] = hmfit::amp_33_int1(fa), fits_int[1] = hmfit::amp_33_int2(fa);
+      fits_int[2] = hmfit::amp_33_int3(fa), fits_int[3] = hmfit::amp_33_int4(fa);
+    } else if constexpr (M == 2) {
+      fits_int[0] = hmfit::amp_32_int1(fa), fits_int[1] = hmfit::amp_32_int2(fa);
+      fits_int[2] = hmfit::amp_32_int3(fa), fits_int[3] = hmfit::amp_32_int4(fa);
     } else {
-      ok = solve_n<8>(a, b) && ok;
-      for (int j = 0; j < 8; ++j) amp.inter[j] = b[j];
+      fits_int[0] = hmfit::amp_44_int1(fa), fits_int[1] = hmfit::amp_44_int2(fa);
+      fits_int[2] = hmfit::amp_44_int3(fa), fits_int[3] = hmfit::amp_44_int4(fa);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[2 + i] = scaled(at(i + 1), w_abs(fits_int[i]));
+  }
+  c[N - 2] = c[N - 1] = scaled(f_rd, rd_value);
+  constexpr double kNodes5[5] = {-1.0, -0.6, 0.2, 1.0, 1.0};
+  constexpr double kNodes8[8] = {-1.0, -1.0, -0.6, -0.2, 0.2, 0.6, 1.0, 1.0};
+  const auto x = [&](int i) { return M == 0 ? kNodes5[i < 5 ? i : 4] : kNodes8[i]; };
+#pragma unroll
+  for (int k = 1; k < N; ++k) {
+#pragma unroll
+    for (int i = N - 1; i >= 1; --i) {
+      if (i < k) continue;
+      if (x(i) == x(i - k)) {
+        c[i] = i == 1 ? d_in : d_rd;
+      } else {
+        c[i] = (c[i] - c[i - 1]) * (1.0 / (x(i) - x(i - k)));
+      }
     }
   }
-  return ok;
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) {
+#pragma unroll
+    for (int i = 0; i < N - 1; ++i) {
+      if (i >= k) c[i] = c[i] - x(k) * c[i + 1];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) amp.inter[j] = j < N ? c[j < N ? j : 0] : R(0.0);
+  return value(f_in) > 0.0 && value(f_rd) > 0.0 && fabs(value(half)) > 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -942,18 +996,20 @@ WFX_HD T ins_phase_int(const T& mf, const Powers<T>& p, const Phase<R>& ph, bool
                        p.one_third, p.two_thirds, mf, p.four_thirds, p.five_thirds, p.two, p.seven_thirds};
   const T log_mf = p.log_;
   T philm(0.0);
+#pragma unroll
   for (int i = leading ? 0 : 1; i < 13; ++i) philm = (ph.phi_l[i] * log_mf + ph.phi[i]) * freqs[i] + philm;
   return philm;
 }
 
 template <class R, class T>
 WFX_HD T ins_dphase(const T& mf, const Powers<T>& p, const Phase<R>& ph) {
-  const R coeffs[13] = {-5.0 / 3.0, -4.0 / 3.0, -1.0, -2.0 / 3.0, -1.0 / 3.0, 0.0, 1.0 / 3.0, 2.0 / 3.0, 1.0,
+  const double coeffs[13] = {-5.0 / 3.0, -4.0 / 3.0, -1.0, -2.0 / 3.0, -1.0 / 3.0, 0.0, 1.0 / 3.0, 2.0 / 3.0, 1.0,
                              4.0 / 3.0, 5.0 / 3.0, 2.0, 7.0 / 3.0};
   const T freqs[13] = {p.m_eight_thirds, p.m_seven_thirds, p.m_two, p.m_five_thirds, p.m_four_thirds, p.m_one,
                        p.m_two_thirds, p.m_one_third, T(1.0), p.one_third, p.two_thirds, mf, p.four_thirds};
   const T log_mf = p.log_;
   T d(0.0);
+#pragma unroll
   for (int i = 0; i < 13; ++i) {
     const T coefficient = ph.phi_l[i] * log_mf + ph.phi[i];
     d = (coefficient * coeffs[i] + ph.phi_l[i]) * freqs[i] + d;
@@ -961,8 +1017,8 @@ WFX_HD T ins_dphase(const T& mf, const Powers<T>& p, const Phase<R>& ph) {
   return d;
 }
 
-template <class R, class T>
-WFX_HD T int_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
+template <class R, int M, class T>
+WFX_HD T int_dphase(const T& ff, const Powers<T>& p, const Mode<R, M>& hm, const Phase<R>& ph) {
   const R fda = hm.f_damp, frd = hm.f_ring;
   const T lor = (ph.c_l * fda) / (fda * fda + (ff - frd) * (ff - frd));
   T d = ph.c1 * p.m_one + ph.c0;
@@ -972,8 +1028,8 @@ WFX_HD T int_dphase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Ph
   return d + lor;
 }
 
-template <class R, class T>
-WFX_HD T int_phase(const T& ff, const Powers<T>& p, const Mode<R>& hm, const Phase<R>& ph) {
+template <class R, int M, class T>
+WFX_HD T int_phase(const T& ff, const Powers<T>& p, const Mode<R, M>& hm, const Phase<R>& ph) {
   const R fda = hm.f_damp, frd = hm.f_ring;
   T x = ph.c0 * ff + ph.c1 * p.log_;
   x = -ph.c2 * p.m_one + x;
@@ -1009,10 +1065,10 @@ WFX_HD R phase_fit(const hmfit::Args<R>& fa, int tag, int i) {
 template <class R>
 WFX_HD R lambda_pn(const hmfit::Args<R>& fa, R eta, int tag) {
   if (eta > 0.01) {
-    const R pi = fit::PI;
+    const double pi = fit::PI;
     R out = 0.0;
     if (tag == 21) out = 2.0 * pi * (-2.0 * fit::LN_2 - 0.5);
-    else if (tag == 33) out = 2.0 / 3.0 * pi * (6.0 * w_log(1.5) + -21.0 / 5.0);
+    else if (tag == 33) out = 2.0 / 3.0 * pi * (6.0 * kLn15 + -21.0 / 5.0);
     else if (tag == 32) out = -((2376.0 * pi * (22.0 * eta - 5.0)) / (11880.0 * eta - 3960.0));
     else out = 45045.0 * pi * (320.0 * (3.0 * eta - 1.0) * fit::LN_2 + (-1193.0 * eta + 336.0)) /
                (2.0 * (5405400.0 * eta - 1801800.0));
@@ -1026,32 +1082,30 @@ WFX_HD R lambda_pn(const hmfit::Args<R>& fa, R eta, int tag) {
   }
 }
 
-// IMRPhenomXHM_PN21AmpSign (hm/phase.py:214-227).
+// IMRPhenomXHM_PN21AmpSign (hm/phase.py:214-227) at M f = 0.008: the
+// coefficients of delta eta, (chi_1 - chi_2 + delta (chi_1 + chi_2)) eta and
+// eta (306 delta - 360 delta eta).
 template <class R>
-WFX_HD bool pn21_amp_sign(R ff, const xas::Internals<R>& w) {
-  const R eta = w.eta, chi1 = w.chi1, chi2 = w.chi2;
-  const R delta = w_sqrt(-4.0 * eta + 1.0);
-  const R sqrt5 = w_sqrt(5.0);
-  const R pi = fit::PI;
-  R out = (-16.0 * delta * eta * ff * w_pow(pi, 1.5)) / (3.0 * sqrt5);
-  out = out + (4.0 * w_pow(2.0, 0.3333333333333333) * (chi1 - chi2 + delta * (chi1 + chi2)) * eta *
-               w_pow(ff, 1.3333333333333333) * w_pow(pi, 1.8333333333333333)) / sqrt5;
-  out = out + (2.0 * w_pow(2.0, 0.6666666666666666) * eta * (306.0 * delta - 360.0 * delta * eta) *
-               w_pow(ff, 1.6666666666666667) * w_pow(pi, 2.1666666666666665)) / (189.0 * sqrt5);
+WFX_HD bool pn21_amp_sign(const xas::Internals<R>& w) {
+  const double eta = value(w.eta), chi1 = value(w.chi1), chi2 = value(w.chi2);
+  const double delta = sqrt(-4.0 * eta + 1.0);
+  double out = -0.1062498980004773 * delta * eta;  // -16 f pi^1.5 / (3 sqrt 5)
+  out = out + 0.02940896476151304 * (chi1 - chi2 + delta * (chi1 + chi2)) * eta;  // 4 2^(1/3) f^(4/3) pi^(11/6) / sqrt 5
+  out = out + 2.871295490843606e-05 * eta * (306.0 * delta - 360.0 * delta * eta);  // 2 2^(2/3) f^(5/3) pi^(13/6) / (189 sqrt 5)
   return out >= 0.0;
 }
 
-template <class R>
-WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R>& hm,
-                                Rotation<R>& rot, Phase<R>& ph) {
+template <class R, int M>
+WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const Mode<R, M>& hm,
+                               const Rotation<R, M>& rot, Phase<R>& ph) {
   using J2 = typename Deriv<R>::J2;
   bool ok = true;
-  const int tag = hm.tag, emm = hm.emm;
+  constexpr int tag = ModeConst<M>::tag, emm = ModeConst<M>::emm;
   const R eta = w.eta, eta_m1 = 1.0 / eta, fring = hm.f_ring, fdamp = hm.f_damp;
   const R fcut = (0.001 * (0.25 / eta - 1.0) + 1.0) * (emm * 1.0) * 0.5 * w.f_meco;
-  const R sqrt3 = w_sqrt(3.0);
+  const double sqrt3 = 1.7320508075688772;
   R freqs[6];
-  if (tag == 32) {
+  if constexpr (tag == 32) {
     const R f_end = -0.5 * w.f_damp + w.f_ring;
     freqs[0] = fcut;
     freqs[1] = (sqrt3 * (fcut - f_end) + 2.0 * (fcut + f_end)) / 4.0;
@@ -1071,6 +1125,7 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
   }
   ph.f_phase_match_in = hm.f_meco_lm;
   R values[6];
+#pragma unroll
   for (int i = 0; i < 6; ++i) values[i] = phase_fit(fa, tag, i) + hm.delta_t;
   const R fcut_rd = ph.f_phase_match_im, fcut_insp = ph.f_phase_match_in;
 
@@ -1079,13 +1134,13 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
     const R non_log[13] = {1.0, 0.0, w.phi2, w.phi3, w.phi4, 0.0, w.phi6, w.phi7, w.phi8, 0.0, 0.0, 0.0, 0.0};
     const R log_terms[13] = {0.0, 0.0, 0.0, 0.0, 0.0, w.phi5l, w.phi6l, 0.0, w.phi8l, 0.0, 0.0, 0.0, 0.0};
     const R pseudo_pn[13] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, w.sigma1, w.sigma2, w.sigma3, w.sigma4, 0.0};
-    const R m_over_2 = emm * 0.5;
-    const R phi_norm = -(3.0 * fit::LALPI_M_FIVE_THIRDS) / 128.0;
+    const double phi_norm = -(3.0 * fit::LALPI_M_FIVE_THIRDS) / 128.0;
     const R fact = phi_norm / eta;
-    const R log_m_over_2 = w_log(m_over_2);
+    const double log_m_over_2 = hm.kLogHalf;
+#pragma unroll
     for (int i = 0; i < 13; ++i) {
       const R nl = non_log[i] * fact, lg = log_terms[i] * fact, ps = pseudo_pn[i] * fact;
-      const R scale = w_pow(m_over_2, (8 - i) / 3.0);
+      const double scale = hm.half(i);
       ph.phi[i] = (-lg * log_m_over_2 + (nl + ps)) * scale;
       ph.phi_l[i] = lg * scale;
     }
@@ -1095,9 +1150,10 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
   ph.c0 = ph.c1 = ph.c2 = ph.c3 = ph.c4 = ph.c_l = 0.0;
 
   // the (2,1) inspiral extends into the intermediate region for high spins
-  if (tag == 21) {
-    const R two_over_m = 2.0 / emm;
+  if constexpr (tag == 21) {
+    const double two_over_m = 2.0 / emm;
     R v[3];
+#pragma unroll
     for (int i = 0; i < 3; ++i) v[i] = 1.0 / eta * dphase22(w, two_over_m * freqs[i], false);
     const R diff12 = v[0] - v[1], diff23 = v[1] - v[2];
     if (w.s_tot_r >= 0.8) {
@@ -1109,15 +1165,17 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
   auto lor = [&](R ff) { return fdamp / (fdamp * fdamp + (ff - fring) * (ff - fring)); };
   R phi0_rd, dphi0_rd;
   const Spheroidal<R>& sp = rot.sp;
-  if (tag != 32) {
+  if constexpr (tag != 32) {
     bool cond_a = eta < kEtaEmr;
     if (emm == hm.ell) cond_a = cond_a || (w.s_tot_r >= 0.8);
     if (tag == 33) cond_a = cond_a || (w.s_tot_r < 0.0);
     const bool cond_b = tag == 21 ? (w.s_tot_r >= 0.8) : false;
-    const int idx2 = cond_a ? 3 : 2;
-    const int idx3 = cond_a ? 4 : (cond_b ? 4 : 3);
-    const int chosen[5] = {0, 1, idx2, idx3, 5};
-    const R wlm = emm == hm.ell ? 2.0 : emm / 3.0;
+    // (the third point: the fourth frequency where cond_a, the fourth: the
+    // fifth where cond_a or cond_b)
+    const bool last3 = cond_a || cond_b;
+    const R f5[5] = {freqs[0], freqs[1], cond_a ? freqs[3] : freqs[2], last3 ? freqs[4] : freqs[3], freqs[5]};
+    const R v5[5] = {values[0], values[1], cond_a ? values[3] : values[2], last3 ? values[4] : values[3], values[5]};
+    const double wlm = emm == hm.ell ? 2.0 : emm / 3.0;
     const R alpha2_fit = hmfit::rd_phase_22_alpha2(fa), alpha_l_fit = hmfit::rd_phase_22_alpha_l(fa);
     ph.rd.alpha2 = 1.0 / (fring * fring) * wlm * alpha2_fit;
     ph.rd.alpha_l = eta_m1 * alpha_l_fit;
@@ -1125,17 +1183,18 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
     phi0_rd = rd_phase(fcut_rd, p_rd, hm, ph.rd, sp);
     dphi0_rd = rd_dphase(fcut_rd, p_rd, hm, ph.rd, sp);
     R a[5][5], b[5];
+#pragma unroll
     for (int i = 0; i < 5; ++i) {
-      const R ff = freqs[chosen[i]];
+      const R ff = f5[i];
       const R ffm1 = 1.0 / ff, ffm2 = ffm1 * ffm1;
       a[i][0] = 1.0;
       a[i][1] = lor(ff);
       a[i][2] = ffm1;
       a[i][3] = ffm2;
       a[i][4] = ffm2 * ffm2;
-      b[i] = values[chosen[i]];
+      b[i] = v5[i];
     }
-    ok = solve_n<5>(a, b) && ok;
+    ok = solve(a, b) && ok;
     ph.c0 = b[0];
     ph.c_l = b[1];
     ph.c1 = b[2];
@@ -1158,6 +1217,7 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
     const R g_c = 0.5 * (1.0 / fcut_insp + 1.0 / fcut_rd);
     const R g_h = 0.5 * (1.0 / fcut_insp - 1.0 / fcut_rd);
     R a[6][6], b[6];
+#pragma unroll
     for (int i = 0; i < 5; ++i) {
       const R v = (1.0 / freqs[i] - g_c) / g_h;
       a[i][0] = 1.0;
@@ -1181,13 +1241,17 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
       a[5][5] = 4.0 * v * v * v * dv;
       b[5] = values[5];
     }
-    ok = solve_n<6>(a, b) && ok;
+    ok = solve(a, b) && ok;
     const R quartic[5] = {b[0], b[2], b[3], b[4], b[5]};
-    R p[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const R comb[5][5] = {{1, 0, 0, 0, 0}, {1, 1, 0, 0, 0}, {1, 2, 1, 0, 0}, {1, 3, 3, 1, 0}, {1, 4, 6, 4, 1}};
-    for (int k = 0; k < 5; ++k) {
-      const R scale = quartic[k] / w_pow(g_h, static_cast<double>(k));
-      for (int j = 0; j <= k; ++j) p[j] = p[j] + scale * comb[k][j] * w_pow(-g_c, static_cast<double>(k - j));
+    // sum_k q_k ((x - g_c) / g_h)^k in powers of x (Horner's rule, from the
+    // highest)
+    R p[5] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
+    const R inv_h = 1.0 / g_h, shift = -g_c * inv_h;
+#pragma unroll
+    for (int k = 4; k >= 0; --k) {
+#pragma unroll
+      for (int j = 4; j >= 1; --j) p[j] = p[j] * shift + p[j - 1] * inv_h;
+      p[0] = p[0] * shift + quartic[k];
     }
     ph.c0 = p[0];
     ph.c_l = b[1];
@@ -1210,14 +1274,15 @@ WFX_HD bool phase_coefficients(const xas::Internals<R>& w, const hmfit::Args<R>&
 
 // The spheroidal (3,2) ringdown aligned with the (2,2) ringdown, without the
 // anchor of the (2,2) in phi0_s (core.py:208-234).
-template <class R>
+template <class R, int M>
 WFX_HD bool spheroidal(const xas::Internals<R>& w, const hmfit::Args<R>& fa, const R* tab22,
-                        const Mode<R>& hm, Spheroidal<R>& sp) {
+                       const Mode<R, M>& hm, Spheroidal<R>& sp) {
   const R fringlm = hm.f_ring, fdamplm = hm.f_damp;
   const R freqs[4] = {w.f_ring, -1.5 * fdamplm + fringlm, -0.5 * fdamplm + fringlm, 0.5 * fdamplm + fringlm};
   R a[4][4];
   R b[4] = {hmfit::rd_phase_32_p1(fa), hmfit::rd_phase_32_p2(fa), hmfit::rd_phase_32_p3(fa),
                   hmfit::rd_phase_32_p4(fa)};
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
     const R ff = freqs[i];
     const R ffm2 = 1.0 / (ff * ff);
@@ -1226,9 +1291,9 @@ WFX_HD bool spheroidal(const xas::Internals<R>& w, const hmfit::Args<R>& fa, con
     a[i][2] = ffm2;
     a[i][3] = ffm2 * ffm2;
   }
-  const bool ok = solve_n<4>(a, b);
+  const bool ok = solve(a, b);
   sp = Spheroidal<R>{b[0], b[1], b[2], b[3], 0.0};
-  const RdPhase<R> none{0.0, 0.0, 0.0};
+  const RdPhase<R> none{R(0.0), R(0.0), R(0.0)};
   {
     const R fref_rd = w.f_ring + w.f_damp;
     const Powers<R> p_ref(fref_rd);
@@ -1290,35 +1355,94 @@ WFX_HD void add_term(R* row, const SPowers<R>& sp, R c, int b, int log_index) {
 // The table of one higher mode (core.py:237-353; MODE_LAYOUT), zero for the
 // odd modes of equal masses and spins. Returns false if a collocation
 // system is singular.
-template <class R>
-WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int, R* out) {
+// The parts of a mode's set-up: its amplitude's slots, and the others (the
+// phase's, with M_ON). They share only the mode's variables (the (3,2): the
+// rotation, of which the phase needs the ringdown amplitude and the amplitude
+// the spheroidal phase), so that different blocks compute them.
+constexpr int kModeAmp = 1, kModePhase = 2;
+
+WFX_HD constexpr bool mode_amp_slot(int k) {
+  return (k >= M_F_AMP_IN && k < M_MIX);
+}
+
+// Whether the odd modes of equal masses and spins vanish (core.py:383-389).
+template <int M, class R>
+WFX_HD bool mode_vanishes(const xas::Internals<R>& w) {
+  return (M == 0 || M == 1) && value(w.q) == 1.0 && value(w.chi1) == value(w.chi2);
+}
+
+template <int M, int PART, class R>
+WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, R* out) {
+#pragma unroll
   for (int k = 0; k < kModeSize; ++k) out[k] = 0.0;
   const hmfit::Args<R> fa = fit_args(w);
   const R psi4_args[4] = {w.eta, w.s_tot_r, w.dchi, sqrt_nonneg(-4.0 * w.eta + 1.0)};
   const R psi4 = fit::fit_call(fit::XAS_PSI4_TO_STRAIN, psi4_args);
-  const Mode<R> hm = mode_struct(w, mode_int, psi4);
-  const bool odd = hm.tag == 21 || hm.tag == 33;
-  if (odd && value(w.q) == 1.0 && value(w.chi1) == value(w.chi2)) return true;  // (core.py:383-389: zeros)
+  const Mode<R, M> hm = mode_struct<M>(w, psi4);
+  if (mode_vanishes<M>(w)) return true;
   Amp<R> amp;
-  Rotation<R> rot{&w, tab22, &hm, &amp, Spheroidal<R>{0.0, 0.0, 0.0, 0.0, 0.0}};
+  Rotation<R, M> rot{&w, tab22, &hm, &amp, Spheroidal<R>{R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)}};
   bool ok = true;
-  if (hm.mixing) ok = spheroidal(w, fa, tab22, hm, rot.sp) && ok;
-  ok = amplitude_coefficients(w, fa, hm, rot, amp) && ok;
+  if constexpr (M == 2) ok = spheroidal(w, fa, tab22, hm, rot.sp) && ok;
+  const R s = w.m_sec;
+  const R amp0 = w.amp0;
+  const Powers<R> p(s);
+  if constexpr (PART == kModeAmp || M == 2) {
+    amplitude_frequencies(w, hm, amp);
+    ok = amplitude_ringdown(fa, hm, amp) && ok;
+  }
+  if constexpr (PART == kModeAmp) {
+    amplitude_inspiral(w, fa, hm, amp);
+    ok = amplitude_intermediate(fa, hm, rot, amp) && ok;
+    // the table (core.py:325-353)
+    out[M_F_AMP_IN] = amp.f_amp_match_in / s;
+    out[M_F_AMP_IM] = amp.f_amp_match_im / s;
+    const R pn_scale = amp.pn_global_factor * amp.amp_norm * p.m_seven_sixths * amp0;
+    const R third[7] = {R(1.0), p.one_third, p.two_thirds, s, p.four_thirds, p.five_thirds, p.two};
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      out[M_PN_RE + k] = amp.pn_re[k] * third[k] * pn_scale;
+      out[M_PN_IM + k] = amp.pn_im[k] * third[k] * pn_scale;
+    }
+    const R fold = amp.pn_dominant * p.m_seven_sixths * amp0;
+    const R r = p.one_third / amp.c_cut, r2 = r * r, r4 = r2 * r2, r7 = r4 * r2 * r;
+    out[M_PSEUDO + 0] = amp.ins[0] * r7 * fold;
+    out[M_PSEUDO + 1] = amp.ins[1] * (r7 * r) * fold;
+    out[M_PSEUDO + 2] = amp.ins[2] * (r7 * r2) * fold;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[M_INTER + j] = amp.inter[j] * p.m_seven_sixths * amp0;
+    out[M_INTER_C] = amp.inter_center / s;
+    out[M_INTER_H] = s / amp.inter_half;
+    const R dfd = hm.f_damp * amp.rd[2];
+    out[M_RD + 0] = amp.rd[0] * hm.f_damp * amp0;
+    out[M_RD + 1] = amp.rd[1] / dfd;
+    out[M_RD + 2] = dfd * dfd;
+    out[M_FALLOFF + 0] = amp.rd[3] * amp0;
+    out[M_FALLOFF + 1] = amp.rd[4] * s;
+    out[M_FALLOFF + 2] = hm.f_amp_rd_falloff / s;
+    if constexpr (M == 2) {
+      const R s_j[4] = {R(1.0), s, p.two, p.three};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) out[M_AUX + j] = amp.rd_aux[j] * s_j[j] * amp0;
+      out[M_F_AUX] = amp.f_rd_aux / s;
+    }
+    return ok;
+  }
   Phase<R> ph;
   ok = phase_coefficients(w, fa, hm, rot, ph) && ok;
 
   // D = deltaphi_lm + (m/2) A (core.py:270-283)
-  const R s = w.m_sec;
-  const R m_over_2 = hm.emm * 0.5;
+  constexpr double m_over_2 = ModeConst<M>::emm * 0.5;
   const R falign = w.eta > kEtaEmr ? 0.6 * m_over_2 * w.f_meco : m_over_2 * w.f_meco;
   R d;
   {
     bool past22;
     const R r22 = rest22(tab22, falign / m_over_2, s, false, past22);
-    const R leading = ph.phi[0] * w_pow(falign, -5.0 / 3.0);
-    const R phi_lm_rest = ph.c1_insp * falign + ins_phase_int(falign, Powers<R>(falign), ph, false) + ph.c_insp;
-    d = (-(3.0 * (fit::PI / 4.0))) * (1.0 - m_over_2) + m_over_2 * r22 - phi_lm_rest - (past22 ? leading : 0.0);
-    if (hm.tag == 21 && pn21_amp_sign(R(0.008), w)) d = d + fit::PI;
+    const Powers<R> pa(falign);
+    const R leading = ph.phi[0] * pa.m_five_thirds;
+    const R phi_lm_rest = ph.c1_insp * falign + ins_phase_int(falign, pa, ph, false) + ph.c_insp;
+    d = (-(3.0 * (fit::PI / 4.0))) * (1.0 - m_over_2) + m_over_2 * r22 - phi_lm_rest - (past22 ? leading : R(0.0));
+    if (M == 0 && pn21_amp_sign(w)) d = d + fit::PI;
   }
 
   // the table (core.py:289-353)
@@ -1326,7 +1450,8 @@ WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int,
   R* rows = out + M_PHASE;
   {
     R* row = rows;  // inspiral
-    const int basis[13] = {-1, B_M4_3, B_M1, B_M2_3, B_M1_3, B_1, B_1_3, B_2_3, B_F, B_4_3, B_5_3, B_F2, B_7_3};
+    constexpr int basis[13] = {-1, B_M4_3, B_M1, B_M2_3, B_M1_3, B_1, B_1_3, B_2_3, B_F, B_4_3, B_5_3, B_F2, B_7_3};
+#pragma unroll
     for (int i = 1; i < 13; ++i) add_term(row, spw, ph.phi[i], basis[i], -1);
     add_term(row, spw, ph.phi_l[5], B_1, B_LOG);
     add_term(row, spw, ph.phi_l[6], B_1_3, B_1_3_LOG);
@@ -1355,18 +1480,17 @@ WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int,
       add_term(row, spw, ph.c_rd + d, B_1, -1);
     }
   }
-  const Powers<R> p(s);
   const R w_at = s / hm.f_damp;
-  if (hm.mixing) {
+  if constexpr (M == 2) {
     out[M_SPH + 0] = rot.sp.alpha0_s * s;
     out[M_SPH + 1] = rot.sp.phi0_s;
     out[M_SPH + 2] = -rot.sp.alpha2_s / s;
     out[M_SPH + 3] = -rot.sp.alpha4_s / 3.0 * p.m_three;
     out[M_ATAN_A + 2] = rot.sp.alpha_l_s;
-    out[M_MIX + 0] = hm.mix[2][0];
-    out[M_MIX + 1] = hm.mix[2][1];
-    out[M_MIX + 2] = hm.mix[3][0];
-    out[M_MIX + 3] = hm.mix[3][1];
+    out[M_MIX + 0] = hm.mix[0][0];
+    out[M_MIX + 1] = hm.mix[0][1];
+    out[M_MIX + 2] = hm.mix[1][0];
+    out[M_MIX + 3] = hm.mix[1][1];
   } else {
     out[M_ATAN_A + 2] = ph.rd.alpha_l;
   }
@@ -1376,34 +1500,6 @@ WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int,
   out[M_SHIFT] = hm.f_ring / s;
   out[M_F_PHASE_IN] = ph.f_phase_match_in / s;
   out[M_F_PHASE_IM] = ph.f_phase_match_im / s;
-  out[M_F_AMP_IN] = amp.f_amp_match_in / s;
-  out[M_F_AMP_IM] = amp.f_amp_match_im / s;
-  const R amp0 = w.amp0;
-  const R pn_scale = amp.pn_global_factor * amp.amp_norm * p.m_seven_sixths * amp0;
-  const R third[7] = {1.0, p.one_third, p.two_thirds, s, p.four_thirds, p.five_thirds, p.two};
-  for (int k = 0; k < 7; ++k) {
-    out[M_PN_RE + k] = amp.pn_re[k] * third[k] * pn_scale;
-    out[M_PN_IM + k] = amp.pn_im[k] * third[k] * pn_scale;
-  }
-  const R fold = amp.pn_dominant * p.m_seven_sixths * amp0;
-  out[M_PSEUDO + 0] = amp.ins[0] / amp.fcut_7_3 * p.seven_thirds * fold;
-  out[M_PSEUDO + 1] = amp.ins[1] / amp.fcut_8_3 * p.eight_thirds * fold;
-  out[M_PSEUDO + 2] = amp.ins[2] / amp.fcut_3 * p.three * fold;
-  for (int j = 0; j < 8; ++j) out[M_INTER + j] = j < amp.n_inter ? amp.inter[j] * p.m_seven_sixths * amp0 : 0.0;
-  out[M_INTER_C] = amp.inter_center / s;
-  out[M_INTER_H] = s / amp.inter_half;
-  const R dfd = hm.f_damp * amp.rd[2];
-  out[M_RD + 0] = amp.rd[0] * hm.f_damp * amp0;
-  out[M_RD + 1] = amp.rd[1] / dfd;
-  out[M_RD + 2] = dfd * dfd;
-  out[M_FALLOFF + 0] = amp.rd[3] * amp0;
-  out[M_FALLOFF + 1] = amp.rd[4] * s;
-  out[M_FALLOFF + 2] = hm.f_amp_rd_falloff / s;
-  if (hm.mixing) {
-    const R s_j[4] = {1.0, s, p.two, p.three};
-    for (int j = 0; j < 4; ++j) out[M_AUX + j] = amp.rd_aux[j] * s_j[j] * amp0;
-    out[M_F_AUX] = amp.f_rd_aux / s;
-  }
   out[M_ON] = 1.0;
   return ok;
 }
@@ -1412,56 +1508,61 @@ WFX_HD bool mode_table(const xas::Internals<R>& w, const R* tab22, int mode_int,
 // The head: the factors (F+, Fx) of each mode h_{l,-m} in the polarizations
 // (reference.py:630-638, _harmonics.py:17-36), amp0 and M in seconds.
 
+WFX_HD constexpr double factorial(int n) {
+  constexpr double f[9] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0};
+  return f[n];
+}
+
 // Wigner's d^l_{m' m}(beta) (the convention of LAL's XLALWignerdMatrix).
-template <class R>
-WFX_HD R wigner_d(int ell, int mp, int m, R beta) {
-  auto fact = [](int n) {
-    R r = 1.0;
-    for (int i = 2; i <= n; ++i) r *= i;
-    return r;
-  };
+template <int ELL, int MP, int M, class R>
+WFX_HD R wigner_d(const R& beta) {
   const R ch = w_cos(beta / 2.0), sh = w_sin(beta / 2.0);
-  const R pre = w_sqrt(fact(ell + mp) * fact(ell - mp) * fact(ell + m) * fact(ell - m));
+  const double pre = sqrt(factorial(ELL + MP) * factorial(ELL - MP) * factorial(ELL + M) * factorial(ELL - M));
   R total = 0.0;
-  const int lo = m - mp > 0 ? m - mp : 0;
-  const int hi = (ell + m) < (ell - mp) ? (ell + m) : (ell - mp);
+  constexpr int lo = M - MP > 0 ? M - MP : 0;
+  constexpr int hi = (ELL + M) < (ELL - MP) ? (ELL + M) : (ELL - MP);
+#pragma unroll
   for (int k = lo; k <= hi; ++k) {
-    const R sign = ((k - m + mp) % 2 == 0) ? 1.0 : -1.0;
-    const R c = sign * pre / (fact(ell + m - k) * fact(k) * fact(ell - k - mp) * fact(k - m + mp));
-    total = total + c * ipow(ch, 2 * ell - 2 * k + m - mp) * ipow(sh, 2 * k - m + mp);
+    const double sign = ((k - M + MP) % 2 == 0) ? 1.0 : -1.0;
+    const double c = sign * pre / (factorial(ELL + M - k) * factorial(k) * factorial(ELL - k - MP) * factorial(k - M + MP));
+    total = total + c * ipow(ch, 2 * ELL - 2 * k + M - MP) * ipow(sh, 2 * k - M + MP);
   }
   return total;
 }
 
 // -2Y_lm(theta, pi/2) as (re, im).
-template <class R>
-WFX_HD void swsh(R theta, int ell, int m, R& re, R& im) {
-  const R norm = w_sqrt((2 * ell + 1) / (4.0 * fit::PI));
-  const R d = norm * wigner_d(ell, m, 2, theta);
-  const R x = static_cast<double>(m) * (fit::PI / 2.0);
-  re = d * w_cos(x);
-  im = d * w_sin(x);
+template <int ELL, int M, class R>
+WFX_HD void swsh(const R& theta, R& re, R& im) {
+  const double norm = sqrt((2 * ELL + 1) / (4.0 * fit::PI));
+  const R d = norm * wigner_d<ELL, M, 2>(theta);
+  const double x = static_cast<double>(M) * (fit::PI / 2.0);
+  re = d * cos(x);
+  im = d * sin(x);
 }
 
 // factors[4 k .. 4 k + 4) = Re F+, Im F+, Re Fx, Im Fx of mode k of
 // (2,2), (2,1), (3,3), (3,2), (4,4).
+template <int ELL, int M, class R>
+WFX_HD void mode_factor(const R& inclination, R* factors) {
+  constexpr double sign = ELL % 2 ? -1.0 : 1.0;
+  R ymr, ymi, yr, yi;
+  swsh<ELL, -M>(inclination, ymr, ymi);
+  swsh<ELL, M>(inclination, yr, yi);
+  const R ysr = yr, ysi = -yi;  // conj
+  // F+ = (ym + sign ystar) / 2, Fx = i (ym - sign ystar) / 2
+  factors[0] = 0.5 * (ymr + sign * ysr);
+  factors[1] = 0.5 * (ymi + sign * ysi);
+  const R dr = ymr - sign * ysr, di = ymi - sign * ysi;
+  factors[2] = -0.5 * di;
+  factors[3] = 0.5 * dr;
+}
 template <class R>
-WFX_HD void mode_factors(R inclination, R* factors) {
-  const int ells[5] = {2, 2, 3, 3, 4}, emms[5] = {2, 1, 3, 2, 4};
-  for (int k = 0; k < 5; ++k) {
-    const int ell = ells[k], emm = emms[k];
-    const R sign = ell % 2 ? -1.0 : 1.0;
-    R ymr, ymi, yr, yi;
-    swsh(inclination, ell, -emm, ymr, ymi);
-    swsh(inclination, ell, emm, yr, yi);
-    const R ysr = yr, ysi = -yi;  // conj
-    // F+ = (ym + sign ystar) / 2, Fx = i (ym - sign ystar) / 2
-    factors[4 * k + 0] = 0.5 * (ymr + sign * ysr);
-    factors[4 * k + 1] = 0.5 * (ymi + sign * ysi);
-    const R dr = ymr - sign * ysr, di = ymi - sign * ysi;
-    factors[4 * k + 2] = -0.5 * di;
-    factors[4 * k + 3] = 0.5 * dr;
-  }
+WFX_HD void mode_factors(const R& inclination, R* factors) {
+  mode_factor<2, 2>(inclination, factors);
+  mode_factor<2, 1>(inclination, factors + 4);
+  mode_factor<3, 3>(inclination, factors + 8);
+  mode_factor<3, 2>(inclination, factors + 12);
+  mode_factor<4, 4>(inclination, factors + 16);
 }
 
 }  // namespace xhm
