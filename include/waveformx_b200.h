@@ -87,6 +87,22 @@ int wfx_version(void);
 /* A static description of a return code or (code > 0) a CUDA error. */
 const char* wfx_status_string(int code);
 
+/* The rows of parameters (B x 8 double: masses, aligned spins, distance,
+ * inclination, phi_ref, f_ref) from eight fields in `precision`: field k of
+ * binary b at fields[k][b * strides[k]] (elements; stride 0 for one value of
+ * every binary). `fields` (device pointers) and `strides` are host arrays.
+ * freqs, f_min: *f_min = freqs[0] in double, or both NULL. */
+int wfx_pack_params(int precision, const void* const* fields, const int64_t* strides, int64_t B, const void* freqs,
+                    double* params, double* f_min, wfx_stream_t stream);
+
+/* The gradient rows of wfx_vjp / wfx_xhm_vjp (B x 9, `precision`) as the
+ * gradients of the fields, in out_precision (not wider than precision), one
+ * after the other in out (13 B elements): masses (B, B), spins (B x 3 twice,
+ * their in-plane components zero), distance, inclination, phi_ref, f_ref and
+ * t_c (B each). */
+int wfx_unpack_gradient(int precision, int out_precision, const void* grad, int64_t B, void* out,
+                        wfx_stream_t stream);
+
 /* The per-binary set-up in FP64 (the coefficient fits, the collocation
  * solves, the connection coefficients, the time shift and the phase
  * alignment at f_ref), one chain per binary. Replaces the table of

@@ -192,3 +192,45 @@ def test_empty_inputs(cuda, approximant):
     assert torch.equal(rows.grad, torch.zeros_like(rows))
     hp, hc = f(binary_of(rows[0].detach().float()), no_freq.float())
     assert tuple(hp.shape) == (0,) and hp.dtype == torch.complex64
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("n", [0, 1, 3, 257])
+def test_fields_without_conversion(cuda, dtype, n):
+    """The drop-in on tensors of one dtype and device (no conversion) equals
+    the general way (the same binary with one field as a list): strain and
+    gradients bit for bit, for one binary (n = 0: fields without an axis) and
+    batches, with expanded, strided and negative-view fields."""
+    import torch
+
+    import waveformx_b200.torch as wt
+
+    real = getattr(torch, dtype)
+    rng = np.random.default_rng(n)
+    rows = max(n, 1)
+    m = np.sort(rng.uniform(10.0, 60.0, (rows, 2)))[:, ::-1]
+    chi = rng.uniform(-0.8, 0.8, (rows, 2))
+    host = {"mass_1": m[:, 0], "mass_2": m[:, 1], "spin_1": np.stack([0 * chi[:, 0], 0 * chi[:, 0], chi[:, 0]], -1),
+            "spin_2": np.stack([0 * chi[:, 0], 0 * chi[:, 0], chi[:, 1]], -1),
+            "luminosity_distance": rng.uniform(100.0, 900.0, rows), "inclination": rng.uniform(0.1, 3.0, rows),
+            "phi_ref": rng.uniform(0.0, 6.0, rows), "f_ref": np.full(rows, 20.0)}
+    grid = torch.linspace(20.0, 400.0, 131, dtype=real, device=cuda)
+    f = wt.polarizations_function("IMRPhenomXAS")
+    out = []
+    for general in (False, True):
+        b = {k: torch.as_tensor(v if n else v[0], dtype=real, device=cuda).clone() for k, v in host.items()}
+        # a strided field, an expanded one and a negative view
+        b["spin_2"] = torch.stack([b["spin_2"], b["spin_2"]], -1)[..., 0]
+        if n:
+            b["f_ref"] = torch.full((), 20.0, dtype=real, device=cuda).expand(n)
+        b["inclination"] = torch._neg_view(-b["inclination"])
+        leaves = {k: b[k].detach().requires_grad_(True) for k in ("mass_1", "spin_1", "phi_ref")}
+        b.update(leaves)
+        if general:
+            b["luminosity_distance"] = list(b["luminosity_distance"].unbind()) if n else [b["luminosity_distance"]]
+        hp, hc = f(b, grid)
+        hp, hc = hp.reshape(rows, -1), hc.reshape(rows, -1)
+        gradients = torch.autograd.grad((hp.abs() ** 2).sum() + hc.real.sum(), list(leaves.values()))
+        out.append([hp.detach(), hc.detach(), *(g.reshape(-1) for g in gradients)])
+    for x, y in zip(*out):
+        assert torch.equal(x, y)

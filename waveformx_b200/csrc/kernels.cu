@@ -16,6 +16,8 @@
 //  * k_contract: per binary, the FP64 sum of its tiles' partial sums and the
 //    product with dtable: the gradient in the parameters.
 //  * k_fwd_f64 / k_adj_f64: the plain FP64 form, one binary per block.
+//  * k_pack_params / k_unpack_gradient: a Binary's fields to the rows of
+//    parameters, the rows of gradients to the fields'.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -1285,6 +1287,58 @@ __global__ void __launch_bounds__(128) k_adj_f64(const double* __restrict__ tabl
 }
 
 // ---------------------------------------------------------------------------
+// the fields of a Binary (the drop-in's inputs) and the rows of parameters
+
+struct FieldPointers {
+  const void* p[8];
+  int64_t stride[8];
+};
+
+// params[b][k] = field k's element b (element strides; zero for one value of
+// every binary) in double, and f_min = the first frequency. One launch where
+// stacking and converting the eight fields took three and some twenty host
+// calls; latency (a few KB).
+template <class S>
+__global__ void __launch_bounds__(kBlock) k_pack_params(FieldPointers f, int64_t B, const S* __restrict__ freqs,
+                                                        double* __restrict__ params, double* __restrict__ f_min) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x;
+  if (i == 0 && freqs != nullptr) *f_min = static_cast<double>(freqs[0]);
+  if (i >= 8 * B) return;
+  const int64_t b = i >> 3;
+  const int k = static_cast<int>(i & 7);
+  const void* from = f.p[0];
+  int64_t stride = f.stride[0];
+#pragma unroll
+  for (int j = 1; j < 8; ++j) {
+    from = k == j ? f.p[j] : from;
+    stride = k == j ? f.stride[j] : stride;
+  }
+  params[i] = static_cast<double>(static_cast<const S*>(from)[b * stride]);
+}
+
+// The gradient's rows (B x 9) as the fields' gradients one after the other:
+// masses (B, B), spins (3 B, 3 B: the in-plane components zero), distance,
+// inclination, phi_ref, f_ref and t_c (B each).
+template <class G, class S>
+__global__ void __launch_bounds__(kBlock) k_unpack_gradient(const G* __restrict__ grad, int64_t B,
+                                                            S* __restrict__ out) {
+  const int64_t b = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x;
+  if (b >= B) return;
+  const G* g = grad + b * kGradColumns;
+  out[b] = static_cast<S>(g[0]);
+  out[B + b] = static_cast<S>(g[1]);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    S* spin = out + (2 + 3 * j) * B + 3 * b;
+    spin[0] = S(0);
+    spin[1] = S(0);
+    spin[2] = static_cast<S>(g[2 + j]);
+  }
+#pragma unroll
+  for (int j = 4; j < kGradColumns; ++j) out[(4 + j) * B + b] = static_cast<S>(g[j]);
+}
+
+// ---------------------------------------------------------------------------
 // host side
 
 int device_sms() {
@@ -1971,6 +2025,45 @@ int wfx_fused_loss_noalloc(int model, int precision, const void* table, const do
   }
   return wfx_fused_loss(model, precision, table, dtable, freqs, offsets, B, n, t_c, data, data_stride, weights,
                         weights_stride, fp, fc, scale, loss, grad, scratch, bytes, stream);
+}
+
+int wfx_pack_params(int precision, const void* const* fields, const int64_t* strides, int64_t B, const void* freqs,
+                    double* params, double* f_min, wfx_stream_t stream) {
+  if (fields == nullptr || strides == nullptr || params == nullptr || B <= 0 || (freqs == nullptr) != (f_min == nullptr))
+    return WFX_EINVAL;
+  FieldPointers f;
+  for (int k = 0; k < 8; ++k) {
+    if (fields[k] == nullptr || strides[k] < 0) return WFX_EINVAL;
+    f.p[k] = fields[k];
+    f.stride[k] = strides[k];
+  }
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const unsigned grid = static_cast<unsigned>((8 * B + kBlock - 1) / kBlock);
+  if (precision == WFX_FP32) {
+    k_pack_params<float><<<grid, kBlock, 0, s>>>(f, B, static_cast<const float*>(freqs), params, f_min);
+  } else if (precision == WFX_FP64) {
+    k_pack_params<double><<<grid, kBlock, 0, s>>>(f, B, static_cast<const double*>(freqs), params, f_min);
+  } else {
+    return WFX_EINVAL;
+  }
+  return launched();
+}
+
+int wfx_unpack_gradient(int precision, int out_precision, const void* grad, int64_t B, void* out,
+                        wfx_stream_t stream) {
+  if (grad == nullptr || out == nullptr || B <= 0) return WFX_EINVAL;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const unsigned grid = static_cast<unsigned>((B + kBlock - 1) / kBlock);
+  if (precision == WFX_FP32 && out_precision == WFX_FP32) {
+    k_unpack_gradient<<<grid, kBlock, 0, s>>>(static_cast<const float*>(grad), B, static_cast<float*>(out));
+  } else if (precision == WFX_FP64 && out_precision == WFX_FP32) {
+    k_unpack_gradient<<<grid, kBlock, 0, s>>>(static_cast<const double*>(grad), B, static_cast<float*>(out));
+  } else if (precision == WFX_FP64 && out_precision == WFX_FP64) {
+    k_unpack_gradient<<<grid, kBlock, 0, s>>>(static_cast<const double*>(grad), B, static_cast<double*>(out));
+  } else {
+    return WFX_EINVAL;
+  }
+  return launched();
 }
 
 }  // extern "C"

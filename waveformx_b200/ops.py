@@ -21,7 +21,8 @@ from . import _lib
 from .exceptions import UnknownApproximantError, UnsupportedError
 
 __all__ = ["APPROXIMANTS", "model_code", "Tables", "setup", "polarizations", "vjp", "fused_loss", "workspace",
-           "setup_jvp_async", "fused_loss_from_params", "fft_length", "overlap", "template_overlap",
+           "setup_jvp_async", "pack_params", "unpack_gradient", "fused_loss_from_params", "fft_length", "overlap",
+           "template_overlap",
            "grid_time_supported", "match_grid_time", "match_refine",
            "polarization_overlap", "template_polarization_overlap", "polarization_refine", "xhm_modes",
            "XHM_MODES", "xhm_dtable", "xhm_vjp", "grid_vjp", "check_offsets", "check_per_frequency",
@@ -55,12 +56,13 @@ def _differentiable(model: int) -> None:
                                "(its gradient: ops.xhm_vjp)")
 
 
+# (plain integers: the prototypes' c_void_p takes them as they are)
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(device: torch.device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def _require(t: torch.Tensor, name: str, dtype=None):
@@ -422,24 +424,59 @@ def setup_jvp_async(approximant: str, params: torch.Tensor, f_min: torch.Tensor,
     stride = 0 if f_min.numel() == 1 else 1
     device = params.device
     rmf = math.nan if reference_mf is None else float(reference_mf)
-    main = torch.cuda.current_stream(device)
     if out is not None:
         _require(out, "out", torch.float64)
         if tuple(out.shape) != (batch, _lib.TABLE_STRIDE, 8):
             raise ValueError(f"out must be ({batch}, {_lib.TABLE_STRIDE}, 8)")
     side = _side_stream(device)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        dtable = out if out is not None else torch.empty((batch, _lib.TABLE_STRIDE, 8), dtype=torch.float64,
-                                                         device=device)
-        _lib.check("wfx_setup_jvp", _lib.library().wfx_setup_jvp(
-            model, _ptr(params), batch, _ptr(f_min), stride, float(amp_scale), rmf, None, None, _ptr(dtable), None,
-            _stream(device)))
-        event = torch.cuda.Event()
-        event.record(side)
+    side.wait_stream(torch.cuda.current_stream(device))
+    dtable = out if out is not None else torch.empty((batch, _lib.TABLE_STRIDE, 8), dtype=torch.float64, device=device)
+    _lib.check("wfx_setup_jvp", _lib.library().wfx_setup_jvp(
+        model, _ptr(params), batch, _ptr(f_min), stride, float(amp_scale), rmf, None, None, _ptr(dtable), None,
+        side.cuda_stream))
+    event = side.record_event()
     if out is None:
-        dtable.record_stream(main)
+        # (allocated on the current stream, used on the second: not reused
+        # before that use is done, though nothing may ever wait for the event)
+        for t in (dtable, params, f_min):
+            t.record_stream(side)
     return dtable, event
+
+
+_POINTERS, _STRIDES = ctypes.c_void_p * 8, ctypes.c_int64 * 8
+
+
+def pack_params(fields, freqs: torch.Tensor):
+    """``(params, f_min)`` of a Binary's eight fields (CUDA tensors of the
+    dtype of ``freqs``: ``(n,)`` or one value, the spins ``(n, 3)`` or
+    ``(3,)``) in one launch: ``(n, 8)`` and ``(1,)`` float64."""
+    batched = fields[0].ndim > 0
+    batch = fields[0].shape[0] if batched else 1
+    if any(map(torch.Tensor.is_neg, fields)):
+        fields = [x.resolve_neg() for x in fields]
+    pointers = [x.data_ptr() for x in fields]
+    for i in (2, 3):
+        pointers[i] += 2 * fields[i].stride(-1) * freqs.element_size()
+    strides = [x.stride(0) for x in fields] if batched else (0,) * 8
+    buffer = torch.empty(8 * batch + 1, dtype=torch.float64, device=freqs.device)
+    params, f_min = buffer[:8 * batch].view(batch, 8), buffer[8 * batch:]
+    _lib.check("wfx_pack_params", _lib.library().wfx_pack_params(
+        _lib.FP32 if freqs.dtype == torch.float32 else _lib.FP64, _POINTERS(*pointers), _STRIDES(*strides), batch,
+        _ptr(freqs), _ptr(params), _ptr(f_min), _stream(freqs.device)))
+    return params, f_min
+
+
+def unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
+    """The nine gradients of a Binary's fields and ``t_c`` (in the order of
+    the fields, the spins ``(n, 3)``) in ``dtype`` from the ``(n, 9)`` rows,
+    in one launch (views of one buffer)."""
+    n = grad.shape[0]
+    out = torch.empty(13 * n, dtype=dtype, device=grad.device)
+    code = lambda t: _lib.FP32 if t == torch.float32 else _lib.FP64  # noqa: E731
+    _lib.check("wfx_unpack_gradient", _lib.library().wfx_unpack_gradient(
+        code(grad.dtype), code(dtype), _ptr(grad), n, _ptr(out), _stream(grad.device)))
+    m1, m2, s1, s2, *rest = out.split([n, n, 3 * n, 3 * n, n, n, n, n, n])
+    return [m1, m2, s1.view(n, 3), s2.view(n, 3), *rest]
 
 
 def fused_loss_from_params(approximant: str, params: torch.Tensor, f_min: torch.Tensor, freqs: torch.Tensor,

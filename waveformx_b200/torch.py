@@ -83,7 +83,8 @@ def _compute_device(device: torch.device) -> torch.device:
 
 class _Polarizations(torch.autograd.Function):
     """``(hplus, hcross)`` of the grid, ``t_c`` and the eight fields (each
-    ``(n,)`` or ``(n, 3)``, batched), with the backward kernel."""
+    ``(n,)`` or ``(n, 3)``, batched; or one binary's, ``()`` or ``(3,)``, with
+    outputs of the grid's length), with the backward kernel."""
 
     @staticmethod
     def forward(ctx, key, out_device, grid, t_c, *fields):
@@ -92,21 +93,22 @@ class _Polarizations(torch.autograd.Function):
         real = grid.dtype
         precision = _lib.FP32 if real == torch.float32 else _lib.FP64
         f = grid.detach().to(device=cdev).contiguous()
-        m1, m2, s1, s2, dist, incl, phi, f_ref = (x.detach().to(device=cdev) for x in fields)
-        params = torch.stack([m1, m2, s1[..., 2], s2[..., 2], dist, incl, phi, f_ref], dim=-1)
-        params = params.to(torch.float64).contiguous()
-        f_min = f[:1].to(torch.float64)
+        single = fields[0].ndim == 0
+        n = 1 if single else fields[0].shape[0]
         needs = any(ctx.needs_input_grad[3:])
         xhm = ops.model_code(approximant) == _lib.XHM
-        ctx.key, ctx.out_device = key, out_device
+        ctx.key, ctx.out_device, ctx.single = key, out_device, single
         ctx.empty = None
-        if params.shape[0] == 0 or f.numel() == 0:
+        if n == 0 or f.numel() == 0:
             # (no binary or no frequency: empty outputs, as the reference's
             # vmapped function gives; nothing to launch)
             complex_dtype = torch.complex64 if precision == _lib.FP32 else torch.complex128
-            ctx.empty = (params.shape[0], f.numel(), real)
-            hp = torch.zeros((params.shape[0], f.numel()), dtype=complex_dtype, device=out_device)
+            ctx.empty = (n, f.numel(), real)
+            hp = torch.zeros((f.numel(),) if single else (n, f.numel()), dtype=complex_dtype, device=out_device)
             return hp, torch.zeros_like(hp)
+        if grid.device != cdev:
+            fields = [x.detach().to(device=cdev) for x in fields]
+        params, f_min = ops.pack_params(fields, f)
         dtable = ready = None
         if needs and not xhm:
             # (the derivatives of the tables on a second stream while the
@@ -123,19 +125,22 @@ class _Polarizations(torch.autograd.Function):
         elif needs or ctx.needs_input_grad[2]:
             # (the grid's derivative: from the FP64 table of the parameters)
             ctx.save_for_backward(tables.table, dtable, f, tc if tc is not None else f[:0], params, f_min)
-        ctx.key, ctx.out_device, ctx.has_tc, ctx.ready, ctx.xhm = key, out_device, tc is not None, ready, xhm
+        ctx.has_tc, ctx.ready, ctx.xhm = tc is not None, ready, xhm
+        if single:
+            hp, hc = hp.view(-1), hc.view(-1)
         return hp.to(out_device), hc.to(out_device)
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, g_hp, g_hc):
         approximant, options = ctx.key
+        need = ctx.needs_input_grad
         if ctx.empty is not None:
             n, n_freq, real = ctx.empty
-            need = ctx.needs_input_grad
+            batch = () if ctx.single else (n,)
             zeros = lambda shape, i: torch.zeros(shape, dtype=real, device=ctx.out_device) if need[i] else None  # noqa: E731
-            fields = [zeros((n, 3) if i in (2, 3) else (n,), 4 + i) for i in range(8)]
-            return (None, None, zeros((n_freq,), 2), zeros((n,), 3), *fields)
+            fields = [zeros((*batch, 3) if i in (2, 3) else batch, 4 + i) for i in range(8)]
+            return (None, None, zeros((n_freq,), 2), zeros(batch, 3), *fields)
         if ctx.xhm:
             params, f_min, f, tc = ctx.saved_tensors
             table = params
@@ -155,28 +160,50 @@ class _Polarizations(torch.autograd.Function):
         # PyTorch's gradient with respect to h is dL/dRe h + i dL/dIm h: the
         # kernels' cotangent convention
         grad_grid = None
-        if ctx.needs_input_grad[2]:
+        if need[2]:
             table64 = ops.setup(approximant, params, f_min, amp_scale=strain_scale(options),
                                 reference_mf=options.reference_mf, precision=_lib.FP64).table
             grad_grid = ops.grid_vjp(approximant, table64, f.to(torch.float64), None,
                                      None if tc is None else tc.to(torch.float64), cot(g_hp), cot(g_hc))
             grad_grid = grad_grid.to(dtype=f.dtype, device=ctx.out_device)
-        if not any(ctx.needs_input_grad[3:]):
+        if not any(need[3:]):
             return (None, None, grad_grid, None) + (None,) * 8
         if ctx.xhm:
             grad = ops.xhm_vjp(params, f_min, f.to(torch.float64), None, None if tc is None else tc.to(torch.float64),
                                cot(g_hp), cot(g_hc), amp_scale=strain_scale(options),
-                               reference_mf=options.reference_mf).to(f.dtype)
+                               reference_mf=options.reference_mf)
         else:
             grad = ops.vjp(approximant, table, dtable, f, None, tc, cot(g_hp), cot(g_hc))
-        grad = grad.to(ctx.out_device)
-        zeros = torch.zeros_like(grad[:, 0])
-        spin = lambda col: torch.stack([zeros, zeros, grad[:, col]], dim=-1)  # noqa: E731
-        by_field = [grad[:, 0], grad[:, 1], spin(2), spin(3), grad[:, 4], grad[:, 5], grad[:, 6], grad[:, 7]]
-        need = ctx.needs_input_grad
-        out = [None, None, grad_grid, grad[:, 8] if (need[3] and ctx.has_tc) else None]
-        out += [g if need[4 + i] else None for i, g in enumerate(by_field)]
+        by_field = ops.unpack_gradient(grad, f.dtype)
+        if ctx.single:
+            by_field = [g.view(3) if i in (2, 3) else g.view(()) for i, g in enumerate(by_field)]
+        *by_field, by_tc = by_field
+        move = lambda g: g if g.device == ctx.out_device else g.to(ctx.out_device)  # noqa: E731
+        out = [None, None, grad_grid, move(by_tc) if (need[3] and ctx.has_tc) else None]
+        out += [move(g) if need[4 + i] else None for i, g in enumerate(by_field)]
         return tuple(out)
+
+
+def _uniform(fields, grid, t_c) -> bool:
+    """Whether the inputs need no conversion: tensors on one device in one of
+    the two precisions, every field with the batch's axis (or none with one).
+    (The general way, some thirty tensor operations that then change nothing,
+    was a third of a call's host time.)"""
+    if not isinstance(grid, torch.Tensor) or grid.dtype not in (torch.float32, torch.float64):
+        return False
+    dtype, device = grid.dtype, grid.device
+    for x in fields:
+        if not isinstance(x, torch.Tensor) or x.dtype != dtype or x.device != device:
+            return False
+    batch = fields[0].shape
+    if len(batch) > 1:
+        return False
+    spin = (*batch, 3)
+    for i, x in enumerate(fields):
+        if x.shape != (spin if i in (2, 3) else batch):
+            return False
+    return t_c is None or (isinstance(t_c, torch.Tensor) and t_c.dtype == dtype and t_c.device == device
+                           and t_c.shape == batch)
 
 
 def _wrap(approximant: str, options: WaveformOptions) -> Callable:
@@ -186,6 +213,8 @@ def _wrap(approximant: str, options: WaveformOptions) -> Callable:
         fields, mapped_tc = _fields(binary)
         if t_c is None:
             t_c = mapped_tc
+        if _uniform(fields, grid, t_c):
+            return _Polarizations.apply((approximant, options), grid.device, grid, t_c, *fields)
         values = [*fields, grid] + ([t_c] if t_c is not None else [])
         tensors = [t for v in values for t in _tensors(v)]
         floats = [t for t in tensors if t.is_floating_point()]
