@@ -15,7 +15,8 @@
 //    reaches memory). Per-tile sums of dL/dtable go to the workspace.
 //  * k_contract: per binary, the FP64 sum of its tiles' partial sums and the
 //    product with dtable: the gradient in the parameters.
-//  * k_fwd_f64 / k_adj_f64: the plain FP64 form, one binary per block.
+//  * k_fwd_f64_shared, k_fwd_f64_ragged: the same in FP64.
+//  * k_adj_f64: the reverse-mode pass in FP64, one binary per block.
 //  * k_pack_params / k_unpack_gradient: a Binary's fields to the rows of
 //    parameters, the rows of gradients to the fields'.
 #include <cuda_runtime.h>
@@ -1142,26 +1143,88 @@ __global__ void __launch_bounds__(kAccSlots) k_contract(const float* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// FP64 plain form: one binary per block
+// FP64 forward on a shared grid
+
+// Block (group, tile): kBlock frequencies, one a thread, of `per` consecutive
+// binaries whose tables are staged once: a frequency's powers (a logarithm,
+// two exponentials and four roots, more FP64 instructions than a binary's own
+// evaluation) are computed once for them, and a single binary spreads over the
+// SMs by tiles. A warp wholly above the XAS cutoff stores zeros without
+// evaluating. Bound by issue (73 % of the slots, the FP64 pipe 44 %). Measured
+// against a block a binary, each with its own powers: IMRPhenomXAS 4.2 us for
+// 1 x 4017 (26.8), 41 for 1000 x 4017 (161), 140 for 4096 x 4017 (623), 10.4
+// for 5 x 60000 (343); IMRPhenomD 181 (621) and TaylorF2 95 (240) for 4096 x
+// 4017.
+constexpr int kF64Binaries = 16;       // binaries per block, at most
+constexpr int64_t kF64Blocks = 1184;   // blocks of a launch before a block takes more than one binary: two waves
+                                       // of four blocks a SM
 
 template <int MODEL>
-__global__ void __launch_bounds__(kBlock) k_fwd_f64(const double* __restrict__ table,
-                                                    const double* __restrict__ freqs,
-                                                    const int64_t* __restrict__ offsets, int64_t n, int64_t B,
-                                                    const double* __restrict__ t_c, double2* __restrict__ hp,
-                                                    double2* __restrict__ hc) {
+__global__ void __launch_bounds__(kBlock, 3) k_fwd_f64_shared(const double* __restrict__ table,
+                                                              const double* __restrict__ freqs, int64_t n, int64_t B,
+                                                              int per, const double* __restrict__ t_c,
+                                                              double2* __restrict__ hp, double2* __restrict__ hc) {
+  __shared__ double sT[kF64Binaries][kTableStride];
+  __shared__ double sTc[kF64Binaries];
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * per;
+  const int count = static_cast<int>(min(static_cast<int64_t>(per), B - base));
+  for (int i = threadIdx.x; i < count * kTableStride; i += kBlock) (&sT[0][0])[i] = table[base * kTableStride + i];
+  if (threadIdx.x < count) sTc[threadIdx.x] = t_c != nullptr ? t_c[base + threadIdx.x] : 0.0;
+  __syncthreads();
+  for (int64_t n0 = static_cast<int64_t>(blockIdx.y) * kBlock; n0 < n; n0 += static_cast<int64_t>(gridDim.y) * kBlock) {
+    const bool in = n0 + threadIdx.x < n;
+    const int64_t i = in ? n0 + threadIdx.x : n0;
+    const Freq<double> q = freq_powers(freqs[i]);
+    double2* out_p = hp + base * n + i;
+    double2* out_c = hc + base * n + i;
+#pragma unroll 1
+    for (int j = 0; j < count; ++j, out_p += n, out_c += n) {
+      const double* T = sT[j];
+      const double kp = T[slot_kp<MODEL>()], kc = T[slot_kc<MODEL>()];
+      double2 vp, vc;
+      bool zero = false;
+      if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, q.f > T[X_F_CUT]);
+      if (zero) {
+        // (0 kp, 0 kc: NaN for a refused binary, as the evaluated form)
+        vp = make_double2(0.0 * kp, 0.0 * kp);
+        vc = make_double2(0.0 * kc, 0.0 * kc);
+      } else {
+        const Point<double> pt = point<MODEL, double>(T, q, sTc[j]);
+        const double ap = kp * pt.amp, ac = kc * pt.amp;
+        vp = make_double2(ap * pt.c, ap * pt.s);
+        vc = make_double2(-ac * pt.s, ac * pt.c);
+      }
+      if (in) {
+        *out_p = vp;
+        *out_c = vc;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 plain form: one binary per block
+
+// The forward on ragged grids: block (binary, part), gridDim.y parts of a
+// binary in steps of kBlock frequencies (a few long binaries fill the SMs).
+template <int MODEL>
+__global__ void __launch_bounds__(kBlock) k_fwd_f64_ragged(const double* __restrict__ table,
+                                                           const double* __restrict__ freqs,
+                                                           const int64_t* __restrict__ offsets, int64_t n, int64_t B,
+                                                           const double* __restrict__ t_c, double2* __restrict__ hp,
+                                                           double2* __restrict__ hc) {
   __shared__ double sT[kTableStride];
   for (int64_t b = blockIdx.x; b < B; b += gridDim.x) {
     __syncthreads();
     if (threadIdx.x < kTableStride) sT[threadIdx.x] = table[b * kTableStride + threadIdx.x];
     __syncthreads();
     const double tc = t_c != nullptr ? t_c[b] : 0.0;
-    const int64_t rs = offsets != nullptr ? min(max(offsets[b], int64_t(0)), n) : b * n;
-    const int64_t re = offsets != nullptr ? min(max(offsets[b + 1], rs), n) : rs + n;
-    const int64_t fbase = offsets != nullptr ? 0 : rs;
+    const int64_t rs = min(max(offsets[b], int64_t(0)), n);
+    const int64_t re = min(max(offsets[b + 1], rs), n);
     const double kp = sT[slot_kp<MODEL>()], kc = sT[slot_kc<MODEL>()];
-    for (int64_t e = rs + threadIdx.x; e < re; e += blockDim.x) {
-      const Freq<double> q = freq_powers(freqs[e - fbase]);
+    for (int64_t e = rs + static_cast<int64_t>(blockIdx.y) * kBlock + threadIdx.x; e < re;
+         e += static_cast<int64_t>(gridDim.y) * kBlock) {
+      const Freq<double> q = freq_powers(freqs[e]);
       const Point<double> pt = point<MODEL, double>(sT, q, tc);
       const double ap = kp * pt.amp, ac = kc * pt.amp;
       hp[e] = make_double2(ap * pt.c, ap * pt.s);
@@ -1169,7 +1232,6 @@ __global__ void __launch_bounds__(kBlock) k_fwd_f64(const double* __restrict__ t
     }
   }
 }
-
 
 // d L / d f for the cotangents (g+, gx) of (h+, hx) (the derivative with
 // respect to the grid of the reference's drop-in, src/waveformx/torch.py:
@@ -1753,12 +1815,34 @@ int wfx_polarizations(int model, int precision, const void* table, const void* f
     return WFX_EINVAL;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (precision == WFX_FP64) {
-    const unsigned grid = static_cast<unsigned>((B < (int64_t(1) << 20) ? B : (int64_t(1) << 20)));
+    const auto* T = static_cast<const double*>(table);
+    const auto* f = static_cast<const double*>(freqs);
+    const auto* tc = static_cast<const double*>(t_c);
+    auto* p = static_cast<double2*>(hp);
+    auto* c = static_cast<double2*>(hc);
     return with_model(model, [&](auto m) {
-      k_fwd_f64<decltype(m)::value><<<grid, kBlock, 0, s>>>(
-          static_cast<const double*>(table), static_cast<const double*>(freqs), offsets, n, B,
-          static_cast<const double*>(t_c), static_cast<double2*>(hp), static_cast<double2*>(hc));
-      return launched();
+      constexpr int64_t kMaxX = (int64_t(1) << 31) - 1, kMaxY = 65535;
+      if (offsets != nullptr) {
+        // (parts of a binary while there are fewer binaries than kF64Blocks,
+        // at most those of its mean length)
+        const int64_t parts = min(max(kF64Blocks / B, int64_t(1)), (n / B + kBlock) / kBlock);
+        const dim3 grid(static_cast<unsigned>(min(B, int64_t(1) << 20)), static_cast<unsigned>(min(parts, kMaxY)));
+        k_fwd_f64_ragged<decltype(m)::value><<<grid, kBlock, 0, s>>>(T, f, offsets, n, B, tc, p, c);
+        return launched();
+      }
+      // (binaries a block: as many as leave kF64Blocks blocks, so that small
+      // batches fill the SMs and large ones share their powers)
+      const int64_t tiles = (n + kBlock - 1) / kBlock;
+      const int per = static_cast<int>(min(max(B * tiles / kF64Blocks, int64_t(1)), static_cast<int64_t>(kF64Binaries)));
+      const int64_t groups = (B + per - 1) / per;
+      for (int64_t g0 = 0; g0 < groups; g0 += kMaxX) {
+        const dim3 grid(static_cast<unsigned>(min(groups - g0, kMaxX)), static_cast<unsigned>(min(tiles, kMaxY)));
+        const int64_t b0 = g0 * per;
+        k_fwd_f64_shared<decltype(m)::value><<<grid, kBlock, 0, s>>>(
+            T + b0 * kTableStride, f, n, B - b0, per, tc != nullptr ? tc + b0 : nullptr, p + b0 * n, c + b0 * n);
+        if (int rc = launched()) return rc;
+      }
+      return 0;
     });
   }
   if (precision != WFX_FP32) return WFX_EINVAL;

@@ -336,7 +336,7 @@ __device__ __forceinline__ double reduced_phase(bool inspiral, const double* T, 
   double phi = (inspiral ? T[t0_slot] * q.y : 0.0) + rest;
   phi = phi - T[anchor_slot];
   phi = phi - kTwoPi * q.f * tc;
-  double turns = rint(phi / kTwoPi);
+  double turns = rint(phi * (1.0 / kTwoPi));
   return phi - turns * kTwoPi;
 }
 
