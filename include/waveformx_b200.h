@@ -95,6 +95,12 @@ const char* wfx_status_string(int code);
 int wfx_pack_params(int precision, const void* const* fields, const int64_t* strides, int64_t B, const void* freqs,
                     double* params, double* f_min, wfx_stream_t stream);
 
+/* bad[b] (B int32) = 1 where binary b's row of hp or hc (complex, (B, n), or
+ * with `offsets` ragged in n flat values) holds a value that is not finite,
+ * else 0. */
+int wfx_nonfinite_rows(int precision, const void* hp, const void* hc, const int64_t* offsets, int64_t B, int64_t n,
+                       int32_t* bad, wfx_stream_t stream);
+
 /* The gradient rows of wfx_vjp / wfx_xhm_vjp (B x 9, `precision`) as the
  * gradients of the fields, in out_precision (not wider than precision), one
  * after the other in out (13 B elements): masses (B, B), spins (B x 3 twice,

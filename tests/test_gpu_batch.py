@@ -145,3 +145,29 @@ def test_ragged_with_empty_rows(cuda, approximant, precision):
         for a, b in ((out.hplus[i], single.hplus[0]), (out.hcross[i], single.hcross[0])):
             a, b = a.cpu().numpy(), b.cpu().numpy()
             np.testing.assert_allclose(a, b, rtol=0, atol=tol * np.abs(b).max())
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("n", [1, 2, 255, 4017])
+def test_nonfinite_rows(cuda, dtype, n):
+    """wfx_nonfinite_rows against torch.isfinite: an infinity or NaN in the
+    real or imaginary part of either array, at a row's ends and middle; rows
+    of odd length (off the 16-byte boundary) and ragged rows, an empty one
+    among them."""
+    import torch
+
+    from waveformx_b200 import ops
+
+    batch = 9
+    hp = torch.randn((batch, n), dtype=getattr(torch, dtype), device=cuda)
+    hc = torch.randn_like(hp)
+    for row, at, value, into in ((1, 0, complex(float("nan"), 0), hp), (3, n - 1, complex(0, float("inf")), hc),
+                                 (4, n // 2, complex(-float("inf"), 0), hc), (8, n - 1, complex(0, float("nan")), hp)):
+        into[row, at] = value
+    expected = ~(torch.isfinite(torch.view_as_real(hp)).flatten(1).all(1)
+                 & torch.isfinite(torch.view_as_real(hc)).flatten(1).all(1))
+    assert torch.equal(ops.nonfinite_rows(hp, hc, None, batch).bool(), expected)
+    # the same values ragged: the first row split in an empty row and itself
+    offsets = torch.tensor([0, 0, *(n * (k + 1) for k in range(batch))], device=cuda)
+    ragged = ops.nonfinite_rows(hp.reshape(-1), hc.reshape(-1), offsets, batch + 1).bool()
+    assert torch.equal(ragged[1:], expected) and not ragged[0]

@@ -122,8 +122,9 @@ def batch_polarizations(approximant: str, grid: Any, parameters: Any, *, threads
     tc_np = None if t_c is None else np.broadcast_to(np.asarray(t_c, dtype=np.float64), (n,))
     rmf = options.reference_mf
     scale = strain_scale(options)
-    out_p, out_c = [], []
+    out_p, out_c, status, bad = [], [], [], []
     status_all = np.zeros(n, dtype=np.int32)
+    finite = np.ones(n, dtype=bool)
     step = n if chunk_size is None else max(1, int(chunk_size))
     if n and len(flat):
         f_dev_all = torch.as_tensor(flat, dtype=real, device=dev)
@@ -139,11 +140,16 @@ def batch_polarizations(approximant: str, grid: Any, parameters: Any, *, threads
                 hp, hc = ops.polarizations(approximant, tables.table, f_dev_all[lo:hi].contiguous(), offs, tc)
             else:
                 hp, hc = ops.polarizations(approximant, tables.table, f_dev_all, None, tc)
-            status_all[start:stop] = tables.status.cpu().numpy()
+            status.append(tables.status)
+            bad.append(ops.nonfinite_rows(hp, hc, offs if ragged else None, stop - start) if hp.numel()
+                       else torch.zeros_like(tables.status))
             out_p.append(hp)
             out_c.append(hc)
-        hplus = torch.cat(out_p)
-        hcross = torch.cat(out_c)
+        hplus = out_p[0] if len(out_p) == 1 else torch.cat(out_p)
+        hcross = out_c[0] if len(out_c) == 1 else torch.cat(out_c)
+        # (read to the host once, after the last chunk is queued)
+        words = torch.cat(status + bad).cpu().numpy()
+        status_all, finite = words[:n], words[n:] == 0
     else:
         hplus = torch.zeros((n, len(flat)) if not ragged else (0,), dtype=cplx, device=dev)
         hcross = torch.zeros_like(hplus)
@@ -152,32 +158,23 @@ def batch_polarizations(approximant: str, grid: Any, parameters: Any, *, threads
         if ok[i]:
             ok[i] = False
             errors[i] = error
-    if ragged:
-        row_of = torch.repeat_interleave(torch.arange(n, device=dev), torch.as_tensor(lengths, device=dev))
-        bad = ~(torch.isfinite(torch.view_as_real(hplus)).all(-1) & torch.isfinite(torch.view_as_real(hcross)).all(-1))
-        finite = torch.ones(n, dtype=torch.bool, device=dev)
-        if bad.any():
-            finite[row_of[bad]] = False
-        finite = finite.cpu().numpy()
-    else:
-        # ((n, N, 2) -> (n,): also for no binary or no frequency)
-        finite = (torch.isfinite(torch.view_as_real(hplus)).all(-1).all(-1)
-                  & torch.isfinite(torch.view_as_real(hcross)).all(-1).all(-1)).cpu().numpy()
     for i in np.flatnonzero(ok & ~finite):
         ok[i] = False
         errors[int(i)] = ModelError(f"{approximant} could not be evaluated for binary {i}")
     if strict and errors:
         raise errors[min(errors)]
-    mask = torch.as_tensor(~ok, device=dev)
+    if not ok.all():
+        mask = torch.as_tensor(~ok, device=dev)
+        if ragged:
+            zero_rows = torch.repeat_interleave(mask, torch.as_tensor(lengths, device=dev))
+            hplus[zero_rows] = 0
+            hcross[zero_rows] = 0
+        else:
+            hplus[mask] = 0
+            hcross[mask] = 0
     if ragged:
-        zero_rows = mask[row_of] if len(flat) else mask[:0]
-        hplus[zero_rows] = 0
-        hcross[zero_rows] = 0
         hplus = list(torch.tensor_split(hplus, offsets_np[1:-1].tolist()))
         hcross = list(torch.tensor_split(hcross, offsets_np[1:-1].tolist()))
-    else:
-        hplus[mask] = 0
-        hcross[mask] = 0
     if output == "numpy":
         conv = lambda x: x.cpu().numpy()  # noqa: E731
         hplus = [conv(x) for x in hplus] if ragged else conv(hplus)

@@ -50,6 +50,7 @@ EXPORTS = {
                                            _P]),
     "wfx_status_string": (ctypes.c_char_p, [_INT]),
     "wfx_pack_params": (_INT, [_INT, _P, _P, _I64, _P, _P, _P, _P]),
+    "wfx_nonfinite_rows": (_INT, [_INT, _P, _P, _P, _I64, _I64, _P, _P]),
     "wfx_unpack_gradient": (_INT, [_INT, _INT, _P, _I64, _P, _P]),
     "wfx_setup": (_INT, [_INT, _P, _I64, _P, _I64, _D, _D, _P, _P, _P, _P]),
     "wfx_setup_jvp": (_INT, [_INT, _P, _I64, _P, _I64, _D, _D, _P, _P, _P, _P, _P]),

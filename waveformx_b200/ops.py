@@ -20,7 +20,7 @@ import torch
 from . import _lib
 from .exceptions import UnknownApproximantError, UnsupportedError
 
-__all__ = ["APPROXIMANTS", "model_code", "Tables", "setup", "polarizations", "vjp", "fused_loss", "workspace",
+__all__ = ["APPROXIMANTS", "model_code", "Tables", "setup", "polarizations", "nonfinite_rows", "vjp", "fused_loss", "workspace",
            "setup_jvp_async", "pack_params", "unpack_gradient", "fused_loss_from_params", "fft_length", "overlap",
            "template_overlap",
            "grid_time_supported", "match_grid_time", "match_refine",
@@ -231,6 +231,19 @@ def polarizations(approximant: str, table: torch.Tensor, freqs: torch.Tensor, of
         model, precision, _ptr(table), _ptr(freqs), _ptr(offsets), batch, n, _ptr(t_c), _ptr(hp), _ptr(hc),
         _ptr(ws), 0 if ws is None else ws.numel(), _stream(table.device)))
     return hp, hc
+
+
+def nonfinite_rows(hp: torch.Tensor, hc: torch.Tensor, offsets: Optional[torch.Tensor], batch: int) -> torch.Tensor:
+    """``(B,)`` int32: 1 where a binary's row of ``hp`` or ``hc`` (``(B, N)``,
+    or flat with ``offsets``) holds a value that is not finite."""
+    _require(hp, "hp")
+    _require(hc, "hc", hp.dtype)
+    bad = torch.empty(batch, dtype=torch.int32, device=hp.device)
+    precision = _lib.FP32 if hp.dtype == torch.complex64 else _lib.FP64
+    n = hp.shape[1] if offsets is None else hp.numel()
+    _lib.check("wfx_nonfinite_rows", _lib.library().wfx_nonfinite_rows(
+        precision, _ptr(hp), _ptr(hc), _ptr(offsets), batch, n, _ptr(bad), _stream(hp.device)))
+    return bad
 
 
 def grid_vjp(approximant: str, table: torch.Tensor, freqs: torch.Tensor, offsets: Optional[torch.Tensor],
