@@ -182,3 +182,46 @@ def test_fused_loss_from_params_is_the_same(cuda, model, ragged):
     loss2, grad2 = ops.fused_loss(approximant, tables.table, tables.dtable, freqs, offsets, t_c, d, w, scale=-0.5)
     assert torch.equal(loss, loss2) and torch.equal(grad, grad2)
     assert torch.equal(status, tables.status)
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("n, batch", [(1, 3), (31, 3), (33, 3), (128, 3), (129, 3), (300, 1600), (700, 6400)])
+def test_fp64_reverse_pass_sums(cuda, model, n, batch):
+    """The FP64 reverse pass of a shared grid at the edges of its spans (128
+    frequencies, 32 a warp), with two and eight binaries a block and several
+    spans a block: the vjp and the fused likelihood of a grid are the sums of
+    those of its frequencies, each taken as a row of its own of a ragged grid
+    (another kernel). Bar: 1e-9 of the sum of the terms' magnitudes (the sums
+    round to 1e-13 of it, and a table's slots cancel by less than 1e4 in the
+    product with the set-up's tangents)."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    base = np.array([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0], [60.0, 15.0, 0.8, 0.5, 1000.0, 2.5, 4.0, 20.0],
+                     [9.0, 7.0, -0.6, 0.2, 200.0, 1.1, 0.3, 20.0]])
+    grid = torch.as_tensor(np.geomspace(20.0, 900.0, n) if n > 1 else np.array([90.0]), device=cuda)
+    rng = np.random.default_rng(n)
+    rows = torch.arange(3, device=cuda).repeat_interleave(n)
+    of = torch.arange(batch, device=cuda) % 3
+    params = torch.as_tensor(base, device=cuda)
+    tables = ops.setup(model, params, grid[:1], precision=_lib.FP64, jvp=True)
+    t_c = torch.tensor([0.01, -0.02, 0.0], dtype=torch.float64, device=cuda)
+    cot = [torch.as_tensor(rng.normal(size=(3, n)) + 1j * rng.normal(size=(3, n)), device=cuda) for _ in range(2)]
+    weights = torch.as_tensor(rng.uniform(0.5, 2.0, n), device=cuda)
+    table, dtable = tables.table[of].contiguous(), tables.dtable[of].contiguous()
+    flat = (tables.table[rows].contiguous(), tables.dtable[rows].contiguous(), grid.repeat(3),
+            torch.arange(3 * n + 1, device=cuda), t_c[rows].contiguous())
+
+    def check(whole, parts):
+        bar = 1e-9 * parts.abs().sum(1)[of]
+        error = (whole - parts.sum(1)[of]).abs()
+        assert bool((error <= bar).all()), (error / bar).max()
+
+    check(ops.vjp(model, table, dtable, grid, None, t_c[of].contiguous(), *(c[of].contiguous() for c in cot)),
+          ops.vjp(model, *flat, *(c.reshape(-1) for c in cot)).reshape(3, n, 9))
+    loss, grad = ops.fused_loss(model, table, dtable, grid, None, t_c[of].contiguous(), cot[0][0].contiguous(), weights,
+                                antenna=(0.6, -0.3), scale=-0.5)
+    loss1, grad1 = ops.fused_loss(model, *flat, cot[0][0].repeat(3), weights.repeat(3), antenna=(0.6, -0.3), scale=-0.5)
+    check(loss[:, None], loss1.reshape(3, n, 1))
+    check(grad, grad1.reshape(3, n, 9))

@@ -16,7 +16,7 @@
 //  * k_contract: per binary, the FP64 sum of its tiles' partial sums and the
 //    product with dtable: the gradient in the parameters.
 //  * k_fwd_f64_shared, k_fwd_f64_ragged: the same in FP64.
-//  * k_adj_f64: the reverse-mode pass in FP64, one binary per block.
+//  * k_rev_f64, k_adj_f64_ragged: the reverse-mode pass in FP64.
 //  * k_nonfinite_rows: which binaries' strain is not finite.
 //  * k_pack_params / k_unpack_gradient: a Binary's fields to the rows of
 //    parameters, the rows of gradients to the fields'.
@@ -34,6 +34,7 @@
 #include "../../include/waveformx_b200.h"
 #include "dual_point.cuh"
 #include "internal.h"
+#include "matrix_sums.cuh"
 #include "point.cuh"
 #include "point_x2.cuh"
 
@@ -1275,8 +1276,379 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 reverse mode on a shared grid
+
+// Block (group, part): up to kRevBinaries consecutive binaries and, kSpan
+// frequencies at a time, the spans part, part + gridDim.y, ... of the grid. A
+// span's powers are computed once for the group's binaries and laid out as the
+// rows of a matrix (matrix_sums.cuh); a warp takes every fourth binary over the
+// span, 32 frequencies at a time: its value, the cotangents of its phase (in
+// the column of its region) and amplitude, and their sums against the rows as
+// matrix products. The sums of each binary wait in shared memory until the
+// block's last span, then its warp contracts them with dtable; with several
+// parts (few binaries) grad and loss, zeroed beforehand, add the parts'
+// atomically. Bound by latency and issue (20 warps a SM; the matrix pipe a
+// quarter busy). Measured against a block a binary with a register per sum and
+// lane (255 registers): IMRPhenomXAS vjp 149 us for 1021 x 4001 (243), the
+// fused likelihood 1512 us for 8192 x 8192 (3722); IMRPhenomD 182 (238) and
+// 2901 (3588), TaylorF2 69 (89) and 996 (1293; 1243 with both tiles of rows);
+// one binary of 4017 frequencies 14.4 (60). Four blocks a SM: 161 us for the
+// first; one wave of blocks: 204.
+constexpr int kRevBlock = kSpan, kRevWarps = kRevBlock / 32;
+constexpr int kRevBinaries = 8;
+constexpr int64_t kRevBlocks = 4 * 4 * 148;  // blocks of a launch before a block takes several spans: four waves of four
+
+enum RevRow : int {
+  R_M3 = 0, R_M2, R_M1, R_MT2, R_MT1, R_ONE, R_T, R_T2, R_F, R_FT, R_FT2, R_FF, R_LOG, R_TLOG, R_FLOG, R_Y, kRevRows,
+  R_F34 = R_M2,                    // (IMRPhenomD: no f^-2, but f^3/4)
+  R_LOG2 = R_M3, R_TLOG2 = R_M2,  // (TaylorF2: neither, the logarithms in the first tile)
+};
+// The tiles of the rows that a model's sums take: TaylorF2's are in the first
+// (f^-5/3 and f as columns).
+template <int MODEL>
+constexpr int kRevTiles = MODEL == kModelTaylorF2 ? 1 : 2;
+static_assert(kRevRows == 16 && R_FF == R_ONE + 6, "two tiles; t^k at R_ONE + k");
+
+struct RevShared {
+  double T[kRevBinaries][kTableStride];
+  double sums[kRevBinaries][kTableStride];  // dL/d(table), kSlotTc, kSlotLoss
+  double rows[kRevRows * kRowStride];
+  double m76[kSpan];
+  double stage[kRevWarps][kStage];
+};
+
+// Adds the columns' products of a binary (stage: [8 row + column] of columns
+// phase by region, amplitude w, w t^7, kp, kc; TaylorF2: the phase's, times
+// f^-5/3 and f, the amplitude's, kp and kc at the same places) to its sums.
+template <int MODEL>
+__device__ __forceinline__ void add_products(double* sums, const double* stage, int lane) {
+  const auto at = [&](int row, int col) { return stage[8 * row + col]; };
+  if constexpr (MODEL == kModelXas) {
+    if (lane < 13) {
+      constexpr int kIns[13] = {R_M1, R_MT2, R_MT1, R_LOG, R_ONE, R_T, R_TLOG, R_T2, R_F, R_FLOG, R_FT, R_FT2, R_FF};
+      int row = R_ONE;
+#pragma unroll
+      for (int k = 0; k < 13; ++k) row = lane == k ? kIns[k] : row;
+      sums[X_PH_INS + lane] += at(row, 0);
+    } else if (lane < 19) {
+      const int k = lane - 13;
+      sums[X_PH_INT + k] += at(k == 0 ? R_ONE : (k == 1 ? R_F : (k == 2 ? R_LOG : (k == 3 ? R_M1 : (k == 4 ? R_M2 : R_M3)))), 1);
+    } else if (lane < 24) {
+      const int k = lane - 19;
+      sums[X_PH_RD + k] += at(k == 0 ? R_ONE : (k == 1 ? R_F : (k == 2 ? R_T2 : (k == 3 ? R_M1 : R_M3))), 2);
+    }
+    if (lane < 10) sums[X_AMP_INS + lane] += lane < 7 ? at(R_ONE + lane, 3) : at(R_ONE + lane - 7, 4);
+  } else if constexpr (MODEL == kModelPhenomD) {
+    if (lane < 12) {
+      constexpr int kIns[12] = {R_ONE, R_M1, R_MT2, R_MT1, R_LOG, R_T, R_TLOG, R_T2, R_F, R_FT, R_FT2, R_FF};
+      int row = R_ONE;
+#pragma unroll
+      for (int k = 0; k < 12; ++k) row = lane == k ? kIns[k] : row;
+      sums[D_PH_INS + lane] += at(row, 0);
+    } else if (lane < 16) {
+      const int k = lane - 12;
+      sums[D_PH_INT + k] += at(k == 0 ? R_ONE : (k == 1 ? R_F : (k == 2 ? R_M3 : R_LOG)), 1);
+    } else if (lane < 20) {
+      const int k = lane - 16;
+      sums[D_PH_RD + k] += at(k == 0 ? R_ONE : (k == 1 ? R_F : (k == 2 ? R_M1 : R_F34)), 2);
+    }
+    if (lane < 10) sums[D_AMP_INS + lane] += lane < 7 ? at(R_ONE + lane, 3) : at(R_ONE + lane - 7, 4);
+  } else {
+    if (lane < 8) {
+      constexpr int kIns[8] = {R_M1, R_MT2, R_MT1, R_LOG2, R_ONE, R_T, R_TLOG2, R_T2};
+      int row = R_ONE;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) row = lane == k ? kIns[k] : row;
+      sums[T_PH + lane] += at(row, 0);
+    } else if (lane == 8) {
+      sums[T_AMP] += at(R_ONE, 3);
+    }
+  }
+  if constexpr (MODEL == kModelTaylorF2) {
+    if (lane == 27) sums[T_T0] += at(R_ONE, 1);
+    if (lane == 28) sums[T_ANCHOR] -= at(R_ONE, 0);
+    if (lane == 29) sums[kSlotTc] -= kTwoPi * at(R_ONE, 2);
+  } else {
+    if (lane == 27) sums[Layout<MODEL>::kT0] += at(R_Y, 0);
+    if (lane == 28) sums[Layout<MODEL>::kAnchor] -= at(R_ONE, 0) + at(R_ONE, 1) + at(R_ONE, 2);
+    if (lane == 29) sums[kSlotTc] -= kTwoPi * (at(R_F, 0) + at(R_F, 1) + at(R_F, 2));
+  }
+  if (lane == 30) sums[Layout<MODEL>::kKp] += at(R_ONE, 5);
+  if (lane == 31) sums[Layout<MODEL>::kKc] += at(R_ONE, 6);
+}
+
+// The terms past the inspiral of one frequency a lane (pb, ab: the cotangents
+// of the phase and of the amplitude, zero for a lane without): eight columns
+// against the rows and eight against ones.
+template <int MODEL>
+__device__ __forceinline__ void past_columns(const double* T, const Freq<double>& q, const Point<double>& pt, double ab,
+                                             double pb, double (&v)[8], double (&w)[8]) {
+  const double f = q.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = w[i] = 0.0;
+  if constexpr (MODEL == kModelXas) {
+    const double y = f - T[X_SHIFT];
+    if (pt.rp > 0) {
+      const int r = pt.rp - 1;
+      const double gz = pb * T[X_ATAN_A + r] * pt.zz;
+      v[7] = -gz * T[X_ATAN_W + r];
+      w[0] = r == 0 ? pb * pt.at : 0.0;
+      w[1] = r == 1 ? pb * pt.at : 0.0;
+      w[2] = r == 0 ? gz * y : 0.0;
+      w[3] = r == 1 ? gz * y : 0.0;
+    }
+    if (pt.ra == 1) {
+      const double inv = 1.0 / pt.a0;
+      v[2] = ab * inv;
+      v[0] = -v[2] * pt.amp;
+      v[1] = v[0] * (f * f);
+    } else if (pt.ra == 2) {
+      const double u = pt.a0, g = ab * pt.amp, inv = 1.0 / (u * u + T[X_AMP_RD_G]);
+      const double ub = g * (-T[X_AMP_RD_GR] - 2.0 * u * inv);
+      v[3] = ab * q.m76 * pt.a1;
+      v[4] = -g * u;
+      v[5] = ub * y;
+      v[6] = -g * inv;
+      v[7] -= ub * T[X_AMP_RD_S];
+    }
+  } else if constexpr (MODEL == kModelPhenomD) {
+    if (pt.rp == 2) {
+      const double gz = pb * T[D_ATAN_A] * pt.zz;
+      v[2] = pb * pt.at;
+      v[3] = gz * (f - T[D_ATAN_SHIFT]);
+      v[4] = -gz * T[D_ATAN_W];
+    }
+    const double am = ab * q.m76;  // (of the amplitude without f^-7/6)
+    if (pt.ra == 1) {
+      v[0] = am;
+      v[1] = am * (f * f);
+    } else if (pt.ra == 2) {
+      const double u = pt.a0, P = T[D_AMP_RD_N] * pt.a1;
+      const double ub = am * P * (-T[D_AMP_RD_GR] - 2.0 * u / (u * u + 1.0));
+      v[5] = am * pt.a1;
+      v[6] = -am * P * u;
+      v[7] = ub * (f - T[D_AMP_RD_SHIFT]);
+      w[0] = -ub * T[D_AMP_RD_S];
+    }
+  }
+}
+
+// Adds those products (stage: of v, then `ones` of w) to the binary's sums.
+template <int MODEL>
+__device__ __forceinline__ void add_past(const double* T, double* sums, double* stage, const double (&d)[2][2],
+                                         const double (&ones)[1][2], int lane) {
+  put_products(stage, d, lane);
+  const auto at = [&](int row, int col) { return stage[8 * row + col]; };
+  // w f^j, j = 0..4: from column 0, from j = 3 on column 1 (w f^2)
+  const double moment = lane < 5 ? at(lane == 0 ? R_ONE : ((lane & 1) ? R_F : R_FF), lane > 2 ? 1 : 0) : 0.0;
+  if constexpr (MODEL == kModelXas) {
+    if (lane < 5) {
+      sums[X_AMP_INT_D + lane] += moment;
+    } else if (lane < 11) {
+      constexpr int kSlot[6] = {X_AMP_INT_N, X_AMP_RD_N, X_AMP_RD_GR, X_AMP_RD_S, X_AMP_RD_G, X_SHIFT};
+      int slot = X_AMP_INT_N;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) slot = lane - 5 == k ? kSlot[k] : slot;
+      sums[slot] += at(R_ONE, lane - 3);
+    }
+    put_products(stage, ones, lane);
+    if (lane < 4) sums[X_ATAN_A + lane] += stage[lane];
+  } else {
+    // y = s f: d_j = s^j moment_j, and dL/ds = (1 / s) sum_j j c_j d_j
+    const double s = T[D_AMP_INT_S];
+    double dj = moment;
+    for (int k = 0; k < lane && k < 4; ++k) dj *= s;
+    if (lane < 5) sums[D_AMP_INT + lane] += dj;
+    double ds = lane < 5 ? lane * T[D_AMP_INT + lane] * dj : 0.0;
+    ds = warp_sum(ds);
+    if (lane == 5) sums[D_AMP_INT_S] += ds / s;
+    if (lane >= 6 && lane < 12) {
+      constexpr int kSlot[6] = {D_ATAN_A, D_ATAN_W, D_ATAN_SHIFT, D_AMP_RD_N, D_AMP_RD_GR, D_AMP_RD_S};
+      int slot = D_ATAN_A;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) slot = lane - 6 == k ? kSlot[k] : slot;
+      sums[slot] += at(R_ONE, lane - 4);
+    }
+    put_products(stage, ones, lane);
+    if (lane == 0) sums[D_AMP_RD_SHIFT] += stage[0];
+  }
+}
+static_assert(X_ATAN_W == X_ATAN_A + 2, "the arc tangents' four slots are contiguous");
+
 template <int MODEL, bool FUSED>
-__global__ void __launch_bounds__(128) k_adj_f64(const double* __restrict__ table, const double* __restrict__ freqs,
+__global__ void __launch_bounds__(kRevBlock, 5)
+    k_rev_f64(const double* __restrict__ table, const double* __restrict__ freqs, int64_t n, int64_t B, int per,
+              const double* __restrict__ t_c, const double2* __restrict__ cot_hp, const double2* __restrict__ cot_hc,
+              FusedArgs fa, const double* __restrict__ dtable, double* grad, double* loss_out) {
+  __shared__ RevShared sh;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const auto* data = static_cast<const double2*>(fa.data);
+  const auto* weights = static_cast<const double*>(fa.weights);
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * per;
+  const int count = static_cast<int>(min(static_cast<int64_t>(per), B - base));
+  for (int i = threadIdx.x; i < count * kTableStride; i += kRevBlock) {
+    (&sh.T[0][0])[i] = table[base * kTableStride + i];
+    (&sh.sums[0][0])[i] = 0.0;
+  }
+  for (int64_t n0 = static_cast<int64_t>(blockIdx.y) * kSpan; n0 < n; n0 += static_cast<int64_t>(gridDim.y) * kSpan) {
+    const int length = static_cast<int>(min(static_cast<int64_t>(kSpan), n - n0));
+    {
+      // (past the span's end: a frequency of it, with zero cotangents)
+      const int i = threadIdx.x;
+      const Freq<double> q = freq_powers(freqs[n0 + (i < length ? i : 0)]);
+      double* r = sh.rows + i;
+      const double mt1 = q.t2 * q.m1, m2 = q.m1 * q.m1;
+      __syncthreads();  // (the last span's rows are read; the first: the tables are staged)
+      constexpr bool kTf2 = MODEL == kModelTaylorF2;
+      r[R_M3 * kRowStride] = kTf2 ? q.lf : m2 * q.m1;
+      r[R_M2 * kRowStride] = kTf2 ? q.t * q.lf : (MODEL == kModelPhenomD ? q.f34 : m2);
+      r[R_M1 * kRowStride] = q.m1;
+      r[R_MT2 * kRowStride] = mt1 * mt1;
+      r[R_MT1 * kRowStride] = mt1;
+      r[R_ONE * kRowStride] = 1.0;
+      r[R_T * kRowStride] = q.t;
+      r[R_T2 * kRowStride] = q.t2;
+      r[R_F * kRowStride] = q.f;
+      r[R_FT * kRowStride] = q.f * q.t;
+      r[R_FT2 * kRowStride] = q.f * q.t2;
+      r[R_FF * kRowStride] = q.f * q.f;
+      r[R_LOG * kRowStride] = q.lf;
+      r[R_TLOG * kRowStride] = q.t * q.lf;
+      r[R_FLOG * kRowStride] = q.f * q.lf;
+      r[R_Y * kRowStride] = q.y;
+      sh.m76[i] = q.m76;
+      __syncthreads();
+    }
+    double* stage = sh.stage[warp];
+    for (int j = warp; j < count; j += kRevWarps) {
+      const double* T = sh.T[j];
+      double* sums = sh.sums[j];
+      const int64_t row = (base + j) * n;
+      const double tc = t_c != nullptr ? t_c[base + j] : 0.0;
+      const double kp = T[slot_kp<MODEL>()], kc = T[slot_kc<MODEL>()];
+      double d1[kRevTiles<MODEL>][2] = {}, d2[2][2] = {}, ones[1][2] = {};
+      double loss = 0.0;
+      bool evaluated = false, past = false;
+      for (int c0 = 0; c0 < length; c0 += 32) {
+        const int i = c0 + lane;
+        const bool in = i < length;
+        const int64_t k = n0 + i;
+        const double* r = sh.rows + i;
+        const double f = r[R_F * kRowStride];
+        bool zero = false;
+        if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, f > T[X_F_CUT]);
+        if (zero && !FUSED) continue;
+        double2 gp = make_double2(0.0, 0.0), gc = gp;
+        if (!FUSED && in) {
+          gp = __ldcs(cot_hp + row + k);
+          gc = __ldcs(cot_hc + row + k);
+        }
+        Freq<double> q;
+        q.f = f;
+        q.t = r[R_T * kRowStride];
+        q.t2 = r[R_T2 * kRowStride];
+        q.m1 = r[R_M1 * kRowStride];
+        q.m3 = r[R_M3 * kRowStride];
+        q.lf = r[R_LOG * kRowStride];
+        q.y = r[R_Y * kRowStride];
+        if constexpr (MODEL == kModelPhenomD) q.f34 = r[R_F34 * kRowStride];
+        q.m76 = sh.m76[i];
+        Point<double> pt;
+        if (zero) {
+          pt.amp = 0.0;
+          pt.c = pt.s = 0.0;
+        } else {
+          pt = point<MODEL, double>(T, q, tc);
+        }
+        if constexpr (FUSED) {
+          if (in) {
+            const double ap = kp * pt.amp, ac = kc * pt.amp;
+            const double2 d = data[fa.data_stride ? row + k : k];
+            const double wt = weights[fa.weights_stride ? row + k : k];
+            const double rx = fa.fp * (ap * pt.c) + fa.fc * (-ac * pt.s) - d.x;
+            const double ry = fa.fp * (ap * pt.s) + fa.fc * (ac * pt.c) - d.y;
+            loss += wt * (rx * rx + ry * ry);
+            const double g = 2.0 * fa.scale * wt;
+            gp = make_double2(fa.fp * g * rx, fa.fp * g * ry);
+            gc = make_double2(fa.fc * g * rx, fa.fc * g * ry);
+          }
+          if (zero || !fa.grad) continue;
+        }
+        evaluated = true;
+        // (IMRPhenomXAS above its cutoff: nothing depends on the table)
+        const bool dead = !in || (MODEL == kModelXas && pt.amp == 0.0);
+        const double A = pt.amp, ap = gp.x * pt.c + gp.y * pt.s, ac = gc.y * pt.c - gc.x * pt.s;
+        const double ab = dead ? 0.0 : kp * ap + kc * ac;
+        const double pb = dead ? 0.0 : A * (kp * (gp.y * pt.c - gp.x * pt.s) - kc * (gc.x * pt.c + gc.y * pt.s));
+        const double w = MODEL == kModelTaylorF2 || pt.ra == 0 ? ab * q.m76 : 0.0;
+        const double t3 = q.t2 * q.t;
+        if constexpr (MODEL == kModelTaylorF2) {
+          put_columns(stage, {pb, pb * q.y, pb * q.f, w, 0.0, dead ? 0.0 : A * ap, dead ? 0.0 : A * ac, 0.0}, lane);
+        } else {
+          put_columns(stage, {pt.rp == 0 ? pb : 0.0, pt.rp == 1 ? pb : 0.0, pt.rp == 2 ? pb : 0.0, w,
+                              w * (t3 * t3 * q.t), dead ? 0.0 : A * ap, dead ? 0.0 : A * ac, 0.0}, lane);
+        }
+        mma_rows<kRevRows>(d1, sh.rows + c0, stage, lane);
+        if constexpr (MODEL != kModelTaylorF2) {
+          if (__any_sync(0xffffffffu, !dead && (pt.rp > 0 || pt.ra > 0))) {
+            past = true;
+            double v[8], o[8];
+            past_columns<MODEL>(T, q, pt, ab, pb, v, o);
+            put_columns(stage, v, lane);
+            mma_rows<kRevRows>(d2, sh.rows + c0, stage, lane);
+            put_columns(stage, o, lane);
+            mma_ones(ones[0], stage, lane);
+          }
+        }
+      }
+      if (evaluated) {
+        put_products(stage, d1, lane);
+        add_products<MODEL>(sums, stage, lane);
+        if constexpr (MODEL != kModelTaylorF2) {
+          if (past) add_past<MODEL>(T, sums, stage, d2, ones, lane);
+        }
+      }
+      if constexpr (FUSED) {
+        loss = warp_sum(loss);
+        if (lane == 0) sums[kSlotLoss] += fa.scale * loss;
+      }
+    }
+  }
+  // each warp contracts its own binaries (the ones it summed): lane (r, d)
+  // takes the slots r + 4 i of direction d
+  const bool whole = gridDim.y == 1;
+  const auto put = [&](double* at, double v) {
+    if (whole) {
+      *at = v;
+    } else {
+      atomicAdd(at, v);
+    }
+  };
+  __syncwarp();
+  for (int j = warp; j < count; j += kRevWarps) {
+    const int64_t b = base + j;
+    const double* sums = sh.sums[j];
+    if (grad != nullptr && dtable != nullptr) {
+      const int d = lane & 7;
+      double g = 0.0;
+#pragma unroll 6
+      for (int k = lane >> 3; k < kTableStride; k += 4) {
+        const double s = sums[k];
+        if (k != kSlotTc && k != kSlotLoss && s != 0.0) g += s * dtable[(b * kTableStride + k) * kDirections + d];
+      }
+      g += __shfl_xor_sync(0xffffffffu, g, 8);
+      g += __shfl_xor_sync(0xffffffffu, g, 16);
+      if (lane < kDirections) put(&grad[b * kGradColumns + lane], g);
+    }
+    if (grad != nullptr && lane == kDirections) put(&grad[b * kGradColumns + kDirections], sums[kSlotTc]);
+    if (loss_out != nullptr && lane == kDirections + 1) put(&loss_out[b], sums[kSlotLoss]);
+  }
+}
+
+// The reverse mode on ragged grids: one binary per block.
+template <int MODEL, bool FUSED>
+__global__ void __launch_bounds__(128) k_adj_f64_ragged(const double* __restrict__ table, const double* __restrict__ freqs,
                                                  const int64_t* __restrict__ offsets, int64_t n, int64_t B,
                                                  const double* __restrict__ t_c, const double2* __restrict__ cot_hp,
                                                  const double2* __restrict__ cot_hc, FusedArgs fa,
@@ -1293,21 +1665,20 @@ __global__ void __launch_bounds__(128) k_adj_f64(const double* __restrict__ tabl
     if (threadIdx.x < kTableStride) sT[threadIdx.x] = table[b * kTableStride + threadIdx.x];
     __syncthreads();
     const double tc = t_c != nullptr ? t_c[b] : 0.0;
-    const int64_t rs = offsets != nullptr ? min(max(offsets[b], int64_t(0)), n) : b * n;
-    const int64_t re = offsets != nullptr ? min(max(offsets[b + 1], rs), n) : rs + n;
-    const int64_t fbase = offsets != nullptr ? 0 : rs;
+    const int64_t rs = min(max(offsets[b], int64_t(0)), n);
+    const int64_t re = min(max(offsets[b + 1], rs), n);
     double acc[kTableStride];
 #pragma unroll
     for (int k = 0; k < kTableStride; ++k) acc[k] = 0.0;
     double loss = 0.0;
     for (int64_t e = rs + threadIdx.x; e < re; e += kAdjBlock) {
-      const Freq<double> q = freq_powers(freqs[e - fbase]);
+      const Freq<double> q = freq_powers(freqs[e]);
       const Point<double> pt = point<MODEL, double>(sT, q, tc);
       double2 gp, gc;
       if constexpr (FUSED) {
         const double ap = sT[slot_kp<MODEL>()] * pt.amp, ac = sT[slot_kc<MODEL>()] * pt.amp;
-        const double2 d = data[fa.data_stride ? e : e - fbase];
-        const double w = weights[fa.weights_stride ? e : e - fbase];
+        const double2 d = data[e];
+        const double w = weights[e];
         const double rx = fa.fp * (ap * pt.c) + fa.fc * (-ac * pt.s) - d.x;
         const double ry = fa.fp * (ap * pt.s) + fa.fc * (ac * pt.c) - d.y;
         loss += w * (rx * rx + ry * ry);
@@ -1927,7 +2298,6 @@ static int adjoint_entry(bool fused, int model, int precision, const void* table
     return WFX_EINVAL;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (precision == WFX_FP64) {
-    const unsigned grid = static_cast<unsigned>((B < (int64_t(1) << 20) ? B : (int64_t(1) << 20)));
     const auto* T = static_cast<const double*>(table);
     const auto* F = static_cast<const double*>(freqs);
     const auto* TC = static_cast<const double*>(t_c);
@@ -1937,10 +2307,34 @@ static int adjoint_entry(bool fused, int model, int precision, const void* table
     auto* L = static_cast<double*>(loss);
     return with_model(model, [&](auto m) {
       constexpr int M = decltype(m)::value;
+      if (offsets != nullptr) {
+        const unsigned grid = static_cast<unsigned>(min(B, int64_t(1) << 20));
+        if (fused) {
+          k_adj_f64_ragged<M, true><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
+        } else {
+          k_adj_f64_ragged<M, false><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
+        }
+        return launched();
+      }
+      // (binaries a block: as many as leave kRevBlocks blocks of one span, up
+      // to kRevBinaries; then spans a block, which cost it one contraction)
+      const int64_t spans = (n + kSpan - 1) / kSpan;
+      const int per = static_cast<int>(min(max(B * spans / kRevBlocks, int64_t(1)), static_cast<int64_t>(kRevBinaries)));
+      const int64_t groups = (B + per - 1) / per;
+      const int64_t each = max(groups * spans / kRevBlocks, int64_t(1));
+      const int64_t parts = min((spans + each - 1) / each, int64_t(65535));
+      if (groups > (int64_t(1) << 31) - 1) return static_cast<int>(WFX_EINVAL);
+      if (parts > 1) {
+        cudaError_t zeroed = cudaSuccess;
+        if (G != nullptr) zeroed = cudaMemsetAsync(G, 0, sizeof(double) * kGradColumns * B, s);
+        if (zeroed == cudaSuccess && L != nullptr) zeroed = cudaMemsetAsync(L, 0, sizeof(double) * B, s);
+        if (zeroed != cudaSuccess) return static_cast<int>(zeroed);
+      }
+      const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(parts));
       if (fused) {
-        k_adj_f64<M, true><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
+        k_rev_f64<M, true><<<grid, kRevBlock, 0, s>>>(T, F, n, B, per, TC, CP, CC, fa, dtable, G, L);
       } else {
-        k_adj_f64<M, false><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
+        k_rev_f64<M, false><<<grid, kRevBlock, 0, s>>>(T, F, n, B, per, TC, CP, CC, fa, dtable, G, L);
       }
       return launched();
     });

@@ -21,6 +21,7 @@
 #include "../../include/waveformx_b200.h"
 #include "dual_point.cuh"
 #include "internal.h"
+#include "matrix_sums.cuh"
 #include "point.cuh"
 #include "setup_xhm.cuh"
 #include "tables.cuh"
@@ -367,9 +368,9 @@ __device__ __forceinline__ void xhm_dual_sum(const Dual* T, const Dual* t0_lm, c
 // directions on dual numbers. Bound by latency: 16 warps a SM issue in 28 % of
 // the cycles (instruction fetch, the elementary functions' chains, the
 // barriers between the stages).
-constexpr int kAdjSpan = kXhmBlock;
+constexpr int kAdjSpan = kSpan;
 constexpr int kAdjWarps = kXhmBlock / 32;
-static_assert(kAdjWarps == xhm::kModes, "a warp for each higher mode");
+static_assert(kAdjSpan == kXhmBlock && kAdjWarps == xhm::kModes, "a thread a frequency, a warp a higher mode");
 // Blocks of a launch before a block takes more than one span of a binary (each
 // block pays one contraction with dtable): four waves of four blocks a SM.
 constexpr int64_t kAdjBlocks = 4 * 4 * 148;
@@ -379,8 +380,6 @@ constexpr int64_t kAdjBlocks = 4 * 4 * 148;
 constexpr int kRowT = xhm::B_1, kRowF = xhm::B_F, kRowF2 = xhm::B_F2;
 constexpr int kRowY = xhm::kBasis, kRowG = kRowY + 1, kRows = kRowG + 4;
 static_assert(kRowT + 7 == xhm::B_7_3 && kRows <= 24, "three tiles of eight rows");
-constexpr int kRowStride = kAdjSpan + 4;  // (doubles; = 4 mod 16: the fragments' loads are conflict-free)
-constexpr int kStageStride = 36;          // (32 frequencies a column, = 4 mod 16)
 // Sums of a warp outside its mode's table: the (2,2)'s slots, then t_c and the
 // head's.
 enum WarpSum : int { W_TC = 58, W_S = 60, W_AMP0 = 61, W_COS = 62, W_SIN = 63, W_FACTOR = 64, W_FACTOR22 = 68 };
@@ -390,64 +389,11 @@ struct AdjShared {
   double rows[kRows * kRowStride];
   double m76[kAdjSpan];
   double h22r[kAdjSpan], h22i[kAdjSpan];  // the (2,2); from the (3,2)'s warp on, its cotangent from the rotation
-  double stage[kAdjWarps][8 * kStageStride];
+  double stage[kAdjWarps][kStage];
   double modes[xhm::kModes * kXhmModeStride64];  // dL/d(mode tables); warp m its own
   double sums[kAdjWarps][kTableStride];
 };
 static_assert(sizeof(AdjShared) <= 48 * 1024, "static shared memory");
-
-// d += a b of one 8 x 4 by 4 x 8 product: lane l holds a[l / 4][l % 4],
-// b[l % 4][l / 4] and d[l / 4][2 (l % 4) + {0, 1}].
-__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(d[0]), "+d"(d[1])
-      : "d"(a), "d"(b));
-}
-
-// Puts eight values a lane into the warp's columns (frequency = lane).
-__device__ __forceinline__ void put_columns(double* stage, const double (&v)[8], int lane) {
-  __syncwarp();
-#pragma unroll
-  for (int n = 0; n < 8; ++n) stage[n * kStageStride + lane] = v[n];
-  __syncwarp();
-}
-
-// d[t] += rows 8 t .. 8 t + 7 times the columns, over 32 frequencies.
-template <int TILES>
-__device__ __forceinline__ void mma_rows(double (&d)[TILES][2], const double* rows, const double* stage, int lane) {
-  const int r = lane >> 2, k = lane & 3;
-  const double* column = stage + r * kStageStride + k;
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const double b = column[4 * s];
-#pragma unroll
-    for (int t = 0; t < TILES; ++t) {
-      // (the last tile's rows past kRows repeat the last row: not read back)
-      const int row = 8 * t + 7 < kRows ? 8 * t + r : min(8 * t + r, kRows - 1);
-      mma_f64(d[t], rows[row * kRowStride + k + 4 * s], b);
-    }
-  }
-}
-
-// d += the sums of the columns, in every row.
-__device__ __forceinline__ void mma_ones(double (&d)[2], const double* stage, int lane) {
-  const double* column = stage + (lane >> 2) * kStageStride + (lane & 3);
-#pragma unroll
-  for (int s = 0; s < 8; ++s) mma_f64(d, 1.0, column[4 * s]);
-}
-
-// Writes d (8 rows each) to the warp's stage as entries [8 row + column].
-template <int TILES>
-__device__ __forceinline__ void put_products(double* stage, const double (&d)[TILES][2], int lane) {
-  __syncwarp();
-#pragma unroll
-  for (int t = 0; t < TILES; ++t) {
-    double* at = stage + 8 * (8 * t + (lane >> 2)) + 2 * (lane & 3);
-    at[0] = d[t][0];
-    at[1] = d[t][1];
-  }
-  __syncwarp();
-}
 
 // The derivatives of a mode's factors from the products of its value (columns
 // 6, 7 of stage) with the cotangents: factor i of Re F+, Im F+, Re Fx, Im Fx.
@@ -613,7 +559,7 @@ __device__ __forceinline__ void mode_reverse(AdjShared& sh, int m, int count, in
       const double h = amp_region == 0 ? ab * m76 : 0.0, inv = root > 0.0 ? h / root : 0.0;
       put_columns(stage, {region == 0 ? pb : 0.0, region == 1 ? pb : 0.0, region == 2 ? pb : 0.0, pr * inv, pi * inv,
                           h * t7, amp * cphi, amp * sphi}, lane);
-      mma_rows(d1, sh.rows + base, stage, lane);
+      mma_rows<kRows>(d1, sh.rows + base, stage, lane);
     }
     if (region == 1) {
       const double gz = pb * M[M_ATAN_A + 1] * zz1;
@@ -671,7 +617,7 @@ __device__ __forceinline__ void mode_reverse(AdjShared& sh, int m, int count, in
         }
         const double w = is_aux ? mb : 0.0;
         put_columns(stage, {psb, w, w * f, m2rb, m2ib, m3rb, m3ib, cos_a}, lane);
-        mma_rows(dm, sh.rows + base, stage, lane);
+        mma_rows<kRows>(dm, sh.rows + base, stage, lane);
       }
       const double d = mb * mag;  // (d lor / d arg = -lor)
       const double dl = is_aux || is_fall ? 0.0 : d, df = is_fall ? d : 0.0;
@@ -785,7 +731,7 @@ __device__ __forceinline__ void reverse_22(AdjShared& sh, const double* rows, in
     const double w = pt.ra == 0 ? ab * q.m76 : 0.0, t2 = q.t * q.t, t8 = t2 * t2 * t2 * t2;
     put_columns(stage, {pt.rp == 0 ? pb : 0.0, pt.rp == 1 ? pb : 0.0, pt.rp == 2 ? pb : 0.0, w, w * t8,
                         direct.im * h.re - direct.re * h.im, h.re, h.im}, lane);
-    mma_rows(d, rows, stage, lane);
+    mma_rows<kRows>(d, rows, stage, lane);
   }
   put_products(stage, d, lane);
   // (the order of X_PH_INS, X_PH_INT and X_PH_RD in rows of HM_BASIS)
@@ -839,7 +785,7 @@ __device__ __forceinline__ void reverse_22(AdjShared& sh, const double* rows, in
   }
   double d2[2][2] = {};
   put_columns(stage, {w, w * (f * f), n, rd_n, rd_gr, ub * y, rd_g, shift}, lane);
-  mma_rows(d2, rows, stage, lane);
+  mma_rows<kRows>(d2, rows, stage, lane);
   double d3[1][2] = {};
   put_columns(stage, {pt.rp == 1 ? at : 0.0, pt.rp == 2 ? at : 0.0, pt.rp == 1 ? gz * y : 0.0,
                       pt.rp == 2 ? gz * y : 0.0, 0.0, 0.0, 0.0, 0.0}, lane);
