@@ -462,6 +462,11 @@ int wfx_polarization_refine(int precision, const void* series, const void* zgrid
 int wfx_match_grid_time(const void* series, int64_t rows, int64_t n, int64_t n_fft, double delta_f, double* t,
                         wfx_stream_t stream);
 
+/* The same for complex128 series (the transforms in double): the power of two
+ * >= max(n, 2048) must be at most 8192 and divide n_fft. */
+int wfx_match_grid_time64(const void* series, int64_t rows, int64_t n, int64_t n_fft, double delta_f, double* t,
+                          wfx_stream_t stream);
+
 /* Step 3 (see wfx_overlap). time: 0 none, 1 from zgrid, 2 from t (the
  * times of wfx_match_grid_time, overwritten by the refined ones). */
 int wfx_match_refine(int precision, const void* series, const void* zgrid, int64_t rows, int64_t n, int64_t n_fft,

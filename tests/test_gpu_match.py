@@ -270,3 +270,34 @@ def test_template_bank_xhm(cuda):
     assert float(tt[5]) == pytest.approx(-0.013, abs=1e-5)
     pm, _ = wm.template_polarization_match("IMRPhenomXHM", p, f, signal, w)
     assert float(pm[5]) == pytest.approx(1.0, abs=2e-5)
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("n", [2, 31, 256, 257, 1025, 4017, 8192, 12000])
+def test_match_at_the_rows_of_the_blocks(cuda, dtype, n):
+    """match() of given waveforms around the sizes at which the refinement's
+    blocks change (256 terms a group, 1 to 16 warps; beyond 8192 in double the
+    row is read by a warp, and the grid is cuFFT's) and the transform's (2048
+    to 16384), every mode, against the oracle. Bar: 1e-6 (complex64: the
+    series' rounding, about n^1/2 6e-8 of the sum of its magnitudes) or 1e-10
+    of the match."""
+    import torch
+
+    from oracle import match as om
+    from waveformx_b200 import match as wm
+
+    rng = np.random.default_rng(n)
+    f = 20.0 + 0.25 * np.arange(n)
+    w = oracle.psd(f)
+    shape = (f / 20.0) ** (-7.0 / 6.0)
+    phase = 2000.0 * (f / 20.0) ** (-5.0 / 3.0)
+    a = shape * np.exp(1j * (phase + 2 * np.pi * np.outer(rng.uniform(-0.3, 0.3, 3), f) + rng.uniform(0, 6, (3, 1))))
+    b = shape * np.exp(1j * phase * (1.0 + 1e-3 * rng.normal(size=(3, 1)))) * (1.0 + 0.05 * rng.normal(size=(3, n)))
+    a, b = a.astype(dtype), b.astype(dtype)
+    real = np.float32 if dtype == "complex64" else np.float64
+    for time, phased in ((True, True), (True, False), (False, True), (False, False)):
+        got = wm.match(torch.as_tensor(a, device=cuda), torch.as_tensor(b, device=cuda), f,
+                       torch.as_tensor(w.astype(real), device=cuda), time=time, phase=phased).cpu().numpy()
+        ref = om.match(a.astype(np.complex128), b.astype(np.complex128), f, w.astype(real).astype(np.float64), time=time,
+                       phase=phased)
+        np.testing.assert_allclose(got, ref, rtol=0, atol=1e-6 if dtype == "complex64" else 1e-10)

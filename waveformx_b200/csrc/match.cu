@@ -295,6 +295,199 @@ __global__ void __launch_bounds__(kMatchBlock) k_match_refine(const typename Cpl
   }
 }
 
+// The refinement from given times (time = 2, or 0: at t = 0) with a row held
+// in the block's registers: its terms are read once for the four evaluations
+// of z (k_match_refine reads them four times, a warp a row), each warp taking
+// `G` groups of 256 terms. Term 256 g + 32 u + l belongs to lane l and to its
+// group's polynomial in R = e^(2 pi i 32 delta_f t), whose value and first two
+// derivatives in R Horner's rule gives together (12 multiply-adds a term; 4
+// where only z is read, the last evaluation): with b = e^(2 pi i f_0 t) at the
+// group's first frequency f_0 (exact, as k_match_refine's) and d = 32 delta_f,
+//   z = sum b p, sum f w = sum b (f_0 p + d R p'),
+//   sum f^2 w = sum b (f_0^2 p + 2 f_0 d R p' + d^2 (R p' + R^2 p'')).
+// Bound by FP64 issue (the pipe 53 % busy at 12 warps a SM): complex64 rows of
+// 4017 terms, 4096 of them 132 us (163 with a warp a row), 500 22.7 (61), one
+// 10.4 (35); 300 rows of 12000 53 (174). (Two groups a lane in single: 148.)
+template <class R>
+struct RefineShape;
+// (kGroups x 8 terms of a lane in 64 registers; blocks of up to kThreads)
+template <>
+struct RefineShape<float> {
+  static constexpr int kGroups = 4;
+};
+template <>
+struct RefineShape<double> {
+  static constexpr int kGroups = 2;
+};
+constexpr int kRefineThreads = 512;
+template <class R>
+constexpr int64_t kRefineTerms = 256 * RefineShape<R>::kGroups * (kRefineThreads / 32);  // the longest row
+
+struct ComplexD {
+  double re, im;
+};
+__device__ __forceinline__ ComplexD mul(ComplexD a, ComplexD b) {
+  return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
+}
+// a b + c
+__device__ __forceinline__ ComplexD mul_add(ComplexD a, ComplexD b, ComplexD c) {
+  return {fma(-a.im, b.im, fma(a.re, b.re, c.re)), fma(a.im, b.re, fma(a.re, b.im, c.im))};
+}
+
+// z, and with `slopes` its first two derivatives in t, at t as k_match_refine's
+// z[0..5], in every thread of the block; buffer: 8 doubles a warp, not the one
+// of the last call.
+template <class C, int G>
+__device__ __forceinline__ void block_z(const C (&c)[G][8], const double (&f0)[G], double t, double delta_f, bool slopes,
+                                        double* buffer, double (&z)[6]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const double d = 32.0 * delta_f;
+  ComplexD rot;
+  cis_turns(d * t, rot.re, rot.im);
+  ComplexD s0{0.0, 0.0}, s1 = s0, s2 = s0;
+  if (slopes) {
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      ComplexD p{0.0, 0.0}, q = p, h = p;  // the polynomial, its derivative and half its second
+#pragma unroll
+      for (int u = 7; u >= 0; --u) {
+        h = mul_add(h, rot, q);
+        q = mul_add(q, rot, p);
+        p = mul_add(p, rot, ComplexD{static_cast<double>(c[i][u].x), static_cast<double>(c[i][u].y)});
+      }
+      ComplexD b;
+      cis_turns(f0[i] * t, b.re, b.im);
+      const double f = f0[i];
+      const ComplexD q1 = mul(q, rot), h1 = mul(mul(h, rot), rot);
+      const ComplexD v1{fma(d, q1.re, f * p.re), fma(d, q1.im, f * p.im)};
+      const ComplexD v2{fma(f, fma(d, q1.re, v1.re), d * d * fma(2.0, h1.re, q1.re)),
+                        fma(f, fma(d, q1.im, v1.im), d * d * fma(2.0, h1.im, q1.im))};
+      s0 = mul_add(b, p, s0);
+      s1 = mul_add(b, v1, s1);
+      s2 = mul_add(b, v2, s2);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      ComplexD p{0.0, 0.0};
+#pragma unroll
+      for (int u = 7; u >= 0; --u)
+        p = mul_add(p, rot, ComplexD{static_cast<double>(c[i][u].x), static_cast<double>(c[i][u].y)});
+      ComplexD b;
+      cis_turns(f0[i] * t, b.re, b.im);
+      s0 = mul_add(b, p, s0);
+    }
+  }
+  // the warp's sums by recursive halving: lane l's bits 4, 3, 2 name the value
+  double v[8] = {s0.re, s0.im, s1.re, s1.im, s2.re, s2.im, 0.0, 0.0};
+#pragma unroll
+  for (int step = 4; step > 0; step >>= 1) {
+    const bool up = lane & (4 * step);
+#pragma unroll
+    for (int i = 0; i < step; ++i) {
+      const double keep = up ? v[i + step] : v[i], send = up ? v[i] : v[i + step];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * step);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((lane & 3) == 0) buffer[8 * warp + (lane >> 2)] = v[0];
+  __syncthreads();
+  double total[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int w = 0; w < warps; ++w) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) total[i] += buffer[8 * w + i];
+  }
+  constexpr double kTau = 2.0 * kPi;
+  z[0] = total[0];
+  z[1] = total[1];
+  z[2] = -kTau * total[3];  // 2 pi i sum f w
+  z[3] = kTau * total[2];
+  z[4] = -kTau * kTau * total[4];
+  z[5] = -kTau * kTau * total[5];
+}
+
+template <class R, int THREADS>
+__global__ void __launch_bounds__(THREADS, 384 / THREADS > 0 ? 384 / THREADS : 1)
+    k_refine_rows(const typename Cplx<R>::type* __restrict__ series, int64_t rows, int64_t n, int64_t n_fft,
+                  const double* __restrict__ freqs, double delta_f, const double* __restrict__ norms, int time, int phase,
+                  int steps, double* __restrict__ match, double* __restrict__ t_out) {
+  using C = typename Cplx<R>::type;
+  constexpr int G = RefineShape<R>::kGroups;
+  __shared__ double buffer[2][8 * (THREADS / 32)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+    const C* row = series + r * n_fft;
+    C c[G][8];
+    double f0[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int64_t k0 = 256 * static_cast<int64_t>(warp + warps * i) + lane;
+      f0[i] = k0 < n ? freqs[k0] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int64_t k = k0 + 32 * u;
+        if (k < n) {
+          c[i][u] = row[k];
+        } else {
+          c[i][u].x = c[i][u].y = R(0);
+        }
+      }
+    }
+    double t = time == 2 ? t_out[r] : 0.0;
+    double z[6];
+    int flip = 0;
+    block_z(c, f0, t, delta_f, time != 0 && steps > 0, buffer[flip], z);
+    if (time) {
+      for (int s = 0; s < steps; ++s) {
+        // match.py:104-115 with the closed-form derivatives
+        double g, h;
+        if (phase) {
+          g = 2.0 * (z[0] * z[2] + z[1] * z[3]);
+          h = 2.0 * (z[2] * z[2] + z[3] * z[3] + z[0] * z[4] + z[1] * z[5]);
+        } else {
+          g = z[2];
+          h = z[4];
+        }
+        const double next = t - (h < 0.0 ? g / h : 0.0);
+        double zn[6];
+        flip ^= 1;
+        block_z(c, f0, next, delta_f, s + 1 < steps, buffer[flip], zn);
+        if (objective(zn, phase) >= objective(z, phase)) {
+          t = next;
+#pragma unroll
+          for (int i = 0; i < 6; ++i) z[i] = zn[i];
+        }
+      }
+    }
+    if (threadIdx.x == 0) {
+      const double best = phase ? sqrt(z[0] * z[0] + z[1] * z[1]) : z[0];
+      match[r] = best / sqrt(norms[2 * r] * norms[2 * r + 1]);
+      if (t_out != nullptr) t_out[r] = t;
+    }
+    __syncthreads();  // (the buffers and t_out are the next row's)
+  }
+}
+
+// k_refine_rows for rows it holds (n <= kRefineTerms): false otherwise.
+template <class R>
+bool launch_refine_rows(const void* series, int64_t rows, int64_t n, int64_t n_fft, const double* freqs, double delta_f,
+                        const double* norms, int time, int phase, int steps, double* match, double* t, cudaStream_t s) {
+  if (n > kRefineTerms<R>) return false;
+  constexpr int64_t kTerms = 256 * RefineShape<R>::kGroups;  // a warp's
+  const int threads = 32 * static_cast<int>((n + kTerms - 1) / kTerms);
+  const unsigned grid = static_cast<unsigned>(rows < (int64_t(1) << 20) ? rows : (int64_t(1) << 20));
+  const auto* c = static_cast<const typename Cplx<R>::type*>(series);
+  if (threads <= 128) {
+    k_refine_rows<R, 128><<<grid, threads, 0, s>>>(c, rows, n, n_fft, freqs, delta_f, norms, time, phase, steps, match, t);
+  } else if (threads <= 256) {
+    k_refine_rows<R, 256><<<grid, threads, 0, s>>>(c, rows, n, n_fft, freqs, delta_f, norms, time, phase, steps, match, t);
+  } else {
+    k_refine_rows<R, 512><<<grid, threads, 0, s>>>(c, rows, n, n_fft, freqs, delta_f, norms, time, phase, steps, match, t);
+  }
+  return true;
+}
+
 // polarization_match's objective square(Re zp, Re zx) (match.py:174-176)
 // of a row: the normalised polarizations' overlap i, and the scales.
 struct PolarizationForm {
@@ -409,7 +602,10 @@ __global__ void __launch_bounds__(kMatchBlock) k_polarization_refine(
 
 // ---------------------------------------------------------------------------
 // The grid's best time without the grid in memory (the match with the phase
-// maximisation, FP32 series). A row's series is zero from n on, so with L
+// maximisation; complex64 series, or complex128 of up to 8192 values, whose
+// transforms run in double: 500 rows of 4017 values, 16384 times, with their
+// refinement 89 us where the library's transform, the grid's arg-max and the
+// refinement took 237). A row's series is zero from n on, so with L
 // the power of two >= max(n, 2048) and n_fft = P L, the inverse transform
 // splits into P transforms of length L of which nothing reads the zeros
 // (decimation in frequency):
@@ -432,43 +628,60 @@ __host__ __device__ constexpr int fft_pad(int i) { return i + (i >> 4); }
 
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v / 2); }
 
-template <int L>
+template <int L, class V>
 struct GridShape {
   static_assert(L == 2048 || L == 4096 || L == 8192 || L == 16384, "transform length");
   static constexpr int kPasses = (ilog2(L) - 1) / 4;    // S
   static constexpr int kLast = L >> (4 * kPasses);       // R
   static constexpr int kThreads = L / 16;                // one first-pass butterfly each
-  static constexpr int kBlocksPerSM = 1024 / kThreads;   // (64 registers a thread)
-  static constexpr size_t kBytes = sizeof(float2) * static_cast<size_t>(fft_pad(L - 1) + 1);
+  // (64 registers a thread; in double 128)
+  static constexpr int kBlocksPerSM = (sizeof(V) == sizeof(float2) ? 1024 : 512) / kThreads;
+  static constexpr size_t kBytes = sizeof(V) * static_cast<size_t>(fft_pad(L - 1) + 1);
 };
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+__device__ __forceinline__ float2 cplx(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 cplx(double a, double b) { return make_double2(a, b); }
+// e^(2 pi i a / b)
+__device__ __forceinline__ void root(int64_t a, int64_t b, float2& w) {
+  sincospif(2.0f * static_cast<float>(a) / static_cast<float>(b), &w.y, &w.x);
+}
+__device__ __forceinline__ void root(int64_t a, int64_t b, double2& w) {
+  sincospi(2.0 * static_cast<double>(a) / static_cast<double>(b), &w.y, &w.x);
 }
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+template <class V>
+__device__ __forceinline__ V cmul(V a, V b) {
+  return cplx(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
 
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+template <class V>
+__device__ __forceinline__ V cadd(V a, V b) { return cplx(a.x + b.x, a.y + b.y); }
+
+template <class V>
+__device__ __forceinline__ V csub(V a, V b) { return cplx(a.x - b.x, a.y - b.y); }
 
 // The 4-point inverse DFT of (a, b, c, d) in place: sum_p x_p i^(p k).
-__device__ __forceinline__ void idft4(float2& a, float2& b, float2& c, float2& d) {
-  const float2 s0 = cadd(a, c), d0 = csub(a, c), s1 = cadd(b, d), d1 = csub(b, d);
+template <class V>
+__device__ __forceinline__ void idft4(V& a, V& b, V& c, V& d) {
+  const V s0 = cadd(a, c), d0 = csub(a, c), s1 = cadd(b, d), d1 = csub(b, d);
   a = cadd(s0, s1);
   c = csub(s0, s1);
-  b = make_float2(d0.x - d1.y, d0.y + d1.x);  // d0 + i d1
-  d = make_float2(d0.x + d1.y, d0.y - d1.x);  // d0 - i d1
+  b = cplx(d0.x - d1.y, d0.y + d1.x);  // d0 + i d1
+  d = cplx(d0.x + d1.y, d0.y - d1.x);  // d0 - i d1
 }
 
 // The 8-point inverse DFT in place, natural order: the 4-point transforms
 // of the even and odd terms, the odd ones turned by e^(2 pi i k / 8).
-__device__ __forceinline__ void idft8(float2 (&x)[8]) {
-  float2 e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6], o0 = x[1], o1 = x[3], o2 = x[5], o3 = x[7];
+template <class V>
+__device__ __forceinline__ void idft8(V (&x)[8]) {
+  using S = decltype(V::x);
+  V e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6], o0 = x[1], o1 = x[3], o2 = x[5], o3 = x[7];
   idft4(e0, e1, e2, e3);
   idft4(o0, o1, o2, o3);
-  constexpr float kR2 = 0.707106781186547524f;
-  o1 = cmul(o1, make_float2(kR2, kR2));
-  o2 = make_float2(-o2.y, o2.x);
-  o3 = cmul(o3, make_float2(-kR2, kR2));
+  constexpr S kR2 = S(0.707106781186547524);
+  o1 = cmul(o1, cplx(kR2, kR2));
+  o2 = cplx(-o2.y, o2.x);
+  o3 = cmul(o3, cplx(-kR2, kR2));
   x[0] = cadd(e0, o0);
   x[4] = csub(e0, o0);
   x[1] = cadd(e1, o1);
@@ -482,24 +695,26 @@ __device__ __forceinline__ void idft8(float2 (&x)[8]) {
 // The 16-point inverse DFT of x: y[k1 + 4 k2] = sum_p x[p] e^(2 pi i p k / 16),
 // p = r + 4 s: a 4-point transform over s, the twiddles e^(2 pi i r k1 / 16),
 // a 4-point transform over r; y returned in natural order.
-__device__ __forceinline__ void idft16(float2 (&x)[16]) {
+template <class V>
+__device__ __forceinline__ void idft16(V (&x)[16]) {
+  using S = decltype(V::x);
 #pragma unroll
   for (int r = 0; r < 4; ++r) idft4(x[r], x[r + 4], x[r + 8], x[r + 12]);
   // (x[r + 4 k1] = A[r][k1])
-  constexpr float kC1 = 0.923879532511286756f, kS1 = 0.382683432365089772f, kR2 = 0.707106781186547524f;
-  x[1 + 4] = cmul(x[1 + 4], make_float2(kC1, kS1));      // r 1, k1 1: e^(2 pi i / 16)
-  x[1 + 8] = cmul(x[1 + 8], make_float2(kR2, kR2));      // r 1, k1 2
-  x[1 + 12] = cmul(x[1 + 12], make_float2(kS1, kC1));    // r 1, k1 3
-  x[2 + 4] = cmul(x[2 + 4], make_float2(kR2, kR2));      // r 2, k1 1
-  x[2 + 8] = make_float2(-x[2 + 8].y, x[2 + 8].x);       // r 2, k1 2: i
-  x[2 + 12] = cmul(x[2 + 12], make_float2(-kR2, kR2));   // r 2, k1 3: e^(2 pi i 6 / 16)
-  x[3 + 4] = cmul(x[3 + 4], make_float2(kS1, kC1));      // r 3, k1 1: e^(2 pi i 3 / 16)
-  x[3 + 8] = cmul(x[3 + 8], make_float2(-kR2, kR2));     // r 3, k1 2
-  x[3 + 12] = cmul(x[3 + 12], make_float2(-kC1, -kS1));  // r 3, k1 3: e^(2 pi i 9 / 16)
+  constexpr S kC1 = S(0.923879532511286756), kS1 = S(0.382683432365089772), kR2 = S(0.707106781186547524);
+  x[1 + 4] = cmul(x[1 + 4], cplx(kC1, kS1));      // r 1, k1 1: e^(2 pi i / 16)
+  x[1 + 8] = cmul(x[1 + 8], cplx(kR2, kR2));      // r 1, k1 2
+  x[1 + 12] = cmul(x[1 + 12], cplx(kS1, kC1));    // r 1, k1 3
+  x[2 + 4] = cmul(x[2 + 4], cplx(kR2, kR2));      // r 2, k1 1
+  x[2 + 8] = cplx(-x[2 + 8].y, x[2 + 8].x);       // r 2, k1 2: i
+  x[2 + 12] = cmul(x[2 + 12], cplx(-kR2, kR2));   // r 2, k1 3: e^(2 pi i 6 / 16)
+  x[3 + 4] = cmul(x[3 + 4], cplx(kS1, kC1));      // r 3, k1 1: e^(2 pi i 3 / 16)
+  x[3 + 8] = cmul(x[3 + 8], cplx(-kR2, kR2));     // r 3, k1 2
+  x[3 + 12] = cmul(x[3 + 12], cplx(-kC1, -kS1));  // r 3, k1 3: e^(2 pi i 9 / 16)
 #pragma unroll
   for (int k1 = 0; k1 < 4; ++k1) idft4(x[4 * k1], x[4 * k1 + 1], x[4 * k1 + 2], x[4 * k1 + 3]);
   // (x[4 k1 + k2] = y[k1 + 4 k2]): to natural order
-  float2 y[16];
+  V y[16];
 #pragma unroll
   for (int k1 = 0; k1 < 4; ++k1) {
 #pragma unroll
@@ -510,10 +725,11 @@ __device__ __forceinline__ void idft16(float2 (&x)[16]) {
 }
 
 // Multiplies y[p] by w^p, p = 1..15, w = e^(2 pi i q / LEN).
-__device__ __forceinline__ void twiddle16(float2 (&y)[16], int q, int LEN) {
-  float2 w1;
-  sincospif(2.0f * static_cast<float>(q) / static_cast<float>(LEN), &w1.y, &w1.x);
-  float2 w = w1;
+template <class V>
+__device__ __forceinline__ void twiddle16(V (&y)[16], int q, int LEN) {
+  V w1;
+  root(q, LEN, w1);
+  V w = w1;
 #pragma unroll
   for (int p = 1; p < 16; ++p) {
     y[p] = cmul(y[p], w);
@@ -523,12 +739,12 @@ __device__ __forceinline__ void twiddle16(float2 (&y)[16], int q, int LEN) {
 
 // A radix-16 pass of the length-L transform over its sub-transforms of
 // length LEN (LEN / 16 > 1) in place.
-template <int L, int LEN>
-__device__ __forceinline__ void fft_pass16(float2* X) {
+template <int L, int LEN, class V>
+__device__ __forceinline__ void fft_pass16(V* X) {
   constexpr int M = LEN / 16;
   for (int u = threadIdx.x; u < L / 16; u += blockDim.x) {
     const int b = u / M, q = u % M, base = b * LEN + q;
-    float2 x[16];
+    V x[16];
 #pragma unroll
     for (int p = 0; p < 16; ++p) x[p] = X[fft_pad(base + p * M)];
     idft16(x);
@@ -539,9 +755,9 @@ __device__ __forceinline__ void fft_pass16(float2* X) {
 }
 
 // The radix-16 passes after the first, down to sub-transforms of length R.
-template <int L, int LEN>
-__device__ __forceinline__ void fft_middle_passes(float2* X) {
-  if constexpr (LEN > GridShape<L>::kLast) {
+template <int L, int LEN, class V>
+__device__ __forceinline__ void fft_middle_passes(V* X) {
+  if constexpr (LEN > GridShape<L, V>::kLast) {
     fft_pass16<L, LEN>(X);
     __syncthreads();
     fft_middle_passes<L, LEN / 16>(X);
@@ -560,37 +776,40 @@ __device__ __forceinline__ int reverse16(int g) {
   return k;
 }
 
-__device__ __forceinline__ void keep_max_f(float& v, int& j, float ov, int oj) {
+template <class S>
+__device__ __forceinline__ void keep_max_f(S& v, int& j, S ov, int oj) {
   if (oj >= 0 && (j < 0 || ov > v || (ov == v && oj < j))) {
     v = ov;
     j = oj;
   }
 }
 
-template <int L>
-__global__ void __launch_bounds__(GridShape<L>::kThreads, GridShape<L>::kBlocksPerSM)
-    k_grid_time(const float2* __restrict__ series, int64_t rows, int64_t n, int64_t n_fft, double delta_f,
+template <int L, class V>
+__global__ void __launch_bounds__(GridShape<L, V>::kThreads, GridShape<L, V>::kBlocksPerSM)
+    k_grid_time(const V* __restrict__ series, int64_t rows, int64_t n, int64_t n_fft, double delta_f,
                 double* __restrict__ t_out) {
-  using G = GridShape<L>;
+  using G = GridShape<L, V>;
+  using S1 = decltype(V::x);
   constexpr int M = L / 16, R = G::kLast, S = G::kPasses;
-  extern __shared__ float2 X[];
-  __shared__ float best_v[32];
+  extern __shared__ double2 dynamic[];
+  V* X = reinterpret_cast<V*>(dynamic);
+  __shared__ S1 best_v[32];
   __shared__ int best_j[32];
   const int P = static_cast<int>(n_fft / L);
   const int q = threadIdx.x;  // (blockDim.x == M)
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float2* c = series + row * n_fft;
-    float v_max = 0.0f;
+    const V* c = series + row * n_fft;
+    S1 v_max = S1(0);
     int j_max = -1;
     for (int r = 0; r < P; ++r) {
       {
         // the first pass: the row turned by e^(2 pi i r m / n_fft)
-        float2 w, step;
-        sincospif(2.0f * static_cast<float>(r * q) / static_cast<float>(n_fft), &w.y, &w.x);
-        sincospif(2.0f * static_cast<float>(r * M) / static_cast<float>(n_fft), &step.y, &step.x);
-        float2 x[16];
+        V w, step;
+        root(r * q, n_fft, w);
+        root(r * M, n_fft, step);
+        V x[16];
 #pragma unroll
-        for (int p = 0; p < 16; ++p) x[p] = (q + p * M < n) ? c[q + p * M] : make_float2(0.f, 0.f);
+        for (int p = 0; p < 16; ++p) x[p] = (q + p * M < n) ? c[q + p * M] : cplx(S1(0), S1(0));
 #pragma unroll
         for (int p = 0; p < 16; ++p) {
           x[p] = cmul(x[p], w);
@@ -605,7 +824,7 @@ __global__ void __launch_bounds__(GridShape<L>::kThreads, GridShape<L>::kBlocksP
       fft_middle_passes<L, L / 16>(X);
       // the last radix and the largest value
       for (int g = threadIdx.x; g < L / R; g += blockDim.x) {
-        float2 x[R];
+        V x[R];
 #pragma unroll
         for (int p = 0; p < R; ++p) x[p] = X[fft_pad(R * g + p)];
         if constexpr (R == 16) {
@@ -615,7 +834,7 @@ __global__ void __launch_bounds__(GridShape<L>::kThreads, GridShape<L>::kBlocksP
         } else if constexpr (R == 4) {
           idft4(x[0], x[1], x[2], x[3]);
         } else {
-          const float2 s = cadd(x[0], x[1]), d = csub(x[0], x[1]);
+          const V s = cadd(x[0], x[1]), d = csub(x[0], x[1]);
           x[0] = s;
           x[1] = d;
         }
@@ -628,7 +847,7 @@ __global__ void __launch_bounds__(GridShape<L>::kThreads, GridShape<L>::kBlocksP
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, v_max, d);
+      const S1 ov = __shfl_xor_sync(0xffffffffu, v_max, d);
       const int oj = __shfl_xor_sync(0xffffffffu, j_max, d);
       keep_max_f(v_max, j_max, ov, oj);
     }
@@ -639,7 +858,7 @@ __global__ void __launch_bounds__(GridShape<L>::kThreads, GridShape<L>::kBlocksP
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      float bv = best_v[0];
+      S1 bv = best_v[0];
       int bj = best_j[0];
       for (int w = 1; w < static_cast<int>(blockDim.x / 32); ++w) keep_max_f(bv, bj, best_v[w], best_j[w]);
       const double denominator = static_cast<double>(n_fft) * delta_f;
@@ -661,24 +880,24 @@ int64_t grid_time_length(int64_t n, int64_t n_fft) {
   return (L <= 16384 && n_fft % L == 0) ? L : 0;
 }
 
-template <int L>
-int launch_grid_time(const float2* series, int64_t rows, int64_t n, int64_t n_fft, double delta_f, double* t,
+template <int L, class V>
+int launch_grid_time(const V* series, int64_t rows, int64_t n, int64_t n_fft, double delta_f, double* t,
                      cudaStream_t s) {
-  using G = GridShape<L>;
+  using G = GridShape<L, V>;
   if (G::kBytes > 48 * 1024) {
     static bool configured[64] = {};
     int dev = 0;
     const cudaError_t rd = cudaGetDevice(&dev);
     if (rd != cudaSuccess) return static_cast<int>(rd);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-      const cudaError_t rc = cudaFuncSetAttribute(k_grid_time<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      const cudaError_t rc = cudaFuncSetAttribute(k_grid_time<L, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   static_cast<int>(G::kBytes));
       if (rc != cudaSuccess) return static_cast<int>(rc);
       if (dev >= 0 && dev < 64) configured[dev] = true;
     }
   }
   const int64_t grid = rows < (int64_t(1) << 20) ? rows : (int64_t(1) << 20);
-  k_grid_time<L><<<static_cast<unsigned>(grid), G::kThreads, G::kBytes, s>>>(series, rows, n, n_fft, delta_f, t);
+  k_grid_time<L, V><<<static_cast<unsigned>(grid), G::kThreads, G::kBytes, s>>>(series, rows, n, n_fft, delta_f, t);
   const cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? 0 : static_cast<int>(err);
 }
@@ -727,6 +946,16 @@ int wfx_match_refine(int precision, const void* series, const void* zgrid, int64
       (time == 2 && t == nullptr) || !(delta_f > 0.0))
     return WFX_EINVAL;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  // (from given times, or at t = 0, a row in a block's registers; from a grid
+  // of z, or a longer row, a warp a row)
+  if (time != 1) {
+    if (precision == WFX_FP64 && launch_refine_rows<double>(series, rows, n, n_fft, freqs, delta_f, norms, time, phase,
+                                                            steps, match, t, s))
+      return launched();
+    if (precision == WFX_FP32 && launch_refine_rows<float>(series, rows, n, n_fft, freqs, delta_f, norms, time, phase,
+                                                           steps, match, t, s))
+      return launched();
+  }
   if (precision == WFX_FP64) {
     k_match_refine<double><<<row_grid((rows + kRowsPerBlock - 1) / kRowsPerBlock), kMatchBlock, 0, s>>>(
         static_cast<const double2*>(series), static_cast<const double2*>(zgrid), rows, n, n_fft, freqs, delta_f,
@@ -756,6 +985,23 @@ int wfx_match_grid_time(const void* series, int64_t rows, int64_t n, int64_t n_f
     case 16384:
       return launch_grid_time<16384>(c, rows, n, n_fft, delta_f, t, s);
     default:
+      return WFX_EINVAL;
+  }
+}
+
+int wfx_match_grid_time64(const void* series, int64_t rows, int64_t n, int64_t n_fft, double delta_f, double* t,
+                          wfx_stream_t stream) {
+  if (series == nullptr || t == nullptr || rows <= 0 || n <= 0 || n_fft < n || !(delta_f > 0.0)) return WFX_EINVAL;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const auto* c = static_cast<const double2*>(series);
+  switch (grid_time_length(n, n_fft)) {
+    case 2048:
+      return launch_grid_time<2048>(c, rows, n, n_fft, delta_f, t, s);
+    case 4096:
+      return launch_grid_time<4096>(c, rows, n, n_fft, delta_f, t, s);
+    case 8192:
+      return launch_grid_time<8192>(c, rows, n, n_fft, delta_f, t, s);
+    default:  // (16384 values in double exceed an SM's shared memory)
       return WFX_EINVAL;
   }
 }

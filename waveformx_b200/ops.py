@@ -582,22 +582,25 @@ def template_overlap(approximant: str, table: torch.Tensor, freqs: torch.Tensor,
     return norms
 
 
-def grid_time_supported(n: int, n_fft: int) -> bool:
+def grid_time_supported(n: int, n_fft: int, dtype: torch.dtype = torch.complex64) -> bool:
     """Whether :func:`match_grid_time` takes ``n`` frequencies on a grid of
     ``n_fft`` times: the power of two ``L >= max(n, 2048)`` is at most 16384
-    and divides ``n_fft`` (the library's rule, ``wfx_match_grid_time``)."""
+    (complex128: 8192) and divides ``n_fft`` (the library's rule,
+    ``wfx_match_grid_time``)."""
     length = max(2048, 1 << (int(n) - 1).bit_length())
-    return length <= 16384 and int(n_fft) % length == 0
+    return length <= (16384 if dtype == torch.complex64 else 8192) and int(n_fft) % length == 0
 
 
 def match_grid_time(series: torch.Tensor, n: int, delta_f: float) -> torch.Tensor:
     """The best time of each row's grid (largest ``|z|``) by the inverse FFT
-    in shared memory, for complex64 ``series`` whose rows are zero from
-    ``n`` on (see :func:`grid_time_supported`): float64 ``(rows,)``."""
-    _require(series, "series", torch.complex64)
+    in shared memory, for ``series`` whose rows are zero from ``n`` on (see
+    :func:`grid_time_supported`; in the precision of ``series``): float64
+    ``(rows,)``."""
+    _require(series, "series", series.dtype)
     rows, n_fft = series.shape
     t = torch.empty(rows, dtype=torch.float64, device=series.device)
-    _lib.check("wfx_match_grid_time", _lib.library().wfx_match_grid_time(
+    name = "wfx_match_grid_time" if series.dtype == torch.complex64 else "wfx_match_grid_time64"
+    _lib.check(name, getattr(_lib.library(), name)(
         _ptr(series), rows, int(n), n_fft, float(delta_f), _ptr(t), _stream(series.device)))
     return t
 
