@@ -225,3 +225,50 @@ def test_fp64_reverse_pass_sums(cuda, model, n, batch):
     loss1, grad1 = ops.fused_loss(model, *flat, cot[0][0].repeat(3), weights.repeat(3), antenna=(0.6, -0.3), scale=-0.5)
     check(loss[:, None], loss1.reshape(3, n, 1))
     check(grad, grad1.reshape(3, n, 9))
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("n, batch", [(1, 2400), (2, 2400), (63, 2401), (65, 2400), (511, 1300), (4001, 2400)])
+def test_fp32_reverse_pass_of_a_batch(cuda, model, n, batch):
+    """The FP32 reverse pass with a tile's powers in shared memory (large
+    batches on a shared grid), at the edges of its chunks (64 frequencies) and
+    tiles, rows of odd length, data shared and per binary, and one refused
+    binary: the module's FP32 bar against the FP64 kernels of the distinct
+    binaries; the loss, a sum of positive terms each within 1e-5 of its size,
+    to 1e-4."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    base = np.array([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0], [60.0, 15.0, 0.8, 0.5, 1000.0, 2.5, 4.0, 20.0],
+                     [9.0, 7.0, -0.6, 0.2, 200.0, 1.1, 0.3, 20.0], [np.nan, 7.0, -0.6, 0.2, 200.0, 1.1, 0.3, 20.0]])
+    grid = torch.as_tensor(np.geomspace(20.0, 2000.0, n) if n > 1 else np.array([90.0]), device=cuda).float()
+    rng = np.random.default_rng(n)
+    of = torch.arange(batch, device=cuda) % 4
+    params = torch.as_tensor(base, device=cuda)
+    t_c = torch.tensor([0.01, -0.02, 0.0, 0.0], dtype=torch.float64, device=cuda)
+    cot = [torch.as_tensor(rng.normal(size=(4, n)) + 1j * rng.normal(size=(4, n)), device=cuda).to(torch.complex64)
+           for _ in range(2)]
+    weights = torch.as_tensor(rng.uniform(0.5, 2.0, (4, n)), device=cuda).float()
+    kw = dict(antenna=(0.6, -0.3), scale=-0.5)
+
+    def run(precision, rows):
+        real, cplx = (torch.float32, torch.complex64) if precision == _lib.FP32 else (torch.float64, torch.complex128)
+        tables = ops.setup(model, params, grid[:1].double(), precision=precision, jvp=True)
+        table, dtable, tc = (x[rows].contiguous() for x in (tables.table, tables.dtable, t_c.to(real)))
+        a, b = (c.to(cplx)[rows].contiguous() for c in cot)
+        w, f = weights.to(real), grid.to(real)
+        yield ops.vjp(model, table, dtable, f, None, tc, a, b)
+        yield from ops.fused_loss(model, table, dtable, f, None, tc, a[0].contiguous(), w[0].contiguous(), **kw)
+        yield from ops.fused_loss(model, table, dtable, f, None, tc, a, w[rows].contiguous(), **kw)
+
+    few = torch.arange(4, device=cuda)
+    for got, exact in zip(run(_lib.FP32, of), run(_lib.FP64, few)):
+        got, exact = got.double(), exact.double()
+        assert torch.isnan(exact[3]).all() and torch.isnan(got[of == 3]).all()
+        got, want = got[of != 3], exact[of[of != 3]]
+        if want.ndim == 1:
+            bar = 1e-4 * want.abs()
+        else:
+            bar = 1e-2 * want.abs() + 1e-3 * want.abs().amax(1, keepdim=True)
+        assert bool(((got - want).abs() <= bar).all()), ((got - want).abs() / bar).max()

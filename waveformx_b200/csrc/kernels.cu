@@ -13,6 +13,8 @@
 //  * k_adj_f32: the reverse-mode pass, for cotangents (vjp) or for the fused
 //    likelihood (cotangent from the data in registers: the strain never
 //    reaches memory). Per-tile sums of dL/dtable go to the workspace.
+//  * k_adj_f32_staged: the same on a shared grid, large batches: a tile's
+//    powers in shared memory for the binaries that a block's warps claim.
 //  * k_contract: per binary, the FP64 sum of its tiles' partial sums and the
 //    product with dtable: the gradient in the parameters.
 //  * k_fwd_f64_shared, k_fwd_f64_ragged: the same in FP64.
@@ -1072,6 +1074,215 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_f32(const float* __restrict__
   }
 }
 
+// k_adj_f32 on a shared grid for batches that give every warp many items: a
+// block keeps a tile's frequency powers in shared memory (their double-float
+// Newton steps, logarithms and exponentials are a third of an evaluation with
+// its derivatives) while its warps claim binaries of that tile from the tile's
+// counter (claims[tile], zero at the launch); when they are claimed the block
+// goes on to the next tile that has some. The chunks of 64 frequencies wholly
+// above a binary's XAS cutoff cost the fused likelihood the sum of w |d|^2,
+// taken once per tile where data and weights are shared, and nothing else.
+// The items, their evaluation and their partial sums are k_adj_f32's. Bound by
+// FP32 issue; two blocks a SM, as the accumulators of a lane allow.
+// Measured with the powers per item and staged: the fused likelihood of 65536
+// binaries x 8192 frequencies, IMRPhenomXAS 3.45 and 2.33 ms, IMRPhenomD 7.25
+// and 4.27 ms, TaylorF2 4.62 and 2.45 ms; of 4096 x 4017, 153 and 121, 247 and
+// 157, 160 and 93 us, and vjp 140 and 120, 273 and 188, 148 and 118 us.
+constexpr int kStagedChunks = static_cast<int>((kAdjTileMax + 63) / 64);
+
+// The staged powers: f, t, f^-1, log f, f^-7/6, f^2/3 (hi, lo), f^-1/3 as
+// basis_products forms it, f^-5/3 (hi, lo), and IMRPhenomD's f^3/4 (hi, lo).
+template <int MODEL>
+__host__ __device__ constexpr int staged_fields() {
+  return MODEL == kModelPhenomD ? 12 : 10;
+}
+
+template <int MODEL>
+__device__ __forceinline__ void stage_powers(float* at, int stride, const Freq<float>& q) {
+  at[0] = q.f;
+  at[stride] = q.t;
+  at[2 * stride] = q.m1;
+  at[3 * stride] = q.lf;
+  at[4 * stride] = q.m76;
+  at[5 * stride] = q.t2;
+  at[6 * stride] = q.t2lo;
+  at[7 * stride] = q.mt1;
+  at[8 * stride] = q.y.hi;
+  at[9 * stride] = q.y.lo;
+  if constexpr (MODEL == kModelPhenomD) {
+    at[10 * stride] = q.f34;
+    at[11 * stride] = q.f34lo;
+  }
+}
+
+template <int MODEL>
+__device__ __forceinline__ void staged_pair(const float* at, int stride, Freq<float>& q0, Freq<float>& q1) {
+  float2 v[staged_fields<MODEL>()];
+#pragma unroll
+  for (int k = 0; k < staged_fields<MODEL>(); ++k) v[k] = *reinterpret_cast<const float2*>(at + k * stride);
+  q0.f = v[0].x, q1.f = v[0].y;
+  q0.t = v[1].x, q1.t = v[1].y;
+  q0.m1 = v[2].x, q1.m1 = v[2].y;
+  q0.lf = v[3].x, q1.lf = v[3].y;
+  q0.m76 = v[4].x, q1.m76 = v[4].y;
+  q0.t2 = v[5].x, q1.t2 = v[5].y;
+  q0.t2lo = v[6].x, q1.t2lo = v[6].y;
+  q0.mt1 = v[7].x, q1.mt1 = v[7].y;
+  q0.y = df{v[8].x, v[9].x}, q1.y = df{v[8].y, v[9].y};
+  if constexpr (MODEL == kModelPhenomD) {
+    q0.f34 = v[10].x, q1.f34 = v[10].y;
+    q0.f34lo = v[11].x, q1.f34lo = v[11].y;
+  }
+  q0.mt2 = q0.mt1 * q0.mt1, q1.mt2 = q1.mt1 * q1.mt1;
+  q0.m2 = q0.m1 * q0.m1, q1.m2 = q1.m1 * q1.m1;
+  q0.m3 = q0.m2 * q0.m1, q1.m3 = q1.m2 * q1.m1;
+}
+
+template <int MODEL, bool FUSED>
+__global__ void __launch_bounds__(kBlock, 2)
+    k_adj_f32_staged(const float* __restrict__ table, const float* __restrict__ freqs, int64_t n, int64_t B,
+                     int tile_len, int tiles, const float* __restrict__ t_c, const float2* __restrict__ cot_hp,
+                     const float2* __restrict__ cot_hc, FusedArgs fa, float* __restrict__ partial,
+                     unsigned* claims) {
+  constexpr AccMap kMap = acc_map<MODEL>();
+  extern __shared__ __align__(16) float powers[];  // [field][tile_len]
+  __shared__ __align__(16) float sT[kBlock / 32][kTableStride];
+  __shared__ float chunk_low[kStagedChunks], chunk_loss[kStagedChunks];
+  __shared__ unsigned claimed;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* T = sT[warp];
+  const float2* data = static_cast<const float2*>(fa.data);
+  const float* weights = static_cast<const float*>(fa.weights);
+  const float fp = static_cast<float>(fa.fp), fc = static_cast<float>(fa.fc);
+  const float two_scale = static_cast<float>(2.0 * fa.scale);
+  // (above a cutoff the likelihood's terms are the same for every binary)
+  const bool shared_terms = FUSED && fa.data_stride == 0 && fa.weights_stride == 0;
+  for (int k = 0; k < tiles; ++k) {
+    const int tile = (static_cast<int>(blockIdx.x % static_cast<unsigned>(tiles)) + k) % tiles;
+    __syncthreads();  // (the last tile's powers are read)
+    if (threadIdx.x == 0) claimed = atomicAdd(claims + tile, 0u);
+    __syncthreads();
+    if (claimed >= B) continue;
+    const int64_t n0 = static_cast<int64_t>(tile) * tile_len;
+    const int length = static_cast<int>(min(static_cast<int64_t>(tile_len), n - n0));
+    const int chunks = (length + 63) / 64;
+    for (int i = threadIdx.x; i < tile_len; i += kBlock) {
+      // (past the end: the tile's first frequency, stored nowhere)
+      stage_powers<MODEL>(powers + i, tile_len, freq_powers(freqs[n0 + (i < length ? i : 0)]));
+    }
+    for (int c = warp; c < chunks; c += kBlock / 32) {
+      float low = INFINITY, sum = 0.0f;
+      bool nan = false;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = 64 * c + 2 * lane + u;
+        if (i < length) {
+          const float f = freqs[n0 + i];
+          low = fminf(low, f);
+          nan = nan || f != f;
+          if (shared_terms) {
+            const float2 d = data[n0 + i];
+            sum += weights[n0 + i] * (d.x * d.x + d.y * d.y);
+          }
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
+      sum = warp_sum(sum);
+      nan = __any_sync(0xffffffffu, nan);
+      if (lane == 0) {
+        chunk_low[c] = nan ? -INFINITY : low;  // (a NaN is above no cutoff)
+        chunk_loss[c] = sum;
+      }
+    }
+    __syncthreads();
+    for (;;) {
+      unsigned claim = 0;
+      if (lane == 0) claim = atomicAdd(claims + tile, 1u);
+      const int64_t b = static_cast<int64_t>(__shfl_sync(0xffffffffu, claim, 0));
+      if (b >= B) break;
+      __syncwarp();
+      if (lane < kTableStride / 4) {
+        reinterpret_cast<float4*>(T)[lane] = __ldg(reinterpret_cast<const float4*>(table + b * kTableStride) + lane);
+      }
+      __syncwarp();
+      if (lane == 0) prepare_model<MODEL>(T, t_c != nullptr ? t_c[b] : 0.0f);
+      __syncwarp();
+      float acc[kTableStride];
+#pragma unroll
+      for (int i = 0; i < kTableStride; ++i) acc[i] = 0.0f;
+      float loss = 0.0f;
+      const int64_t row = b * n + n0;
+      const bool even = (row & 1) == 0;  // (the row's pairs are 16-byte aligned)
+      // two elements of the row (zero where out of range)
+      const auto row_pair = [&](const float2* x, int r, bool v0, bool v1) {
+        if (even) return load_pair(x + row, r, v0, v1);
+        const float2 a = v0 ? __ldcs(x + row + r) : make_float2(0.f, 0.f);
+        const float2 c = v1 ? __ldcs(x + row + r + 1) : make_float2(0.f, 0.f);
+        return make_float4(a.x, a.y, c.x, c.y);
+      };
+      for (int c = 0; c < chunks; ++c) {
+        const int r = 64 * c + 2 * lane;
+        const bool v0 = r < length, v1 = r + 1 < length;
+        bool zero = false;
+        float4 vp, vc;
+        if constexpr (MODEL == kModelXas) {
+          zero = chunk_low[c] > T[X_F_CUT];
+          if (zero) {
+            if (!FUSED) continue;
+            const float zp = 0.0f * T[X_KP], zc = 0.0f * T[X_KC];  // (NaN for a refused binary)
+            if (shared_terms) {
+              if (lane == 0) loss += chunk_loss[c] + (fp * zp + fc * zc);
+              continue;
+            }
+            vp = make_float4(zp, zp, zp, zp);
+            vc = make_float4(zc, zc, zc, zc);
+          }
+        }
+        Freq<float> q0, q1;
+        Point<float> p0, p1;
+        if (!zero) {
+          // (a lane past the end: the tile's first pair, nothing added)
+          staged_pair<MODEL>(powers + (v0 ? r : 0), tile_len, q0, q1);
+          point_pair<MODEL, float, false>(T, q0, q1, TcF{}, p0, p1);
+          if constexpr (FUSED) project<MODEL>(T, p0, p1, vp, vc);
+        }
+        float4 gp, gc;
+        if constexpr (FUSED) {
+          // r = fp h+ + fc hx - d; loss += w |r|^2; g = 2 scale w r
+          float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (fa.data_stride) {
+            d = row_pair(data, r, v0, v1);
+          } else {
+            const float2 a = data[n0 + (v0 ? r : 0)], e = data[n0 + (v1 ? r + 1 : 0)];
+            d = make_float4(a.x, a.y, e.x, e.y);
+          }
+          const float* w = weights + (fa.weights_stride ? row : n0);
+          const float w0 = v0 ? w[r] : 0.0f, w1 = v1 ? w[r + 1] : 0.0f;
+          const float r0x = fp * vp.x + fc * vc.x - d.x, r0y = fp * vp.y + fc * vc.y - d.y;
+          const float r1x = fp * vp.z + fc * vc.z - d.z, r1y = fp * vp.w + fc * vc.w - d.w;
+          loss += w0 * (r0x * r0x + r0y * r0y) + w1 * (r1x * r1x + r1y * r1y);
+          if (!fa.grad || zero) continue;
+          const float g0 = two_scale * w0, g1 = two_scale * w1;
+          gp = make_float4(fp * g0 * r0x, fp * g0 * r0y, fp * g1 * r1x, fp * g1 * r1y);
+          gc = make_float4(fc * g0 * r0x, fc * g0 * r0y, fc * g1 * r1x, fc * g1 * r1y);
+        } else {
+          gp = row_pair(cot_hp, r, v0, v1);
+          gc = row_pair(cot_hc, r, v0, v1);
+        }
+        if (v0) adjoint<MODEL, float>(T, q0, p0, gp.x, gp.y, gc.x, gc.y, acc);
+        if (v1) adjoint<MODEL, float>(T, q1, p1, gp.z, gp.w, gc.z, gc.w, acc);
+      }
+      acc[kSlotLoss] = static_cast<float>(fa.scale) * loss;
+      float v[kAccSlots];
+#pragma unroll
+      for (int c = 0; c < kAccSlots; ++c) v[c] = kMap.slot[c] >= 0 ? acc[kMap.slot[c]] : 0.0f;
+      const float2 sums = warp_reduce_scatter(v, lane);
+      reinterpret_cast<float2*>(partial + (b * tiles + tile) * kAccSlots)[lane] = sums;
+    }
+  }
+}
+
 // The table slot of each compact accumulator, per model (-1 for none), for
 // kernels that index it at run time.
 template <int MODEL>
@@ -1869,7 +2080,8 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 // go, so short items balance the SMs of a small batch (1024 x 4017: 8192
 // items of 504 frequencies, 68.6 us, against 2048 of 2010, 82.9 us, and
 // 75.3 us with 4096 of 1006; 16384 of 252: 72.3 us), while long ones cost
-// fewer stagings and reductions where items are plenty (65536 x 8192:
+// fewer stagings and reductions where items are plenty (65536 x 8192, each
+// item with its own powers:
 // 3.67 ms with tiles of 1640, 4.02 ms with 820, 4.69 ms with 410).
 constexpr int64_t kAdjItems = 8192;
 
@@ -1882,6 +2094,22 @@ int64_t adj_tile_len(int64_t B, int64_t n) {
     if (B * tiles >= kAdjItems) break;
   }
   return len;
+}
+
+// The staged reverse pass is taken where its resident warps get an item each
+// and a tile's powers serve enough binaries: 256, or 1024 of IMRPhenomXAS,
+// whose binaries leave the tiles above their cutoffs unread (measured, with
+// the powers per item and staged, in us: IMRPhenomD 128 x 30000 78 and 80,
+// 300 x 8192 59 and 48; TaylorF2 128 x 30000 56 and 64, 300 x 8192 41 and 35;
+// IMRPhenomXAS 512 x 8192 54 and 55, vjp 48 and 53, 768 x 8192 70 and 68, vjp
+// 61 and 64, 1024 x 8192 86 and 76, vjp 75 and 69, 1024 x 1000 31 and 31; below
+// an item a warp, 1000 frequencies of 300 to 1024 binaries, no difference).
+// kAdjClaims: the tiles whose counters a workspace holds.
+constexpr int64_t kAdjClaims = 64;
+
+bool adj_staged(int model, int64_t B, int64_t tiles) {
+  const int64_t binaries = model == kModelXas ? 1024 : 256;
+  return B >= binaries && tiles <= kAdjClaims && B * tiles >= 2 * (kBlock / 32) * max(device_sms(), 1);
 }
 
 struct Workspace {
@@ -1916,8 +2144,9 @@ Workspace carve(void* base, int64_t B, int64_t n, bool ragged, int64_t tile_len,
   if (partials) {
     w.partial = reinterpret_cast<float*>(p ? p + used : nullptr);
     used += align256(sizeof(float) * kAccSlots * items);
+    // (or k_adj_f32_staged's 32-bit counter of each tile)
     w.claim = reinterpret_cast<unsigned long long*>(p ? p + used : nullptr);
-    used += align256(sizeof(unsigned long long));
+    used += align256(sizeof(unsigned) * kAdjClaims);
   }
   w.items = items;
   w.bytes = used;
@@ -2010,6 +2239,31 @@ int polarizations_f32(const float* table, const float* freqs, const int64_t* off
   return ragged_f32<MODEL>(table, freqs, offsets, B, n, t_c, hp, hc, scratch, ragged_config(MODEL, B, n), s);
 }
 
+// k_adj_f32_staged on the resident blocks (two a SM: a tile's powers take up to
+// 98 KB of shared memory, allowed once per device).
+template <int MODEL, bool FUSED>
+int launch_adj_staged(const float* table, const float* freqs, int64_t n, int64_t B, int64_t tile_len, int64_t tiles,
+                      const float* t_c, const float2* cot_hp, const float2* cot_hc, FusedArgs fa, const Workspace& w,
+                      cudaStream_t s) {
+  constexpr int kDevices = 64;
+  constexpr int kMost = static_cast<int>(sizeof(float)) * staged_fields<MODEL>() * static_cast<int>(kAdjTileMax);
+  static std::atomic<bool> configured[kDevices] = {};
+  int dev = 0;
+  const cudaError_t rd = cudaGetDevice(&dev);
+  if (rd != cudaSuccess) return static_cast<int>(rd);
+  if (dev < 0 || dev >= kDevices || !configured[dev].load()) {
+    const cudaError_t rc = cudaFuncSetAttribute(k_adj_f32_staged<MODEL, FUSED>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+    if (rc != cudaSuccess) return static_cast<int>(rc);
+    if (dev >= 0 && dev < kDevices) configured[dev].store(true);
+  }
+  const size_t bytes = sizeof(float) * staged_fields<MODEL>() * static_cast<size_t>(tile_len);
+  k_adj_f32_staged<MODEL, FUSED><<<static_cast<unsigned>(2 * max(device_sms(), 1)), kBlock, bytes, s>>>(
+      table, freqs, n, B, static_cast<int>(tile_len), static_cast<int>(tiles), t_c, cot_hp, cot_hc, fa, w.partial,
+      reinterpret_cast<unsigned*>(w.claim));
+  return launched();
+}
+
 // The stages of the FP32 reverse pass: the per-item sums (the reverse
 // kernel), their contraction with dtable, or both in turn.
 enum AdjointStage : int { kStagePartials = 1, kStageContract = 2, kStageAll = 3 };
@@ -2029,7 +2283,8 @@ int adjoint_f32(bool fused, const float* table, const double* dtable, const floa
     }
     // one warp per work item, at most the blocks that are resident at once
     const int64_t wanted = (upper + kBlock / 32 - 1) / (kBlock / 32);
-    const cudaError_t zeroed = cudaMemsetAsync(w.claim, 0, sizeof(unsigned long long), s);
+    const bool staged = !ragged && adj_staged(MODEL, B, tpb);
+    const cudaError_t zeroed = cudaMemsetAsync(w.claim, 0, staged ? sizeof(unsigned) * tpb : sizeof(unsigned long long), s);
     if (zeroed != cudaSuccess) return static_cast<int>(zeroed);
 #define WFX_ADJ(R, F)                                                                                          \
   do {                                                                                                        \
@@ -2044,6 +2299,9 @@ int adjoint_f32(bool fused, const float* table, const double* dtable, const floa
       } else {
         WFX_ADJ(true, false);
       }
+    } else if (staged) {
+      const auto launch = fused ? launch_adj_staged<MODEL, true> : launch_adj_staged<MODEL, false>;
+      if (int rc = launch(table, freqs, n, B, tile_len, tpb, t_c, cot_hp, cot_hc, fa, w, s)) return rc;
     } else {
       if (fused) {
         WFX_ADJ(false, true);
