@@ -230,3 +230,37 @@ def test_zero_above_the_cutoff(cuda, precision):
             assert np.all(hp[i][above] == 0) and np.all(hc[i][above] == 0)
             assert np.all(np.abs(hp[i][~above][:-1]) > 0)
         assert np.all(np.isnan(hp[2])) and np.all(np.isnan(hc[2]))
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("batch", [1, 40, 17000])
+def test_fp32_ragged_items(cuda, model, batch):
+    """A ragged batch with more work items than blocks, empty rows, rows of
+    one frequency and rows just past a tile (1022), in rows whose frequencies
+    ascend (a warp in one region) and in the same rows shuffled (a warp in
+    several): against the FP64 kernels, to the module's bar on the largest
+    value of a row (2e-4)."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    rng = np.random.default_rng(batch)
+    lengths = np.array([1023, 0, 1, 33, 1022, 2, 513, 300])[np.arange(batch) % 8]
+    params = draw_batch(rng, 8)[np.arange(batch) % 8]
+    offsets = np.concatenate([[0], np.cumsum(lengths)])
+    total = 4.925490947641267e-06 * (params[:, 0] + params[:, 1])
+    k = np.arange(offsets[-1]) - np.repeat(offsets[:-1], lengths)
+    flat = 20.0 * (np.repeat(0.32 / total, lengths) / 20.0) ** (k / np.repeat(np.maximum(lengths - 1, 1), lengths))
+    rows = torch.as_tensor(np.repeat(np.arange(batch), lengths), device=cuda)
+    offs = torch.as_tensor(offsets, device=cuda)
+    shuffled = flat[np.lexsort((rng.random(flat.size), rows.cpu().numpy()))]
+    p = torch.as_tensor(params, device=cuda)
+    f_min = torch.full((batch,), 20.0, dtype=torch.float64, device=cuda)
+    for grid in (flat, shuffled):
+        f = torch.as_tensor(grid, device=cuda).float()
+        got, want = (ops.polarizations(model, ops.setup(model, p, f_min, precision=precision).table, g, offs)
+                     for precision, g in ((_lib.FP32, f), (_lib.FP64, f.double())))
+        for a, b in zip(got, want):
+            largest = torch.zeros(batch, dtype=torch.float64, device=cuda)
+            largest.scatter_reduce_(0, rows, b.abs(), "amax")
+            assert bool(((a - b).abs() <= 2e-4 * largest[rows]).all())

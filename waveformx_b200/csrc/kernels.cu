@@ -125,15 +125,10 @@ __device__ __forceinline__ void eval_fixed(const S* T, const Freq<S>* q, typenam
 }
 
 // Two adjacent frequencies of one binary: evaluated in lockstep (each table
-// coefficient read once) when they share their regions, else one by one.
-// When every lane of the warp holds frequencies of the same (phase,
-// amplitude) regions (all but the few warps that straddle a boundary), the
-// evaluation compiled for those regions runs: no branch on them. Every lane
-// of the warp must call it (a vote).
-//
-// SPECIALIZE = false: no vote and no specialized copies (the reverse pass,
-// whose larger code is fetch-bound already).
-template <int MODEL, class S, bool SPECIALIZE = true, bool TURNS = false>
+// coefficient read once) when they share their regions, else one by one
+// (the reverse pass, whose larger code is fetch-bound already, and the
+// forward's warps that straddle a boundary).
+template <int MODEL, class S, bool TURNS = false>
 __device__ __forceinline__ void point_pair(const S* T, const Freq<S>& q0, const Freq<S>& q1,
                                            typename TcOf<S>::type tc, Point<S>& p0, Point<S>& p1) {
   int rp0, ra0, rp1, ra1;
@@ -147,41 +142,9 @@ __device__ __forceinline__ void point_pair(const S* T, const Freq<S>& q0, const 
     tf2_regions(T, q0.f, rp0, ra0);
     tf2_regions(T, q1.f, rp1, ra1);
   }
-  const int code = rp0 * 3 + ra0;
   const bool same = rp0 == rp1 && ra0 == ra1;
-  const int lead = __shfl_sync(0xffffffffu, code, 0);
   const Freq<S> q[2] = {q0, q1};
   Point<S> p[2];
-  if (SPECIALIZE && __all_sync(0xffffffffu, same && code == lead)) {
-    switch (lead) {
-      case 8:
-        eval_fixed<MODEL, S, 2, 2, TURNS>(T, q, tc, p);
-        break;
-      case 7:
-        eval_fixed<MODEL, S, 2, 1, TURNS>(T, q, tc, p);
-        break;
-      case 4:
-        eval_fixed<MODEL, S, 1, 1, TURNS>(T, q, tc, p);
-        break;
-      case 3:
-        eval_fixed<MODEL, S, 1, 0, TURNS>(T, q, tc, p);
-        break;
-      case 0:
-        eval_fixed<MODEL, S, 0, 0, TURNS>(T, q, tc, p);
-        break;
-      default:
-        if constexpr (MODEL == kModelXas) {
-          xas_eval<S, 2, -1, -1, TURNS>(T, q, rp0, ra0, tc, p);
-        } else if constexpr (MODEL == kModelPhenomD) {
-          phd_eval<S, 2, -1, -1, TURNS>(T, q, rp0, ra0, tc, p);
-        } else {
-          tf2_eval<S, 2, -1, -1, TURNS>(T, q, rp0, ra0, tc, p);
-        }
-    }
-    p0 = p[0];
-    p1 = p[1];
-    return;
-  }
   if (same) {
     if constexpr (MODEL == kModelXas) {
       xas_eval<S, 2, -1, -1, TURNS>(T, q, rp0, ra0, tc, p);
@@ -424,7 +387,7 @@ template <int MODEL, bool TURNS>
 __device__ __forceinline__ void span_pair(const float* T, const Freq<float>& q0, const Freq<float>& q1,
                                           const SpanRegions& sr, Point<float>& p0, Point<float>& p1) {
   if (!sr.uniform) {
-    point_pair<MODEL, float, false, TURNS>(T, q0, q1, TcF{}, p0, p1);
+    point_pair<MODEL, float, TURNS>(T, q0, q1, TcF{}, p0, p1);
     return;
   }
   const Freq<float> q[2] = {q0, q1};
@@ -493,6 +456,71 @@ __device__ __forceinline__ bool pair_packed(const C& T, const Freq2& q, const Sp
     }
   }
   return false;
+}
+
+// The powers in one lane of a Freq2.
+__device__ __forceinline__ Freq<float> lane_powers(const Freq2& p, bool y) {
+  Freq<float> q;
+  q.f = y ? p.f.y : p.f.x;
+  q.t = y ? p.t.y : p.t.x;
+  q.m1 = y ? p.m1.y : p.m1.x;
+  q.lf = y ? p.lf.y : p.lf.x;
+  q.m76 = y ? p.m76.y : p.m76.x;
+  q.t2 = y ? p.t2.y : p.t2.x;
+  q.t2lo = y ? p.t2lo.y : p.t2lo.x;
+  q.m3 = y ? p.m3.y : p.m3.x;
+  q.y = y ? df{p.yhi.y, p.ylo.y} : df{p.yhi.x, p.ylo.x};
+  q.f34 = y ? p.f34.y : p.f34.x;
+  q.f34lo = y ? p.f34lo.y : p.f34lo.x;
+  return q;
+}
+
+// The pair at frequencies whose powers no other binary of the block shares:
+// where every frequency of the warp has the same regions (one of those that
+// eval_fixed serves), point_pair's evaluation with the powers that it reads
+// and no others. False elsewhere. Every lane of the warp calls it.
+template <int MODEL>
+__device__ __forceinline__ bool pair_from_frequencies(const float* T, float f0, float f1, float4& hp, float4& hc) {
+  int rp0, ra0, rp1, ra1;
+  if constexpr (MODEL == kModelXas) {
+    xas_regions(T, f0, rp0, ra0);
+    xas_regions(T, f1, rp1, ra1);
+  } else if constexpr (MODEL == kModelPhenomD) {
+    phd_regions(T, f0, rp0, ra0);
+    phd_regions(T, f1, rp1, ra1);
+  } else {
+    tf2_regions(T, f0, rp0, ra0);
+    tf2_regions(T, f1, rp1, ra1);
+  }
+  const int code = rp0 * 3 + ra0;
+  const int lead = __shfl_sync(0xffffffffu, code, 0);
+  if (!__all_sync(0xffffffffu, code == lead && rp1 * 3 + ra1 == lead)) return false;
+  const auto eval = [&](auto rp, auto ra) {
+    const Freq2 p = freq_powers2(make_float2(f0, f1));
+    const Freq<float> q[2] = {lane_powers(p, false), lane_powers(p, true)};
+    Point<float> pt[2];
+    eval_fixed<MODEL, float, decltype(rp)::value, decltype(ra)::value, true>(T, q, TcF{}, pt);
+    project<MODEL>(T, pt[0], pt[1], hp, hc);
+    return true;
+  };
+  using I0 = std::integral_constant<int, 0>;
+  using I1 = std::integral_constant<int, 1>;
+  using I2 = std::integral_constant<int, 2>;
+  if constexpr (MODEL == kModelTaylorF2) return eval(I0{}, I0{});
+  switch (lead) {
+    case 8:
+      return eval(I2{}, I2{});
+    case 7:
+      return eval(I2{}, I1{});
+    case 4:
+      return eval(I1{}, I1{});
+    case 3:
+      return eval(I1{}, I0{});
+    case 0:
+      return eval(I0{}, I0{});
+    default:
+      return false;
+  }
 }
 
 // Shared-grid forward. Block (group, tile): kFwdTile frequencies of a group
@@ -769,31 +797,48 @@ __global__ void __launch_bounds__(kBlock) k_template_norms(const float2* __restr
   }
 }
 
-template <int MODEL, bool RAGGED>
-__global__ void __launch_bounds__(kBlock) k_fwd_f32_tiles(const float* __restrict__ table,
+// Ragged forward: each block takes work items (binary, tile of its
+// frequencies) in turn: the first by its number, the next ones from the
+// counter *claim (zero at the launch), read while the item before is
+// evaluated (with blocks that step by the grid's size instead, the blocks past
+// the resident ones ran in a second wave on a part of the chip). Bound by issue
+// and the latency of the special functions: 188 instructions an evaluation,
+// three fifths of them the frequency's powers, so that an evaluation takes
+// those of its region alone (pair_from_frequencies), in pairs on the packed
+// instructions, and 6 blocks reside on an SM (5 of TaylorF2). 16384 binaries
+// of 278 million frequencies: IMRPhenomXAS 2566 us with every power, 2115
+// with the region's, 1977 with claimed items (5 blocks, 1840 with 6), 1567
+// with items of 4094 frequencies; IMRPhenomD 3094, 2492, 2302, 1932; TaylorF2
+// 2187, 2116, 1957, 1685 (849 at the copy's bandwidth). The results are the
+// same bits in all of them.
+template <int MODEL>
+__global__ void __launch_bounds__(kBlock, MODEL == kModelTaylorF2 ? 5 : 6) k_fwd_f32_tiles(const float* __restrict__ table,
                                                           const float* __restrict__ freqs,
                                                           const int64_t* __restrict__ offsets,
                                                           const int64_t* __restrict__ tile_prefix,
                                                           const int32_t* __restrict__ tile_map, int64_t n, int64_t B,
-                                                          int64_t tile_len, int64_t tiles_per_binary, int64_t capacity,
+                                                          int64_t tile_len, int64_t capacity,
                                                           const float* __restrict__ t_c, float2* __restrict__ hp,
-                                                          float2* __restrict__ hc) {
-  __shared__ __align__(16) float sT[kTableStride];
-  // (ragged: never more items than the workspace holds, whatever tile_prefix says)
-  const int64_t total = RAGGED ? min(tile_prefix[B], capacity) : B * tiles_per_binary;
-  for (int64_t item = blockIdx.x; item < total; item += gridDim.x) {
-    const Item it = item_of<RAGGED>(item, offsets, tile_prefix, tile_map, n, tile_len, tiles_per_binary);
-    __syncthreads();
-    if (threadIdx.x < kTableStride / 4) {
-      reinterpret_cast<float4*>(sT)[threadIdx.x] =
-          reinterpret_cast<const float4*>(table + it.b * kTableStride)[threadIdx.x];
+                                                          float2* __restrict__ hc, unsigned long long* claim) {
+  __shared__ __align__(16) float T[kTableStride];
+  __shared__ unsigned long long claimed;
+  const int lane = static_cast<int>(threadIdx.x);
+  // (never more items than the workspace holds, whatever tile_prefix says)
+  const int64_t total = min(tile_prefix[B], capacity);
+  const bool more = total > static_cast<int64_t>(gridDim.x);  // (than each block's first)
+  for (int64_t item = blockIdx.x; item < total;) {
+    const Item it = item_of<true>(item, offsets, tile_prefix, tile_map, n, tile_len, 0);
+    unsigned long long next = 0;
+    if (lane == 0 && more) next = atomicAdd(claim, 1ull);
+    if (lane < kTableStride / 4) {
+      reinterpret_cast<float4*>(T)[lane] = reinterpret_cast<const float4*>(table + it.b * kTableStride)[lane];
     }
     __syncthreads();
-    if (threadIdx.x == 0) prepare_model<MODEL, true>(sT, t_c != nullptr ? t_c[it.b] : 0.0f);
+    if (lane == 0) prepare_model<MODEL, true>(T, t_c != nullptr ? t_c[it.b] : 0.0f);
     __syncthreads();
     // (item-local 32-bit offsets r from s2, the even element at or below
-    // the item's start; the block runs the same trip count, lanes past the
-    // end evaluate the grid's first frequency and store nothing)
+    // the item's start; the block runs the same trip count, lanes past
+    // the end evaluate the item's last frequency and store nothing)
     const int64_t s2 = it.s & ~static_cast<int64_t>(1);
     const int lo_off = static_cast<int>(it.s - s2), hi_off = static_cast<int>(it.e - s2);
     const int npairs = (hi_off + 1) / 2;
@@ -801,23 +846,27 @@ __global__ void __launch_bounds__(kBlock) k_fwd_f32_tiles(const float* __restric
     float2* out_p = hp + s2;
     float2* out_c = hc + s2;
     for (int base = 0; base < npairs; base += kBlock) {
-      const int pr = base + static_cast<int>(threadIdx.x), r = 2 * pr;
+      const int pr = base + lane, r = 2 * pr;
       const bool in = pr < npairs;
       const bool v0 = in && r >= lo_off && r < hi_off, v1 = in && r + 1 >= lo_off && r + 1 < hi_off;
-      const float* a0 = v0 ? fr + r : (v1 ? fr + r + 1 : freqs);
+      const float* a0 = v0 ? fr + r : (v1 ? fr + r + 1 : fr + hi_off - 1);
       const float* a1 = v1 ? fr + r + 1 : a0;
       const float f0 = *a0, f1 = *a1;
       float4 vp, vc;
-      if (!all_above_cutoff<MODEL>(sT, f0, f1, vp, vc)) {
+      if (!all_above_cutoff<MODEL>(T, f0, f1, vp, vc) && !pair_from_frequencies<MODEL>(T, f0, f1, vp, vc)) {
         const Freq<float> q0 = freq_powers(f0);
         const Freq<float> q1 = freq_powers(f1);
         Point<float> p0, p1;
-        point_pair<MODEL, float, true, true>(sT, q0, q1, TcF{}, p0, p1);
-        project<MODEL>(sT, p0, p1, vp, vc);
+        point_pair<MODEL, float, true>(T, q0, q1, TcF{}, p0, p1);
+        project<MODEL>(T, p0, p1, vp, vc);
       }
       store_pair(out_p, r, vp, v0, v1);
       store_pair(out_c, r, vc, v0, v1);
     }
+    if (!more) break;
+    if (lane == 0) claimed = next;
+    __syncthreads();
+    item = static_cast<int64_t>(gridDim.x) + static_cast<int64_t>(claimed);
   }
 }
 
@@ -830,48 +879,74 @@ __global__ void __launch_bounds__(kBlock) k_fwd_f32_tiles(const float* __restric
 // 0 (no work item), else *error = 0. Valid offsets give at most
 // n / tile_len + B items (each binary's ceil(len / tile_len) <= len /
 // tile_len + 1), which carve() holds.
-__global__ void k_tile_prefix(const int64_t* __restrict__ offsets, int64_t B, int64_t n, int64_t tile_len,
-                              int64_t* prefix, int32_t* error) {
-  __shared__ int64_t sums[1024];
-  __shared__ int bad;
-  const int t = threadIdx.x;
-  const int64_t chunk = (B + blockDim.x - 1) / blockDim.x;
-  const int64_t lo = min(B, t * chunk), hi = min(B, lo + chunk);
-  if (t == 0) bad = 0;
-  __syncthreads();
-  bool ok = t != 0 || (offsets[0] >= 0 && offsets[B] == n);
-  for (int64_t b = lo; b < hi; ++b) ok = ok && offsets[b] <= offsets[b + 1];
-  if (!ok) bad = 1;
-  __syncthreads();
-  if (bad) {
-    for (int64_t b = lo; b < hi; ++b) prefix[b] = 0;
-    if (t == 0) {
-      prefix[B] = 0;
-      *error = WFX_EOFFSETS;
+// Bound by latency: 16 rows a thread, a stride of the block apart, loaded
+// together and scanned by warps (16384 rows: 43 us with 16 consecutive rows a
+// thread and three passes over them, whose reads touch a line a lane; now 13).
+constexpr int kPrefixRows = 16, kPrefixWarps = 32;
+
+__global__ void __launch_bounds__(32 * kPrefixWarps) k_tile_prefix(const int64_t* __restrict__ offsets, int64_t B,
+                                                                   int64_t n, int64_t tile_len, int64_t* prefix,
+                                                                   int32_t* error, unsigned long long* claim) {
+  constexpr int kThreads = 32 * kPrefixWarps;
+  __shared__ int64_t sums[kPrefixRows * kPrefixWarps], tops[kPrefixRows];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const auto scan = [&](int64_t v) {  // inclusive, over the warp
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, v, d);
+      v += lane >= d ? u : 0;
     }
-    return;
-  }
-  if (t == 0) *error = 0;
-  int64_t s = 0;
-  for (int64_t b = lo; b < hi; ++b) {
-    const int64_t len = offsets[b + 1] - offsets[b];
-    s += (len + tile_len - 1) / tile_len;
-  }
-  sums[t] = s;
-  __syncthreads();
-  for (int d = 1; d < static_cast<int>(blockDim.x); d <<= 1) {
-    int64_t v = t >= d ? sums[t - d] : 0;
+    return v;
+  };
+  const int64_t first = offsets[0], last = offsets[B];
+  bool ok = (first >= 0) & (last == n);
+  int64_t total = 0;
+  for (int64_t base = 0; base < B; base += kPrefixRows * kThreads) {
+    int64_t count[kPrefixRows];
+#pragma unroll
+    for (int k = 0; k < kPrefixRows; ++k) {
+      const int64_t b = base + k * kThreads + t;
+      count[k] = b < B ? offsets[b + 1] - offsets[b] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPrefixRows; ++k) {
+      if (base + k * kThreads >= B) continue;  // (no rows: count[k] is zero)
+      ok = ok && count[k] >= 0;
+      const int64_t up = count[k] + tile_len - 1;
+      // (32-bit division where it fits)
+      count[k] = up < (int64_t(1) << 32) ? static_cast<uint32_t>(up) / static_cast<uint32_t>(tile_len) : up / tile_len;
+      const int64_t through = scan(count[k]);
+      if (lane == 31) sums[k * kPrefixWarps + warp] = through;
+      count[k] = through - count[k];
+    }
     __syncthreads();
-    sums[t] += v;
+    // the warps' sums, in the rows' order: k first, then the warp
+    if (warp < kPrefixRows) {
+      const int64_t v = base + warp * kThreads < B ? sums[t] : 0, through = scan(v);
+      sums[t] = through - v;
+      if (lane == 31) tops[warp] = through;
+    }
     __syncthreads();
+    int64_t before = total;
+#pragma unroll
+    for (int k = 0; k < kPrefixRows; ++k) {
+      if (base + k * kThreads >= B) continue;
+      const int64_t b = base + k * kThreads + t;
+      if (b < B) prefix[b] = before + sums[k * kPrefixWarps + warp] + count[k];
+      before += tops[k];
+    }
+    total = before;
+    if (base + kPrefixRows * kThreads < B) __syncthreads();  // (sums and tops are read)
   }
-  int64_t run = t > 0 ? sums[t - 1] : 0;
-  for (int64_t b = lo; b < hi; ++b) {
-    prefix[b] = run;
-    const int64_t len = offsets[b + 1] - offsets[b];
-    run += (len + tile_len - 1) / tile_len;
+  const bool bad = __syncthreads_or(!ok);
+  if (bad) {
+    for (int64_t b = t; b < B; b += kThreads) prefix[b] = 0;
   }
-  if (t == static_cast<int>(blockDim.x) - 1) prefix[B] = sums[t];
+  if (t == 0) {
+    prefix[B] = bad ? 0 : total;
+    *error = bad ? WFX_EOFFSETS : 0;
+    *claim = 0;
+  }
 }
 
 // map[k] = the binary of work item k, for k below the workspace's capacity.
@@ -1026,7 +1101,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_f32(const float* __restrict__
       if (!zero) {
         q0 = freq_powers(f0);
         q1 = freq_powers(f1);
-        point_pair<MODEL, float, false>(T, q0, q1, TcF{}, p0, p1);
+        point_pair<MODEL, float>(T, q0, q1, TcF{}, p0, p1);
         if constexpr (FUSED) project<MODEL>(T, p0, p1, vp, vc);
       }
       float4 gp, gc;
@@ -1244,7 +1319,7 @@ __global__ void __launch_bounds__(kBlock, 2)
         if (!zero) {
           // (a lane past the end: the tile's first pair, nothing added)
           staged_pair<MODEL>(powers + (v0 ? r : 0), tile_len, q0, q1);
-          point_pair<MODEL, float, false>(T, q0, q1, TcF{}, p0, p1);
+          point_pair<MODEL, float>(T, q0, q1, TcF{}, p0, p1);
           if constexpr (FUSED) project<MODEL>(T, p0, p1, vp, vc);
         }
         float4 gp, gc;
@@ -2114,6 +2189,7 @@ bool adj_staged(int model, int64_t B, int64_t tiles) {
 
 struct Workspace {
   int32_t* error;  // ragged: the offsets' status word, at the start of the workspace
+  unsigned long long* next;  // ragged: the forward's next work item, in the status word's 256 bytes
   int64_t* tile_prefix;
   int32_t* tile_map;
   float* partial;
@@ -2133,6 +2209,7 @@ Workspace carve(void* base, int64_t B, int64_t n, bool ragged, int64_t tile_len,
   if (ragged) {
     items = n / tile_len + B + 1;
     w.error = reinterpret_cast<int32_t*>(p ? p + used : nullptr);
+    w.next = reinterpret_cast<unsigned long long*>(p ? p + used + sizeof(unsigned long long) : nullptr);
     used += align256(sizeof(int32_t));
     w.tile_prefix = reinterpret_cast<int64_t*>(p ? p + used : nullptr);
     used += align256(sizeof(int64_t) * (B + 1));
@@ -2154,7 +2231,7 @@ Workspace carve(void* base, int64_t B, int64_t n, bool ragged, int64_t tile_len,
 }
 
 int build_items(const int64_t* offsets, int64_t B, int64_t n, int64_t tile_len, Workspace& w, cudaStream_t s) {
-  k_tile_prefix<<<1, 1024, 0, s>>>(offsets, B, n, tile_len, w.tile_prefix, w.error);
+  k_tile_prefix<<<1, 32 * kPrefixWarps, 0, s>>>(offsets, B, n, tile_len, w.tile_prefix, w.error, w.next);
   k_tile_map<<<static_cast<unsigned>((B + 255) / 256), 256, 0, s>>>(w.tile_prefix, B, w.items, w.tile_map);
   return launched();
 }
@@ -2169,7 +2246,20 @@ struct RaggedConfig {
   int64_t tile_len;
   int64_t blocks_per_sm;
 };
-constexpr RaggedConfig kRaggedDefault{4 * kBlock - 2, 8};
+// Untuned: the longest item of 1022, 2046 and 4094 frequencies that still
+// gives the launched blocks two each (an item costs 1.5 us of its block for
+// the chain of reads to its table and the table's preparation). Measured, in
+// us, with items of 1022, 2046 and 4094, IMRPhenomXAS: 1.1 million frequencies
+// 24.9, 26.5, 26.8; 5.1 million 49.5, 49.5, 52.6; 16.8 million 128, 117, 119;
+// 278 million 1840, 1653, 1567.
+RaggedConfig ragged_default(int64_t n) {
+  constexpr int64_t kBlocks = 8;
+  int64_t len = 4 * kBlock - 2;
+  for (const int64_t longer : {8 * kBlock - 2, 16 * kBlock - 2}) {
+    if (n / longer >= 2 * kBlocks * max(device_sms(), 1)) len = longer;
+  }
+  return {len, kBlocks};
+}
 constexpr int64_t kRaggedTileCandidates[] = {2 * kBlock - 2, 4 * kBlock - 2, 8 * kBlock - 2, 16 * kBlock - 2};
 constexpr int64_t kRaggedBlocksCandidates[] = {2, 4, 8, 16};
 
@@ -2196,7 +2286,7 @@ RaggedConfig ragged_config(int model, int64_t B, int64_t n) {
   const TuneKey key = tune_key(model, B, n);
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   const auto it = g_tune.find(key);
-  return it == g_tune.end() ? kRaggedDefault : it->second;
+  return it == g_tune.end() ? ragged_default(n) : it->second;
 }
 
 bool valid_config(const RaggedConfig& c) {
@@ -2211,9 +2301,9 @@ int ragged_f32(const float* table, const float* freqs, const int64_t* offsets, i
   Workspace w = carve(scratch, B, n, true, kRaggedTileMin, false);
   if (int rc = build_items(offsets, B, n, c.tile_len, w, s)) return rc;
   const int64_t upper = n / c.tile_len + B + 1;
-  const int64_t grid = min(upper, static_cast<int64_t>(max(device_sms(), 1)) * c.blocks_per_sm);
-  k_fwd_f32_tiles<MODEL, true><<<static_cast<unsigned>(grid), kBlock, 0, s>>>(
-      table, freqs, offsets, w.tile_prefix, w.tile_map, n, B, c.tile_len, 0, w.items, t_c, hp, hc);
+  const int64_t resident = static_cast<int64_t>(max(device_sms(), 1)) * c.blocks_per_sm;
+  k_fwd_f32_tiles<MODEL><<<static_cast<unsigned>(min(upper, resident)), kBlock, 0, s>>>(
+      table, freqs, offsets, w.tile_prefix, w.tile_map, n, B, c.tile_len, w.items, t_c, hp, hc, w.next);
   return launched();
 }
 
@@ -2689,7 +2779,7 @@ int wfx_autotune_ragged(int model, const void* table, const void* freqs, const i
     if (start) cudaEventDestroy(start);
     return static_cast<int>(cudaGetLastError());
   }
-  RaggedConfig best = kRaggedDefault;
+  RaggedConfig best = ragged_default(n);
   float best_ms = -1.0f;
   int rc = 0;
   for (const int64_t tile : kRaggedTileCandidates) {
@@ -2741,7 +2831,7 @@ int wfx_tuning(int model, int64_t B, int64_t n, int64_t* config, int set) {
     return 1;
   }
   const auto it = g_tune.find(key);
-  const RaggedConfig c = it == g_tune.end() ? kRaggedDefault : it->second;
+  const RaggedConfig c = it == g_tune.end() ? ragged_default(n) : it->second;
   config[0] = c.tile_len;
   config[1] = c.blocks_per_sm;
   return it == g_tune.end() ? 0 : 1;

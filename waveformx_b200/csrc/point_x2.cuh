@@ -63,6 +63,74 @@ __device__ __forceinline__ float2 round_nearest2(float2 x) {
   return add2(add2(x, bc2(kMagic)), bc2(-kMagic));
 }
 
+// A double-float in each lane, and the double-float operations of point.cuh.
+struct df2 {
+  float2 hi, lo;
+};
+__device__ __forceinline__ df2 quick_two_sum2(float2 a, float2 b) {
+  const float2 s = add2(a, b);
+  return {s, sub2(b, sub2(s, a))};
+}
+__device__ __forceinline__ df2 two_prod2(float2 a, float2 b) {
+  const float2 p = mul2(a, b);
+  return {p, fma2(a, b, neg2(p))};
+}
+__device__ __forceinline__ df2 df_mul2(df2 a, df2 b) {
+  const df2 p = two_prod2(a.hi, b.hi);
+  return quick_two_sum2(p.hi, fma2(a.hi, b.lo, fma2(a.lo, b.hi, p.lo)));
+}
+__device__ __forceinline__ df2 df_mul2(df2 a, float2 b) {
+  const df2 p = two_prod2(a.hi, b);
+  return quick_two_sum2(p.hi, fma2(a.lo, b, p.lo));
+}
+
+// freq_powers of two frequencies, each lane's roundings as there. A caller
+// that reads some of the powers pays for those: inlined where the regions are
+// known at compile time (xas_pair_x2 and phd_pair_x2 read the double-float
+// f^-5/3 in the inspiral alone, f^1/3 in none of the intermediate's terms).
+__device__ __forceinline__ Freq2 freq_powers2(float2 f) {
+  Freq2 q;
+  q.f = f;
+  q.m1 = make_float2(__frcp_rn(f.x), __frcp_rn(f.y));
+  q.lf = make_float2(logf(f.x), logf(f.y));
+  const float2 e = mul2(q.lf, bc2(1.0f / 3.0f));
+  const float2 t = make_float2(expf(e.x), expf(e.y));
+  const float2 cube = mul2(mul2(t, t), t);
+  q.t = mul2(mul2(t, fma2(neg2(cube), q.m1, bc2(4.0f))), bc2(1.0f / 3.0f));
+  q.m76 = mul2(q.m1, make_float2(rsqrtf(q.t.x), rsqrtf(q.t.y)));
+  const float2 g = mul2(bc2(-5.0f / 3.0f), q.lf);
+  const float2 y0 = make_float2(expf(g.x), expf(g.y));
+  const df2 ff = two_prod2(f, f);
+  const df2 f5 = df_mul2(df_mul2(ff, ff), f);
+  const df2 y3 = df_mul2(two_prod2(y0, y0), y0);
+  const df2 w = df_mul2(y3, f5);
+  const float2 r = sub2(sub2(bc2(1.0f), w.hi), w.lo);
+  const df2 y = quick_two_sum2(y0, mul2(mul2(y0, r), bc2(1.0f / 3.0f)));
+  q.yhi = y.hi;
+  q.ylo = y.lo;
+  // (f^2/3 and f^3/4: the Newton steps of df_pow23 and df_pow34)
+  const float2 t2 = mul2(q.t, q.t);
+  const df2 c3 = df_mul2(two_prod2(t2, t2), t2);
+  const float2 r2 = add2(sub2(ff.hi, c3.hi), sub2(ff.lo, c3.lo));
+  const float2 d2 = mul2(mul2(bc2(3.0f), t2), t2);
+  const df2 t23 = quick_two_sum2(t2, make_float2(__fdividef(r2.x, d2.x), __fdividef(r2.y, d2.y)));
+  q.t2 = t23.hi;
+  q.t2lo = t23.lo;
+  const float2 root = make_float2(sqrtf(f.x), sqrtf(f.y));
+  const float2 h0 = mul2(root, make_float2(sqrtf(root.x), sqrtf(root.y)));
+  const df2 f3 = df_mul2(ff, f);
+  const df2 h2 = two_prod2(h0, h0);
+  const df2 h4 = df_mul2(h2, h2);
+  const float2 r4 = add2(sub2(f3.hi, h4.hi), sub2(f3.lo, h4.lo));
+  const float2 d4 = mul2(mul2(mul2(bc2(4.0f), h0), h0), h0);
+  const df2 f34 = quick_two_sum2(h0, make_float2(__fdividef(r4.x, d4.x), __fdividef(r4.y, d4.y)));
+  q.f34 = f34.hi;
+  q.f34lo = f34.lo;
+  const float2 m2 = mul2(q.m1, q.m1);
+  q.m3 = mul2(m2, q.m1);
+  return q;
+}
+
 // phase_turns in both lanes (big = 0 when BIG is false).
 template <bool BIG, class C>
 __device__ __forceinline__ float2 phase_turns2(const C& T, int cs, int ls, int llo, const Freq2& q, float2 big_hi,
