@@ -144,7 +144,7 @@ int wfx_xhm_setup(const double* params, int64_t B, const double* f_min, int64_t 
 /* IMRPhenomXHM's set-up with its forward-mode derivative along the eight
  * parameters (the tables and tangents of the reference's XHM VJP,
  * models/xhm/mlx/_api.py:42-48 and 63-69): the set-up of every part on dual
- * numbers, one thread per binary, part and parameter. dtable (B x
+ * numbers, a part of the row per block, a parameter per thread. dtable (B x
  * WFX_XHM_STRIDE64 x 8 double): d row64[b][k] / d params[b][j] at
  * [(b * WFX_XHM_STRIDE64 + k) * 8 + j]; zero along f_ref where it is 0 (the
  * first frequency or reference_mf / M stands for it). table64, table32 and
