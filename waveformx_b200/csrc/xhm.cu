@@ -933,7 +933,7 @@ static_assert((H_FACTORS & 3) == 0, "factor i of mode k at H_FACTORS + 4 k + i")
 // IMRPhenomXHM's derivative with respect to the grid (the reference's
 // drop-in differentiates its model with respect to the frequencies,
 // src/waveformx/torch.py:87-91; models/xhm/model.py:40 takes the set-up's
-// first frequency without a derivative): the FP64 evaluation of k_xhm_jvp
+// first frequency without a derivative): the FP64 evaluation of k_xhm
 // with the table's tangents zero and the frequency's powers carrying d/df
 // (freq_powers_dual), e^(-2 pi i f t_c) differentiated in f too, contracted
 // with the cotangents: d[b][j] = Re(conj(g+) dh+/df + conj(gx) dhx/df).
