@@ -301,3 +301,24 @@ def test_match_at_the_rows_of_the_blocks(cuda, dtype, n):
         ref = om.match(a.astype(np.complex128), b.astype(np.complex128), f, w.astype(real).astype(np.float64), time=time,
                        phase=phased)
         np.testing.assert_allclose(got, ref, rtol=0, atol=1e-6 if dtype == "complex64" else 1e-10)
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_match_of_conjugate_views(cuda, dtype):
+    """Waveforms as conjugate views, and a psd as a negative one, match as
+    their values do."""
+    import torch
+
+    from waveformx_b200 import match as wm
+
+    c = getattr(torch, dtype)
+    a = _t(cuda, chirp()).to(c)
+    b = torch.stack([_t(cuda, shifted(chirp(0.01 * k), 0.01 * k, 0.3)).to(c) for k in range(3)])
+    psd = _t(cuda, PSD).to(a.real.dtype)
+    lazy = torch._neg_view(-psd)
+    for x, y in ((a.conj(), b.conj()), (a, b.conj()), (a.conj(), b)):
+        got = wm.match(x, y, FREQUENCIES, lazy, return_time=True)
+        expected = wm.match(x.resolve_conj(), y.resolve_conj(), FREQUENCIES, psd, return_time=True)
+        assert all(torch.equal(u, v) for u, v in zip(got, expected))
+    got = wm.polarization_match(a.conj(), b.conj(), b, FREQUENCIES, lazy)
+    assert torch.equal(got, wm.polarization_match(a.conj().resolve_conj(), b.conj().resolve_conj(), b, FREQUENCIES, psd))

@@ -234,3 +234,79 @@ def test_fields_without_conversion(cuda, dtype, n):
         out.append([hp.detach(), hc.detach(), *(g.reshape(-1) for g in gradients)])
     for x, y in zip(*out):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("approximant", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2", "IMRPhenomXHM"])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("batched", [False, True])
+def test_losses_with_the_strain_under_conj(cuda, approximant, dtype, batched):
+    """A loss with the strain under ``conj`` sends the backward a conjugate
+    view: its gradients are those of the same loss with the other factor
+    conjugated. Bar: 200 terms' rounding in any order, 1e-12 (float64) or 1e-5
+    of a field's largest; the conjugate cotangent's gradients differ in the
+    first digit."""
+    import torch
+
+    import waveformx_b200.torch as wt
+    from waveformx_b200 import match
+
+    real = getattr(torch, dtype)
+    rows = torch.tensor(BATCH if batched else ALIGNED, dtype=real, device=cuda)
+    grid = torch.linspace(20.0, 400.0, 200, dtype=real, device=cuda)
+    rng = np.random.default_rng(5)
+    d = torch.as_tensor(rng.normal(size=200) + 1j * rng.normal(size=200), device=cuda).to(
+        torch.complex64 if dtype == "float32" else torch.complex128)
+    w = torch.as_tensor(oracle.psd(np.linspace(20.0, 400.0, 200)), device=cuda).to(real)
+    f = wt.polarizations_function(approximant)
+
+    def gradient(loss):
+        x = rows.clone().requires_grad_(True)
+        t_c = torch.full(rows.shape[:-1], 0.01, dtype=real, device=cuda, requires_grad=True)
+        hp, hc = f(binary_of(x), grid, t_c=t_c)
+        return torch.autograd.grad(loss(hp) + 0.5 * loss(hc), (x, t_c))
+
+    pairs = [(lambda h: (h.conj() * d * w).real.sum(), lambda h: (h * d.conj() * w).real.sum()),
+             (lambda h: (torch.conj(h) @ d).imag.sum(), lambda h: -(h @ torch.conj(d)).imag.sum()),
+             (lambda h: match.inner_product(d, h, grid, w).sum(), lambda h: match.inner_product(h, d, grid, w).sum())]
+    tol = 1e-12 if dtype == "float64" else 1e-5
+    for under, other in pairs:
+        for a, b in zip(gradient(under), gradient(other)):
+            scale = b.abs().amax(0) if batched else b.abs()
+            assert bool((b != 0).any()) and bool(((a - b).abs() <= tol * scale).all())
+
+
+def test_inputs_that_are_negative_views(cuda):
+    """The grid and ``t_c`` as negative views (contiguous, and negated as they
+    are read) give the strain of their values."""
+    import torch
+
+    import waveformx_b200.torch as wt
+
+    f = wt.polarizations_function("IMRPhenomXAS")
+    grid = torch.linspace(20.0, 400.0, 65, dtype=torch.float64, device=cuda)
+    t_c = torch.tensor([0.01, -0.02, 0.3], dtype=torch.float64, device=cuda)
+    b = binary_of(torch.tensor(BATCH, dtype=torch.float64, device=cuda))
+    expected = f(b, grid, t_c=t_c)
+    for got in (f(b, torch._neg_view(-grid), t_c=t_c), f(b, grid, t_c=torch._neg_view(-t_c))):
+        assert all(torch.equal(x, y) for x, y in zip(got, expected))
+
+
+def test_operations_refuse_lazy_views(cuda):
+    """The tensor operations, which read their arguments' memory, refuse
+    conjugate and negative views."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    p = torch.as_tensor(np.ascontiguousarray(aligned(BATCH)), device=cuda)
+    grid = torch.linspace(20.0, 400.0, 65, dtype=torch.float64, device=cuda)
+    t = ops.setup("IMRPhenomXAS", p, grid[:1], precision=_lib.FP64, jvp=True)
+    g = torch.randn((3, 65), dtype=torch.complex128, device=cuda)
+    with pytest.raises(ValueError, match="conjugate"):
+        ops.vjp("IMRPhenomXAS", t.table, t.dtable, grid, None, None, g.conj(), g)
+    with pytest.raises(ValueError, match="negative"):
+        ops.polarizations("IMRPhenomXAS", t.table, torch._neg_view(-grid))
+    # (those that convert their cotangents take them)
+    a = ops.grid_vjp("IMRPhenomXAS", t.table, grid, None, None, g.conj(), g)
+    b = ops.grid_vjp("IMRPhenomXAS", t.table, grid, None, None, g.conj().resolve_conj(), g)
+    torch.testing.assert_close(a, b, rtol=1e-12, atol=0)

@@ -37,7 +37,7 @@ class CapturedPolarizations:
         self.approximant = approximant
         self.batch = int(batch)
         self.device = freqs.device
-        self.freqs = freqs.contiguous()
+        self.freqs = ops.plain(freqs)
         self.offsets = None if offsets is None else offsets.to(self.device, torch.int64).contiguous()
         if self.offsets is not None:
             # (checked here, outside any capture: the check reads them to the host)
@@ -136,7 +136,7 @@ class CapturedLikelihood:
         self.approximant = approximant
         self.batch = int(batch)
         self.device = freqs.device
-        self.freqs = freqs.contiguous()
+        self.freqs = ops.plain(freqs)
         self.offsets = None if offsets is None else offsets.to(self.device, torch.int64).contiguous()
         if self.offsets is not None:
             # (checked here, outside any capture: the check reads them to the host)

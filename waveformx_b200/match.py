@@ -42,7 +42,7 @@ NEWTON_STEPS = 3
 
 
 def _grid(frequencies, device, dtype):
-    f = torch.as_tensor(frequencies, device=device).to(torch.float64).contiguous()
+    f = ops.plain(torch.as_tensor(frequencies, device=device).to(torch.float64))
     if f.ndim != 1 or f.numel() < 2:
         raise ValueError("frequencies must be a uniform grid of at least two values")
     return f, float(f[1] - f[0]), f.to(dtype).contiguous()
@@ -102,7 +102,7 @@ def match(a: torch.Tensor, b: torch.Tensor, frequencies, psd, *, time: bool = Tr
     n = f64.numel()
     if a.shape[-1] != n or b.shape[-1] != n:
         raise ValueError("the last axis of a and b must hold one value per frequency")
-    s = torch.as_tensor(psd, device=a.device, dtype=a.real.dtype).contiguous()
+    s = ops.plain(torch.as_tensor(psd, device=a.device, dtype=a.real.dtype))
     shape = torch.broadcast_shapes(a.shape[:-1], b.shape[:-1])
     rows = 1
     for d in shape:
@@ -110,7 +110,7 @@ def match(a: torch.Tensor, b: torch.Tensor, frequencies, psd, *, time: bool = Tr
 
     def flat(x):
         # (a one-dimensional waveform is one vector for every row)
-        return x.contiguous() if x.ndim == 1 else x.expand(*shape, n).reshape(rows, n).contiguous()
+        return ops.plain(x if x.ndim == 1 else x.expand(*shape, n).reshape(rows, n))
 
     flat_a, flat_b = flat(a), flat(b)
     n_fft = ops.fft_length(n, pad)
@@ -142,14 +142,14 @@ def polarization_match(signal: torch.Tensor, hplus: torch.Tensor, hcross: torch.
             raise TypeError("signal, hplus and hcross must all be complex64 or all complex128")
     f64, delta_f, _ = _grid(frequencies, signal.device, signal.real.dtype)
     n = f64.numel()
-    s = torch.as_tensor(psd, device=signal.device, dtype=signal.real.dtype).contiguous()
+    s = ops.plain(torch.as_tensor(psd, device=signal.device, dtype=signal.real.dtype))
     shape = torch.broadcast_shapes(signal.shape[:-1], hplus.shape[:-1], hcross.shape[:-1])
     rows = 1
     for d in shape:
         rows *= d
 
     def flat(x):
-        return x.contiguous() if x.ndim == 1 else x.expand(*shape, n).reshape(rows, n).contiguous()
+        return ops.plain(x if x.ndim == 1 else x.expand(*shape, n).reshape(rows, n))
 
     n_fft = ops.fft_length(n, pad)
     series = _series_buffer(2 * rows, n_fft, signal.dtype, signal.device)
@@ -178,15 +178,15 @@ def template_polarization_match(approximant: str, params: torch.Tensor, frequenc
     _require_cuda(params, "params")
     f64, delta_f, f32 = _grid(frequencies, params.device, torch.float32)
     n = f64.numel()
-    sig = torch.as_tensor(signal, device=params.device).to(torch.complex64).contiguous()
+    sig = ops.plain(torch.as_tensor(signal, device=params.device).to(torch.complex64))
     if sig.numel() != n:
         raise ValueError("signal must hold one value per frequency")
-    s = torch.as_tensor(psd, device=params.device).to(torch.float32).contiguous()
+    s = ops.plain(torch.as_tensor(psd, device=params.device).to(torch.float32))
     tables = ops.setup(approximant, params, f64[:1], amp_scale=amp_scale, reference_mf=reference_mf,
                        precision=_lib.FP32)
     n_fft = ops.fft_length(n, pad)
     series = _series_buffer(2 * params.shape[0], n_fft, torch.complex64, params.device)
-    tc = None if t_c is None else torch.as_tensor(t_c, device=params.device).to(torch.float32).contiguous()
+    tc = None if t_c is None else ops.plain(torch.as_tensor(t_c, device=params.device).to(torch.float32))
     if ops.model_code(approximant) == _lib.XHM:
         hp, hc = ops.polarizations(approximant, tables.table, f32, None, tc)
         norms = ops.polarization_overlap(sig, hp.contiguous(), hc.contiguous(), s, delta_f, series)
@@ -211,15 +211,15 @@ def template_match(approximant: str, params: torch.Tensor, frequencies, signal: 
     _require_cuda(params, "params")
     f64, delta_f, f32 = _grid(frequencies, params.device, torch.float32)
     n = f64.numel()
-    sig = torch.as_tensor(signal, device=params.device).to(torch.complex64).contiguous()
+    sig = ops.plain(torch.as_tensor(signal, device=params.device).to(torch.complex64))
     if sig.numel() != n:
         raise ValueError("signal must hold one value per frequency")
-    s = torch.as_tensor(psd, device=params.device).to(torch.float32).contiguous()
+    s = ops.plain(torch.as_tensor(psd, device=params.device).to(torch.float32))
     tables = ops.setup(approximant, params, f64[:1], amp_scale=amp_scale, reference_mf=reference_mf,
                        precision=_lib.FP32)
     n_fft = ops.fft_length(n, pad)
     series = _series_buffer(params.shape[0], n_fft, torch.complex64, params.device)
-    tc = None if t_c is None else torch.as_tensor(t_c, device=params.device).to(torch.float32).contiguous()
+    tc = None if t_c is None else ops.plain(torch.as_tensor(t_c, device=params.device).to(torch.float32))
     if ops.model_code(approximant) == _lib.XHM:
         # (IMRPhenomXHM: its templates' strain from its kernel, then the
         # series of the given waveforms)

@@ -26,7 +26,7 @@ __all__ = ["APPROXIMANTS", "model_code", "Tables", "setup", "polarizations", "no
            "grid_time_supported", "match_grid_time", "match_refine",
            "polarization_overlap", "template_polarization_overlap", "polarization_refine", "xhm_modes",
            "XHM_MODES", "xhm_dtable", "xhm_vjp", "grid_vjp", "check_offsets", "check_per_frequency",
-           "offsets_problem"]
+           "offsets_problem", "plain"]
 
 #: The approximants of this path and their codes in the C ABI.
 APPROXIMANTS = {"IMRPhenomXAS": _lib.XAS, "IMRPhenomD": _lib.PHENOMD, "TaylorF2": _lib.TAYLORF2,
@@ -72,7 +72,17 @@ def _require(t: torch.Tensor, name: str, dtype=None):
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
+    if t.is_conj() or t.is_neg():
+        raise ValueError(f"{name} must not be a lazy conjugate or negative view (resolve_conj(), resolve_neg()): "
+                         "the kernels read its memory")
     return t
+
+
+def plain(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as contiguous memory that holds its values: a conjugate or
+    negative view, which is contiguous but negates as it is read, written
+    out."""
+    return t.resolve_conj().resolve_neg().contiguous()
 
 
 def workspace(op: int, model: int, precision: int, batch: int, n: int, ragged: bool,
@@ -259,8 +269,8 @@ def grid_vjp(approximant: str, table: torch.Tensor, freqs: torch.Tensor, offsets
         _require(t_c, "t_c", torch.float64)
     if offsets is not None:
         check_offsets(offsets, batch, n)
-    cp = cot_hp.to(torch.complex128).contiguous()
-    cc = cot_hc.to(torch.complex128).contiguous()
+    cp = plain(cot_hp.to(torch.complex128))
+    cc = plain(cot_hc.to(torch.complex128))
     out = torch.empty(n, dtype=torch.float64, device=table.device)
     _lib.check("wfx_grid_vjp", _lib.library().wfx_grid_vjp(
         model, _ptr(table), _ptr(freqs), _ptr(offsets), batch, n, _ptr(t_c), _ptr(cp), _ptr(cc), _ptr(out),
@@ -326,8 +336,8 @@ def xhm_vjp(params: torch.Tensor, f_min: torch.Tensor, freqs: torch.Tensor, offs
     batch, n = params.shape[0], freqs.numel()
     if t_c is not None:
         _require(t_c, "t_c", torch.float64)
-    cp = cot_hp.to(torch.complex128).contiguous()
-    cc = cot_hc.to(torch.complex128).contiguous()
+    cp = plain(cot_hp.to(torch.complex128))
+    cc = plain(cot_hc.to(torch.complex128))
     max_len = n
     if offsets is not None:
         check_offsets(offsets, batch, n)

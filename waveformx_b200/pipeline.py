@@ -113,7 +113,7 @@ def polarizations_batches(approximant: str, params: torch.Tensor, freqs: torch.T
     if not (isinstance(params, torch.Tensor) and params.is_cuda and params.dtype == torch.float64
             and params.ndim == 3 and params.shape[2] == 8 and params.shape[0] > 0 and params.shape[1] > 0):
         raise ValueError("params must be a (K, B, 8) float64 CUDA tensor with K, B > 0")
-    params = params.contiguous()
+    params = ops.plain(params)
     K, batch = params.shape[0], params.shape[1]
     device = params.device
     real = torch.float32 if precision == _lib.FP32 else torch.float64
@@ -134,11 +134,11 @@ def polarizations_batches(approximant: str, params: torch.Tensor, freqs: torch.T
             f_min = freqs[:1].to(torch.float64)
         else:
             f_min = freqs[offsets[:-1].clamp(max=max(n - 1, 0))].to(torch.float64)
-    f_min = f_min.to(device, torch.float64).contiguous()
+    f_min = ops.plain(f_min.to(device, torch.float64))
     if f_min.numel() not in (1, batch):
         raise ValueError("f_min must have one value or one per binary")
     if t_c is not None:
-        t_c = torch.as_tensor(t_c, dtype=real, device=device).contiguous()
+        t_c = ops.plain(torch.as_tensor(t_c, dtype=real, device=device))
         if t_c.numel() != K * batch:
             raise ValueError("t_c must be (K, B)")
     ring = K if ring is None else int(ring)
@@ -222,7 +222,7 @@ def likelihood_batches(approximant: str, params: torch.Tensor, freqs: torch.Tens
     if not (isinstance(params, torch.Tensor) and params.is_cuda and params.dtype == torch.float64
             and params.ndim == 3 and params.shape[2] == 8 and params.shape[0] > 0 and params.shape[1] > 0):
         raise ValueError("params must be a (K, B, 8) float64 CUDA tensor with K, B > 0")
-    params = params.contiguous()
+    params = ops.plain(params)
     K, batch = params.shape[0], params.shape[1]
     device = params.device
     ops._require(freqs, "freqs", torch.float32)
@@ -239,11 +239,11 @@ def likelihood_batches(approximant: str, params: torch.Tensor, freqs: torch.Tens
             f_min = freqs[:1].to(torch.float64)
         else:
             f_min = freqs[offsets[:-1].clamp(max=max(n - 1, 0))].to(torch.float64)
-    f_min = f_min.to(device, torch.float64).contiguous()
+    f_min = ops.plain(f_min.to(device, torch.float64))
     if f_min.numel() not in (1, batch):
         raise ValueError("f_min must have one value or one per binary")
     if t_c is not None:
-        t_c = torch.as_tensor(t_c, dtype=torch.float32, device=device).contiguous()
+        t_c = ops.plain(torch.as_tensor(t_c, dtype=torch.float32, device=device))
         if t_c.numel() != K * batch:
             raise ValueError("t_c must be (K, B)")
     if group is None:
@@ -327,7 +327,7 @@ def polarizations_stream(approximant: str, batches: Iterable, freqs: torch.Tenso
         else:
             first = offsets[:-1].clamp(max=max(freqs.numel() - 1, 0))
             f_min = freqs[first].to(torch.float64)
-    f_min = f_min.to(device, torch.float64).contiguous()
+    f_min = ops.plain(f_min.to(device, torch.float64))
     rmf = float("nan") if reference_mf is None else float(reference_mf)
     lib = _lib.library()
     main = torch.cuda.current_stream(device)
@@ -357,7 +357,7 @@ def polarizations_stream(approximant: str, batches: Iterable, freqs: torch.Tenso
                 and params.ndim == 2 and params.shape[1] == 8 and params.shape[0] > 0):
             ops._require(params, "params", torch.float64)
             raise ValueError("params must be (B, 8) with B > 0")
-        params = params.contiguous()
+        params = ops.plain(params)
         if batch is None:
             batch = params.shape[0]
             if f_min.numel() not in (1, batch):
@@ -390,7 +390,7 @@ def polarizations_stream(approximant: str, batches: Iterable, freqs: torch.Tenso
 
     def forward(slot, t_c):
         if t_c is not None:
-            t_c = torch.as_tensor(t_c, dtype=real, device=device)
+            t_c = torch.as_tensor(t_c, dtype=real, device=device).resolve_neg()
             ops._require(t_c, "t_c", real)
             if t_c.numel() != batch:
                 raise ValueError("t_c must have one value per binary")
@@ -458,7 +458,7 @@ def likelihood_stream(approximant: str, batches: Iterable, freqs: torch.Tensor, 
         else:
             first = offsets[:-1].clamp(max=max(freqs.numel() - 1, 0))
             f_min = freqs[first].to(torch.float64)
-    f_min = f_min.to(device, torch.float64).contiguous()
+    f_min = ops.plain(f_min.to(device, torch.float64))
     rmf = float("nan") if reference_mf is None else float(reference_mf)
     lib = _lib.library()
     main_handle = torch.cuda.current_stream(device).cuda_stream
@@ -475,7 +475,7 @@ def likelihood_stream(approximant: str, batches: Iterable, freqs: torch.Tensor, 
                 and params.ndim == 2 and params.shape[1] == 8 and params.shape[0] > 0):
             ops._require(params, "params", torch.float64)
             raise ValueError("params must be (B, 8) with B > 0")
-        params = params.contiguous()
+        params = ops.plain(params)
         if not state:
             batch = params.shape[0]
             if f_min.numel() not in (1, batch):
@@ -505,7 +505,7 @@ def likelihood_stream(approximant: str, batches: Iterable, freqs: torch.Tensor, 
     def fused(slot, t_c):
         batch = state["batch"]
         if t_c is not None:
-            t_c = torch.as_tensor(t_c, dtype=torch.float32, device=device)
+            t_c = torch.as_tensor(t_c, dtype=torch.float32, device=device).resolve_neg()
             ops._require(t_c, "t_c", torch.float32)
             if t_c.numel() != batch:
                 raise ValueError("t_c must have one value per binary")

@@ -92,7 +92,7 @@ class _Polarizations(torch.autograd.Function):
         cdev = _compute_device(grid.device)
         real = grid.dtype
         precision = _lib.FP32 if real == torch.float32 else _lib.FP64
-        f = grid.detach().to(device=cdev).contiguous()
+        f = ops.plain(grid.detach().to(device=cdev))
         single = fields[0].ndim == 0
         n = 1 if single else fields[0].shape[0]
         needs = any(ctx.needs_input_grad[3:])
@@ -117,7 +117,7 @@ class _Polarizations(torch.autograd.Function):
                                                 reference_mf=options.reference_mf)
         tables = ops.setup(approximant, params, f_min, amp_scale=strain_scale(options),
                            reference_mf=options.reference_mf, precision=precision)
-        tc = None if t_c is None else t_c.detach().to(device=cdev, dtype=real).contiguous()
+        tc = None if t_c is None else ops.plain(t_c.detach().to(device=cdev, dtype=real))
         hp, hc = ops.polarizations(approximant, tables.table, f, None, tc)
         if (needs or ctx.needs_input_grad[2]) and xhm:
             # (IMRPhenomXHM: its backward takes the set-up's tangents itself)
@@ -155,7 +155,8 @@ class _Polarizations(torch.autograd.Function):
         def cot(g):
             if g is None:
                 return torch.zeros(shape, dtype=complex_dtype, device=table.device)
-            return g.to(device=table.device, dtype=complex_dtype).contiguous()
+            # (a loss with the strain under conj sends a conjugate view)
+            return ops.plain(g.to(device=table.device, dtype=complex_dtype))
 
         # PyTorch's gradient with respect to h is dL/dRe h + i dL/dIm h: the
         # kernels' cotangent convention
