@@ -310,3 +310,36 @@ def test_operations_refuse_lazy_views(cuda):
     a = ops.grid_vjp("IMRPhenomXAS", t.table, grid, None, None, g.conj(), g)
     b = ops.grid_vjp("IMRPhenomXAS", t.table, grid, None, None, g.conj().resolve_conj(), g)
     torch.testing.assert_close(a, b, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("approximant", ["IMRPhenomXAS", "IMRPhenomXHM"])
+@pytest.mark.parametrize("device", ["cuda", "cpu"])
+@pytest.mark.parametrize("batched", [False, True])
+def test_in_place_operations_on_the_strain(cuda, approximant, device, batched):
+    """A strain that requires a gradient can be masked, scaled and added to in
+    place, one binary's as a batch's, from a grid on either device: the
+    gradients of the same operations out of place."""
+    import torch
+
+    import waveformx_b200.torch as wt
+
+    rows = torch.tensor(BATCH if batched else ALIGNED, dtype=torch.float64, device=device)
+    grid = torch.linspace(20.0, 400.0, 120, dtype=torch.float64, device=device)
+    window = torch.hann_window(120, dtype=torch.float64, device=device)
+    f = wt.polarizations_function(approximant)
+    out = []
+    for in_place in (True, False):
+        x = rows.clone().requires_grad_(True)
+        hp, hc = f(binary_of(x), grid)
+        if in_place:
+            hp *= window
+            hp[..., grid < 50.0] = 0
+            hc.mul_(0.5).add_(hp)
+        else:
+            hp = torch.where(grid < 50.0, 0.0, hp * window)
+            hc = 0.5 * hc + hp
+        (hp.abs() ** 2).sum().backward(retain_graph=True)
+        hc.real.sum().backward()
+        out.append((hp.detach(), hc.detach(), x.grad))
+    for a, b in zip(*out):
+        torch.testing.assert_close(a, b, rtol=1e-12, atol=1e-12 * float(b.abs().max()))

@@ -81,6 +81,12 @@ def _compute_device(device: torch.device) -> torch.device:
     return torch.device("cuda", torch.cuda.current_device())
 
 
+def _no_view(t: torch.Tensor) -> torch.Tensor:
+    """``t``'s memory as a tensor that is no view: autograd refuses in-place
+    operations on a view that a Function returns (``hp *= window``)."""
+    return t.data
+
+
 class _Polarizations(torch.autograd.Function):
     """``(hplus, hcross)`` of the grid, ``t_c`` and the eight fields (each
     ``(n,)`` or ``(n, 3)``, batched; or one binary's, ``()`` or ``(3,)``, with
@@ -127,7 +133,7 @@ class _Polarizations(torch.autograd.Function):
             ctx.save_for_backward(tables.table, dtable, f, tc if tc is not None else f[:0], params, f_min)
         ctx.has_tc, ctx.ready, ctx.xhm = tc is not None, ready, xhm
         if single:
-            hp, hc = hp.view(-1), hc.view(-1)
+            hp, hc = _no_view(hp.view(-1)), _no_view(hc.view(-1))
         return hp.to(out_device), hc.to(out_device)
 
     @staticmethod
