@@ -343,3 +343,27 @@ def test_in_place_operations_on_the_strain(cuda, approximant, device, batched):
         out.append((hp.detach(), hc.detach(), x.grad))
     for a, b in zip(*out):
         torch.testing.assert_close(a, b, rtol=1e-12, atol=1e-12 * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_gradients_of_the_fields_are_tensors_of_their_own(cuda, batched):
+    """An in-place change of one field's ``.grad`` leaves the others as they
+    were, their use in another graph included."""
+    import torch
+
+    import waveformx_b200.torch as wt
+    import waveformx_b200 as wb
+
+    rows = np.asarray(BATCH if batched else ALIGNED)
+    fields = [torch.tensor(np.asarray(v), dtype=torch.float64, device=cuda, requires_grad=True) for v in binary_of(rows)]
+    hp, hc = wt.polarizations_function("IMRPhenomXAS")(wb.Binary(*fields), torch.linspace(20.0, 400.0, 65, dtype=torch.float64,
+                                                                                       device=cuda))
+    ((hp.abs() ** 2).sum() + hc.real.sum()).backward()
+    factor = torch.ones((), dtype=torch.float64, device=cuda, requires_grad=True)
+    held = [x.grad.clone() for x in fields]
+    total = sum((factor * x.grad).sum() for x in fields[1:])  # (keeps the gradients for factor's)
+    fields[0].grad.zero_()
+    total.backward()
+    assert all(torch.equal(x.grad, g) for x, g in zip(fields[1:], held[1:]))
+    torch.testing.assert_close(factor.grad, sum(g.sum() for g in held[1:]), rtol=1e-12, atol=0)
+    fields[2].grad.mul_(factor)  # (as of a tensor with a history)

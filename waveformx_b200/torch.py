@@ -185,7 +185,9 @@ class _Polarizations(torch.autograd.Function):
         if ctx.single:
             by_field = [g.view(3) if i in (2, 3) else g.view(()) for i, g in enumerate(by_field)]
         *by_field, by_tc = by_field
-        move = lambda g: g if g.device == ctx.out_device else g.to(ctx.out_device)  # noqa: E731
+        # (no views of the one buffer, whose version an in-place change of one
+        # field's .grad would move on for all)
+        move = lambda g: _no_view(g) if g.device == ctx.out_device else g.to(ctx.out_device)  # noqa: E731
         out = [None, None, grad_grid, move(by_tc) if (need[3] and ctx.has_tc) else None]
         out += [move(g) if need[4 + i] else None for i, g in enumerate(by_field)]
         return tuple(out)
