@@ -322,3 +322,15 @@ def test_match_of_conjugate_views(cuda, dtype):
         assert all(torch.equal(u, v) for u, v in zip(got, expected))
     got = wm.polarization_match(a.conj(), b.conj(), b, FREQUENCIES, lazy)
     assert torch.equal(got, wm.polarization_match(a.conj().resolve_conj(), b.conj().resolve_conj(), b, FREQUENCIES, psd))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64", "int64"])
+def test_grid_time_refuses_other_types(cuda, dtype):
+    """A series that is not complex holds half the bytes that the transform
+    reads: a TypeError."""
+    import torch
+
+    from waveformx_b200 import ops
+
+    with pytest.raises(TypeError, match="complex64"):
+        ops.match_grid_time(torch.zeros((2, 8192), dtype=getattr(torch, dtype), device=cuda), 2048, 0.25)

@@ -604,9 +604,9 @@ def grid_time_supported(n: int, n_fft: int, dtype: torch.dtype = torch.complex64
 def match_grid_time(series: torch.Tensor, n: int, delta_f: float) -> torch.Tensor:
     """The best time of each row's grid (largest ``|z|``) by the inverse FFT
     in shared memory, for ``series`` whose rows are zero from ``n`` on (see
-    :func:`grid_time_supported`; in the precision of ``series``): float64
-    ``(rows,)``."""
-    _require(series, "series", series.dtype)
+    :func:`grid_time_supported`; complex64, or complex128 with the transforms
+    in double): float64 ``(rows,)``."""
+    _require(series, "series", torch.complex128 if series.dtype == torch.complex128 else torch.complex64)
     rows, n_fft = series.shape
     t = torch.empty(rows, dtype=torch.float64, device=series.device)
     name = "wfx_match_grid_time" if series.dtype == torch.complex64 else "wfx_match_grid_time64"
