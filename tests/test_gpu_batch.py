@@ -171,3 +171,40 @@ def test_nonfinite_rows(cuda, dtype, n):
     offsets = torch.tensor([0, 0, *(n * (k + 1) for k in range(batch))], device=cuda)
     ragged = ops.nonfinite_rows(hp.reshape(-1), hc.reshape(-1), offsets, batch + 1).bool()
     assert torch.equal(ragged[1:], expected) and not ragged[0]
+
+
+def test_row_kernels_refuse_other_arguments(cuda):
+    """The kernels of rows check what they are given: types, shapes and
+    devices that would be read past their ends or as something else."""
+    import torch
+
+    from waveformx_b200 import ops
+
+    z = torch.zeros((3, 64), dtype=torch.complex64, device=cuda)
+    offsets = torch.tensor([0, 64, 128, 192], device=cuda)
+    for hp, hc, o, error in ((z.real.contiguous(), z.real.contiguous(), None, TypeError),
+                             (z, z.to(torch.complex128), None, TypeError), (z, z[:2], None, ValueError),
+                             (z[:2], z[:2], None, ValueError), (z.reshape(-1), z.reshape(-1), None, ValueError),
+                             (z.reshape(-1), z.reshape(-1), offsets[:-1], ValueError),
+                             (z.reshape(-1), z.reshape(-1), offsets.int(), TypeError)):
+        with pytest.raises(error):
+            ops.nonfinite_rows(hp, hc, o, 3)
+    one, spin = torch.ones(3, dtype=torch.float64, device=cuda), torch.zeros((3, 3), dtype=torch.float64, device=cuda)
+    good = [one, one, spin, spin, one, one, one, one]
+    freqs = torch.linspace(20.0, 40.0, 5, dtype=torch.float64, device=cuda)
+    params, f_min = ops.pack_params(good, freqs)
+    assert params.shape == (3, 8) and float(f_min) == 20.0
+    for k, bad, error in ((0, one.float(), TypeError), (1, one.cpu(), TypeError), (2, one, ValueError),
+                          (3, spin[:2], ValueError), (7, one[:2], ValueError)):
+        with pytest.raises(error):
+            ops.pack_params([bad if i == k else x for i, x in enumerate(good)], freqs)
+    with pytest.raises(TypeError):
+        ops.pack_params([x.to(torch.int64) for x in good], freqs.to(torch.int64))
+    with pytest.raises(ValueError):
+        ops.pack_params(good[:7], freqs)
+    for grad, dtype, error in ((torch.zeros((3, 8), device=cuda), torch.float32, ValueError),
+                               (torch.zeros((3, 9), device=cuda), torch.float64, TypeError),
+                               (torch.zeros((3, 9), device=cuda).double(), torch.float16, TypeError),
+                               (torch.zeros((3, 9), dtype=torch.float16, device=cuda), torch.float32, TypeError)):
+        with pytest.raises(error):
+            ops.unpack_gradient(grad, dtype)

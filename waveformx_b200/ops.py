@@ -246,10 +246,18 @@ def polarizations(approximant: str, table: torch.Tensor, freqs: torch.Tensor, of
 def nonfinite_rows(hp: torch.Tensor, hc: torch.Tensor, offsets: Optional[torch.Tensor], batch: int) -> torch.Tensor:
     """``(B,)`` int32: 1 where a binary's row of ``hp`` or ``hc`` (``(B, N)``,
     or flat with ``offsets``) holds a value that is not finite."""
-    _require(hp, "hp")
-    _require(hc, "hc", hp.dtype)
+    precision = _lib.FP64 if hp.dtype == torch.complex128 else _lib.FP32
+    complex_dtype = torch.complex64 if precision == _lib.FP32 else torch.complex128
+    _require(hp, "hp", complex_dtype)
+    _require(hc, "hc", complex_dtype)
+    if hc.shape != hp.shape or (offsets is None and (hp.ndim != 2 or hp.shape[0] != batch)):
+        raise ValueError(f"hp and hc must be ({batch}, N), or flat with offsets, got {tuple(hp.shape)} and "
+                         f"{tuple(hc.shape)}")
+    if offsets is not None:
+        _require(offsets, "offsets", torch.int64)
+        if offsets.numel() != batch + 1:
+            raise ValueError(f"offsets must have B + 1 = {batch + 1} entries")
     bad = torch.empty(batch, dtype=torch.int32, device=hp.device)
-    precision = _lib.FP32 if hp.dtype == torch.complex64 else _lib.FP64
     n = hp.shape[1] if offsets is None else hp.numel()
     _lib.check("wfx_nonfinite_rows", _lib.library().wfx_nonfinite_rows(
         precision, _ptr(hp), _ptr(hc), _ptr(offsets), batch, n, _ptr(bad), _stream(hp.device)))
@@ -471,8 +479,25 @@ _POINTERS, _STRIDES = ctypes.c_void_p * 8, ctypes.c_int64 * 8
 
 def pack_params(fields, freqs: torch.Tensor):
     """``(params, f_min)`` of a Binary's eight fields (CUDA tensors of the
-    dtype of ``freqs``: ``(n,)`` or one value, the spins ``(n, 3)`` or
-    ``(3,)``) in one launch: ``(n, 8)`` and ``(1,)`` float64."""
+    dtype of ``freqs``, float32 or float64: ``(n,)`` or one value, the spins
+    ``(n, 3)`` or ``(3,)``) in one launch: ``(n, 8)`` and ``(1,)`` float64,
+    ``f_min`` the first of ``freqs``."""
+    _require(freqs, "freqs", torch.float32 if freqs.dtype == torch.float32 else torch.float64)
+    if len(fields) != 8:
+        raise ValueError("a Binary has eight fields")
+    batch = fields[0].shape
+    if len(batch) > 1 or 0 in batch or freqs.numel() == 0:
+        raise ValueError("the fields must hold one value or a batch, the frequencies at least one")
+    for i, x in enumerate(fields):
+        if x.dtype != freqs.dtype or x.device != freqs.device:
+            raise TypeError(f"every field must be {freqs.dtype} on {freqs.device}, got {x.dtype} on {x.device}")
+        if x.shape != ((*batch, 3) if i in (2, 3) else batch):
+            raise ValueError(f"field {i} must be {tuple(batch)}, a spin with three components, got {tuple(x.shape)}")
+    return _pack_params(fields, freqs)
+
+
+def _pack_params(fields, freqs: torch.Tensor):
+    """:func:`pack_params` of fields that are as it asks."""
     batched = fields[0].ndim > 0
     batch = fields[0].shape[0] if batched else 1
     if any(map(torch.Tensor.is_neg, fields)):
@@ -493,6 +518,11 @@ def unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
     """The nine gradients of a Binary's fields and ``t_c`` (in the order of
     the fields, the spins ``(n, 3)``) in ``dtype`` from the ``(n, 9)`` rows,
     in one launch (views of one buffer)."""
+    _require(grad, "grad", torch.float32 if grad.dtype == torch.float32 else torch.float64)
+    if grad.ndim != 2 or grad.shape[1] != _lib.GRAD_COLUMNS:
+        raise ValueError(f"grad must be (n, {_lib.GRAD_COLUMNS})")
+    if dtype not in (torch.float32, grad.dtype):
+        raise TypeError(f"the gradients of {grad.dtype} rows are float32 or {grad.dtype}")
     n = grad.shape[0]
     out = torch.empty(13 * n, dtype=dtype, device=grad.device)
     code = lambda t: _lib.FP32 if t == torch.float32 else _lib.FP64  # noqa: E731

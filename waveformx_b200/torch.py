@@ -114,7 +114,7 @@ class _Polarizations(torch.autograd.Function):
             return hp, torch.zeros_like(hp)
         if grid.device != cdev:
             fields = [x.detach().to(device=cdev) for x in fields]
-        params, f_min = ops.pack_params(fields, f)
+        params, f_min = ops._pack_params(fields, f)
         dtable = ready = None
         if needs and not xhm:
             # (the derivatives of the tables on a second stream while the
