@@ -367,3 +367,33 @@ def test_gradients_of_the_fields_are_tensors_of_their_own(cuda, batched):
     assert all(torch.equal(x.grad, g) for x, g in zip(fields[1:], held[1:]))
     torch.testing.assert_close(factor.grad, sum(g.sum() for g in held[1:]), rtol=1e-12, atol=0)
     fields[2].grad.mul_(factor)  # (as of a tensor with a history)
+
+
+@pytest.mark.parametrize("needs", [False, True])
+@pytest.mark.parametrize("general", [False, True])
+def test_grids_of_another_rank(cuda, needs, general):
+    """A grid without an axis is an IndexError, and one whose first entry is
+    neither one frequency nor one a binary a ValueError, with tensors of one
+    type and with fields that are converted; a column is its frequencies."""
+    import torch
+
+    import waveformx_b200.torch as wt
+
+    f = wt.polarizations_function("IMRPhenomXAS")
+    grid = torch.linspace(20.0, 400.0, 60, dtype=torch.float64, device=cuda)
+    for rows in (BATCH, ALIGNED):
+        x = torch.tensor(rows, dtype=torch.float64, device=cuda, requires_grad=needs)
+        b = binary_of(x)
+        if general:
+            b = b._replace(luminosity_distance=500.0)
+        with pytest.raises(IndexError):
+            f(b, grid[0])
+        for shape in ((30, 2), (12, 5), (3, 20)):
+            with pytest.raises(ValueError, match="f_min"):
+                f(b, grid.reshape(shape))
+        for a, c in zip(f(b, grid.reshape(60, 1)), f(b, grid)):
+            assert a.shape == c.shape and torch.equal(a, c)
+    with pytest.raises(ValueError, match="f_min"):
+        from waveformx_b200 import ops
+
+        ops.setup_jvp_async("IMRPhenomXAS", torch.ones((3, 8), dtype=torch.float64, device=cuda), grid[:2])

@@ -452,6 +452,10 @@ def setup_jvp_async(approximant: str, params: torch.Tensor, f_min: torch.Tensor,
     _require(params, "params", torch.float64)
     _require(f_min, "f_min", torch.float64)
     batch = params.shape[0]
+    if params.ndim != 2 or params.shape[1] != 8 or batch == 0:
+        raise ValueError("params must be (B, 8) with B > 0")
+    if f_min.numel() not in (1, batch):
+        raise ValueError("f_min must have one value or one per binary")
     stride = 0 if f_min.numel() == 1 else 1
     device = params.device
     rmf = math.nan if reference_mf is None else float(reference_mf)

@@ -115,6 +115,10 @@ class _Polarizations(torch.autograd.Function):
         if grid.device != cdev:
             fields = [x.detach().to(device=cdev) for x in fields]
         params, f_min = ops._pack_params(fields, f)
+        if f.ndim != 1:
+            # (a grid of another rank: its first entry, as many frequencies as
+            # the set-up takes, or an error)
+            f_min = f[:1].to(torch.float64)
         dtable = ready = None
         if needs and not xhm:
             # (the derivatives of the tables on a second stream while the
