@@ -272,3 +272,40 @@ def test_fp32_reverse_pass_of_a_batch(cuda, model, n, batch):
         else:
             bar = 1e-2 * want.abs() + 1e-3 * want.abs().amax(1, keepdim=True)
         assert bool(((got - want).abs() <= bar).all()), ((got - want).abs() / bar).max()
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("n, batch", [(60, 3), (300, 1), (1001, 37), (129, 1000), (4017, 1), (20000, 5), (4001, 1021)])
+def test_fp64_reverse_pass_repeats(cuda, model, n, batch, monkeypatch):
+    """The FP64 vjp and fused likelihood of a shared grid repeat their bits,
+    with a binary's frequencies in one block, in a cluster of two to eight and
+    in parts that the workspace gathers, and without a workspace. The two ways
+    are the same sums in another order: 1e-8 of a binary's largest component
+    (the sums round to 1e-13 of their terms' magnitudes, which the contraction
+    cancels by less than 1e5)."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    rng = np.random.default_rng(n)
+    params = torch.as_tensor(draw_batch(rng, batch), device=cuda)
+    grid = torch.linspace(20.0, 900.0, n, dtype=torch.float64, device=cuda)
+    t = ops.setup(model, params, grid[:1], precision=_lib.FP64, jvp=True)
+    cot = [torch.randn((batch, n), dtype=torch.complex128, device=cuda) for _ in range(2)]
+    data, weights = torch.randn(n, dtype=torch.complex128, device=cuda), torch.rand(n, dtype=torch.float64, device=cuda)
+
+    def run():
+        loss, grad = ops.fused_loss(model, t.table, t.dtable, grid, None, None, data, weights)
+        alone, _ = ops.fused_loss(model, t.table, None, grid, None, None, data, weights)
+        return ops.vjp(model, t.table, t.dtable, grid, None, None, *cot), grad, loss[:, None], alone[:, None]
+
+    ways = []
+    for workspace in (ops.workspace, lambda *arguments: None):
+        monkeypatch.setattr(ops, "workspace", workspace)
+        first = run()
+        for _ in range(6):
+            assert all(torch.equal(a, b) for a, b in zip(run(), first))
+        assert torch.equal(first[2], first[3])
+        ways.append(first)
+    for a, b in zip(*ways):
+        assert bool(((a - b).abs() <= 1e-8 * b.abs().amax(1, keepdim=True)).all())

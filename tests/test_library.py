@@ -202,3 +202,19 @@ def test_reverse_pass_items_follow_the_batch():
     assert 2 * 4096 <= items(4096, 4017) < 2 * 4096 + 64
     assert 4 * 2048 <= items(2048, 4017) < 4 * 2048 + 64
     assert items(16, 4017) >= 8 * 16
+
+
+def test_reverse64_workspace():
+    """The FP64 reverse pass's optional workspace: none for what one block or
+    one wave of clusters holds, else ten values a binary and part, whose
+    number the blocks of a launch bound."""
+    from waveformx_b200 import _lib
+
+    size = _lib.library().wfx_reverse64_workspace_bytes
+    assert size(0, 100) == size(3, 0) == size(-1, 100) == 0
+    assert size(1, 1) == size(1, 128) == size(20000, 128) == 0
+    assert size(37, 1001) == 0 and size(1, 1024) == 0
+    assert size(1, 4017) == 32 * 80 and size(1, 60000) == 469 * 80
+    for batch in (1, 7, 100, 1021, 8192, 300000):
+        for n in (129, 4001, 100000, 5000000):
+            assert size(batch, n) <= 2 * 16 * 148 * 8 * 80

@@ -22,6 +22,7 @@
 //  * k_nonfinite_rows: which binaries' strain is not finite.
 //  * k_pack_params / k_unpack_gradient: a Binary's fields to the rows of
 //    parameters, the rows of gradients to the fields'.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -1572,9 +1573,11 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
 // span, 32 frequencies at a time: its value, the cotangents of its phase (in
 // the column of its region) and amplitude, and their sums against the rows as
 // matrix products. The sums of each binary wait in shared memory until the
-// block's last span, then its warp contracts them with dtable; with several
-// parts (few binaries) grad and loss, zeroed beforehand, add the parts'
-// atomically. Bound by latency and issue (20 warps a SM; the matrix pipe a
+// block's last span, then a warp contracts them with dtable. Several parts (few
+// binaries) add up in a fixed order, so that a call repeats its bits (their
+// atomic sums did not): with `partial` each part stores its contractions there
+// for k_sum_parts; without it a group's parts are a cluster, and a binary's
+// warp first adds their sums from the blocks' shared memory. Bound by latency and issue (20 warps a SM; the matrix pipe a
 // quarter busy). Measured against a block a binary with a register per sum and
 // lane (255 registers): IMRPhenomXAS vjp 149 us for 1021 x 4001 (243), the
 // fused likelihood 1512 us for 8192 x 8192 (3722); IMRPhenomD 182 (238) and
@@ -1583,7 +1586,10 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
 // first; one wave of blocks: 204.
 constexpr int kRevBlock = kSpan, kRevWarps = kRevBlock / 32;
 constexpr int kRevBinaries = 8;
-constexpr int64_t kRevBlocks = 4 * 4 * 148;  // blocks of a launch before a block takes several spans: four waves of four
+constexpr int64_t kRevBlocks = 16 * 148;  // blocks of a launch before a block takes several spans: about three waves
+                                          // of the five resident on a SM
+constexpr int kRevParts = 8;              // blocks of a cluster, at most (the portable size)
+constexpr int kPartColumns = kGradColumns + 1;  // of `partial`: the gradient's, the loss
 
 enum RevRow : int {
   R_M3 = 0, R_M2, R_M1, R_MT2, R_MT1, R_ONE, R_T, R_T2, R_F, R_FT, R_FT2, R_FF, R_LOG, R_TLOG, R_FLOG, R_Y, kRevRows,
@@ -1762,11 +1768,12 @@ __device__ __forceinline__ void add_past(const double* T, double* sums, double* 
 }
 static_assert(X_ATAN_W == X_ATAN_A + 2, "the arc tangents' four slots are contiguous");
 
-template <int MODEL, bool FUSED>
+// (CLUSTER: the parts of a group are a cluster)
+template <int MODEL, bool FUSED, bool CLUSTER>
 __global__ void __launch_bounds__(kRevBlock, 5)
     k_rev_f64(const double* __restrict__ table, const double* __restrict__ freqs, int64_t n, int64_t B, int per,
               const double* __restrict__ t_c, const double2* __restrict__ cot_hp, const double2* __restrict__ cot_hc,
-              FusedArgs fa, const double* __restrict__ dtable, double* grad, double* loss_out) {
+              FusedArgs fa, const double* __restrict__ dtable, double* grad, double* loss_out, double* partial) {
   __shared__ RevShared sh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const auto* data = static_cast<const double2*>(fa.data);
@@ -1901,20 +1908,36 @@ __global__ void __launch_bounds__(kRevBlock, 5)
       }
     }
   }
-  // each warp contracts its own binaries (the ones it summed): lane (r, d)
-  // takes the slots r + 4 i of direction d
-  const bool whole = gridDim.y == 1;
-  const auto put = [&](double* at, double v) {
-    if (whole) {
-      *at = v;
-    } else {
-      atomicAdd(at, v);
-    }
-  };
-  __syncwarp();
-  for (int j = warp; j < count; j += kRevWarps) {
+  // each warp contracts its own binaries (the ones it summed), or in a cluster
+  // of `parts` blocks part p's warps the binaries p, p + parts, ...: lane
+  // (r, d) takes the slots r + 4 i of direction d
+  const auto cluster = cooperative_groups::this_cluster();
+  const int parts = CLUSTER ? static_cast<int>(gridDim.y) : 1, part = CLUSTER ? static_cast<int>(blockIdx.y) : 0;
+  if constexpr (CLUSTER) {
+    cluster.sync();
+  } else {
+    __syncwarp();
+  }
+  for (int j = part + parts * warp; j < count; j += parts * kRevWarps) {
     const int64_t b = base + j;
     const double* sums = sh.sums[j];
+    double* at = grad != nullptr ? grad + b * kGradColumns : nullptr;
+    double* loss_at = loss_out != nullptr ? loss_out + b : nullptr;
+    if (!CLUSTER && partial != nullptr) {
+      at = partial + (blockIdx.y * B + b) * kPartColumns;
+      loss_at = at + kGradColumns;
+    }
+    if constexpr (CLUSTER) {
+      double* total = sh.stage[warp];
+      __syncwarp();
+      for (int k = lane; k < kTableStride; k += 32) {
+        double s = 0.0;
+        for (int p = 0; p < parts; ++p) s += cluster.map_shared_rank(&sh.sums[j][0], p)[k];
+        total[k] = s;
+      }
+      __syncwarp();
+      sums = total;
+    }
     if (grad != nullptr && dtable != nullptr) {
       const int d = lane & 7;
       double g = 0.0;
@@ -1925,11 +1948,30 @@ __global__ void __launch_bounds__(kRevBlock, 5)
       }
       g += __shfl_xor_sync(0xffffffffu, g, 8);
       g += __shfl_xor_sync(0xffffffffu, g, 16);
-      if (lane < kDirections) put(&grad[b * kGradColumns + lane], g);
+      if (lane < kDirections) at[lane] = g;
     }
-    if (grad != nullptr && lane == kDirections) put(&grad[b * kGradColumns + kDirections], sums[kSlotTc]);
-    if (loss_out != nullptr && lane == kDirections + 1) put(&loss_out[b], sums[kSlotLoss]);
+    if (grad != nullptr && lane == kDirections) at[kDirections] = sums[kSlotTc];
+    if (loss_out != nullptr && lane == kDirections + 1) *loss_at = sums[kSlotLoss];
   }
+  if constexpr (CLUSTER) cluster.sync();  // (the other blocks have read this one's sums)
+}
+
+// grad and loss (either may be null): a warp a binary and column, the parts'
+// contractions in a fixed order (lane l the parts l, l + 32, ...).
+__global__ void __launch_bounds__(kBlock) k_sum_parts(const double* __restrict__ partial, int64_t B, int parts,
+                                                      double* grad, double* loss_out) {
+  const int64_t i = (static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x) >> 5;
+  if (i >= B * kPartColumns) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t b = i / kPartColumns;
+  const int c = static_cast<int>(i % kPartColumns);
+  double* at = c < kGradColumns ? (grad != nullptr ? grad + b * kGradColumns + c : nullptr)
+                                : (loss_out != nullptr ? loss_out + b : nullptr);
+  if (at == nullptr) return;
+  double s = 0.0;
+  for (int p = lane; p < parts; p += 32) s += partial[p * B * kPartColumns + i];
+  s = warp_sum(s);
+  if (lane == 0) *at = s;
 }
 
 // The reverse mode on ragged grids: one binary per block.
@@ -2354,6 +2396,73 @@ int launch_adj_staged(const float* table, const float* freqs, int64_t n, int64_t
   return launched();
 }
 
+// How k_rev_f64 splits B binaries of n frequencies: `per` binaries a block,
+// as many as leave kRevBlocks blocks of one span, up to kRevBinaries; then
+// several spans a block, which cost it one contraction. Where a cluster's parts
+// give the same split and its blocks are a wave at most, the clusters are as
+// fast as k_sum_parts' second launch (XAS vjp 37 x 1001: 15.3 and 16.6 us;
+// 1000 x 129, in waves: 43 and 31): no workspace.
+struct RevShape {
+  int64_t groups, parts;
+  int per;
+  size_t bytes;  // of `partial`
+};
+RevShape rev_shape(int64_t B, int64_t n) {
+  const int64_t spans = (n + kSpan - 1) / kSpan;
+  RevShape r;
+  r.per = static_cast<int>(min(max(B * spans / kRevBlocks, int64_t(1)), static_cast<int64_t>(kRevBinaries)));
+  r.groups = (B + r.per - 1) / r.per;
+  const int64_t each = max(r.groups * spans / kRevBlocks, int64_t(1));
+  r.parts = min((spans + each - 1) / each, int64_t(65535));
+  const bool cluster = r.parts <= kRevParts && r.groups * r.parts <= kRevBlocks / 4;
+  r.bytes = cluster ? 0 : sizeof(double) * kPartColumns * static_cast<size_t>(B * r.parts);
+  if (r.parts == 1) r.bytes = 0;
+  return r;
+}
+
+// k_rev_f64, its parts' sums in `partial` where `bytes` hold them, else in
+// clusters: kRevParts parts at most, a power of two, and fewer binaries a block
+// for as many blocks (1, 2, or a multiple of its warps).
+template <int MODEL, bool FUSED>
+int launch_rev_f64(const double* table, const double* freqs, int64_t n, int64_t B, const double* t_c,
+                   const double2* cot_hp, const double2* cot_hc, FusedArgs fa, const double* dtable, double* grad,
+                   double* loss, void* partial, size_t bytes, cudaStream_t s) {
+  RevShape r = rev_shape(B, n);
+  const bool stored = r.bytes > 0 && partial != nullptr && bytes >= r.bytes &&
+                      (reinterpret_cast<uintptr_t>(partial) & 7u) == 0;
+  if (r.parts > 1 && !stored) {
+    const int64_t most = min((n + kSpan - 1) / kSpan, static_cast<int64_t>(kRevParts));
+    const int64_t per = B * most / kRevBlocks;
+    r.per = per >= kRevBinaries ? kRevBinaries : (per >= kRevWarps ? kRevWarps : (per >= 2 ? 2 : 1));
+    r.groups = (B + r.per - 1) / r.per;
+    r.parts = 1;
+    while (r.parts < most && r.parts * r.groups < kRevBlocks) r.parts *= 2;
+  }
+  if (r.groups > (int64_t(1) << 31) - 1) return WFX_EINVAL;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = cluster.val.clusterDim.z = 1;
+  cluster.val.clusterDim.y = static_cast<unsigned>(r.parts);
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(static_cast<unsigned>(r.groups), static_cast<unsigned>(r.parts));
+  config.blockDim = dim3(kRevBlock);
+  config.stream = s;
+  config.attrs = &cluster;
+  const bool clustered = !stored && r.parts > 1;
+  config.numAttrs = clustered ? 1 : 0;
+  const cudaError_t rc =
+      cudaLaunchKernelEx(&config, clustered ? k_rev_f64<MODEL, FUSED, true> : k_rev_f64<MODEL, FUSED, false>, table,
+                         freqs, n, B, r.per, t_c, cot_hp, cot_hc, fa, dtable, grad, loss,
+                         stored ? static_cast<double*>(partial) : nullptr);
+  if (rc != cudaSuccess) return static_cast<int>(rc);
+  if (stored) {
+    const int64_t warps = B * kPartColumns;
+    k_sum_parts<<<static_cast<unsigned>((warps + kBlock / 32 - 1) / (kBlock / 32)), kBlock, 0, s>>>(
+        static_cast<const double*>(partial), B, static_cast<int>(r.parts), grad, loss);
+  }
+  return launched();
+}
+
 // The stages of the FP32 reverse pass: the per-item sums (the reverse
 // kernel), their contraction with dtable, or both in turn.
 enum AdjointStage : int { kStagePartials = 1, kStageContract = 2, kStageAll = 3 };
@@ -2558,6 +2667,8 @@ size_t wfx_workspace_bytes(int op, int model, int precision, int64_t B, int64_t 
   return 0;
 }
 
+size_t wfx_reverse64_workspace_bytes(int64_t B, int64_t n) { return B <= 0 || n <= 0 ? 0 : rev_shape(B, n).bytes; }
+
 int wfx_grid_vjp(int model, const double* table, const double* freqs, const int64_t* offsets, int64_t B, int64_t n,
                  const double* t_c, const void* cot_hp, const void* cot_hc, double* grad_f, wfx_stream_t stream) {
   if (table == nullptr || freqs == nullptr || cot_hp == nullptr || cot_hc == nullptr || grad_f == nullptr || B <= 0 ||
@@ -2664,27 +2775,8 @@ static int adjoint_entry(bool fused, int model, int precision, const void* table
         }
         return launched();
       }
-      // (binaries a block: as many as leave kRevBlocks blocks of one span, up
-      // to kRevBinaries; then spans a block, which cost it one contraction)
-      const int64_t spans = (n + kSpan - 1) / kSpan;
-      const int per = static_cast<int>(min(max(B * spans / kRevBlocks, int64_t(1)), static_cast<int64_t>(kRevBinaries)));
-      const int64_t groups = (B + per - 1) / per;
-      const int64_t each = max(groups * spans / kRevBlocks, int64_t(1));
-      const int64_t parts = min((spans + each - 1) / each, int64_t(65535));
-      if (groups > (int64_t(1) << 31) - 1) return static_cast<int>(WFX_EINVAL);
-      if (parts > 1) {
-        cudaError_t zeroed = cudaSuccess;
-        if (G != nullptr) zeroed = cudaMemsetAsync(G, 0, sizeof(double) * kGradColumns * B, s);
-        if (zeroed == cudaSuccess && L != nullptr) zeroed = cudaMemsetAsync(L, 0, sizeof(double) * B, s);
-        if (zeroed != cudaSuccess) return static_cast<int>(zeroed);
-      }
-      const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(parts));
-      if (fused) {
-        k_rev_f64<M, true><<<grid, kRevBlock, 0, s>>>(T, F, n, B, per, TC, CP, CC, fa, dtable, G, L);
-      } else {
-        k_rev_f64<M, false><<<grid, kRevBlock, 0, s>>>(T, F, n, B, per, TC, CP, CC, fa, dtable, G, L);
-      }
-      return launched();
+      const auto launch = fused ? launch_rev_f64<M, true> : launch_rev_f64<M, false>;
+      return launch(T, F, n, B, TC, CP, CC, fa, dtable, G, L, workspace, workspace_bytes, s);
     });
   }
   if (precision != WFX_FP32) return WFX_EINVAL;
