@@ -309,3 +309,41 @@ def test_fp64_reverse_pass_repeats(cuda, model, n, batch, monkeypatch):
         ways.append(first)
     for a, b in zip(*ways):
         assert bool(((a - b).abs() <= 1e-8 * b.abs().amax(1, keepdim=True)).all())
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2", "IMRPhenomXHM"])
+def test_fp64_reverse_pass_beside_odd_frequencies(cuda, model):
+    """A frequency whose powers overflow where nothing reads them (above
+    IMRPhenomXAS's cutoff, infinity included; with a zero cotangent) leaves the
+    gradient of the others: the grid's without it, to 1e-9 of the largest
+    component (150 terms summed in another order, cancelling by less than 1e5).
+    One at which the waveform is not finite gives NaN."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    p = torch.tensor([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0]], dtype=torch.float64, device=cuda)
+    f_min = torch.tensor([20.0], dtype=torch.float64, device=cuda)
+    grid = torch.linspace(20.0, 900.0, 150, dtype=torch.float64, device=cuda)
+    g = torch.full((1, 150), 0.3 + 0.2j, dtype=torch.complex128, device=cuda)
+    rest = torch.arange(150, device=cuda) != 70
+    t = None if model == "IMRPhenomXHM" else ops.setup(model, p, f_min, precision=_lib.FP64, jvp=True)
+
+    def gradient(f, g):
+        if t is None:
+            return ops.xhm_vjp(p, f_min, f, None, None, g, g)
+        return ops.vjp(model, t.table, t.dtable, f, None, None, g, g)
+
+    expected = gradient(grid[rest], g[:, rest].contiguous())
+    cut = model == "IMRPhenomXAS"
+    for odd, weight in ((1e120, 0.0), (1e140, 0.0), (1e160, 0.0), (1e200, 0.0), (1e-104, 0.0),
+                        *(((1e160, 1.0), (float("inf"), 0.0), (float("inf"), 1.0)) if cut else ())):
+        f, w = grid.clone(), g.clone()
+        f[70] = odd
+        w[:, 70] *= weight
+        got = gradient(f, w)
+        assert bool(((got - expected).abs() <= 1e-9 * expected.abs().max()).all()), (odd, weight, got)
+    for odd in (0.0, -5.0, float("nan"), -float("inf"), *(() if cut else (float("inf"),))):
+        f = grid.clone()
+        f[70] = odd
+        assert bool(torch.isnan(gradient(f, g)).all()), odd

@@ -1606,7 +1606,7 @@ struct RevShared {
   double T[kRevBinaries][kTableStride];
   double sums[kRevBinaries][kTableStride];  // dL/d(table), kSlotTc, kSlotLoss
   double rows[kRevRows * kRowStride];
-  double m76[kSpan];
+  double f[kSpan], m76[kSpan];
   double stage[kRevWarps][kStage];
 };
 
@@ -1671,8 +1671,8 @@ __device__ __forceinline__ void add_products(double* sums, const double* stage, 
 }
 
 // The terms past the inspiral of one frequency a lane (pb, ab: the cotangents
-// of the phase and of the amplitude, zero for a lane without): eight columns
-// against the rows and eight against ones.
+// of the phase and of the amplitude): eight columns against the rows and eight
+// against ones.
 template <int MODEL>
 __device__ __forceinline__ void past_columns(const double* T, const Freq<double>& q, const Point<double>& pt, double ab,
                                              double pb, double (&v)[8], double (&w)[8]) {
@@ -1794,23 +1794,24 @@ __global__ void __launch_bounds__(kRevBlock, 5)
       const double mt1 = q.t2 * q.m1, m2 = q.m1 * q.m1;
       __syncthreads();  // (the last span's rows are read; the first: the tables are staged)
       constexpr bool kTf2 = MODEL == kModelTaylorF2;
-      r[R_M3 * kRowStride] = kTf2 ? q.lf : m2 * q.m1;
-      r[R_M2 * kRowStride] = kTf2 ? q.t * q.lf : (MODEL == kModelPhenomD ? q.f34 : m2);
-      r[R_M1 * kRowStride] = q.m1;
-      r[R_MT2 * kRowStride] = mt1 * mt1;
-      r[R_MT1 * kRowStride] = mt1;
+      r[R_M3 * kRowStride] = row_entry(kTf2 ? q.lf : m2 * q.m1);
+      r[R_M2 * kRowStride] = row_entry(kTf2 ? q.t * q.lf : (MODEL == kModelPhenomD ? q.f34 : m2));
+      r[R_M1 * kRowStride] = row_entry(q.m1);
+      r[R_MT2 * kRowStride] = row_entry(mt1 * mt1);
+      r[R_MT1 * kRowStride] = row_entry(mt1);
       r[R_ONE * kRowStride] = 1.0;
-      r[R_T * kRowStride] = q.t;
-      r[R_T2 * kRowStride] = q.t2;
-      r[R_F * kRowStride] = q.f;
-      r[R_FT * kRowStride] = q.f * q.t;
-      r[R_FT2 * kRowStride] = q.f * q.t2;
-      r[R_FF * kRowStride] = q.f * q.f;
-      r[R_LOG * kRowStride] = q.lf;
-      r[R_TLOG * kRowStride] = q.t * q.lf;
-      r[R_FLOG * kRowStride] = q.f * q.lf;
-      r[R_Y * kRowStride] = q.y;
-      sh.m76[i] = q.m76;
+      r[R_T * kRowStride] = row_entry(q.t);
+      r[R_T2 * kRowStride] = row_entry(q.t2);
+      r[R_F * kRowStride] = row_entry(q.f);
+      r[R_FT * kRowStride] = row_entry(q.f * q.t);
+      r[R_FT2 * kRowStride] = row_entry(q.f * q.t2);
+      r[R_FF * kRowStride] = row_entry(q.f * q.f);
+      r[R_LOG * kRowStride] = row_entry(q.lf);
+      r[R_TLOG * kRowStride] = row_entry(q.t * q.lf);
+      r[R_FLOG * kRowStride] = row_entry(q.f * q.lf);
+      r[R_Y * kRowStride] = row_entry(q.y);
+      sh.f[i] = q.f;
+      sh.m76[i] = row_m76(q.f, q.y, q.m76);
       __syncthreads();
     }
     double* stage = sh.stage[warp];
@@ -1828,7 +1829,7 @@ __global__ void __launch_bounds__(kRevBlock, 5)
         const bool in = i < length;
         const int64_t k = n0 + i;
         const double* r = sh.rows + i;
-        const double f = r[R_F * kRowStride];
+        const double f = sh.f[i];
         bool zero = false;
         if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, f > T[X_F_CUT]);
         if (zero && !FUSED) continue;
@@ -1869,8 +1870,10 @@ __global__ void __launch_bounds__(kRevBlock, 5)
           if (zero || !fa.grad) continue;
         }
         evaluated = true;
-        // (IMRPhenomXAS above its cutoff: nothing depends on the table)
+        // (IMRPhenomXAS above its cutoff: nothing depends on the table. A lane
+        // without a term is in no region, whatever its powers hold)
         const bool dead = !in || (MODEL == kModelXas && pt.amp == 0.0);
+        if (dead) pt.rp = pt.ra = -1;
         const double A = pt.amp, ap = gp.x * pt.c + gp.y * pt.s, ac = gc.y * pt.c - gc.x * pt.s;
         const double ab = dead ? 0.0 : kp * ap + kc * ac;
         const double pb = dead ? 0.0 : A * (kp * (gp.y * pt.c - gp.x * pt.s) - kc * (gc.x * pt.c + gc.y * pt.s));
@@ -1880,11 +1883,12 @@ __global__ void __launch_bounds__(kRevBlock, 5)
           put_columns(stage, {pb, pb * q.y, pb * q.f, w, 0.0, dead ? 0.0 : A * ap, dead ? 0.0 : A * ac, 0.0}, lane);
         } else {
           put_columns(stage, {pt.rp == 0 ? pb : 0.0, pt.rp == 1 ? pb : 0.0, pt.rp == 2 ? pb : 0.0, w,
-                              w * (t3 * t3 * q.t), dead ? 0.0 : A * ap, dead ? 0.0 : A * ac, 0.0}, lane);
+                              pt.ra == 0 ? w * (t3 * t3 * q.t) : 0.0, dead ? 0.0 : A * ap, dead ? 0.0 : A * ac, 0.0},
+                      lane);
         }
         mma_rows<kRevRows>(d1, sh.rows + c0, stage, lane);
         if constexpr (MODEL != kModelTaylorF2) {
-          if (__any_sync(0xffffffffu, !dead && (pt.rp > 0 || pt.ra > 0))) {
+          if (__any_sync(0xffffffffu, pt.rp > 0 || pt.ra > 0)) {
             past = true;
             double v[8], o[8];
             past_columns<MODEL>(T, q, pt, ab, pb, v, o);

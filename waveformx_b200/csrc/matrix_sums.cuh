@@ -18,6 +18,18 @@ constexpr int kRowStride = kSpan + 4;  // (doubles; = 4 mod 16: the fragments' l
 constexpr int kStageStride = 36;       // (32 frequencies a column, = 4 mod 16)
 constexpr int kStage = 8 * kStageStride;
 
+// An entry of the rows: zero where it is not finite, so that it adds nothing to
+// the sums of a column that is zero there (a power that overflows in a region
+// that does not read it). Where the value itself is not finite its columns are.
+__device__ __forceinline__ double row_entry(double x) { return isfinite(x) ? x : 0.0; }
+
+// f^-7/6 as the amplitudes take it beside such rows: NaN where f or f^-5/3 is
+// not finite (f <= 0, NaN, an infinity), since the powers read back from the
+// rows no longer say so.
+__device__ __forceinline__ double row_m76(double f, double y, double m76) {
+  return isfinite(f) && isfinite(y) ? m76 : NAN;
+}
+
 // d += a b of one 8 x 4 by 4 x 8 product: lane l holds a[l / 4][l % 4],
 // b[l % 4][l / 4] and d[l / 4][2 (l % 4) + {0, 1}].
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {

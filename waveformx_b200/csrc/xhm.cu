@@ -728,7 +728,8 @@ __device__ __forceinline__ void reverse_22(AdjShared& sh, const double* rows, in
   const double f = q.f, y = f - T[X_SHIFT];
   double d[3][2] = {};
   {
-    const double w = pt.ra == 0 ? ab * q.m76 : 0.0, t2 = q.t * q.t, t8 = t2 * t2 * t2 * t2;
+    const bool inspiral = !zero && pt.ra == 0;
+    const double w = inspiral ? ab * q.m76 : 0.0, t2 = q.t * q.t, t8 = inspiral ? t2 * t2 * t2 * t2 : 0.0;
     put_columns(stage, {pt.rp == 0 ? pb : 0.0, pt.rp == 1 ? pb : 0.0, pt.rp == 2 ? pb : 0.0, w, w * t8,
                         direct.im * h.re - direct.re * h.im, h.re, h.im}, lane);
     mma_rows<kRows>(d, rows, stage, lane);
@@ -784,11 +785,11 @@ __device__ __forceinline__ void reverse_22(AdjShared& sh, const double* rows, in
     shift -= ub * T[X_AMP_RD_S];
   }
   double d2[2][2] = {};
-  put_columns(stage, {w, w * (f * f), n, rd_n, rd_gr, ub * y, rd_g, shift}, lane);
+  put_columns(stage, {w, past && pt.ra == 1 ? w * (f * f) : 0.0, n, rd_n, rd_gr, past ? ub * y : 0.0, rd_g, shift}, lane);
   mma_rows<kRows>(d2, rows, stage, lane);
   double d3[1][2] = {};
-  put_columns(stage, {pt.rp == 1 ? at : 0.0, pt.rp == 2 ? at : 0.0, pt.rp == 1 ? gz * y : 0.0,
-                      pt.rp == 2 ? gz * y : 0.0, 0.0, 0.0, 0.0, 0.0}, lane);
+  put_columns(stage, {pt.rp == 1 ? at : 0.0, pt.rp == 2 ? at : 0.0, past && pt.rp == 1 ? gz * y : 0.0,
+                      past && pt.rp == 2 ? gz * y : 0.0, 0.0, 0.0, 0.0, 0.0}, lane);
   mma_ones(d3[0], stage, lane);
   put_products(stage, d2, lane);
   if (lane < 5) {
@@ -846,30 +847,30 @@ __global__ void __launch_bounds__(kXhmBlock, 4)
       }
       double* q = sh.rows + i;
       const double t2 = p.t * p.t, mt1 = t2 * p.m1, m2 = p.m1 * p.m1, ff = p.f * p.f, ft = p.f * p.t;
-      q[B_M3 * kRowStride] = m2 * p.m1;
-      q[B_M2 * kRowStride] = m2;
-      q[B_M4_3 * kRowStride] = p.m1 * mt1;
-      q[B_M1 * kRowStride] = p.m1;
-      q[B_M2_3 * kRowStride] = mt1 * mt1;
-      q[B_M1_3 * kRowStride] = mt1;
+      q[B_M3 * kRowStride] = row_entry(m2 * p.m1);
+      q[B_M2 * kRowStride] = row_entry(m2);
+      q[B_M4_3 * kRowStride] = row_entry(p.m1 * mt1);
+      q[B_M1 * kRowStride] = row_entry(p.m1);
+      q[B_M2_3 * kRowStride] = row_entry(mt1 * mt1);
+      q[B_M1_3 * kRowStride] = row_entry(mt1);
       q[B_1 * kRowStride] = 1.0;
-      q[B_1_3 * kRowStride] = p.t;
-      q[B_2_3 * kRowStride] = t2;
-      q[B_F * kRowStride] = p.f;
-      q[B_4_3 * kRowStride] = ft;
-      q[B_5_3 * kRowStride] = p.f * t2;
-      q[B_F2 * kRowStride] = ff;
-      q[B_7_3 * kRowStride] = ff * p.t;
-      q[B_LOG * kRowStride] = p.lf;
-      q[B_1_3_LOG * kRowStride] = p.t * p.lf;
-      q[B_F_LOG * kRowStride] = p.f * p.lf;
-      q[B_4_3_LOG * kRowStride] = ft * p.lf;
-      q[kRowY * kRowStride] = p.y;
+      q[B_1_3 * kRowStride] = row_entry(p.t);
+      q[B_2_3 * kRowStride] = row_entry(t2);
+      q[B_F * kRowStride] = row_entry(p.f);
+      q[B_4_3 * kRowStride] = row_entry(ft);
+      q[B_5_3 * kRowStride] = row_entry(p.f * t2);
+      q[B_F2 * kRowStride] = row_entry(ff);
+      q[B_7_3 * kRowStride] = row_entry(ff * p.t);
+      q[B_LOG * kRowStride] = row_entry(p.lf);
+      q[B_1_3_LOG * kRowStride] = row_entry(p.t * p.lf);
+      q[B_F_LOG * kRowStride] = row_entry(p.f * p.lf);
+      q[B_4_3_LOG * kRowStride] = row_entry(ft * p.lf);
+      q[kRowY * kRowStride] = row_entry(p.y);
       q[kRowG * kRowStride] = gp.re;
       q[(kRowG + 1) * kRowStride] = gp.im;
       q[(kRowG + 2) * kRowStride] = gc.re;
       q[(kRowG + 3) * kRowStride] = gc.im;
-      sh.m76[i] = p.m76;
+      sh.m76[i] = row_m76(p.f, p.y, p.m76);
       sh.h22r[i] = h22.re;
       sh.h22i[i] = h22.im;
       __syncthreads();
