@@ -393,11 +393,26 @@ __device__ __forceinline__ void block_z(const C (&c)[G][8], const double (&f0)[G
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
   if ((lane & 3) == 0) buffer[8 * warp + (lane >> 2)] = v[0];
   __syncthreads();
-  double total[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int w = 0; w < warps; ++w) {
+  // the warps' sums, in every warp alike: lane l takes the value l % 8 of the
+  // warps l / 8, l / 8 + 4, ..., with the roundings of the additions beside them
+  // (plain additions of a few large sums were most of z's error, which decides
+  // whether the last Newton step is taken)
+  double sum = 0.0, rest = 0.0;
+  const auto add = [&](double x) {
+    const double s = sum + x, y = s - sum;
+    rest += (sum - (s - y)) + (x - y);
+    sum = s;
+  };
+  for (int w = lane >> 3; w < warps; w += 4) add(buffer[8 * w + (lane & 7)]);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) total[i] += buffer[8 * w + i];
+  for (int o = 8; o < 32; o <<= 1) {
+    const double other = __shfl_xor_sync(0xffffffffu, sum, o);
+    rest += __shfl_xor_sync(0xffffffffu, rest, o);
+    add(other);
   }
+  double total[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) total[i] = __shfl_sync(0xffffffffu, sum + rest, i);
   constexpr double kTau = 2.0 * kPi;
   z[0] = total[0];
   z[1] = total[1];
