@@ -372,3 +372,43 @@ def test_refined_matches_are_as_accurate_as_a_warps(cuda):
         exact = np.hypot((re * wc - im * ws).sum(1), (re * ws + im * wc).sum(1)) / norm
         rms.append(float(np.sqrt(np.mean(((value.cpu().numpy() - exact) / exact) ** 2))))
     assert rms[0] <= 1.03 * rms[1], rms
+
+
+def test_matches_on_streams_and_threads(cuda):
+    """Calls of one shape on several streams and threads at a time keep their
+    series apart: the matches of the same calls one after the other."""
+    import threading
+
+    import torch
+
+    from waveformx_b200 import match as wm
+
+    n, rows = 4017, 200
+    f = 20.0 + 0.25 * np.arange(n)
+    w = torch.ones(n, dtype=torch.float64, device=cuda)
+    inputs = [[torch.randn((rows, n), dtype=torch.complex128, device=cuda) + 1.0 for _ in range(2)] for _ in range(3)]
+    expected = [wm.match(a, b, f, w, return_time=True) for a, b in inputs]
+    streams = [torch.cuda.Stream() for _ in range(wm._SERIES.STREAMS + 2)]
+    buffers = []
+    for s in streams:
+        with torch.cuda.stream(s):
+            buffers.append(wm._series_buffer(2, 2048, torch.complex64, cuda))
+    assert len({x.data_ptr() for x in buffers}) == len(streams) and len(wm._SERIES.kept) == wm._SERIES.STREAMS
+    torch.cuda.synchronize()
+    got = [[] for _ in inputs]
+
+    def calls(k):
+        with torch.cuda.stream(streams[k]):
+            for _ in range(8):
+                got[k].append(wm.match(*inputs[k], f, w, return_time=True))
+        streams[k].synchronize()
+
+    threads = [threading.Thread(target=calls, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(3):
+        assert len(got[k]) == 8
+        for value, t in got[k]:
+            assert torch.equal(value, expected[k][0]) and torch.equal(t, expected[k][1])

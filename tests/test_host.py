@@ -145,3 +145,27 @@ def test_offsets_and_per_frequency_checks():
         check_per_frequency(torch.zeros(39), "weights", 4, 10, False)
     with pytest.raises(ValueError, match="data"):
         check_per_frequency(torch.zeros(9), "data", 4, 10, True)
+
+
+def test_series_buffers_of_threads():
+    """A match's series buffer is kept from one call of a thread to its next,
+    a call of another shape replaces it, and a thread beside it has its own."""
+    import threading
+
+    import torch
+
+    from waveformx_b200 import match
+
+    first = match._series_buffer(2, 8, torch.complex64, "cpu")
+    assert match._series_buffer(2, 8, torch.complex64, "cpu") is first and not first.any()
+    others = []
+    threads = [threading.Thread(target=lambda: others.append(match._series_buffer(2, 8, torch.complex64, "cpu")))
+               for _ in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len({x.data_ptr() for x in (first, *others)}) == 4
+    other = match._series_buffer(3, 8, torch.complex64, "cpu")
+    assert other.shape == (3, 8) and match._series_buffer(3, 8, torch.complex64, "cpu") is other
+    assert match._series_buffer(2, 8, torch.complex64, "cpu") is not first

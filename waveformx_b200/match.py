@@ -27,6 +27,8 @@ refinement are FP64 either way).
 
 from __future__ import annotations
 
+import threading
+from collections import OrderedDict
 from typing import Optional, Tuple
 
 import torch
@@ -62,19 +64,38 @@ def inner_product(a: torch.Tensor, b: torch.Tensor, frequencies, psd) -> torch.T
     return 4 * delta_f * torch.sum((a * torch.conj(b)).real / s, dim=-1)
 
 
-_SERIES: dict = {}
+class _SeriesBuffers(threading.local):
+    """A thread's series buffers: each of its last streams' last one, by
+    device and stream."""
+
+    STREAMS = 4
+
+    def __init__(self):
+        self.kept = OrderedDict()
+
+    def clear(self):
+        self.kept.clear()
+
+
+_SERIES = _SeriesBuffers()
 
 
 def _series_buffer(rows: int, n_fft: int, dtype, device) -> torch.Tensor:
     """A ``(rows, n_fft)`` buffer whose columns from ``n`` stay zero: the
     kernels write only the first ``n`` of each row, so one zeroed buffer
-    per shape serves every call (the last one is kept)."""
-    key = (rows, n_fft, dtype, device)
-    buf = _SERIES.get(key)
-    if buf is None:
-        _SERIES.clear()
+    per shape serves every call of this thread on the current stream (each
+    stream's last one is kept; another thread's or stream's call, which may
+    run beside this one, has its own)."""
+    device = torch.device(device)
+    stream = torch._C._cuda_getCurrentRawStream(device.index) if device.type == "cuda" else None
+    kept = _SERIES.kept
+    buf = kept.pop((device, stream), None)
+    if buf is None or buf.shape != (rows, n_fft) or buf.dtype != dtype:
+        buf = None  # (the one before goes first)
         buf = torch.zeros((rows, n_fft), dtype=dtype, device=device)
-        _SERIES[key] = buf
+    kept[device, stream] = buf
+    while len(kept) > _SERIES.STREAMS:
+        kept.popitem(last=False)
     return buf
 
 
