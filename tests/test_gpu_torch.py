@@ -397,3 +397,41 @@ def test_grids_of_another_rank(cuda, needs, general):
         from waveformx_b200 import ops
 
         ops.setup_jvp_async("IMRPhenomXAS", torch.ones((3, 8), dtype=torch.float64, device=cuda), grid[:2])
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2", "IMRPhenomXHM"])
+def test_gradients_with_saved_tensor_hooks_and_on_other_streams(cuda, model):
+    """The gradients of a batch with its saved tensors moved to the host (the
+    set-up's derivatives, which a second stream forms, among them), and with
+    the whole call on another stream than the default, several calls under
+    way: those of the plain call, 1e-12 of a field's largest."""
+    import torch
+
+    import waveformx_b200.torch as wt
+
+    rng = np.random.default_rng(4)
+    m = np.sort(rng.uniform(10.0, 60.0, (2000, 2)))[:, ::-1]
+    x = torch.as_tensor(np.concatenate([m, np.zeros((2000, 2)), rng.uniform(-0.8, 0.8, (2000, 1)), np.zeros((2000, 2)),
+                                        rng.uniform(-0.8, 0.8, (2000, 1)), rng.uniform(100.0, 900.0, (2000, 1)),
+                                        rng.uniform(0.1, 3.0, (2000, 2)), np.full((2000, 1), 20.0)], 1), device=cuda)
+    grid = torch.linspace(20.0, 400.0, 33, dtype=torch.float64, device=cuda)
+    f = wt.polarizations_function(model)
+
+    def gradient(rows):
+        leaf = rows.clone().requires_grad_(True)
+        hp, hc = f(binary_of(leaf), grid)
+        return torch.autograd.grad((hp.abs() ** 2).sum() + hc.real.sum(), leaf)[0]
+
+    expected = [gradient(x), gradient(x[::2])]
+    with torch.autograd.graph.save_on_cpu():
+        got = [gradient(x), gradient(x[::2])]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for s in streams:
+            with torch.cuda.stream(s):
+                got += [gradient(x), gradient(x[::2])]
+    torch.cuda.synchronize()
+    for k, g in enumerate(got):
+        e = expected[k % 2]
+        assert bool(((g - e).abs() <= 1e-12 * e.abs().amax(0)).all())

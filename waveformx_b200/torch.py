@@ -134,6 +134,9 @@ class _Polarizations(torch.autograd.Function):
             ctx.save_for_backward(params, f_min, f, tc if tc is not None else f[:0])
         elif needs or ctx.needs_input_grad[2]:
             # (the grid's derivative: from the FP64 table of the parameters)
+            if ready is not None and torch._C._autograd._top_saved_tensors_default_hooks(False) is not None:
+                # (saved-tensor hooks read dtable on this stream, now)
+                torch.cuda.current_stream(cdev).wait_event(ready)
             ctx.save_for_backward(tables.table, dtable, f, tc if tc is not None else f[:0], params, f_min)
         ctx.has_tc, ctx.ready, ctx.xhm = tc is not None, ready, xhm
         if single:
