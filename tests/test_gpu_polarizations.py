@@ -264,3 +264,31 @@ def test_fp32_ragged_items(cuda, model, batch):
             largest = torch.zeros(batch, dtype=torch.float64, device=cuda)
             largest.scatter_reduce_(0, rows, b.abs(), "amax")
             assert bool(((a - b).abs() <= 2e-4 * largest[rows]).all())
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("batch, n", [(2401, 257), (1203, 4001), (19001, 1), (2368, 256), (4800, 300)])
+def test_fp64_forward_of_groups(cuda, model, batch, n):
+    """The FP64 forward on a shared grid with two to sixteen binaries a block,
+    a last group short of them, odd lengths, t_c and a refused binary: every
+    row is the same binary's evaluated alone, bit for bit."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    base = torch.tensor([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0], [60.0, 15.0, 0.8, 0.5, 1000.0, 2.5, 4.0, 20.0],
+                         [9.0, 7.0, -0.6, 0.2, 200.0, 1.1, 0.3, 20.0], [150.0, 90.0, 0.1, 0.4, 800.0, 0.4, 2.0, 20.0],
+                         [float("nan"), 7.0, -0.6, 0.2, 200.0, 1.1, 0.3, 20.0]], dtype=torch.float64, device=cuda)
+    grid = torch.linspace(20.0, 900.0, n, dtype=torch.float64, device=cuda)
+    t_c = torch.tensor([0.01, -0.02, 0.0, 0.3, 0.1], dtype=torch.float64, device=cuda)
+    table = ops.setup(model, base, grid[:1], precision=_lib.FP64).table
+    of = (torch.arange(batch, device=cuda) * 7 + torch.arange(batch, device=cuda) // 5) % 5
+    for tc in (t_c, None):
+        got = ops.polarizations(model, table[of].contiguous(), grid, None, None if tc is None else tc[of].contiguous())
+        for row in range(5):
+            alone = ops.polarizations(model, table[row:row + 1].contiguous(), grid, None,
+                                      None if tc is None else tc[row:row + 1])
+            for a, b in zip(got, alone):
+                a, b = torch.view_as_real(a[of == row]), torch.view_as_real(b)
+                assert bool(((a == b) | (torch.isnan(a) & torch.isnan(b))).all())
+                assert bool(torch.isnan(b).any()) == (row == 4)
