@@ -66,7 +66,7 @@ def _stream(device: torch.device):
 
 
 def _require(t: torch.Tensor, name: str, dtype=None):
-    if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
+    if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise TypeError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype != dtype:
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
@@ -82,7 +82,9 @@ def plain(t: torch.Tensor) -> torch.Tensor:
     """``t`` as contiguous memory that holds its values: a conjugate or
     negative view, which is contiguous but negates as it is read, written
     out."""
-    return t.resolve_conj().resolve_neg().contiguous()
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t.contiguous()
 
 
 def workspace(op: int, model: int, precision: int, batch: int, n: int, ragged: bool,
