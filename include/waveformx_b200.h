@@ -182,10 +182,11 @@ int wfx_grid_vjp(int model, const double* table, const double* freqs, const int6
  * d (mass_1, mass_2, chi_1, chi_2, luminosity_distance, inclination,
  * phi_ref, f_ref, t_c) for the cotangents cot_hp, cot_hc (complex128, dL/dRe
  * h + i dL/dIm h, the layout of wfx_xhm_polarizations) of the FP64
- * evaluation: forward-mode derivatives of the evaluation along each column
- * of dtable (B x WFX_XHM_STRIDE64 x 8 double: d table / d parameter, the
- * caller's), contracted with the cotangents. Grids as
- * wfx_xhm_polarizations. */
+ * evaluation: the sums of dL/d(table) over the frequencies, contracted with
+ * dtable (B x WFX_XHM_STRIDE64 x 8 double: d table / d parameter, the
+ * caller's). Grids as wfx_xhm_polarizations. The blocks that share a long
+ * binary add their parts in the order in which they finish: the last bits of
+ * a call may differ from those of the one before. */
 int wfx_xhm_vjp(const double* table, const double* dtable, const double* freqs, const int64_t* offsets, int64_t B,
                 int64_t n, int64_t max_len, const double* t_c, const void* cot_hp, const void* cot_hc, double* grad,
                 wfx_stream_t stream);
@@ -206,7 +207,7 @@ int wfx_phase_difference(int model, const double* params, int64_t B, const doubl
  *   WFX_FP32: table float, freqs float, t_c float, hp/hc complex64: FP32
  *     with double-float phase;
  *   WFX_FP64: table double, freqs double, t_c double, hp/hc complex128: the
- *     plain FP64 form (one binary per block).
+ *     plain FP64 form.
  * The FP32 ragged form (offsets != NULL) runs one persistent launch over
  * (binary, tile) work items whose index lives in the workspace
  * (wfx_workspace_bytes(WFX_OP_POLARIZATIONS, ...)); the other forms need no

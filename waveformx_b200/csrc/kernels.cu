@@ -1577,13 +1577,15 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
 // binaries) add up in a fixed order, so that a call repeats its bits (their
 // atomic sums did not): with `partial` each part stores its contractions there
 // for k_sum_parts; without it a group's parts are a cluster, and a binary's
-// warp first adds their sums from the blocks' shared memory. Bound by latency and issue (20 warps a SM; the matrix pipe a
-// quarter busy). Measured against a block a binary with a register per sum and
-// lane (255 registers): IMRPhenomXAS vjp 149 us for 1021 x 4001 (243), the
-// fused likelihood 1512 us for 8192 x 8192 (3722); IMRPhenomD 182 (238) and
-// 2901 (3588), TaylorF2 69 (89) and 996 (1293; 1243 with both tiles of rows);
-// one binary of 4017 frequencies 14.4 (60). Four blocks a SM: 161 us for the
-// first; one wave of blocks: 204.
+// warp first adds their sums from the blocks' shared memory. Bound by latency
+// and issue (45 % of the slots at 16 warps a SM, the matrix pipe 31 % busy).
+// Measured, the call, against a block a binary with a register per sum and
+// lane (255 registers): IMRPhenomXAS vjp 148 us for 1021 x 4001 (243), the fused
+// likelihood 1537 us for 8192 x 8192 (3722); IMRPhenomD 185 (238) and 2930
+// (3588), TaylorF2 71 (89) and 1014 (1293); one binary of 4017 frequencies 14.5
+// to 16.5 (60). 1 to 3 % of these are the parts' order and the entries that are
+// not finite. In clusters, without the workspace: 30.9 us for one binary of 4017
+// frequencies, 293 for 1021 x 4001 (176 on the same draw).
 constexpr int kRevBlock = kSpan, kRevWarps = kRevBlock / 32;
 constexpr int kRevBinaries = 8;
 constexpr int64_t kRevBlocks = 16 * 148;  // blocks of a launch before a block takes several spans: about three waves

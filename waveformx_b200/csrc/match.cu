@@ -305,9 +305,11 @@ __global__ void __launch_bounds__(kMatchBlock) k_match_refine(const typename Cpl
 // group's first frequency f_0 (exact, as k_match_refine's) and d = 32 delta_f,
 //   z = sum b p, sum f w = sum b (f_0 p + d R p'),
 //   sum f^2 w = sum b (f_0^2 p + 2 f_0 d R p' + d^2 (R p' + R^2 p'')).
-// Bound by FP64 issue (the pipe 53 % busy at 12 warps a SM): complex64 rows of
-// 4017 terms, 4096 of them 132 us (163 with a warp a row), 500 22.7 (61), one
-// 10.4 (35); 300 rows of 12000 53 (174). (Two groups a lane in single: 148.)
+// Bound by FP64 issue (the pipe 51 % busy at 12 warps a SM): complex64 rows of
+// 4017 terms, 4096 of them 136 us (163 with a warp a row), 500 24 (61), one 10.4
+// (35); 300 rows of 12000 51 (174). (Two groups a lane in single: 148.) z's
+// error, and with it the times', is below the other kernel's: 1.47e-16 and
+// 6.0e-12 s rms over 4000 rows of 4017 (1.54e-16 and 6.4e-12).
 template <class R>
 struct RefineShape;
 // (kGroups x 8 terms of a lane in 64 registers; blocks of up to kThreads)

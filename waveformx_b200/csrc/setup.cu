@@ -326,10 +326,8 @@ __global__ void __launch_bounds__(kWholeBlock, MIN_BLOCKS) k_setup_whole(const d
 // to 1024 binaries, a mode a block 102 to 112; 58 to 64 us (98 at 4096) with
 // the amplitudes apart from the phases, the amplitudes' collocation points as
 // divided differences and the powers of constants as numbers. The tangents:
-// 154 us at 250 binaries, 223 at 1024, 726 at 4096, from 394, 720 and 2053
-// (four dual-number directions rather than eight besides). (The duals do not
-// write the values too: a form that did, saving the values' launch, did not
-// come to an end on the device, though its host build did.)
+// 154 us at 250 binaries, 230 at 1024, 724 at 4096, from 394, 720 and 2053
+// (four dual-number directions rather than eight besides).
 constexpr int kXhmSetupBlock = 64;
 constexpr int kXhmParts = 9;
 

@@ -365,7 +365,7 @@ __device__ __forceinline__ void xhm_dual_sum(const Dual* T, const Dual* t0_lm, c
 // 32 frequencies, in 12 registers a lane). With a register per sum and lane
 // instead, the kernel held 255 registers, two blocks a SM: 856 us for 250 x
 // 4017 against 439 (705 held to 128 registers), and 2156 for the eight
-// directions on dual numbers. Bound by latency: 16 warps a SM issue in 28 % of
+// directions on dual numbers. Bound by latency: 15 warps a SM issue in 35 % of
 // the cycles (instruction fetch, the elementary functions' chains, the
 // barriers between the stages).
 constexpr int kAdjSpan = kSpan;

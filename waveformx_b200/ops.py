@@ -313,9 +313,10 @@ def xhm_modes(table: torch.Tensor, freqs: torch.Tensor, t_c: Optional[torch.Tens
 def xhm_dtable(params: torch.Tensor, f_min: torch.Tensor, *, amp_scale: float = 1e21,
                reference_mf: Optional[float] = None) -> torch.Tensor:
     """IMRPhenomXHM's ``d table / d params`` ``(B, 544, 8)`` float64 of its
-    FP64 row: its set-up on dual numbers (one thread per binary, part and
-    parameter); zero along ``f_ref`` where ``f_ref = 0`` (the first frequency
-    or ``reference_mf / M`` then stands for it, as in the reference)."""
+    FP64 row: its set-up on dual numbers (a part of the row per block, a
+    parameter per thread); zero along ``f_ref`` where ``f_ref = 0`` (the
+    first frequency or ``reference_mf / M`` then stands for it, as in the
+    reference)."""
     _require(params, "params", torch.float64)
     _require(f_min, "f_min", torch.float64)
     batch = params.shape[0]
@@ -338,9 +339,8 @@ def xhm_vjp(params: torch.Tensor, f_min: torch.Tensor, freqs: torch.Tensor, offs
     (mass_1, mass_2, chi_1, chi_2, luminosity_distance, inclination, phi_ref,
     f_ref, t_c) for the cotangents ``dL/dRe h + i dL/dIm h`` of (hplus,
     hcross), from the FP64 evaluation on ``freqs`` (float64; ragged with
-    ``offsets``): its forward-mode derivatives along the set-up's tangents
-    (the set-up on dual numbers, :func:`xhm_dtable`), contracted with the
-    cotangents in the kernel."""
+    ``offsets``): the reverse pass over the modes, its sums contracted with
+    the set-up's tangents (:func:`xhm_dtable`) in the kernel."""
     _require(params, "params", torch.float64)
     _require(freqs, "freqs", torch.float64)
     tables = setup("IMRPhenomXHM", params, f_min, amp_scale=amp_scale, reference_mf=reference_mf,
