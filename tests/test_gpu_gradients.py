@@ -347,3 +347,49 @@ def test_fp64_reverse_pass_beside_odd_frequencies(cuda, model):
         f = grid.clone()
         f[70] = odd
         assert bool(torch.isnan(gradient(f, g)).all()), odd
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("kind", ["band", "above", "odd"])
+def test_fp64_shared_grids_are_not_finite_where_ragged_ones_are_not(cuda, model, kind):
+    """Refused binaries (a zero distance, a mass ratio beyond the fits, spins
+    above one, a NaN mass) and odd frequencies (infinities, NaN, zero, a
+    negative one) on a shared grid, in the band and wholly above
+    IMRPhenomXAS's cutoffs, against the same rows as a ragged grid (the kernels
+    of a binary a block): strain, vjp, likelihood and its gradient are NaN in
+    the same places, and equal elsewhere (strain 1e-12 of a row's largest;
+    sums 1e-9, as the module's other comparison of the two)."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    base = np.array([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0], [36.0, 29.0, 0.3, -0.1, 0.0, 0.7, 1.2, 20.0],
+                     [1500.0, 1.0, 0.0, 0.0, 500.0, 0.7, 1.2, 20.0], [36.0, 29.0, 1.5, -0.1, 500.0, 0.7, 1.2, 20.0],
+                     [np.nan, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0], [60.0, 15.0, 0.8, 0.5, 1000.0, 2.5, 4.0, 20.0]])
+    n, batch = 300, 6 * 400
+    f = np.linspace(20.0, 900.0, n) if kind != "above" else np.linspace(3000.0, 4500.0, n)
+    if kind == "odd":
+        f[[7, 90]], f[200:264] = (0.0, -5.0), np.inf
+        f[130] = np.nan
+    grid = torch.as_tensor(f, device=cuda)
+    t = ops.setup(model, torch.as_tensor(base, device=cuda), torch.tensor([20.0], dtype=torch.float64, device=cuda),
+                  precision=_lib.FP64, jvp=True)
+    of = torch.arange(batch, device=cuda) % 6
+    rng = np.random.default_rng(0)
+    g = torch.as_tensor(rng.normal(size=(6, n)) + 1j * rng.normal(size=(6, n)), device=cuda)
+    w = torch.as_tensor(rng.uniform(0.5, 2.0, n), device=cuda)
+    offsets = torch.arange(7, device=cuda) * n
+    table, dtable = t.table[of].contiguous(), t.dtable[of].contiguous()
+    for rows, tab, dtab in ((torch.arange(6, device=cuda), t.table, t.dtable), (of, table, dtable)):
+        shared = [*ops.polarizations(model, tab, grid), ops.vjp(model, tab, dtab, grid, None, None, *(g[rows].contiguous(),) * 2),
+                  *ops.fused_loss(model, tab, dtab, grid, None, None, g[0].contiguous(), w)]
+        ragged = [*(h.reshape(6, n) for h in ops.polarizations(model, t.table, grid.repeat(6), offsets)),
+                  ops.vjp(model, t.table, t.dtable, grid.repeat(6), offsets, None, *(g.reshape(-1),) * 2),
+                  *ops.fused_loss(model, t.table, t.dtable, grid.repeat(6), offsets, None, g[0].repeat(6), w.repeat(6))]
+        for k, (a, b) in enumerate(zip(shared, ragged)):
+            a, b = (torch.view_as_real(x) if x.is_complex() else x for x in (a, b[rows]))
+            assert torch.equal(torch.isnan(a), torch.isnan(b)), k
+            a, b = torch.nan_to_num(a, 0.0, 0.0, 0.0).flatten(1 if a.ndim > 1 else 0), torch.nan_to_num(b, 0.0, 0.0, 0.0).flatten(
+                1 if b.ndim > 1 else 0)
+            scale = b.abs().amax(1, keepdim=True) if b.ndim > 1 else b.abs()
+            assert bool(((a - b).abs() <= (1e-12 if k < 2 else 1e-9) * scale).all()), k

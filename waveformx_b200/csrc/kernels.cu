@@ -1448,6 +1448,10 @@ constexpr int kF64Binaries = 16;       // binaries per block, at most
 constexpr int64_t kF64Blocks = 1184;   // blocks of a launch before a block takes more than one binary: two waves
                                        // of four blocks a SM
 
+// f as a warp compares it with the XAS cutoff before it evaluates nothing: an
+// infinite frequency is above every cutoff, but its phase is not a number.
+__device__ __forceinline__ double above_cutoff(double f) { return isinf(f) ? NAN : f; }
+
 template <int MODEL>
 __global__ void __launch_bounds__(kBlock, 3) k_fwd_f64_shared(const double* __restrict__ table,
                                                               const double* __restrict__ freqs, int64_t n, int64_t B,
@@ -1464,6 +1468,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_fwd_f64_shared(const double* __re
     const bool in = n0 + threadIdx.x < n;
     const int64_t i = in ? n0 + threadIdx.x : n0;
     const Freq<double> q = freq_powers(freqs[i]);
+    const double f_above = above_cutoff(q.f);
     double2* out_p = hp + base * n + i;
     double2* out_c = hc + base * n + i;
 #pragma unroll 1
@@ -1472,7 +1477,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_fwd_f64_shared(const double* __re
       const double kp = T[slot_kp<MODEL>()], kc = T[slot_kc<MODEL>()];
       double2 vp, vc;
       bool zero = false;
-      if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, q.f > T[X_F_CUT]);
+      if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, f_above > T[X_F_CUT]);
       if (zero) {
         // (0 kp, 0 kc: NaN for a refused binary, as the evaluated form)
         vp = make_double2(0.0 * kp, 0.0 * kp);
@@ -1833,7 +1838,7 @@ __global__ void __launch_bounds__(kRevBlock, 5)
         const double* r = sh.rows + i;
         const double f = sh.f[i];
         bool zero = false;
-        if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, f > T[X_F_CUT]);
+        if constexpr (MODEL == kModelXas) zero = __all_sync(0xffffffffu, above_cutoff(f) > T[X_F_CUT]);
         if (zero && !FUSED) continue;
         double2 gp = make_double2(0.0, 0.0), gc = gp;
         if (!FUSED && in) {
@@ -1946,14 +1951,18 @@ __global__ void __launch_bounds__(kRevBlock, 5)
     }
     if (grad != nullptr && dtable != nullptr) {
       const int d = lane & 7;
+      // (a refused binary's tangents may not be finite where nothing is summed)
+      const bool every = isnan(sh.T[j][slot_kp<MODEL>()]);
       double g = 0.0;
 #pragma unroll 6
       for (int k = lane >> 3; k < kTableStride; k += 4) {
         const double s = sums[k];
-        if (k != kSlotTc && k != kSlotLoss && s != 0.0) g += s * dtable[(b * kTableStride + k) * kDirections + d];
+        if (k != kSlotTc && k != kSlotLoss && (s != 0.0 || every)) g += s * dtable[(b * kTableStride + k) * kDirections + d];
       }
       g += __shfl_xor_sync(0xffffffffu, g, 8);
       g += __shfl_xor_sync(0xffffffffu, g, 16);
+      // (nor has a loss that is not finite a gradient)
+      if (FUSED) g += 0.0 * sums[kSlotLoss];
       if (lane < kDirections) at[lane] = g;
     }
     if (grad != nullptr && lane == kDirections) at[kDirections] = sums[kSlotTc];
