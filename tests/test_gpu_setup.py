@@ -108,3 +108,29 @@ def test_jvp_same_in_small_and_large_batches(cuda, model):
         small = _setup(cuda, MODELS[model], params[lo:lo + 16], np.full(16, 20.0), jvp=True)
         for a, b in ((small.table, big.table), (small.dtable, big.dtable), (small.status, big.status)):
             np.testing.assert_array_equal(a.cpu().numpy(), b[lo:lo + 16].cpu().numpy())
+
+
+def test_set_up_on_the_second_stream_of_another_device(cuda, monkeypatch):
+    """The dual-number set-up on its device's second stream is launched with
+    that device current, whichever the caller's is (a device index of the
+    caller's own stands in for a second device)."""
+    import torch
+
+    from waveformx_b200 import ops
+
+    entered = []
+
+    class Guard(torch.cuda.device):
+        def __enter__(self):
+            entered.append(self.idx)
+            return super().__enter__()
+
+    p = torch.tensor([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0]], dtype=torch.float64, device=cuda)
+    f_min = torch.tensor([20.0], dtype=torch.float64, device=cuda)
+    expected, event = ops.setup_jvp_async("IMRPhenomXAS", p, f_min)
+    event.synchronize()
+    monkeypatch.setattr(torch.cuda, "device", Guard)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 7)
+    dtable, event = ops.setup_jvp_async("IMRPhenomXAS", p, f_min)
+    event.synchronize()
+    assert cuda.index in entered and torch.equal(dtable, expected)

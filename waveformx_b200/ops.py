@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+from contextlib import nullcontext
 from dataclasses import dataclass
 from typing import Optional
 
@@ -471,9 +472,11 @@ def setup_jvp_async(approximant: str, params: torch.Tensor, f_min: torch.Tensor,
     side = _side_stream(device)
     side.wait_stream(torch.cuda.current_stream(device))
     dtable = out if out is not None else torch.empty((batch, _lib.TABLE_STRIDE, 8), dtype=torch.float64, device=device)
-    _lib.check("wfx_setup_jvp", _lib.library().wfx_setup_jvp(
-        model, _ptr(params), batch, _ptr(f_min), stride, float(amp_scale), rmf, None, None, _ptr(dtable), None,
-        side.cuda_stream))
+    # (a launch on a stream of another device than the current one is refused)
+    with nullcontext() if torch.cuda.current_device() == device.index else torch.cuda.device(device):
+        _lib.check("wfx_setup_jvp", _lib.library().wfx_setup_jvp(
+            model, _ptr(params), batch, _ptr(f_min), stride, float(amp_scale), rmf, None, None, _ptr(dtable), None,
+            side.cuda_stream))
     event = side.record_event()
     if out is None:
         # (allocated on the current stream, used on the second: not reused
