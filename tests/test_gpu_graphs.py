@@ -132,3 +132,35 @@ def test_likelihood_capture_refusals(cuda):
         captured(np.zeros((3, 8)))
     with pytest.raises(TypeError):
         captured(draw_batch(np.random.default_rng(1), 4), t_c=torch.zeros(4, device=cuda))
+
+
+@pytest.mark.parametrize("n, batch", [(100, 3), (1001, 37), (4017, 9)])
+def test_fp64_reverse_pass_in_a_graph(cuda, n, batch):
+    """The FP64 likelihood and vjp captured, with a binary's frequencies in a
+    block, a cluster and the workspace's parts: a replay on new parameters
+    gives the bits of the call."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    rng = np.random.default_rng(n)
+    params = torch.as_tensor(draw_batch(rng, batch), device=cuda)
+    other = torch.as_tensor(draw_batch(rng, batch), device=cuda)
+    grid = torch.linspace(20.0, 900.0, n, dtype=torch.float64, device=cuda)
+    data, w = torch.randn(n, dtype=torch.complex128, device=cuda), torch.rand(n, dtype=torch.float64, device=cuda)
+    g = torch.randn((batch, n), dtype=torch.complex128, device=cuda)
+
+    def run():
+        t = ops.setup("IMRPhenomXAS", params, grid[:1], precision=_lib.FP64, jvp=True)
+        return (*ops.fused_loss("IMRPhenomXAS", t.table, t.dtable, grid, None, None, data, w),
+                ops.vjp("IMRPhenomXAS", t.table, t.dtable, grid, None, None, g, g))
+
+    run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run()
+    params.copy_(other)
+    graph.replay()
+    got = [x.clone() for x in captured]
+    assert all(torch.equal(a, b) for a, b in zip(got, run()))
