@@ -130,7 +130,7 @@ def test_set_up_on_the_second_stream_of_another_device(cuda, monkeypatch):
     expected, event = ops.setup_jvp_async("IMRPhenomXAS", p, f_min)
     event.synchronize()
     monkeypatch.setattr(torch.cuda, "device", Guard)
-    monkeypatch.setattr(torch.cuda, "current_device", lambda: 7)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 7)
     dtable, event = ops.setup_jvp_async("IMRPhenomXAS", p, f_min)
     event.synchronize()
     assert cuda.index in entered and torch.equal(dtable, expected)

@@ -430,6 +430,7 @@ def fused_loss(approximant: str, table: torch.Tensor, dtable: Optional[torch.Ten
     return loss, grad
 
 
+_HERE = nullcontext()
 _SIDE_STREAMS: dict = {}
 
 
@@ -473,7 +474,7 @@ def setup_jvp_async(approximant: str, params: torch.Tensor, f_min: torch.Tensor,
     side.wait_stream(torch.cuda.current_stream(device))
     dtable = out if out is not None else torch.empty((batch, _lib.TABLE_STRIDE, 8), dtype=torch.float64, device=device)
     # (a launch on a stream of another device than the current one is refused)
-    with nullcontext() if torch.cuda.current_device() == device.index else torch.cuda.device(device):
+    with _HERE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device):
         _lib.check("wfx_setup_jvp", _lib.library().wfx_setup_jvp(
             model, _ptr(params), batch, _ptr(f_min), stride, float(amp_scale), rmf, None, None, _ptr(dtable), None,
             side.cuda_stream))
@@ -535,6 +536,11 @@ def unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
         raise ValueError(f"grad must be (n, {_lib.GRAD_COLUMNS})")
     if dtype not in (torch.float32, grad.dtype):
         raise TypeError(f"the gradients of {grad.dtype} rows are float32 or {grad.dtype}")
+    return _unpack_gradient(grad, dtype)
+
+
+def _unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
+    """:func:`unpack_gradient` of rows that are as it asks."""
     n = grad.shape[0]
     out = torch.empty(13 * n, dtype=dtype, device=grad.device)
     code = lambda t: _lib.FP32 if t == torch.float32 else _lib.FP64  # noqa: E731
