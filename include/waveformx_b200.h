@@ -320,7 +320,7 @@ size_t wfx_workspace_bytes(int op, int model, int precision, int64_t B, int64_t 
 /* The workspace with which wfx_vjp and wfx_fused_loss in WFX_FP64 on a shared
  * grid spread a binary's frequencies over as many blocks as the device has
  * room for (0: a block holds them). It is optional, as every workspace of the
- * FP64 forms: with less, clusters of at most eight blocks share a binary's
+ * FP64 forms: with less, clusters of at most sixteen blocks share a binary's
  * frequencies. Either way a call's bits repeat. */
 size_t wfx_reverse64_workspace_bytes(int64_t B, int64_t n);
 

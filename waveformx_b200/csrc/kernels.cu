@@ -1589,13 +1589,14 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
 // likelihood 1537 us for 8192 x 8192 (3722); IMRPhenomD 185 (238) and 2930
 // (3588), TaylorF2 71 (89) and 1014 (1293); one binary of 4017 frequencies 14.5
 // to 16.5 (60). 1 to 3 % of these are the parts' order and the entries that are
-// not finite. In clusters, without the workspace: 30.9 us for one binary of 4017
-// frequencies, 293 for 1021 x 4001 (176 on the same draw).
+// not finite. In clusters, without the workspace: 24 us for one binary of 4017
+// frequencies, 222 for 1021 x 4001 (178 on the same draw; 31 and 293 in clusters
+// of eight with more and smaller blocks).
 constexpr int kRevBlock = kSpan, kRevWarps = kRevBlock / 32;
 constexpr int kRevBinaries = 8;
 constexpr int64_t kRevBlocks = 16 * 148;  // blocks of a launch before a block takes several spans: about three waves
                                           // of the five resident on a SM
-constexpr int kRevParts = 8;              // blocks of a cluster, at most (the portable size)
+constexpr int kRevParts = 16;             // blocks of a cluster, at most
 constexpr int kPartColumns = kGradColumns + 1;  // of `partial`: the gradient's, the loss
 
 enum RevRow : int {
@@ -2414,9 +2415,9 @@ int launch_adj_staged(const float* table, const float* freqs, int64_t n, int64_t
 // How k_rev_f64 splits B binaries of n frequencies: `per` binaries a block,
 // as many as leave kRevBlocks blocks of one span, up to kRevBinaries; then
 // several spans a block, which cost it one contraction. Where a cluster's parts
-// give the same split and its blocks are a wave at most, the clusters are as
-// fast as k_sum_parts' second launch (XAS vjp 37 x 1001: 15.3 and 16.6 us;
-// 1000 x 129, in waves: 43 and 31): no workspace.
+// (of the portable eight at most) give the same split and its blocks are a wave
+// at most, the clusters are as fast as k_sum_parts' second launch (XAS vjp 37 x
+// 1001: 15.3 and 16.6 us; 1000 x 129, in waves: 35 to 43 and 31): no workspace.
 struct RevShape {
   int64_t groups, parts;
   int per;
@@ -2429,15 +2430,41 @@ RevShape rev_shape(int64_t B, int64_t n) {
   r.groups = (B + r.per - 1) / r.per;
   const int64_t each = max(r.groups * spans / kRevBlocks, int64_t(1));
   r.parts = min((spans + each - 1) / each, int64_t(65535));
-  const bool cluster = r.parts <= kRevParts && r.groups * r.parts <= kRevBlocks / 4;
+  const bool cluster = r.parts <= 8 && r.groups * r.parts <= kRevBlocks / 4;
   r.bytes = cluster ? 0 : sizeof(double) * kPartColumns * static_cast<size_t>(B * r.parts);
   if (r.parts == 1) r.bytes = 0;
   return r;
 }
 
+// The blocks of a cluster that the device takes of k_rev_f64: kRevParts where
+// it has that many SMs beside one another (allowed once per device), else the
+// portable eight.
+template <int MODEL, bool FUSED>
+int rev_cluster(int* most) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices] = {};
+  int dev = 0;
+  cudaError_t rc = cudaGetDevice(&dev);
+  if (rc != cudaSuccess) return static_cast<int>(rc);
+  *most = dev >= 0 && dev < kDevices ? known[dev].load() : 0;
+  if (*most > 0) return 0;
+  const auto kernel = k_rev_f64<MODEL, FUSED, true>;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(1, kRevParts);
+  config.blockDim = dim3(kRevBlock);
+  int size = 0;
+  rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (rc == cudaSuccess) rc = cudaOccupancyMaxPotentialClusterSize(&size, kernel, &config);
+  if (rc != cudaSuccess) return static_cast<int>(rc);
+  *most = size >= kRevParts ? kRevParts : 8;
+  if (dev >= 0 && dev < kDevices) known[dev].store(*most);
+  return 0;
+}
+
 // k_rev_f64, its parts' sums in `partial` where `bytes` hold them, else in
-// clusters: kRevParts parts at most, a power of two, and fewer binaries a block
-// for as many blocks (1, 2, or a multiple of its warps).
+// clusters: a power of two parts, and as many binaries a block (1, 2, or a
+// multiple of its warps) as leave a wave of blocks, since a span costs a block
+// little more for eight binaries than for one.
 template <int MODEL, bool FUSED>
 int launch_rev_f64(const double* table, const double* freqs, int64_t n, int64_t B, const double* t_c,
                    const double2* cot_hp, const double2* cot_hc, FusedArgs fa, const double* dtable, double* grad,
@@ -2446,9 +2473,11 @@ int launch_rev_f64(const double* table, const double* freqs, int64_t n, int64_t 
   const bool stored = r.bytes > 0 && partial != nullptr && bytes >= r.bytes &&
                       (reinterpret_cast<uintptr_t>(partial) & 7u) == 0;
   if (r.parts > 1 && !stored) {
-    const int64_t most = min((n + kSpan - 1) / kSpan, static_cast<int64_t>(kRevParts));
-    const int64_t per = B * most / kRevBlocks;
-    r.per = per >= kRevBinaries ? kRevBinaries : (per >= kRevWarps ? kRevWarps : (per >= 2 ? 2 : 1));
+    int blocks = 0;
+    if (int rc = rev_cluster<MODEL, FUSED>(&blocks)) return rc;
+    const int64_t most = min((n + kSpan - 1) / kSpan, static_cast<int64_t>(blocks));
+    const int64_t per = 3 * B * most / kRevBlocks;
+    r.per = per > kRevWarps ? kRevBinaries : (per > 2 ? kRevWarps : (per == 2 ? 2 : 1));
     r.groups = (B + r.per - 1) / r.per;
     r.parts = 1;
     while (r.parts < most && r.parts * r.groups < kRevBlocks) r.parts *= 2;
