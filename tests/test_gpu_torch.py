@@ -435,3 +435,33 @@ def test_gradients_with_saved_tensor_hooks_and_on_other_streams(cuda, model):
     for k, g in enumerate(got):
         e = expected[k % 2]
         assert bool(((g - e).abs() <= 1e-12 * e.abs().amax(0)).all())
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_host_inputs_take_one_copy_back_of_the_gradient(cuda, batched, monkeypatch):
+    """With a grid and a binary on the host, a call copies the two strains
+    back, and its backward the fields' gradients in one copy (each waits for
+    the device)."""
+    import torch
+
+    import waveformx_b200 as wb
+    import waveformx_b200.torch as wt
+
+    fields = [torch.tensor(np.asarray(v), dtype=torch.float64, requires_grad=True)
+              for v in binary_of(np.asarray(BATCH if batched else ALIGNED))]
+    f = wt.polarizations_function("IMRPhenomXAS")
+    grid = torch.linspace(20.0, 400.0, 65, dtype=torch.float64)
+    copies, to = [], torch.Tensor.to
+
+    def counted(self, *args, **kw):
+        out = to(self, *args, **kw)
+        if self.is_cuda and not out.is_cuda:
+            copies.append(out.shape)
+        return out
+
+    monkeypatch.setattr(torch.Tensor, "to", counted)
+    hp, hc = f(wb.Binary(*fields), grid)
+    assert len(copies) == 2
+    gradients = torch.autograd.grad((hp.abs() ** 2).sum() + hc.real.sum(), fields)
+    assert len(copies) == 3
+    assert all(g.device.type == "cpu" and g.shape == x.shape for g, x in zip(gradients, fields))

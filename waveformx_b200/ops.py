@@ -539,13 +539,16 @@ def unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
     return _unpack_gradient(grad, dtype)
 
 
-def _unpack_gradient(grad: torch.Tensor, dtype: torch.dtype):
-    """:func:`unpack_gradient` of rows that are as it asks."""
+def _unpack_gradient(grad: torch.Tensor, dtype: torch.dtype, device: Optional[torch.device] = None):
+    """:func:`unpack_gradient` of rows that are as it asks; the fields'
+    gradients on ``device`` (one copy)."""
     n = grad.shape[0]
     out = torch.empty(13 * n, dtype=dtype, device=grad.device)
     code = lambda t: _lib.FP32 if t == torch.float32 else _lib.FP64  # noqa: E731
     _lib.check("wfx_unpack_gradient", _lib.library().wfx_unpack_gradient(
         code(grad.dtype), code(dtype), _ptr(grad), n, _ptr(out), _stream(grad.device)))
+    if device is not None:
+        out = out.to(device)
     m1, m2, s1, s2, *rest = out.split([n, n, 3 * n, 3 * n, n, n, n, n, n])
     return [m1, m2, s1.view(n, 3), s2.view(n, 3), *rest]
 

@@ -188,15 +188,14 @@ class _Polarizations(torch.autograd.Function):
                                reference_mf=options.reference_mf)
         else:
             grad = ops.vjp(approximant, table, dtable, f, None, tc, cot(g_hp), cot(g_hc))
-        by_field = ops._unpack_gradient(grad, f.dtype)
+        by_field = ops._unpack_gradient(grad, f.dtype, ctx.out_device)
         if ctx.single:
             by_field = [g.view(3) if i in (2, 3) else g.view(()) for i, g in enumerate(by_field)]
         *by_field, by_tc = by_field
         # (no views of the one buffer, whose version an in-place change of one
         # field's .grad would move on for all)
-        move = _no_view if f.device == ctx.out_device else (lambda g: g.to(ctx.out_device))  # noqa: E731
-        out = [None, None, grad_grid, move(by_tc) if (need[3] and ctx.has_tc) else None]
-        out += [move(g) if need[4 + i] else None for i, g in enumerate(by_field)]
+        out = [None, None, grad_grid, _no_view(by_tc) if (need[3] and ctx.has_tc) else None]
+        out += [_no_view(g) if need[4 + i] else None for i, g in enumerate(by_field)]
         return tuple(out)
 
 
