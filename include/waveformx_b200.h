@@ -317,12 +317,12 @@ int wfx_pipeline_likelihood_run(wfx_pipeline_t pipeline, int model, int64_t K, c
  * form reads or writes outside its buffers whatever the offsets hold. */
 size_t wfx_workspace_bytes(int op, int model, int precision, int64_t B, int64_t n, int ragged);
 
-/* The workspace with which wfx_vjp and wfx_fused_loss in WFX_FP64 on a shared
- * grid spread a binary's frequencies over as many blocks as the device has
- * room for (0: a block holds them). It is optional, as every workspace of the
- * FP64 forms: with less, clusters of at most sixteen blocks share a binary's
+/* The workspace with which wfx_vjp and wfx_fused_loss of `model` in WFX_FP64 on
+ * a shared grid spread a binary's frequencies over as many blocks as the device
+ * has room for (0: a block holds them). It is optional, as every workspace of
+ * the FP64 forms: with less, clusters of at most sixteen blocks share a binary's
  * frequencies. Either way a call's bits repeat. */
-size_t wfx_reverse64_workspace_bytes(int64_t B, int64_t n);
+size_t wfx_reverse64_workspace_bytes(int model, int64_t B, int64_t n);
 
 /* The offsets check of the last FP32 ragged call (wfx_polarizations,
  * wfx_vjp, wfx_fused_loss, wfx_fused_loss_partials, wfx_autotune_ragged)

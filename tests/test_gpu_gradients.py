@@ -312,7 +312,8 @@ def test_fp64_reverse_pass_repeats(cuda, model, n, batch, monkeypatch):
 
 
 @pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2", "IMRPhenomXHM"])
-def test_fp64_reverse_pass_beside_odd_frequencies(cuda, model):
+@pytest.mark.parametrize("batch", [1, 2000])
+def test_fp64_reverse_pass_beside_odd_frequencies(cuda, model, batch):
     """A frequency whose powers overflow where nothing reads them (above
     IMRPhenomXAS's cutoff, infinity included; with a zero cotangent) leaves the
     gradient of the others: the grid's without it, to 1e-9 of the largest
@@ -322,10 +323,10 @@ def test_fp64_reverse_pass_beside_odd_frequencies(cuda, model):
 
     from waveformx_b200 import _lib, ops
 
-    p = torch.tensor([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0]], dtype=torch.float64, device=cuda)
+    p = torch.tensor([[36.0, 29.0, 0.3, -0.1, 500.0, 0.7, 1.2, 20.0]], dtype=torch.float64, device=cuda).repeat(batch, 1)
     f_min = torch.tensor([20.0], dtype=torch.float64, device=cuda)
     grid = torch.linspace(20.0, 900.0, 150, dtype=torch.float64, device=cuda)
-    g = torch.full((1, 150), 0.3 + 0.2j, dtype=torch.complex128, device=cuda)
+    g = torch.full((batch, 150), 0.3 + 0.2j, dtype=torch.complex128, device=cuda)
     rest = torch.arange(150, device=cuda) != 70
     t = None if model == "IMRPhenomXHM" else ops.setup(model, p, f_min, precision=_lib.FP64, jvp=True)
 
@@ -393,3 +394,35 @@ def test_fp64_shared_grids_are_not_finite_where_ragged_ones_are_not(cuda, model,
                 1 if b.ndim > 1 else 0)
             scale = b.abs().amax(1, keepdim=True) if b.ndim > 1 else b.abs()
             assert bool(((a - b).abs() <= (1e-12 if k < 2 else 1e-9) * scale).all()), k
+
+
+@pytest.mark.parametrize("model", ["IMRPhenomXAS", "IMRPhenomD", "TaylorF2"])
+@pytest.mark.parametrize("n, batch", [(65, 3), (300, 40), (2049, 1), (2080, 3), (2175, 70), (4017, 51), (700, 600), (257, 1001)])
+def test_fp64_reverse_pass_against_a_binary_a_block(cuda, model, n, batch):
+    """The FP64 vjp and fused likelihood of a shared grid where four or two
+    warps share a binary's span, with a last group of one, where a warp takes a
+    binary, and where a block does, at remainders of spans and of a warp's
+    frequencies, against the same rows as a ragged grid (a binary a block): the
+    same sums in another order, 1e-8 of a binary's largest component (they
+    round to 1e-13 of their terms' magnitudes, which the contraction cancels
+    by less than 1e5)."""
+    import torch
+
+    from waveformx_b200 import _lib, ops
+
+    rng = np.random.default_rng(n)
+    params = torch.as_tensor(draw_batch(rng, batch), device=cuda)
+    grid = torch.linspace(20.0, 900.0, n, dtype=torch.float64, device=cuda)
+    t = ops.setup(model, params, grid[:1], precision=_lib.FP64, jvp=True)
+    t_c = torch.as_tensor(rng.uniform(-0.1, 0.1, batch), device=cuda)
+    cot = [torch.randn((batch, n), dtype=torch.complex128, device=cuda) for _ in range(2)]
+    w = torch.rand((batch, n), dtype=torch.float64, device=cuda)
+    offsets = torch.arange(batch + 1, device=cuda) * n
+    flat = (t.table, t.dtable, grid.repeat(batch), offsets, t_c)
+    shared = [ops.vjp(model, t.table, t.dtable, grid, None, t_c, *cot),
+              *ops.fused_loss(model, t.table, t.dtable, grid, None, t_c, cot[0], w, antenna=(0.6, -0.3), scale=-0.5)]
+    ragged = [ops.vjp(model, *flat, *(c.reshape(-1) for c in cot)),
+              *ops.fused_loss(model, *flat, cot[0].reshape(-1), w.reshape(-1), antenna=(0.6, -0.3), scale=-0.5)]
+    for a, b in zip(shared, ragged):
+        scale = b.abs().amax(1, keepdim=True) if b.ndim > 1 else b.abs()
+        assert bool(((a - b).abs() <= 1e-8 * scale).all())

@@ -205,16 +205,18 @@ def test_reverse_pass_items_follow_the_batch():
 
 
 def test_reverse64_workspace():
-    """The FP64 reverse pass's optional workspace: none for what one block or
-    one wave of clusters holds, else ten values a binary and part, whose
+    """The FP64 reverse pass's optional workspace: none for what one block of
+    a binary or of a span takes, else ten values a binary and part, whose
     number the blocks of a launch bound."""
     from waveformx_b200 import _lib
 
     size = _lib.library().wfx_reverse64_workspace_bytes
-    assert size(0, 100) == size(3, 0) == size(-1, 100) == 0
-    assert size(1, 1) == size(1, 128) == size(20000, 128) == 0
-    assert size(37, 1001) == 0 and size(1, 1024) == 0
-    assert size(1, 4017) == 32 * 80 and size(1, 60000) == 469 * 80
-    for batch in (1, 7, 100, 1021, 8192, 300000):
-        for n in (129, 4001, 100000, 5000000):
-            assert size(batch, n) <= 2 * 16 * 148 * 8 * 80
+    for model in (_lib.XAS, _lib.PHENOMD, _lib.TAYLORF2):
+        assert size(model, 0, 100) == size(model, 3, 0) == size(model, -1, 100) == 0
+        assert size(model, 1, 1) == size(model, 1, 128) == size(model, 20000, 128) == 0
+        assert size(model, 37, 257) == 0  # (a wave of blocks with a binary each)
+        assert size(model, 1, 4017) == 32 * 80 and size(model, 1, 60000) == 469 * 80
+        for batch in (1, 7, 100, 1021, 8192, 300000):
+            for n in (129, 4001, 100000, 5000000):
+                assert size(model, batch, n) <= 2 * 16 * 148 * 8 * 80
+    assert size(_lib.XHM, 1, 4017) == 0

@@ -57,7 +57,7 @@ EXPORTS = {
     "wfx_polarizations": (_INT, [_INT, _INT, _P, _P, _P, _I64, _I64, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "wfx_workspace_bytes": (ctypes.c_size_t, [_INT, _INT, _INT, _I64, _I64, _INT]),
     "wfx_ragged_status": (_INT, [_P, _P]),
-    "wfx_reverse64_workspace_bytes": (ctypes.c_size_t, [_I64, _I64]),
+    "wfx_reverse64_workspace_bytes": (ctypes.c_size_t, [_INT, _I64, _I64]),
     "wfx_vjp": (_INT, [_INT, _INT, _P, _P, _P, _P, _I64, _I64, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "wfx_fused_loss": (_INT, [_INT, _INT, _P, _P, _P, _P, _I64, _I64, _P, _P, _INT, _P, _INT, _D, _D, _D, _P, _P,
                               _P, ctypes.c_size_t, _P]),

@@ -18,7 +18,7 @@
 //  * k_contract: per binary, the FP64 sum of its tiles' partial sums and the
 //    product with dtable: the gradient in the parameters.
 //  * k_fwd_f64_shared, k_fwd_f64_ragged: the same in FP64.
-//  * k_rev_f64, k_adj_f64_ragged: the reverse-mode pass in FP64.
+//  * k_rev_f64, k_adj_f64: the reverse-mode pass in FP64.
 //  * k_nonfinite_rows: which binaries' strain is not finite.
 //  * k_pack_params / k_unpack_gradient: a Binary's fields to the rows of
 //    parameters, the rows of gradients to the fields'.
@@ -1584,18 +1584,21 @@ __global__ void __launch_bounds__(kBlock) k_grid_vjp(const double* __restrict__ 
 // for k_sum_parts; without it a group's parts are a cluster, and a binary's
 // warp first adds their sums from the blocks' shared memory. Bound by latency
 // and issue (45 % of the slots at 16 warps a SM, the matrix pipe 31 % busy).
-// Measured, the call, against a block a binary with a register per sum and
-// lane (255 registers): IMRPhenomXAS vjp 148 us for 1021 x 4001 (243), the fused
-// likelihood 1537 us for 8192 x 8192 (3722); IMRPhenomD 185 (238) and 2930
-// (3588), TaylorF2 71 (89) and 1014 (1293); one binary of 4017 frequencies 14.5
-// to 16.5 (60). 1 to 3 % of these are the parts' order and the entries that are
-// not finite. In clusters, without the workspace: 24 us for one binary of 4017
-// frequencies, 222 for 1021 x 4001 (178 on the same draw; 31 and 293 in clusters
-// of eight with more and smaller blocks).
+// Measured, the call, against k_adj_f64 (a block a binary, a register per sum
+// and lane, 255 registers), which takes the small batches of few frequencies
+// (rev_small): IMRPhenomXAS vjp 151 us for 1021 x 4001 (243), the fused
+// likelihood 1558 us for 8192 x 8192 (3722); IMRPhenomD 187 (238) and 2930
+// (3588), TaylorF2 72 (89) and 1015 (1293); one binary of 4017 frequencies 12.4
+// (63). 1 to 3 % of these are the parts' order and the entries that are not
+// finite. One or two binaries a block share its warps: 1 x 4017 16.5 us with a
+// warp a binary, 100 x 4017 33 (52, with blocks of one binary, three of its four
+// warps idle). In clusters, without the workspace: 16.5 us for one binary of 4017
+// frequencies, 223 for 1021 x 4001 (178 on the same draw).
 constexpr int kRevBlock = kSpan, kRevWarps = kRevBlock / 32;
 constexpr int kRevBinaries = 8;
 constexpr int64_t kRevBlocks = 16 * 148;  // blocks of a launch before a block takes several spans: about three waves
                                           // of the five resident on a SM
+constexpr int64_t kRevWave = 5 * 148;     // blocks resident
 constexpr int kRevParts = 16;             // blocks of a cluster, at most
 constexpr int kPartColumns = kGradColumns + 1;  // of `partial`: the gradient's, the loss
 
@@ -1776,8 +1779,9 @@ __device__ __forceinline__ void add_past(const double* T, double* sums, double* 
 }
 static_assert(X_ATAN_W == X_ATAN_A + 2, "the arc tangents' four slots are contiguous");
 
-// (CLUSTER: the parts of a group are a cluster)
-template <int MODEL, bool FUSED, bool CLUSTER>
+// (SHARE: the warps share the frequencies of groups of one or two binaries;
+// CLUSTER: the parts of a group are a cluster)
+template <int MODEL, bool FUSED, bool SHARE, bool CLUSTER>
 __global__ void __launch_bounds__(kRevBlock, 5)
     k_rev_f64(const double* __restrict__ table, const double* __restrict__ freqs, int64_t n, int64_t B, int per,
               const double* __restrict__ t_c, const double2* __restrict__ cot_hp, const double2* __restrict__ cot_hc,
@@ -1788,10 +1792,11 @@ __global__ void __launch_bounds__(kRevBlock, 5)
   const auto* weights = static_cast<const double*>(fa.weights);
   const int64_t base = static_cast<int64_t>(blockIdx.x) * per;
   const int count = static_cast<int>(min(static_cast<int64_t>(per), B - base));
-  for (int i = threadIdx.x; i < count * kTableStride; i += kRevBlock) {
-    (&sh.T[0][0])[i] = table[base * kTableStride + i];
-    (&sh.sums[0][0])[i] = 0.0;
-  }
+  // (warps a binary)
+  const int shift = !SHARE ? 0 : (count == 1 ? 2 : (count == 2 ? 1 : 0)), share = 1 << shift;
+  static_assert(kRevWarps == 4, "a binary's warps");
+  for (int i = threadIdx.x; i < count * kTableStride; i += kRevBlock) (&sh.T[0][0])[i] = table[base * kTableStride + i];
+  for (int i = threadIdx.x; i < count * share * kTableStride; i += kRevBlock) (&sh.sums[0][0])[i] = 0.0;
   for (int64_t n0 = static_cast<int64_t>(blockIdx.y) * kSpan; n0 < n; n0 += static_cast<int64_t>(gridDim.y) * kSpan) {
     const int length = static_cast<int>(min(static_cast<int64_t>(kSpan), n - n0));
     {
@@ -1823,16 +1828,17 @@ __global__ void __launch_bounds__(kRevBlock, 5)
       __syncthreads();
     }
     double* stage = sh.stage[warp];
-    for (int j = warp; j < count; j += kRevWarps) {
+    for (int i0 = warp; i0 < count * share; i0 += kRevWarps) {
+      const int j = i0 >> shift;
       const double* T = sh.T[j];
-      double* sums = sh.sums[j];
+      double* sums = sh.sums[i0];
       const int64_t row = (base + j) * n;
       const double tc = t_c != nullptr ? t_c[base + j] : 0.0;
       const double kp = T[slot_kp<MODEL>()], kc = T[slot_kc<MODEL>()];
       double d1[kRevTiles<MODEL>][2] = {}, d2[2][2] = {}, ones[1][2] = {};
       double loss = 0.0;
       bool evaluated = false, past = false;
-      for (int c0 = 0; c0 < length; c0 += 32) {
+      for (int c0 = 32 * (i0 & (share - 1)); c0 < length; c0 += 32 * share) {
         const int i = c0 + lane;
         const bool in = i < length;
         const int64_t k = n0 + i;
@@ -1925,6 +1931,16 @@ __global__ void __launch_bounds__(kRevBlock, 5)
   // (r, d) takes the slots r + 4 i of direction d
   const auto cluster = cooperative_groups::this_cluster();
   const int parts = CLUSTER ? static_cast<int>(gridDim.y) : 1, part = CLUSTER ? static_cast<int>(blockIdx.y) : 0;
+  if constexpr (SHARE) {  // (a binary's warps' sums into its first one's)
+    __syncthreads();
+    for (int j = warp; j < count; j += kRevWarps) {
+      for (int k = lane; k < kTableStride; k += 32) {
+        double s = 0.0;
+        for (int q = 0; q < share; ++q) s += sh.sums[(j << shift) + q][k];
+        sh.sums[j << shift][k] = s;
+      }
+    }
+  }
   if constexpr (CLUSTER) {
     cluster.sync();
   } else {
@@ -1932,7 +1948,7 @@ __global__ void __launch_bounds__(kRevBlock, 5)
   }
   for (int j = part + parts * warp; j < count; j += parts * kRevWarps) {
     const int64_t b = base + j;
-    const double* sums = sh.sums[j];
+    const double* sums = sh.sums[j << shift];
     double* at = grad != nullptr ? grad + b * kGradColumns : nullptr;
     double* loss_at = loss_out != nullptr ? loss_out + b : nullptr;
     if (!CLUSTER && partial != nullptr) {
@@ -1944,7 +1960,7 @@ __global__ void __launch_bounds__(kRevBlock, 5)
       __syncwarp();
       for (int k = lane; k < kTableStride; k += 32) {
         double s = 0.0;
-        for (int p = 0; p < parts; ++p) s += cluster.map_shared_rank(&sh.sums[j][0], p)[k];
+        for (int p = 0; p < parts; ++p) s += cluster.map_shared_rank(&sh.sums[j << shift][0], p)[k];
         total[k] = s;
       }
       __syncwarp();
@@ -1990,9 +2006,11 @@ __global__ void __launch_bounds__(kBlock) k_sum_parts(const double* __restrict__
   if (lane == 0) *at = s;
 }
 
-// The reverse mode on ragged grids: one binary per block.
-template <int MODEL, bool FUSED>
-__global__ void __launch_bounds__(128) k_adj_f64_ragged(const double* __restrict__ table, const double* __restrict__ freqs,
+// The reverse mode with a binary a block, a register per sum and lane: on
+// ragged grids, and on shared ones where a wave of blocks holds the batch and
+// few frequencies each (rev_small).
+template <int MODEL, bool FUSED, bool RAGGED>
+__global__ void __launch_bounds__(128) k_adj_f64(const double* __restrict__ table, const double* __restrict__ freqs,
                                                  const int64_t* __restrict__ offsets, int64_t n, int64_t B,
                                                  const double* __restrict__ t_c, const double2* __restrict__ cot_hp,
                                                  const double2* __restrict__ cot_hc, FusedArgs fa,
@@ -2009,20 +2027,21 @@ __global__ void __launch_bounds__(128) k_adj_f64_ragged(const double* __restrict
     if (threadIdx.x < kTableStride) sT[threadIdx.x] = table[b * kTableStride + threadIdx.x];
     __syncthreads();
     const double tc = t_c != nullptr ? t_c[b] : 0.0;
-    const int64_t rs = min(max(offsets[b], int64_t(0)), n);
-    const int64_t re = min(max(offsets[b + 1], rs), n);
+    const int64_t rs = RAGGED ? min(max(offsets[b], int64_t(0)), n) : b * n;
+    const int64_t re = RAGGED ? min(max(offsets[b + 1], rs), n) : rs + n;
+    const int64_t fbase = RAGGED ? 0 : rs;
     double acc[kTableStride];
 #pragma unroll
     for (int k = 0; k < kTableStride; ++k) acc[k] = 0.0;
     double loss = 0.0;
     for (int64_t e = rs + threadIdx.x; e < re; e += kAdjBlock) {
-      const Freq<double> q = freq_powers(freqs[e]);
+      const Freq<double> q = freq_powers(freqs[e - fbase]);
       const Point<double> pt = point<MODEL, double>(sT, q, tc);
       double2 gp, gc;
       if constexpr (FUSED) {
         const double ap = sT[slot_kp<MODEL>()] * pt.amp, ac = sT[slot_kc<MODEL>()] * pt.amp;
-        const double2 d = data[e];
-        const double w = weights[e];
+        const double2 d = data[RAGGED || fa.data_stride ? e : e - fbase];
+        const double w = weights[RAGGED || fa.weights_stride ? e : e - fbase];
         const double rx = fa.fp * (ap * pt.c) + fa.fc * (-ac * pt.s) - d.x;
         const double ry = fa.fp * (ap * pt.s) + fa.fc * (ac * pt.c) - d.y;
         loss += w * (rx * rx + ry * ry);
@@ -2412,28 +2431,52 @@ int launch_adj_staged(const float* table, const float* freqs, int64_t n, int64_t
   return launched();
 }
 
-// How k_rev_f64 splits B binaries of n frequencies: `per` binaries a block,
-// as many as leave kRevBlocks blocks of one span, up to kRevBinaries; then
-// several spans a block, which cost it one contraction. Where a cluster's parts
-// (of the portable eight at most) give the same split and its blocks are a wave
-// at most, the clusters are as fast as k_sum_parts' second launch (XAS vjp 37 x
-// 1001: 15.3 and 16.6 us; 1000 x 129, in waves: 35 to 43 and 31): no workspace.
+// How k_rev_f64 splits B binaries of n frequencies: a wave of blocks of one
+// span with up to four binaries, one a warp, then eight; then several spans a
+// block, which cost it one contraction.
 struct RevShape {
   int64_t groups, parts;
   int per;
   size_t bytes;  // of `partial`
 };
+int rev_binaries(int64_t spans) {
+  const int64_t per = spans / kRevWave;
+  return per > kRevWarps ? kRevBinaries : (per > 2 ? kRevWarps : (per == 2 ? 2 : 1));
+}
 RevShape rev_shape(int64_t B, int64_t n) {
   const int64_t spans = (n + kSpan - 1) / kSpan;
   RevShape r;
-  r.per = static_cast<int>(min(max(B * spans / kRevBlocks, int64_t(1)), static_cast<int64_t>(kRevBinaries)));
+  r.per = rev_binaries(B * spans);
   r.groups = (B + r.per - 1) / r.per;
   const int64_t each = max(r.groups * spans / kRevBlocks, int64_t(1));
   r.parts = min((spans + each - 1) / each, int64_t(65535));
-  const bool cluster = r.parts <= 8 && r.groups * r.parts <= kRevBlocks / 4;
-  r.bytes = cluster ? 0 : sizeof(double) * kPartColumns * static_cast<size_t>(B * r.parts);
-  if (r.parts == 1) r.bytes = 0;
+  r.bytes = r.parts > 1 ? sizeof(double) * kPartColumns * static_cast<size_t>(B * r.parts) : 0;
   return r;
+}
+
+// Whether k_adj_f64 takes a shared grid rather than k_rev_f64: up to two waves
+// of its blocks (two a SM, four of TaylorF2) with few spans each, whose time,
+// `wave` and `wave_span` a span, is less than k_rev_f64's, `fixed` and `span` a
+// binary and span over the whole chip. Fitted to both kernels over 1 to 4000
+// binaries of 1 to 4017 frequencies (the common unit is k_adj_f64's time of a
+// span): the choice is within 0.2 %, 0.9 % and 0.5 % of the faster one on average.
+// IMRPhenomXAS vjp, k_adj_f64 and k_rev_f64, us: 1 x 65 8.3 and 9.3, 296 x 300
+// 12.4 and 18.6, 296 x 1000 22.6 and 24.7; 37 x 1000 21.5 and 16.5, 300 x 300 20.6
+// and 18.6, 296 x 2000 37.0 and 35.0, 1000 x 129 30.8 and 24.7, 1 x 4017 66 and
+// 12.4.
+bool rev_small(int model, int64_t B, int64_t n) {
+  struct Fit {
+    int64_t resident;
+    double spans, wave, wave_span, fixed, span;
+  };
+  constexpr Fit kFits[3] = {{2 * 148, 12, 3.5, 1.0, 7.0, 0.0025},   // IMRPhenomXAS
+                            {2 * 148, 8, 4.0, 1.5, 9.0, 0.006},     // IMRPhenomD
+                            {4 * 148, 12, 3.5, 1.0, 10.0, 0.0015}};  // TaylorF2
+  const Fit& f = kFits[model == kModelXas ? 0 : (model == kModelPhenomD ? 1 : 2)];
+  const double waves = static_cast<double>((B + f.resident - 1) / f.resident);
+  const double spans = static_cast<double>((n + kSpan - 1) / kSpan);
+  return waves <= 2.0 && spans <= f.spans &&
+         waves * (f.wave + f.wave_span * spans) < f.fixed + f.span * static_cast<double>(B) * spans;
 }
 
 // The blocks of a cluster that the device takes of k_rev_f64: kRevParts where
@@ -2448,12 +2491,15 @@ int rev_cluster(int* most) {
   if (rc != cudaSuccess) return static_cast<int>(rc);
   *most = dev >= 0 && dev < kDevices ? known[dev].load() : 0;
   if (*most > 0) return 0;
-  const auto kernel = k_rev_f64<MODEL, FUSED, true>;
+  const auto kernel = k_rev_f64<MODEL, FUSED, true, true>;  // (both take the same shared memory)
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(1, kRevParts);
   config.blockDim = dim3(kRevBlock);
   int size = 0;
   rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (rc == cudaSuccess) {
+    rc = cudaFuncSetAttribute(k_rev_f64<MODEL, FUSED, false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }
   if (rc == cudaSuccess) rc = cudaOccupancyMaxPotentialClusterSize(&size, kernel, &config);
   if (rc != cudaSuccess) return static_cast<int>(rc);
   *most = size >= kRevParts ? kRevParts : 8;
@@ -2476,8 +2522,7 @@ int launch_rev_f64(const double* table, const double* freqs, int64_t n, int64_t 
     int blocks = 0;
     if (int rc = rev_cluster<MODEL, FUSED>(&blocks)) return rc;
     const int64_t most = min((n + kSpan - 1) / kSpan, static_cast<int64_t>(blocks));
-    const int64_t per = 3 * B * most / kRevBlocks;
-    r.per = per > kRevWarps ? kRevBinaries : (per > 2 ? kRevWarps : (per == 2 ? 2 : 1));
+    r.per = rev_binaries(B * most);
     r.groups = (B + r.per - 1) / r.per;
     r.parts = 1;
     while (r.parts < most && r.parts * r.groups < kRevBlocks) r.parts *= 2;
@@ -2494,10 +2539,12 @@ int launch_rev_f64(const double* table, const double* freqs, int64_t n, int64_t 
   config.attrs = &cluster;
   const bool clustered = !stored && r.parts > 1;
   config.numAttrs = clustered ? 1 : 0;
-  const cudaError_t rc =
-      cudaLaunchKernelEx(&config, clustered ? k_rev_f64<MODEL, FUSED, true> : k_rev_f64<MODEL, FUSED, false>, table,
-                         freqs, n, B, r.per, t_c, cot_hp, cot_hc, fa, dtable, grad, loss,
-                         stored ? static_cast<double*>(partial) : nullptr);
+  // (compiled apart: shared warps cost a large batch 2 to 8 %)
+  const auto kernel =
+      r.per <= 2 ? (clustered ? k_rev_f64<MODEL, FUSED, true, true> : k_rev_f64<MODEL, FUSED, true, false>)
+                 : (clustered ? k_rev_f64<MODEL, FUSED, false, true> : k_rev_f64<MODEL, FUSED, false, false>);
+  const cudaError_t rc = cudaLaunchKernelEx(&config, kernel, table, freqs, n, B, r.per, t_c, cot_hp, cot_hc, fa, dtable,
+                                            grad, loss, stored ? static_cast<double*>(partial) : nullptr);
   if (rc != cudaSuccess) return static_cast<int>(rc);
   if (stored) {
     const int64_t warps = B * kPartColumns;
@@ -2711,7 +2758,9 @@ size_t wfx_workspace_bytes(int op, int model, int precision, int64_t B, int64_t 
   return 0;
 }
 
-size_t wfx_reverse64_workspace_bytes(int64_t B, int64_t n) { return B <= 0 || n <= 0 ? 0 : rev_shape(B, n).bytes; }
+size_t wfx_reverse64_workspace_bytes(int model, int64_t B, int64_t n) {
+  return check_model(model) || B <= 0 || n <= 0 || rev_small(model, B, n) ? 0 : rev_shape(B, n).bytes;
+}
 
 int wfx_grid_vjp(int model, const double* table, const double* freqs, const int64_t* offsets, int64_t B, int64_t n,
                  const double* t_c, const void* cot_hp, const void* cot_hc, double* grad_f, wfx_stream_t stream) {
@@ -2812,11 +2861,13 @@ static int adjoint_entry(bool fused, int model, int precision, const void* table
       constexpr int M = decltype(m)::value;
       if (offsets != nullptr) {
         const unsigned grid = static_cast<unsigned>(min(B, int64_t(1) << 20));
-        if (fused) {
-          k_adj_f64_ragged<M, true><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
-        } else {
-          k_adj_f64_ragged<M, false><<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
-        }
+        const auto kernel = fused ? k_adj_f64<M, true, true> : k_adj_f64<M, false, true>;
+        kernel<<<grid, 128, 0, s>>>(T, F, offsets, n, B, TC, CP, CC, fa, dtable, G, L);
+        return launched();
+      }
+      if (rev_small(M, B, n)) {
+        const auto kernel = fused ? k_adj_f64<M, true, false> : k_adj_f64<M, false, false>;
+        kernel<<<static_cast<unsigned>(B), 128, 0, s>>>(T, F, nullptr, n, B, TC, CP, CC, fa, dtable, G, L);
         return launched();
       }
       const auto launch = fused ? launch_rev_f64<M, true> : launch_rev_f64<M, false>;

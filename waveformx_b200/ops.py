@@ -92,7 +92,7 @@ def workspace(op: int, model: int, precision: int, batch: int, n: int, ragged: b
               device: torch.device) -> Optional[torch.Tensor]:
     """A scratch buffer for ``op`` (None if none is needed)."""
     if precision == _lib.FP64 and not ragged and op != _lib.OP_POLARIZATIONS:
-        nbytes = int(_lib.library().wfx_reverse64_workspace_bytes(batch, n))
+        nbytes = int(_lib.library().wfx_reverse64_workspace_bytes(model, batch, n))
     else:
         nbytes = int(_lib.library().wfx_workspace_bytes(op, model, precision, batch, n, int(ragged)))
     return None if nbytes == 0 else torch.empty(nbytes, dtype=torch.uint8, device=device)
